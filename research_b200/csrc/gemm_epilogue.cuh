@@ -1,0 +1,19 @@
+// Activations that the products' epilogues apply to fp32 sums.
+#pragma once
+#include "common.cuh"
+
+namespace rb {
+
+__device__ __forceinline__ float clamped_glu_epi(float g, float u, float limit) {
+  g = fminf(g, limit);
+  u = fminf(fmaxf(u, -limit), limit);
+  return g / (1.f + __expf(-1.702f * g)) * (u + 1.f);
+}
+
+// silu(gate) * up with the rounding points of the unfused path: bf16(gate), bf16(silu), bf16(up); the caller rounds the product.
+__device__ __forceinline__ float swiglu_epi(float gate, float up) {
+  const float g = __bfloat162float(__float2bfloat16_rn(gate)), u = __bfloat162float(__float2bfloat16_rn(up));
+  return __bfloat162float(__float2bfloat16_rn(g / (1.f + __expf(-g)))) * u;
+}
+
+}  // namespace rb

@@ -26,6 +26,7 @@
 // owner's epilogue warps then sum the P partial tiles (their own memory, local reads) and
 // write the result (all-reduce: to every peer). This is the GEMM -> reduce-scatter path.
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 #include "gemm_sm100.h"
 
 #include <stdlib.h>
@@ -196,12 +197,6 @@ __device__ __forceinline__ void epi_store_row_chunk(const GemmParams& p, const f
       }
     }
   }
-}
-
-__device__ __forceinline__ float clamped_glu_epi(float g, float u, float limit) {
-  g = fminf(g, limit);
-  u = fminf(fmaxf(u, -limit), limit);
-  return g / (1.f + __expf(-1.702f * g)) * (u + 1.f);
 }
 
 // Counter-based random stream of the sampler (identical to rb_sample_logprob: splitmix64 row key,
@@ -824,14 +819,8 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
                         clamped_glu_epi(__uint_as_float(g[j + 2 * e + 1]) * rscale, __uint_as_float(u[j + 2 * e + 1]) * rscale, p.glu_limit));
                     continue;
                   }
-                  // same rounding points as the unfused path: bf16(gate), bf16(silu), bf16(up), bf16(product)
-                  const float g0 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(g[j + 2 * e]) * rscale));
-                  const float g1 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(g[j + 2 * e + 1]) * rscale));
-                  const float u0 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[j + 2 * e]) * rscale));
-                  const float u1 = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[j + 2 * e + 1]) * rscale));
-                  const float s0 = __bfloat162float(__float2bfloat16_rn(g0 / (1.f + __expf(-g0))));
-                  const float s1 = __bfloat162float(__float2bfloat16_rn(g1 / (1.f + __expf(-g1))));
-                  o[e] = pack_bf16x2(s0 * u0, s1 * u1);
+                  o[e] = pack_bf16x2(swiglu_epi(__uint_as_float(g[j + 2 * e]) * rscale, __uint_as_float(u[j + 2 * e]) * rscale),
+                                     swiglu_epi(__uint_as_float(g[j + 2 * e + 1]) * rscale, __uint_as_float(u[j + 2 * e + 1]) * rscale));
                 }
                 *reinterpret_cast<uint4*>(dst + j) = make_uint4(o[0], o[1], o[2], o[3]);
               }

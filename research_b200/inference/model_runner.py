@@ -489,16 +489,16 @@ class ModelRunner(RunnerBase):
         gu = self.a_gu[:n] if static else None
         act = self.a_act[:n] if static else None
         if self.fuse_swiglu:
-            act = ops.gemm(src[:n], lw.wgu, out=act, bn=self.swiglu_bn, swiglu=True, norm_eps=eps)
+            act = ops.gemm(src[:n], lw.wgu, out=act, bn=self.swiglu_bn, swiglu=True, norm_eps=eps, constant_b=True)
         else:
-            gu = ops.gemm(src[:n], lw.wgu, out=gu, norm_eps=eps)
+            gu = ops.gemm(src[:n], lw.wgu, out=gu, norm_eps=eps, constant_b=True)
             act = ops.swiglu(gu, out=act)
         self._row_parallel(act, lw.wd, x[:n])
 
     def _row_parallel(self, a: torch.Tensor, w: torch.Tensor, x: torch.Tensor) -> None:
         """x += a @ w.T, summed over tensor-parallel ranks when sharded."""
         if self.tp is None or self.tp_size == 1:
-            ops.gemm(a, w, residual=x, out=x)
+            ops.gemm(a, w, residual=x, out=x, constant_b=True)
         else:
             self.tp.gemm_all_reduce(a, w, x)
 
@@ -506,10 +506,10 @@ class ModelRunner(RunnerBase):
         cfg = self.cfg
         for li, lw in enumerate(self.layers):
             if self.fold_norm:
-                qkv = ops.gemm(x[:n], lw.wqkv, bias=lw.bqkv, out=self.a_qkv[:n] if static else None, norm_eps=cfg.rms_norm_eps)
+                qkv = ops.gemm(x[:n], lw.wqkv, bias=lw.bqkv, out=self.a_qkv[:n] if static else None, norm_eps=cfg.rms_norm_eps, constant_b=True)
             else:
                 ops.rmsnorm(x[:n], lw.ln1, cfg.rms_norm_eps, out=h[:n])
-                qkv = ops.gemm(h[:n], lw.wqkv, bias=lw.bqkv, out=self.a_qkv[:n] if static else None)
+                qkv = ops.gemm(h[:n], lw.wqkv, bias=lw.bqkv, out=self.a_qkv[:n] if static else None, constant_b=True)
             q = ops.rope_kv_append(qkv, positions, slots, self.rope, self.k_cache[li], self.v_cache[li], self.Hq,
                                    self.Hkv, self.D, lw.q_norm, lw.k_norm, cfg.rms_norm_eps,
                                    q_out=self.a_q[:n] if static else None)
@@ -583,7 +583,7 @@ class ModelRunner(RunnerBase):
             ops.lm_head_sample(h, self.lm_head, temps, seeds, 0, None, self.d_out_tokens[:n], self.d_out_logprobs[:n],
                                workspace=self.sample_ws)
             return
-        logits = ops.gemm(h, self.lm_head, out=self.a_logits[:n], out_f32=True)
+        logits = ops.gemm(h, self.lm_head, out=self.a_logits[:n], out_f32=True, constant_b=True)
         self._sample(logits, temps, seeds, n)
 
     # ------------------------------------------------------------------ packed batches

@@ -49,11 +49,11 @@ class DensePart(Part):
         T = inp.shape[0]
         act = self.act[:T * w.ffp].view(T, w.ffp)
         if self.r.bf16:
-            ops.gemm(inp, w.wgu, out=act, bn=GLU_BN, swiglu=True, glu_limit=w.spec.limit)
+            ops.gemm(inp, w.wgu, out=act, bn=GLU_BN, swiglu=True, glu_limit=w.spec.limit, constant_b=True)
         else:
-            gu = ops.gemm(inp, w.wgu, out=self.gu[:T * 2 * w.ffp].view(T, 2 * w.ffp))
+            gu = ops.gemm(inp, w.wgu, out=self.gu[:T * 2 * w.ffp].view(T, 2 * w.ffp), constant_b=True)
             ops.clamped_glu(gu, w.spec.limit, out=act)
-        ops.gemm(act, w.wd, out=y, out_f32=True)
+        ops.gemm(act, w.wd, out=y, out_f32=True, constant_b=True)
         return {"y2": y}
 
 
@@ -82,9 +82,9 @@ class PolyNormPart(Part):
     def forward(self, w: PolyNormWeights, inp, y, small=None) -> dict:
         T = inp.shape[0]
         z, a = (t[:T * w.ffp].view(T, w.ffp) for t in (self.z, self.a))
-        ops.gemm(inp, w.wu, out=z)
+        ops.gemm(inp, w.wu, out=z, constant_b=True)
         ops.poly_norm(z, w.act, w.spec.ff, self.r.cfg.norm_eps, a)
-        ops.gemm(a, w.wd, out=y, out_f32=True)
+        ops.gemm(a, w.wd, out=y, out_f32=True, constant_b=True)
         return {"y2": y}
 
 

@@ -107,7 +107,7 @@ class GroupedPart(Part):
         return self.proj[:T * w.geo.proj].view(T, w.geo.proj)
 
     def project(self, w: GroupedWeights, inp, tail) -> None:
-        ops.gemm(inp, w.wproj, bias=w.bproj, out=self._projected(w, inp.shape[0]), tail=tail)
+        ops.gemm(inp, w.wproj, bias=w.bproj, out=self._projected(w, inp.shape[0]), tail=tail, constant_b=True)
 
     def attend(self, w: GroupedWeights, cache: GroupedCache, out, b, splits, small, factor: float = 1.0, proj=None) -> None:
         """Heads' outputs (gated, times ``factor``) into ``out [T, H * dp]``, after ``project`` (or from the rows ``proj``)."""
@@ -122,4 +122,4 @@ class GroupedPart(Part):
         T, n = b.num_tokens, w.geo.heads * w.geo.dp
         out = self.out[:T * n].view(T, n)
         self.attend(w, cache, out, b, plan, small)
-        ops.gemm(out, w.wo, out=y, out_f32=True)
+        ops.gemm(out, w.wo, out=y, out_f32=True, constant_b=True)

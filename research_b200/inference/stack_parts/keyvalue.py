@@ -74,7 +74,7 @@ class KeyValuePart(Part):
         return self.proj[:T * w.geo.proj].view(T, w.geo.proj)
 
     def project(self, w: KeyValueWeights, inp, tail) -> None:
-        ops.gemm(inp, w.wproj, bias=w.bproj, out=self._projected(w, inp.shape[0]), tail=tail)
+        ops.gemm(inp, w.wproj, bias=w.bproj, out=self._projected(w, inp.shape[0]), tail=tail, constant_b=True)
 
     def forward(self, w: KeyValueWeights, cache, inp, y, b, splits, small=None) -> None:
         T, g, m = b.num_tokens, w.geo, w.spec
@@ -83,4 +83,4 @@ class KeyValuePart(Part):
         ops.kv_append(proj, g, b.positions, b.slots, m.q_temp.coef, m.q_temp.every, cache)
         ops.kv_attention(proj, g, cache, b.block_tables, b.cu_q, b.seq_lens, w.sink, out, scale=m.scale, rows=T, max_q=b.max_new,
                          n_single=b.n_single, workspace=self.workspace, splits=splits.get(g, 1))
-        ops.gemm(out, w.wo, bias=w.bo, out=y, out_f32=True)
+        ops.gemm(out, w.wo, bias=w.bo, out=y, out_f32=True, constant_b=True)

@@ -129,9 +129,9 @@ class LatentPart(Part):
     def forward(self, w: LatentWeights, cache, inp, y, b, plan, small=None) -> None:
         n_short, short_attn, long_attn = plan
         T, g, f = b.num_tokens, w.geo, self.bufs[w.geo]
-        ops.gemm(inp, w.wproj, out=f.proj[:T], out_f32=True)
+        ops.gemm(inp, w.wproj, out=f.proj[:T], out_f32=True, constant_b=True)
         ops.latent_append(f.proj[:T], g, w.q_norm, w.kv_norm, self.r.cfg.norm_eps, b.positions, b.slots, w.table, cache, f.cq, f.gate)
-        q = ops.gemm(f.cq[:T], w.wuq, out=f.q[:T])
+        q = ops.gemm(f.cq[:T], w.wuq, out=f.q[:T], constant_b=True)
         ops.latent_query(q, g, b.positions, w.table, n_short, f.qn, f.qa)
         if n_short > 0:
             ops.head_gemm_absorb(f.qn, w.wuk, f.qa, n_short)
@@ -139,7 +139,7 @@ class LatentPart(Part):
             ops.head_gemm_expand(f.ol, w.wuv, f.attn, n_short)
         if n_short < T:
             long_attn(w, cache, f)
-        ops.gemm(f.attn[:T], w.wo, out=y, out_f32=True)
+        ops.gemm(f.attn[:T], w.wo, out=y, out_f32=True, constant_b=True)
 
     def _short_attention(self, rows: int, max_q: int, cu_q, seq_lens, block_tables, plans: dict | None = None):
         """Attention on the cached latents for the first ``rows`` rows of the batch."""

@@ -87,7 +87,7 @@ class ParallelPart(Part):
         out = self.out[:T * w.wo.shape[1]].view(T, -1)
         self.left.attend(w.left, cache[0], out[:, :n], b, plan[0], small, w.spec.left_scale)
         self.right.mix(w.right, cache[1], inp, out[:, n:], b, plan[1])
-        ops.gemm(out, w.wo, out=y, out_f32=True)
+        ops.gemm(out, w.wo, out=y, out_f32=True, constant_b=True)
 
 
 @dataclass
@@ -156,14 +156,14 @@ class NormedPairPart(Part):
         return self.proj[:T * n].view(T, n)
 
     def project(self, w: NormedPairWeights, inp, tail) -> None:
-        ops.gemm(inp, w.wproj, bias=w.bproj, out=self._projected(w, inp.shape[0]), silu_cols=w.right.geo.silu_cols, tail=tail)
+        ops.gemm(inp, w.wproj, bias=w.bproj, out=self._projected(w, inp.shape[0]), silu_cols=w.right.geo.silu_cols, tail=tail, constant_b=True)
 
     def forward(self, w: NormedPairWeights, cache, inp, y, b, plan, small=None) -> dict:
         T, n = b.num_tokens, w.left.geo.heads * w.left.geo.dp
         proj = self._projected(w, T)
         out = self.left.out[:T * n].view(T, n)
         self.left.attend(w.left, cache[0], out, b, plan[0], None, proj=proj[:, w.right.geo.proj:])
-        ops.gemm(out, w.left.wo, out=y, out_f32=True)
+        ops.gemm(out, w.left.wo, out=y, out_f32=True, constant_b=True)
         other = self.r.y2[:T]
         self.right.mix(w.right, cache[1], proj, small, other, b, plan[1])
         return {"y1": y, "pair": (other, w.left_out, w.right_out)}

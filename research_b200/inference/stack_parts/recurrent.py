@@ -87,7 +87,7 @@ class RecurrentPart(Part):
         return self.proj[:T * w.geo.proj].view(T, w.geo.proj)
 
     def project(self, w: RecurrentWeights, inp, tail) -> None:
-        ops.gemm(inp, w.wproj, out=self._projected(w, inp.shape[0]), silu_cols=w.geo.silu_cols, tail=tail)
+        ops.gemm(inp, w.wproj, out=self._projected(w, inp.shape[0]), silu_cols=w.geo.silu_cols, tail=tail, constant_b=True)
 
     def forward(self, w: RecurrentWeights, state: RecurrentState, inp, y, b, plan, small=None) -> None:
         T, g = b.num_tokens, w.geo
@@ -96,7 +96,7 @@ class RecurrentPart(Part):
         o, out = self.o[:T * n].view(T, n), self.out[:T * n].view(T, n)
         self.recur(w, state, proj, small, o, b, plan)
         ops.gated_norm(o, w.norm, proj[:, g.offsets[3]:], g, self.r.cfg.norm_eps, out, g.gated)
-        ops.gemm(out, w.wo, out=y, out_f32=True)
+        ops.gemm(out, w.wo, out=y, out_f32=True, constant_b=True)
 
     def plan(self, b):
         """(sequences and rows that run token by token, chunk table of the rest)"""
@@ -212,16 +212,16 @@ class TimeMixPart(Part):
             ops.head_gemm_expand(self.mixed[:4], w.wproj, proj, T)       # (the whole buffer: its destination table is kept)
             return proj[:T]
         for i in range(4):
-            ops.gemm(self.mixed[i, :T], w.wproj[i * n:(i + 1) * n], out=proj[:T, i * n:(i + 1) * n])
+            ops.gemm(self.mixed[i, :T], w.wproj[i * n:(i + 1) * n], out=proj[:T, i * n:(i + 1) * n], constant_b=True)
         return proj[:T]
 
     def decay_logits(self, w: TimeMixWeights, T: int) -> torch.Tensor:
         """``W_w2 tanh(W_w1 mix)`` in fp32."""
         n = w.geo.heads * w.geo.kp
         inner, tanh = self.inner[:T * w.rank].view(T, -1), self.tanh[:T * w.rank * self.parts].view(T, -1)
-        ops.gemm(self.mixed[4, :T], w.w1, out=inner, out_f32=True)
+        ops.gemm(self.mixed[4, :T], w.w1, out=inner, out_f32=True, constant_b=True)
         ops.tanh_parts(inner, tanh)
-        return ops.gemm(tanh, w.w2, out=self.z[:T * n].view(T, n), out_f32=True)
+        return ops.gemm(tanh, w.w2, out=self.z[:T * n].view(T, n), out_f32=True, constant_b=True)
 
     def recur(self, w: TimeMixWeights, cache: TimeMixState, proj, z, out, b, plan) -> None:
         T, g, eps = b.num_tokens, w.geo, self.r.cfg.norm_eps
@@ -242,7 +242,7 @@ class TimeMixPart(Part):
         T, n = b.num_tokens, w.geo.heads * w.geo.vp
         out = self.out[:T * n].view(T, n)
         self.mix(w, cache, inp, out, b, plan)
-        ops.gemm(out, w.wo, out=y, out_f32=True)
+        ops.gemm(out, w.wo, out=y, out_f32=True, constant_b=True)
 
 
 class ForgetMixWeights:
@@ -298,7 +298,7 @@ class ForgetMixPart(Part):
         T, n = b.num_tokens, w.geo.heads * w.geo.vp
         out = self.out[:T * n].view(T, n)
         self.recur(w, state, proj, z, out, b, plan)
-        ops.gemm(out, w.wo, out=y, out_f32=True)
+        ops.gemm(out, w.wo, out=y, out_f32=True, constant_b=True)
 
     def recur(self, w: ForgetMixWeights, state: RecurrentState, proj, z, out, b, plan) -> None:
         T, g, eps = b.num_tokens, w.geo, self.r.cfg.norm_eps
@@ -396,7 +396,7 @@ class DeltaPart(Part):
         return self.proj[:T * w.geo.proj].view(T, w.geo.proj)
 
     def project(self, w: DeltaWeights, inp, tail) -> None:
-        ops.gemm(inp, w.wproj, out=self._projected(w, inp.shape[0]), tail=tail)
+        ops.gemm(inp, w.wproj, out=self._projected(w, inp.shape[0]), tail=tail, constant_b=True)
 
     def prepare(self, w: DeltaWeights, cache: DeltaState, small, b) -> tuple[torch.Tensor, DeltaRule]:
         """What the recurrence reads, after ``project``."""
@@ -425,4 +425,4 @@ class DeltaPart(Part):
         rows, rule = self.prepare(w, cache, small, b)
         self.recur(w, cache, rows, rule, o, b, plan)
         ops.gated_norm(o, w.norm, self._projected(w, T)[:, g.offsets[3]:], g, self.r.cfg.norm_eps, out, True, silu=True)
-        ops.gemm(out, w.wo, out=y, out_f32=True)
+        ops.gemm(out, w.wo, out=y, out_f32=True, constant_b=True)

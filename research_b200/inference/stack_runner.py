@@ -230,7 +230,7 @@ class StackRunner(RunnerBase):
     # ------------------------------------------------------------------ layers
     def _small_rows(self, inp: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
         """The narrow projections of ``inp``, fp32."""
-        return ops.gemm(inp, w, out=self._small_buffer(inp.shape[0], w), out_f32=True)
+        return ops.gemm(inp, w, out=self._small_buffer(inp.shape[0], w), out_f32=True, constant_b=True)
 
     def _small_buffer(self, T: int, w: torch.Tensor) -> torch.Tensor:
         return self._small[:T * w.shape[0]].view(T, w.shape[0])
@@ -256,7 +256,7 @@ class StackRunner(RunnerBase):
 
     def _enter_pass(self, T: int) -> None:
         """``x = W [x; embedding output]``: a pass of the loop begins (the stream's copy is in ``x_loop`` already)."""
-        ops.gemm(self.x_loop[:T], self.loop_in, out=self.x[:T], out_f32=True)
+        ops.gemm(self.x_loop[:T], self.loop_in, out=self.x[:T], out_f32=True, constant_b=True)
 
     def _embed(self, b: PackedBatch, first_copy: torch.Tensor | None) -> None:
         """Embedding output into the stream, its second half of ``x_loop`` and, if given, another copy."""
@@ -319,9 +319,9 @@ class StackRunner(RunnerBase):
         """``y = W_proj (gelu_tanh(W_gate x) * e)`` with the layer's part ``e`` of the tokens' side embedding."""
         T = b.num_tokens
         z, a = self.side_z[:T], self.side_a[:T]
-        ops.gemm(xb, w.gate, out=z, out_f32=True)
+        ops.gemm(xb, w.gate, out=z, out_f32=True, constant_b=True)
         ops.token_side(z, b.tokens[:T], self.side_embed, w.col, a, self.side_dim)
-        ops.gemm(a, w.proj, out=y, out_f32=True)
+        ops.gemm(a, w.proj, out=y, out_f32=True, constant_b=True)
 
     def _post_norm_layers(self, b: PackedBatch, plans: dict) -> None:
         T, d, eps = b.num_tokens, self.cfg.hidden_size, self.cfg.norm_eps
@@ -357,9 +357,9 @@ class StackRunner(RunnerBase):
         """``logits`` (rows padded to ``vp`` columns) of the final-normed rows ``h``, soft-capped."""
         cap = self.cfg.logit_softcap
         if self.bf16 and cap > 0:
-            ops.gemm(h, self.head, out=logits, out_f32=True, softcap=cap)
+            ops.gemm(h, self.head, out=logits, out_f32=True, softcap=cap, constant_b=True)
         else:
-            ops.gemm(h, self.head, out=logits, out_f32=True)
+            ops.gemm(h, self.head, out=logits, out_f32=True, constant_b=True)
             if cap > 0:
                 ops.softcap(logits, cap)
         return logits[:, :self.cfg.vocab_size]

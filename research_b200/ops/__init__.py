@@ -70,7 +70,7 @@ def set_pdl(on: bool) -> None:
     attention, SwiGLU, embedding, sampling): consecutive kernels overlap prologue and tail."""
     from .. import _native
 
-    for lib, fn in (("rb_gemm", "rb_gemm_set_pdl"), ("rb_ops", "rb_ops_set_pdl"), ("rb_attn", "rb_attn_set_pdl"),
+    for lib, fn in (("rb_gemm", "rb_gemm_set_pdl"), ("rb_skinny", "rb_skinny_set_pdl"), ("rb_ops", "rb_ops_set_pdl"), ("rb_attn", "rb_attn_set_pdl"),
                     ("rb_latent", "rb_latent_set_pdl"), ("rb_gemm_f32", "rb_gemm_f32_set_pdl"),
                     ("rb_recurrent", "rb_recurrent_set_pdl"), ("rb_moe", "rb_moe_set_pdl")):
         if _native.available(lib):      # a partial build has only the libraries its models need

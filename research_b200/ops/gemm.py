@@ -127,6 +127,42 @@ def _lib2() -> ctypes.CDLL:
     return lib
 
 
+def _lib_skinny() -> ctypes.CDLL:
+    lib = _native.load("rb_skinny")
+    if not getattr(lib, "_rb_typed", False):
+        vp, i, ll, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+        lib.rb_skinny.argtypes = [vp] * 5 + [i] * 3 + [ll] * 4 + [i, i, i, f, i, f, f, i, vp, i, ll, i, vp]
+        lib.rb_skinny.restype = i
+        lib._rb_typed = True
+    return lib
+
+
+# rows -> most elements of B, for csrc/skinny_sm100.cu
+_SKINNY = ((8, 1 << 62), (16, 120_000_000), (32, 17_000_000))
+
+
+def _skinny_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail) -> bool:
+    """Few rows (csrc/skinny_sm100.cu): weights streamed by every warp on its own. Each 8 rows cost it another pass of activations
+    through L1 beside the weights, so past 8 rows the tcgen05 kernel is the better one where the matrix is large enough for its tiles
+    to fill the machine. Microseconds of a chain of captured launches over weights that are not in L2, tcgen05 kernel / this one:
+    2 rows: 896 x 896 8.2 / 2.5, 4096 x 4096 17.5 / 7.5, 28672 x 4096 71 / 46, 151936 x 896 59.5 / 54; 16 rows: 28672 x 4096
+    54.1 / 50.5, 151936 x 896 61.5 / 71.8; 32 rows: 896 x 896 8.2 / 6.1, 4096 x 4096 17.2 / 14.6, 6144 x 4096 21.5 / 23.6. What it
+    does not take (a layout the vector loads need, what the other kernel refuses or leaves unsaid) is left to the other kernel."""
+    if M > 32 or N * K > next(most for rows, most in _SKINNY if M <= rows):
+        return False
+    if N % 8 or K % 16 or a.stride(0) % 16 or b.stride(0) % 16 or a.data_ptr() % 32 or b.data_ptr() % 32:
+        return False
+    if residual is not None and (residual.stride(1) != 1 or residual.dtype != torch.bfloat16):
+        return False
+    if bias is not None and (bias.dtype != torch.bfloat16 or not bias.is_contiguous()):
+        return False
+    if swiglu:
+        return bn in (64, 128, 256) and N % bn == 0 and bias is None and residual is None and not out_f32 and not silu_cols and tail is None and softcap == 0
+    if silu_cols % 32 or (tail is not None and ((N - tail.shape[1]) % 32 or tail.stride(0) % 4 or tail.dtype != torch.float32 or tail.stride(1) != 1)):
+        return False
+    return bn == 0
+
+
 _GEMM2 = os.environ.get("RB_GEMM2", "1") != "0"
 _GEMM2_GATHER = os.environ.get("RB_GEMM2_GATHER", "1") != "0"     # gather-carrying launches on the two-CTA kernel too
 _GATHER_CHUNKS = int(os.environ.get("RB_GATHER_CHUNKS", "8"))      # pieces a gathered part is published in (tiles start per piece)
@@ -249,6 +285,7 @@ def gemm(
     softcap: float = 0.0,
     silu_cols: int = 0,
     tail: torch.Tensor | None = None,
+    constant_b: bool = False,
 ) -> torch.Tensor:
     """``C[M,N] = alpha * op(A) @ op(B)^T (+bias) (+ beta * residual)``.
 
@@ -269,6 +306,9 @@ def gemm(
     ``glu_limit`` makes the fused gate|up epilogue (``swiglu=True``) the clamped unit of ``elementwise.clamped_glu``;
     ``softcap`` stores ``softcap * tanh(C / softcap)``. ``silu_cols``: the first so many columns are stored as ``silu(C)``.
     ``tail`` (fp32 ``[M, n]``) receives the last ``n`` columns of the product, which ``out`` then lacks.
+
+    ``constant_b``: no kernel still running on the stream writes ``b`` (model weights). Under programmatic launches its first
+    loads then overlap the kernel before this one.
 
     K-major operands are ``[rows, K]`` row-major (a torch ``Linear`` weight is a K-major B);
     MN-major operands are ``[K, rows]`` row-major. On CUDA this launches the tcgen05 kernel;
@@ -350,6 +390,15 @@ def gemm(
     if out is None:
         out = torch.empty(M, N // 2 if swiglu else N - (tail.shape[1] if tail is not None else 0), dtype=torch.float32 if out_f32 else torch.bfloat16, device=a.device)
     assert out.stride(1) == 1
+    if (gather is None and wait_flag is None and not (a_mn_major or b_mn_major) and alpha == 1.0 and beta == 1.0 and max_ctas == 0 and split_k in (0, 1)
+            and not cluster_split and _skinny_takes(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail)):
+        rc = _lib_skinny().rb_skinny(
+            a.data_ptr(), b.data_ptr(), out.data_ptr(), ptr(bias), ptr(residual), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+            residual.stride(0) if residual is not None else 0, int(out_f32), bn // 2 if swiglu else 0, int(glu_limit is not None), glu_limit or 0.0,
+            int(norm_eps is not None), norm_eps or 0.0, softcap, silu_cols, ptr(tail), N - tail.shape[1] if tail is not None else 0,
+            tail.stride(0) if tail is not None else 0, int(constant_b), stream_handle(a.device))
+        check_rc(rc, "rb_skinny")
+        return out
     args = RbGemmArgs()
     args.A[0] = a.data_ptr()
     args.B[0] = b.data_ptr()

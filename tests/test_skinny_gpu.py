@@ -1,0 +1,120 @@
+"""Products with few rows (csrc/skinny_sm100.cu) against 64-bit sums and against the tcgen05 kernel, over the forms both take."""
+
+import pytest
+import torch
+
+from research_b200 import ops
+
+pytestmark = pytest.mark.gpu
+gemm_mod = ops.gemm_mod
+
+
+def _strided(rows, cols, pad, gen, scale=1.0):
+    return (torch.randn(rows, cols + pad, device="cuda", generator=gen) * scale).bfloat16()[:, :cols]
+
+
+def _reference(a, b, bias=None, residual=None, norm_eps=None, swiglu=False, bn=0, glu_limit=None, softcap=0.0, silu_cols=0, **_):
+    """(result, bound on the sums' rounding), 64 bits; the bound is 2 K 2^-24 of the absolute sums, the worst order of fp32 additions."""
+    x, w = a.double(), b.double()
+    if norm_eps is not None:
+        x = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + norm_eps)
+    y, spread = x @ w.T, (x.abs() @ w.abs().T) * 2 * a.shape[1] * 2.0 ** -24
+    if bias is not None:
+        y = y + bias.double()
+    if residual is not None:
+        y = y + residual.double()
+    if swiglu:
+        v, s = y.view(len(y), -1, 2, bn // 2), spread.view(len(y), -1, 2, bn // 2)
+        g, u = v[:, :, 0], v[:, :, 1]
+        size = (g.abs() + 1) * (u.abs() + 2)
+        # three roundings to bf16 on the way, and the sums' own error through both factors
+        spread = (3 * 2.0 ** -9 * size + 2 * (s[:, :, 0] * (u.abs() + 2) + s[:, :, 1] * (g.abs() + 1))).reshape(len(y), -1)
+        if glu_limit is not None:
+            g, u = g.clamp(max=glu_limit), u.clamp(-glu_limit, glu_limit)
+            y = g * torch.sigmoid(1.702 * g) * (u + 1)
+        else:
+            y = torch.nn.functional.silu(g) * u
+        y = y.reshape(len(a), -1)
+    if softcap > 0:
+        y = softcap * torch.tanh(y / softcap)
+    if silu_cols:
+        y[:, :silu_cols] = torch.nn.functional.silu(y[:, :silu_cols])
+    return y, spread
+
+
+FORMS = {
+    "plain": {},
+    "f32": {"out_f32": True},
+    "bias_residual": {"bias": True, "residual": True},
+    "norm_bias": {"bias": True, "norm_eps": 1e-5},
+    "softcap": {"out_f32": True, "softcap": 5.0},
+    "silu_tail": {"silu_cols": 32, "tail": 8},
+    "swiglu": {"swiglu": True, "bn": 64},
+    "swiglu_norm": {"swiglu": True, "bn": 128, "norm_eps": 1e-6},
+    "clamped": {"swiglu": True, "bn": 256, "glu_limit": 1.5},
+}
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("N,K", [(8, 16), (72, 48), (136, 1040), (896, 4864), (4096, 64)])
+def test_few_rows(form, M, N, K, monkeypatch):
+    kw = dict(FORMS[form])
+    if kw.get("swiglu"):
+        N = -(-N // kw["bn"]) * kw["bn"]
+    if kw.get("tail"):
+        N += 64 - N % 32 + kw["tail"]
+    gen = torch.Generator(device="cuda").manual_seed(M * 1000 + N + K)
+    a, b = _strided(M, K, 16, gen), _strided(N, K, 32 if N < 1000 else 0, gen, K ** -0.5)
+    if kw.pop("bias", False):
+        kw["bias"] = torch.randn(N, device="cuda", generator=gen).bfloat16()
+    if kw.pop("residual", False):
+        kw["residual"] = _strided(M, N, 8, gen)
+    tails = [torch.empty(M, kw["tail"] + 8, device="cuda")[:, :kw["tail"]] for _ in range(2)] if kw.get("tail") else [None, None]
+
+    def run(tail):
+        args = {k: v for k, v in kw.items() if k != "tail"}
+        return ops.gemm(a, b, tail=tail, **args)
+
+    assert gemm_mod._skinny_takes(a, b, kw.get("bias"), kw.get("residual"), M, N, K, kw.get("bn", 0), kw.get("swiglu", False),
+                                  kw.get("out_f32", False), kw.get("softcap", 0.0), kw.get("silu_cols", 0), tails[0])
+    y, spread = _reference(a, b, **{k: v for k, v in kw.items() if k != "tail"})
+    n = N - kw["tail"] if kw.get("tail") else y.shape[1]
+    out = run(tails[0])
+    half = 0.0 if kw.get("out_f32") else 2.0 ** -8
+    # activations of softcap and silu: a few units in the last place of their fp32 value
+    room = spread + half * y.abs() + 1e-6 * (1 + y.abs())
+    assert ((out.double() - y[:, :n]).abs() <= room[:, :n]).all()
+    if tails[0] is not None:
+        assert ((tails[0].double() - y[:, n:]).abs() <= (spread + 1e-6)[:, n:]).all()
+    monkeypatch.setattr(gemm_mod, "_SKINNY", ((32, 0),))
+    other = run(tails[1])
+    assert ((out.double() - other.double()).abs() <= 2 * room[:, :n]).all()
+
+
+def test_few_rows_under_capture_with_constant_weights():
+    """First loads of the weights before the launch dependency is waited for: a chain in which every product reads the one before."""
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    ws = [(torch.randn(512, 512, device="cuda", generator=gen) / 512 ** 0.5).bfloat16() for _ in range(6)]
+    x = torch.randn(4, 512, device="cuda", generator=gen).bfloat16()
+    bufs = [torch.empty(4, 512, device="cuda", dtype=torch.bfloat16) for _ in ws]
+
+    def body():
+        h = x
+        for w, o in zip(ws, bufs):
+            h = ops.gemm(h, w, out=o, constant_b=True)
+        return h
+
+    want = body().clone()
+    ops.set_pdl(True)
+    try:
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            body()
+    finally:
+        ops.set_pdl(False)
+    for _ in range(20):
+        for o in bufs:
+            o.zero_()
+        graph.replay()
+        assert torch.equal(bufs[-1], want)
