@@ -444,71 +444,146 @@ __global__ void __launch_bounds__(FA_THREADS, 1) flash_fwd_kernel(const __grid_c
 
 
 // ------------------------------------------------------------------------------------------
-// Forward, two query tiles per CTA ("ping-pong"): 256 query rows of one head, handled as tiles a and b
-// with one softmax warpgroup each (warps 2-5 and 6-9, a full score row per thread). Both tiles share the
-// K/V tiles in shared memory (loaded once for 256 rows), and while one warpgroup is in its softmax the
-// tensor core works for the other tile, so neither the TMEM read, the P store nor the polling of the MMA
-// thread sits on a critical path. TMEM: S_a, S_b (128 columns each), O_a, O_b (D columns each).
+// Forward, two query tiles per CTA: 256 query rows of one head, handled as tiles a and b with one softmax warpgroup
+// each (a full score row per thread). Both tiles share the K/V tiles in shared memory, and while one warpgroup is in
+// its softmax the tensor core works for the other tile.
+//
+// What bounds it: per 128 x 128 tile the exponentials take 1024 cycles of the SM's special-function unit and the two
+// products 1024 (D = 128) or 512 (D = 64) of the tensor core, so everything else has to hide under these:
+//  * P goes to tensor memory (packed bf16) and is the A operand from there. From shared memory the two 128 x 128
+//    operands of a product alone need the SM's whole shared-memory bandwidth, and P's stores would come on top.
+//    D = 128 fills tensor memory with S_a S_b O_a O_b, so P takes the place of its scores and the next scores wait for
+//    P V; D = 64 has room for P beside S, and the next scores are computed under the softmax.
+//  * P is handed over in halves: P V starts on the first 64 keys while the exponentials of the others run.
+//  * Three warpgroups of 168 registers a thread, redistributed to 88 / 208 / 208: the softmax threads keep their 128 scores
+//    in registers without spills.
+//  * Pairs of fp32 values per instruction (fma / add .f32x2), three-way maxima.
+//  * A CTA stays and takes the next query tile from the launch's own queue (cluster launch control: it cancels a CTA that
+//    has not started and does its work), so set-up, the first loads and the epilogue overlap; longest tiles first.
+// Measured rates stand beside the dispatch in launch_flash_fwd.
 // ------------------------------------------------------------------------------------------
 template <int D>
 struct Flash2Cfg {
   static constexpr int kTileBytes = FA_BN * D * 2;
-  static constexpr int kPBytes = FA_BM * FA_BN * 2;
-  static constexpr int kSmemBytes = 1024 + 2 * kTileBytes + FA_KV_SLOTS * kTileBytes + 2 * kPBytes;
+  static constexpr int kSlots = D == 128 ? 4 : 6;
+  static constexpr int kSmemBytes = 1024 + 2 * kTileBytes + kSlots * kTileBytes;
+};
+constexpr int FA2_THREADS = 384;
+constexpr int FA2_REGS_LAUNCH = 168, FA2_REGS_OTHER = 88, FA2_REGS_SOFTMAX = 208;     // 88 + 2 x 208 = 3 x 168
+
+struct FlashItem {       // one query tile pair
+  int b, h, q0, q_begin, q_len, kv_len, k_begin, off, kvh, t_begin, n_a, n_b;
+  __device__ __forceinline__ bool valid() const { return q0 < q_len; }
+  __device__ __forceinline__ int n() const { return max(n_a, n_b); }
 };
 
+__device__ __forceinline__ FlashItem flash_item(const FlashFwdParams& p, int x, int y, int z) {
+  FlashItem t;
+  // blocks start in the order of their index: the late tiles of all heads and sequences, which see the most keys, first
+  const int heads = p.Hq, lin = (z * gridDim.y + y) * gridDim.x + x, per = heads * gridDim.z;
+  const int q_tile = gridDim.x - 1 - lin / per, rest = lin % per;
+  t.b = rest / heads;
+  t.h = rest % heads;
+  t.q_begin = p.cu_q[t.b];
+  t.q_len = p.cu_q[t.b + 1] - t.q_begin;
+  t.q0 = q_tile * 2 * FA_BM;
+  t.kv_len = p.paged ? p.seq_lens[t.b] : (p.cu_k[t.b + 1] - p.cu_k[t.b]);
+  t.k_begin = p.paged ? 0 : p.cu_k[t.b];
+  t.off = t.kv_len - t.q_len;
+  t.kvh = t.h / (p.Hq / p.Hkv);
+  // key tiles: both query tiles start at tile a's first visible tile; each stops at its own last one
+  t.t_begin = flash_first_key(p, t.off + t.q0) / FA_BN;
+  const int hi_a = p.causal ? min(t.kv_len, t.off + t.q0 + FA_BM) : t.kv_len;
+  const int hi_b = p.causal ? min(t.kv_len, t.off + t.q0 + 2 * FA_BM) : t.kv_len;
+  t.n_a = max((hi_a + FA_BN - 1) / FA_BN - t.t_begin, 0);
+  t.n_b = t.q0 + FA_BM < t.q_len ? max((hi_b + FA_BN - 1) / FA_BN - t.t_begin, 0) : 0;
+  return t;
+}
+
+// D[tmem] (+)= A[tmem] * B[smem]: A is 128 lanes x 8 columns of packed bf16 pairs.
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t pair(float lo, float hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ void unpair(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// ---- cluster launch control: take over the work of a CTA of this launch that has not started -------------------------
+__device__ __forceinline__ void clc_try_cancel(uint32_t response, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(response), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool clc_read(uint32_t response, int& x, int& y, int& z) {
+  uint32_t got;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\t.reg .pred P;\n\t"
+      "ld.shared.b128 r, [%4];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 P, r;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t"
+      "mov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+      "@P clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, _}, r;\n\t}"
+      : "=r"(got), "=r"(x), "=r"(y), "=r"(z)
+      : "r"(response)
+      : "memory");
+  return got != 0;
+}
+
 template <int D>
-__global__ void __launch_bounds__(FA_THREADS, 1) flash_fwd2_kernel(const __grid_constant__ FlashFwdParams p) {
+__global__ void __launch_bounds__(FA2_THREADS, 1) flash_fwd2_kernel(const __grid_constant__ FlashFwdParams p) {
   using Cfg = Flash2Cfg<D>;
   constexpr int DCH = D / 64;
+  constexpr int SLOTS = Cfg::kSlots;
   constexpr int CHUNK_BYTES = FA_BN * 128;
+  constexpr bool EARLY = D == 64;          // P has columns of its own: the next scores need not wait for P V
+  constexpr uint32_t TM_O = 2 * FA_BN, TM_P = EARLY ? 2 * FA_BN + 2 * D : 0, TM_P_STEP = EARLY ? FA_BN / 2 : FA_BN;
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t q_full, kv_full[FA_KV_SLOTS], kv_empty[FA_KV_SLOTS];
-  __shared__ __align__(8) uint64_t s_full[2], s_empty[2], p_full[2], p_empty[2], o_done[2];
+  __shared__ __align__(16) uint4 next_item[2];
+  __shared__ __align__(8) uint64_t q_full, q_empty, kv_full[SLOTS], kv_empty[SLOTS];
+  __shared__ __align__(8) uint64_t s_full[2], s_empty[2], p_full[2][2], o_done[2], item_full[2], item_empty[2];
   __shared__ uint32_t tmem_base_smem;
   __shared__ int abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.z, h = blockIdx.y;
-  const int q_tile = gridDim.x - 1 - blockIdx.x;
-  const int q_begin = p.cu_q[b];
-  const int q_len = p.cu_q[b + 1] - q_begin;
-  const int q0 = q_tile * 2 * FA_BM;
-  if (q0 >= q_len) return;
-  const int kv_len = p.paged ? p.seq_lens[b] : (p.cu_k[b + 1] - p.cu_k[b]);
-  const int k_begin = p.paged ? 0 : p.cu_k[b];
-  const int off = kv_len - q_len;
-  const int kvh = h / (p.Hq / p.Hkv);
-  const bool has_b = q0 + FA_BM < q_len;
-  // key tiles: both query tiles start at tile a's first visible tile; each stops at its own last one
-  const int lo = flash_first_key(p, off + q0);
-  const int t_begin = lo / FA_BN;
-  const int hi_a = p.causal ? min(kv_len, off + q0 + FA_BM) : kv_len;
-  const int hi_b = p.causal ? min(kv_len, off + q0 + 2 * FA_BM) : kv_len;
-  const int n_a = max((hi_a + FA_BN - 1) / FA_BN - t_begin, 0);
-  const int n_b = has_b ? max((hi_b + FA_BN - 1) / FA_BN - t_begin, 0) : 0;
-  const int n_tiles = max(n_a, n_b);
-
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t q_s = smem_base;                                   // Q_a then Q_b
   const uint32_t kv_s = q_s + 2 * Cfg::kTileBytes;
-  const uint32_t p_off = 2 * Cfg::kTileBytes + FA_KV_SLOTS * Cfg::kTileBytes;   // P_a then P_b
-  const uint32_t p_s = smem_base + p_off;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
     mbar_init(smem_u32(&q_full), 1);
-    for (int i = 0; i < FA_KV_SLOTS; ++i) {
+    mbar_init(smem_u32(&q_empty), 1);
+    for (int i = 0; i < SLOTS; ++i) {
       mbar_init(smem_u32(&kv_full[i]), 1);
       mbar_init(smem_u32(&kv_empty[i]), 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&s_full[i]), 1);
       mbar_init(smem_u32(&s_empty[i]), 4);
-      mbar_init(smem_u32(&p_full[i]), 4);
-      mbar_init(smem_u32(&p_empty[i]), 1);
+      mbar_init(smem_u32(&p_full[i][0]), 4);
+      mbar_init(smem_u32(&p_full[i][1]), 4);
       mbar_init(smem_u32(&o_done[i]), 1);
+      mbar_init(smem_u32(&item_full[i]), 1);
+      mbar_init(smem_u32(&item_empty[i]), 10);      // TMA warp, MMA thread, 8 softmax warps
     }
     fence_mbar_init();
   }
@@ -522,264 +597,354 @@ __global__ void __launch_bounds__(FA_THREADS, 1) flash_fwd2_kernel(const __grid_
   const uint32_t tmem_base = tmem_base_smem;
   volatile int* abortp = &abort_flag;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (elect_one_sync()) {
+  // The n-th item of this CTA (n > 0), by every role for itself: false when there is none or a wait ran out.
+  auto take = [&](int n, FlashItem& t, bool arrive) -> bool {
+    const int slot = (n - 1) & 1;
+    if (!mbar_wait_backoff(smem_u32(&item_full[slot]), ((n - 1) >> 1) & 1u, abortp, p.status, ST_TIMEOUT_SMEM_FULL)) return false;
+    int x, y, z;
+    const bool got = clc_read(smem_u32(&next_item[slot]), x, y, z);
+    fence_proxy_async_smem();          // read before the next answer is written over it
+    if (arrive) mbar_arrive(smem_u32(&item_empty[slot]));
+    if (got) t = flash_item(p, x, y, z);
+    return got;
+  };
+  auto take_warp = [&](int n, FlashItem& t) -> bool {      // all lanes read, then one arrives
+    const bool got = __all_sync(0xffffffffu, take(n, t, false));
+    if (lane == 0 && got) mbar_arrive(smem_u32(&item_empty[(n - 1) & 1]));
+    return got;
+  };
+
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FA2_REGS_OTHER));
+    FlashItem t = flash_item(p, blockIdx.x, blockIdx.y, blockIdx.z);
+    if (warp == 0) {
+      // ------------------------------------------------------------------ TMA producer: the whole warp, a box a lane
       bool ok = true;
-      mbar_expect_tx(smem_u32(&q_full), (has_b ? 2 : 1) * Cfg::kTileBytes);
-      for (int x = 0; x < (has_b ? 2 : 1); ++x)
-#pragma unroll
-        for (int c = 0; c < DCH; ++c)
-          tma_load_2d(q_s + x * Cfg::kTileBytes + c * CHUNK_BYTES, &p.q_map, smem_u32(&q_full), h * D + c * 64,
-                      q_begin + q0 + x * FA_BM);
       uint32_t it = 0;
-      auto load_tile = [&](int j, int which) -> bool {
-        const int k0 = (t_begin + j) * FA_BN;
-        const int slot = it % FA_KV_SLOTS;
-        if (!mbar_wait_backoff(smem_u32(&kv_empty[slot]), ((it / FA_KV_SLOTS) & 1u) ^ 1u, abortp, p.status, ST_TIMEOUT_SMEM_EMPTY))
-          return false;
-        const uint32_t fb = smem_u32(&kv_full[slot]);
-        const uint32_t dst = kv_s + slot * Cfg::kTileBytes;
+      int q_loads = 0;
+      auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+        return __all_sync(0xffffffffu, mbar_wait_backoff(smem_u32(bar), parity, abortp, p.status, ST_TIMEOUT_SMEM_EMPTY));
+      };
+      auto load_tile = [&](int j, int which) -> bool {          // which 0: K tile, 1: V tile
+        const int k0 = (t.t_begin + j) * FA_BN, slot = it % SLOTS;
+        if (!wait(&kv_empty[slot], ((it / SLOTS) & 1u) ^ 1u)) return false;
+        const uint32_t fb = smem_u32(&kv_full[slot]), dst = kv_s + slot * Cfg::kTileBytes;
         const CUtensorMap* map = which == 0 ? &p.k_map : &p.v_map;
-        mbar_expect_tx(fb, Cfg::kTileBytes);
+        if (lane == 0) mbar_expect_tx(fb, Cfg::kTileBytes);
+        __syncwarp();
         if (!p.paged) {
-#pragma unroll
-          for (int c = 0; c < DCH; ++c) tma_load_2d(dst + c * CHUNK_BYTES, map, fb, kvh * D + c * 64, k_begin + k0);
-        } else {
-          const int* bt = p.block_tables + (long long)b * p.max_blocks;
-          const int n_blk = (kv_len + 15) >> 4;
-#pragma unroll 1
-          for (int i = 0; i < FA_BN / 16; ++i) {
-            const int bi = (k0 >> 4) + i;
-            int blk = p.num_blocks;
-            if (bi < n_blk) {
-              blk = bt[bi];
-              if (blk < 0 || blk >= p.num_blocks) { set_status(p.status, ST_BAD_INDEX); blk = p.num_blocks; }
-            }
-            const int y = (blk * p.Hkv + kvh) * 16;
-#pragma unroll
-            for (int c = 0; c < DCH; ++c) tma_load_2d(dst + c * CHUNK_BYTES + i * 2048, map, fb, c * 64, y);
+          if (lane < DCH) tma_load_2d(dst + lane * CHUNK_BYTES, map, fb, t.kvh * D + lane * 64, t.k_begin + k0);
+        } else if (lane < 8 * DCH) {
+          const int i = lane / DCH, c = lane % DCH, bi = (k0 >> 4) + i;
+          int blk = p.num_blocks;                               // out of range: the copy fills zeros
+          if (bi < (t.kv_len + 15) >> 4) {
+            blk = p.block_tables[(long long)t.b * p.max_blocks + bi];
+            if (blk < 0 || blk >= p.num_blocks) { set_status(p.status, ST_BAD_INDEX); blk = p.num_blocks; }
           }
+          tma_load_2d(dst + c * CHUNK_BYTES + i * 2048, map, fb, c * 64, (blk * p.Hkv + t.kvh) * 16);
         }
+        __syncwarp();
         ++it;
         return true;
       };
-      if (n_tiles > 0) ok = load_tile(0, 0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        if (j + 1 < n_tiles) { ok = load_tile(j + 1, 0); if (!ok) break; }
-        ok = load_tile(j, 1);
-      }
-      if (!ok) {
-        const uint32_t first = it > (uint32_t)FA_KV_SLOTS ? it - FA_KV_SLOTS : 0;
-        for (uint32_t j = first; j < it; ++j) {
-          const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(smem_u32(&kv_full[j % FA_KV_SLOTS]), (j / FA_KV_SLOTS) & 1u))
-            if (globaltimer_ns() - t0 > 50000000ull) break;
-        }
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (elect_one_sync()) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(FA_BM, FA_BN, 0, 0);
-      constexpr uint32_t idesc_o = make_idesc_bf16(FA_BM, D, 0, 1);
-      bool ok = mbar_wait_backoff(smem_u32(&q_full), 0, abortp, p.status, ST_TIMEOUT_SMEM_FULL);
-      uint32_t it = 0;                       // K/V tiles consumed, in the producer's order
-      const int n_x[2] = {n_a, n_b};
-      // S_x(j) = Q_x K_j^T into TMEM columns x*128; the K tile sits in ring slot `slot`
-      auto issue_s = [&](int x, int j, int slot) -> bool {
-        if (!mbar_wait_backoff(smem_u32(&s_empty[x]), (uint32_t)((j & 1) ^ 1), abortp, p.status, ST_TIMEOUT_TMEM_EMPTY)) return false;
-        tc_fence_after();
-        const uint32_t ks = kv_s + slot * Cfg::kTileBytes, qs = q_s + x * Cfg::kTileBytes;
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t adesc = make_smem_desc_sw128(qs + (k >> 2) * CHUNK_BYTES + (k & 3) * 32, 16, 1024);
-          const uint64_t bdesc = make_smem_desc_sw128(ks + (k >> 2) * CHUNK_BYTES + (k & 3) * 32, 16, 1024);
-          umma_bf16(tmem_base + x * FA_BN, adesc, bdesc, idesc_s, k > 0 ? 1u : 0u);
-        }
-        umma_commit(smem_u32(&s_full[x]));
-        return true;
-      };
-      auto issue_pv = [&](int x, int j, int slot) -> bool {
-        if (!mbar_wait_backoff(smem_u32(&p_full[x]), (uint32_t)(j & 1), abortp, p.status, ST_TIMEOUT_TMEM_FULL)) return false;
-        tc_fence_after();
-        const uint32_t vs = kv_s + slot * Cfg::kTileBytes, ps = p_s + x * Cfg::kPBytes;
-#pragma unroll
-        for (int k = 0; k < FA_BN / 16; ++k) {
-          const uint64_t adesc = make_smem_desc_sw128(ps + (k >> 2) * CHUNK_BYTES + (k & 3) * 32, 16, 1024);
-          const uint64_t bdesc = make_smem_desc_sw128(vs + k * 2048, CHUNK_BYTES, 1024);
-          umma_bf16(tmem_base + 2 * FA_BN + x * D, adesc, bdesc, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-        }
-        umma_commit(smem_u32(&p_empty[x]));
-        umma_commit(smem_u32(&o_done[x]));
-        return true;
-      };
-      auto wait_kv = [&](int slot, uint32_t idx) -> bool {
-        return mbar_wait_backoff(smem_u32(&kv_full[slot]), (idx / FA_KV_SLOTS) & 1u, abortp, p.status, ST_TIMEOUT_SMEM_FULL);
-      };
-      if (ok && n_tiles > 0) {
-        const int slot = it % FA_KV_SLOTS;
-        ok = wait_kv(slot, it);
-        if (ok && n_x[0] > 0) ok = issue_s(0, 0, slot);
-        if (ok && n_x[1] > 0) ok = issue_s(1, 0, slot);
-        if (ok) umma_commit(smem_u32(&kv_empty[slot]));
-        ++it;
-      }
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        int kslot = -1;
-        if (j + 1 < n_tiles) {
-          kslot = it % FA_KV_SLOTS;
-          ok = wait_kv(kslot, it);
-          ++it;
-          if (ok && j + 1 < n_x[0]) ok = issue_s(0, j + 1, kslot);
+      for (int n = 0; ok;) {
+        if (t.valid()) {
+          const int tiles = t.q0 + FA_BM < t.q_len ? 2 : 1, nt = t.n();
+          ok = wait(&q_empty, (q_loads & 1u) ^ 1u);
+          if (!ok) break;
+          if (lane == 0) mbar_expect_tx(smem_u32(&q_full), tiles * Cfg::kTileBytes);
+          __syncwarp();
+          if (lane < tiles * DCH) {
+            const int x = lane / DCH, c = lane % DCH;
+            tma_load_2d(q_s + x * Cfg::kTileBytes + c * CHUNK_BYTES, &p.q_map, smem_u32(&q_full), t.h * D + c * 64, t.q_begin + t.q0 + x * FA_BM);
+          }
+          __syncwarp();
+          ++q_loads;
+          // in the order of use
+          if (nt > 0) ok = load_tile(0, 0);
+          for (int j = 0; j < nt && ok; ++j) {
+            if constexpr (EARLY) {
+              if (j + 1 < nt) ok = load_tile(j + 1, 0);
+              if (ok) ok = load_tile(j, 1);
+            } else {
+              ok = load_tile(j, 1);
+              if (ok && j + 1 < nt) ok = load_tile(j + 1, 0);
+            }
+          }
           if (!ok) break;
         }
-        const int vslot = it % FA_KV_SLOTS;
-        ok = wait_kv(vslot, it);
-        ++it;
-        if (!ok) break;
-        if (j < n_x[0]) { ok = issue_pv(0, j, vslot); if (!ok) break; }
-        if (kslot >= 0) {
-          if (j + 1 < n_x[1]) { ok = issue_s(1, j + 1, kslot); if (!ok) break; }
-          umma_commit(smem_u32(&kv_empty[kslot]));     // K_{j+1} is free once both score products have run
+        ++n;
+        if (!take_warp(n, t)) break;
+      }
+      if (!ok && lane == 0) {   // drain: no bulk copy may land after the CTA has gone
+        auto drain = [&](uint64_t* bar, uint32_t parity) {
+          const uint64_t t0 = globaltimer_ns();
+          while (!mbar_try_wait(smem_u32(bar), parity))
+            if (globaltimer_ns() - t0 > 50000000ull) break;
+        };
+        if (q_loads > 0) drain(&q_full, (q_loads - 1) & 1u);
+        for (uint32_t j = it > (uint32_t)SLOTS ? it - SLOTS : 0; j < it; ++j) drain(&kv_full[j % SLOTS], (j / SLOTS) & 1u);
+      }
+    } else if (warp == 1) {
+      // ------------------------------------------------------------------ MMA issuer
+      if (elect_one_sync()) {
+        constexpr uint32_t idesc_s = make_idesc_bf16(FA_BM, FA_BN, 0, 0);   // Q, K both K-major
+        constexpr uint32_t idesc_o = make_idesc_bf16(FA_BM, D, 0, 1);       // P in tensor memory, V MN-major
+        bool ok = true;
+        uint32_t it = 0, s_count[2] = {0, 0}, p_count[2] = {0, 0};
+        int q_loads = 0;
+        auto wait = [&](uint64_t* bar, uint32_t parity, int code) { return mbar_wait_backoff(smem_u32(bar), parity, abortp, p.status, code); };
+        auto wait_kv = [&](uint32_t idx) { return wait(&kv_full[idx % SLOTS], (idx / SLOTS) & 1u, ST_TIMEOUT_SMEM_FULL); };
+        auto issue_s = [&](int x, uint32_t idx) -> bool {
+          if constexpr (EARLY) {
+            if (!wait(&s_empty[x], (s_count[x] & 1u) ^ 1u, ST_TIMEOUT_TMEM_EMPTY)) return false;
+          }
+          ++s_count[x];
+          tc_fence_after();
+          const uint32_t ks = kv_s + (idx % SLOTS) * Cfg::kTileBytes, qs = q_s + x * Cfg::kTileBytes;
+#pragma unroll
+          for (int k = 0; k < D / 16; ++k) {
+            const uint64_t adesc = make_smem_desc_sw128(qs + (k >> 2) * CHUNK_BYTES + (k & 3) * 32, 16, 1024);
+            const uint64_t bdesc = make_smem_desc_sw128(ks + (k >> 2) * CHUNK_BYTES + (k & 3) * 32, 16, 1024);
+            umma_bf16(tmem_base + x * FA_BN, adesc, bdesc, idesc_s, k > 0 ? 1u : 0u);
+          }
+          umma_commit(smem_u32(&s_full[x]));
+          return true;
+        };
+        auto issue_pv = [&](int x, int j, uint32_t idx) -> bool {
+          const uint32_t vs = kv_s + (idx % SLOTS) * Cfg::kTileBytes;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            if (!wait(&p_full[x][half], p_count[x] & 1u, ST_TIMEOUT_TMEM_FULL)) return false;
+            tc_fence_after();
+#pragma unroll
+            for (int k = half * 4; k < half * 4 + 4; ++k)
+              umma_bf16_ts(tmem_base + TM_O + x * D, tmem_base + TM_P + x * TM_P_STEP + k * 8, make_smem_desc_sw128(vs + k * 2048, CHUNK_BYTES, 1024),
+                           idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+          }
+          ++p_count[x];
+          umma_commit(smem_u32(&o_done[x]));
+          return true;
+        };
+        auto release = [&](uint32_t idx) { umma_commit(smem_u32(&kv_empty[idx % SLOTS])); };
+        for (int n = 0; ok;) {
+          if (t.valid()) {
+            const int nt = t.n();
+            const int n_x[2] = {t.n_a, t.n_b};
+            ok = wait(&q_full, q_loads & 1u, ST_TIMEOUT_SMEM_FULL);
+            ++q_loads;
+            if (!ok) break;
+            if (nt > 0) {
+              ok = wait_kv(it);
+              if (ok && n_x[0] > 0) ok = issue_s(0, it);
+              if (ok && n_x[1] > 0) ok = issue_s(1, it);
+              if (!ok) break;
+              release(it++);
+            }
+            if (nt <= 1) umma_commit(smem_u32(&q_empty));
+            for (int j = 0; j < nt && ok; ++j) {
+              const bool more = j + 1 < nt;
+              if constexpr (EARLY) {
+                if (more) {
+                  ok = wait_kv(it);
+                  if (ok && j + 1 < n_x[0]) ok = issue_s(0, it);
+                  if (ok && j + 1 < n_x[1]) ok = issue_s(1, it);
+                  if (!ok) break;
+                  release(it++);
+                  if (j + 2 == nt) umma_commit(smem_u32(&q_empty));
+                }
+                ok = wait_kv(it);
+                if (ok && j < n_x[0]) ok = issue_pv(0, j, it);
+                if (ok && j < n_x[1]) ok = issue_pv(1, j, it);
+                if (!ok) break;
+                release(it++);
+              } else {
+                const uint32_t iv = it++, ik = it;
+                if (more) ++it;
+                ok = wait_kv(iv);
+                for (int x = 0; x < 2 && ok; ++x) {
+                  if (j < n_x[x]) ok = issue_pv(x, j, iv);
+                  if (ok && x == 1) release(iv);
+                  if (ok && more && x == 0) ok = wait_kv(ik);
+                  if (ok && j + 1 < n_x[x]) ok = issue_s(x, ik);
+                }
+                if (!ok) break;
+                if (more) {
+                  release(ik);
+                  if (j + 2 == nt) umma_commit(smem_u32(&q_empty));
+                }
+              }
+            }
+            if (!ok) break;
+          }
+          ++n;
+          if (!take(n, t, true)) break;
         }
-        if (j < n_x[1]) { ok = issue_pv(1, j, vslot); if (!ok) break; }
-        umma_commit(smem_u32(&kv_empty[vslot]));
+      }
+    } else if (warp == 2) {
+      // ------------------------------------------------------------------ next items, two answers ahead at most
+      if (elect_one_sync()) {
+        for (int n = 1;; ++n) {
+          const int slot = (n - 1) & 1;
+          const uint32_t use = (n - 1) >> 1;
+          if (!mbar_wait_backoff(smem_u32(&item_empty[slot]), (use & 1u) ^ 1u, abortp, p.status, ST_TIMEOUT_SMEM_EMPTY)) break;
+          mbar_expect_tx(smem_u32(&item_full[slot]), 16);
+          clc_try_cancel(smem_u32(&next_item[slot]), smem_u32(&item_full[slot]));
+          // the answer is waited for in any case: it must not land after the CTA has gone
+          const uint64_t t0 = globaltimer_ns();
+          bool there;
+          while (!(there = mbar_try_wait_hint(smem_u32(&item_full[slot]), use & 1u, 2000u)))
+            if (globaltimer_ns() - t0 > RB_WAIT_BUDGET_NS) break;
+          if (!there) {
+            *abortp = 1;
+            set_status(p.status, ST_TIMEOUT_SMEM_FULL);
+            break;
+          }
+          int x, y, z;
+          if (!clc_read(smem_u32(&next_item[slot]), x, y, z)) break;
+          fence_proxy_async_smem();
+        }
       }
     }
   } else {
     // ------------------------------------------------------------------ softmax + epilogue, one warpgroup per query tile
-    const int x = (warp - 2) >> 2;               // 0: tile a, 1: tile b
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FA2_REGS_SOFTMAX));
+    FlashItem t = flash_item(p, blockIdx.x, blockIdx.y, blockIdx.z);
+    const int x = (warp >> 2) - 1;               // 0: tile a, 1: tile b
     const int qd = warp & 3;
     const int r = qd * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(qd * 32) << 16;
-    const int q0x = q0 + x * FA_BM;
-    const int qpos = off + q0x + r;
-    const int k_first = flash_first_key(p, qpos), last_first = flash_first_key(p, off + q0x + FA_BM - 1);
-    const int n_mine = x == 0 ? n_a : n_b;
     const uint32_t tmem_s = tmem_base + x * FA_BN + lane_addr;
-    const uint32_t tmem_o = tmem_base + 2 * FA_BN + x * D + lane_addr;
-    uint8_t* prow = smem_al + p_off + x * Cfg::kPBytes + r * 128;
-    float m_used = -INFINITY, l = 0.f;
+    const uint32_t tmem_o = tmem_base + TM_O + x * D + lane_addr;
+    const uint32_t tmem_p = tmem_base + TM_P + x * TM_P_STEP + lane_addr;
+    const uint64_t scale2 = pair(p.scale_log2, p.scale_log2);
+    uint32_t count = 0;                          // key tiles of this query tile so far, all items
     bool ok = true;
-    for (int j = 0; j < n_mine; ++j) {
-      const int k0 = (t_begin + j) * FA_BN;
-      ok = mbar_wait_backoff(smem_u32(&s_full[x]), (uint32_t)(j & 1), abortp, p.status, ST_TIMEOUT_TMEM_FULL);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
-      const bool need_mask = (k0 + FA_BN > kv_len) || (p.causal && k0 + FA_BN - 1 > off + q0x) ||
-                             k0 < last_first;
-      uint32_t v[FA_BN];
-#pragma unroll
-      for (int c = 0; c < FA_BN / 32; ++c)
-        tmem_ld_32x32(tmem_s + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&v[c * 32]));
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&s_empty[x]));       // the next score product may overwrite S now
-      if (need_mask) {
-#pragma unroll
-        for (int i = 0; i < FA_BN; ++i) {
-          const int kj = k0 + i;
-          const bool dead = kj >= kv_len || (p.causal && kj > qpos) || kj < k_first;
-          if (dead) v[i] = 0xff800000u;
-        }
-      }
-      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int i = 0; i < FA_BN; i += 4) {
-        mx[0] = fmaxf(mx[0], __uint_as_float(v[i]));
-        mx[1] = fmaxf(mx[1], __uint_as_float(v[i + 1]));
-        mx[2] = fmaxf(mx[2], __uint_as_float(v[i + 2]));
-        mx[3] = fmaxf(mx[3], __uint_as_float(v[i + 3]));
-      }
-      const float m_new = fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2);
-      const bool need = m_new > m_used + FA_RESCALE_THRESHOLD || (m_used == -INFINITY && m_new != -INFINITY);
-      if (__any_sync(0xffffffffu, need)) {
-        if (j > 0) {
-          ok = mbar_wait_backoff(smem_u32(&o_done[x]), (uint32_t)((j - 1) & 1), abortp, p.status, ST_TIMEOUT_TMEM_FULL);
-          ok = __all_sync(0xffffffffu, ok);
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+      return __all_sync(0xffffffffu, mbar_wait_backoff(smem_u32(bar), parity, abortp, p.status, ST_TIMEOUT_TMEM_FULL));
+    };
+    for (int n = 0; ok;) {
+      const int q0x = t.q0 + x * FA_BM;
+      if (t.valid() && q0x < t.q_len) {
+        const int qpos = t.off + q0x + r;
+        const int k_first = flash_first_key(p, qpos), last_first = flash_first_key(p, t.off + q0x + FA_BM - 1);
+        const int n_mine = x == 0 ? t.n_a : t.n_b;
+        float m_used = -INFINITY, l = 0.f;
+        for (int j = 0; j < n_mine; ++j, ++count) {
+          const int k0 = (t.t_begin + j) * FA_BN;
+          ok = wait(&s_full[x], count & 1u);
           if (!ok) break;
           tc_fence_after();
-          const float alpha = need ? fast_exp2((m_used == -INFINITY ? m_new : m_used) - m_new) : 1.f;
+          const bool need_mask = (k0 + FA_BN > t.kv_len) || (p.causal && k0 + FA_BN - 1 > t.off + q0x) || k0 < last_first;
+          uint32_t v[FA_BN];
+#pragma unroll
+          for (int c = 0; c < FA_BN / 32; ++c) tmem_ld_32x32(tmem_s + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&v[c * 32]));
+          tmem_ld_wait();
+          if constexpr (EARLY) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&s_empty[x]));       // the next scores may take the columns now
+          }
+          if (need_mask) {
+            // keys k_first <= k <= last of this row
+            const int last = (p.causal ? min(t.kv_len - 1, qpos) : t.kv_len - 1) - k0, first = k_first - k0;
+#pragma unroll
+            for (int i = 0; i < FA_BN; ++i)
+              if (i > last || i < first) v[i] = 0xff800000u;
+          }
+          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+          for (int i = 0; i < FA_BN; i += 8) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) mx[u] = max3(mx[u], __uint_as_float(v[i + 2 * u]), __uint_as_float(v[i + 2 * u + 1]));
+          }
+          const float m_new = fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2);
+          const bool need = m_new > m_used + FA_RESCALE_THRESHOLD || (m_used == -INFINITY && m_new != -INFINITY);
+          if (EARLY && j > 0) {      // the previous P V has read P and written O (D = 128: these scores came after it)
+            ok = wait(&o_done[x], (count - 1) & 1u);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          if (__any_sync(0xffffffffu, need)) {
+            if (j > 0) {
+              const float alpha = need ? fast_exp2((m_used == -INFINITY ? m_new : m_used) - m_new) : 1.f;
 #pragma unroll 1
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t o[32];
+              for (int c = 0; c < D / 16; ++c) {
+                uint32_t o[16];
+                tmem_ld_32x16(tmem_o + c * 16, o);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                tmem_st_32x16(tmem_o + c * 16, o);
+              }
+              l *= alpha;
+            }
+            if (need) m_used = m_new;
+          }
+          const float mref = m_used == -INFINITY ? 0.f : m_used;
+          const uint64_t neg2 = pair(-mref, -mref);
+          uint64_t ls[2] = {0, 0};       // four running sums, keys 4 i + 0 .. 3
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            uint32_t w[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const int e = half * 64 + 2 * i;
+              float a, b;
+              unpair(fma2(pair(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), scale2, neg2), a, b);
+              a = fast_exp2(a);
+              b = fast_exp2(b);
+              ls[i & 1] = add2(ls[i & 1], pair(a, b));
+              w[i] = pack_bf16x2(a, b);
+            }
+            tmem_st_32x32(tmem_p + half * 32, w);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&p_full[x][half]));
+          }
+          float s0, s1, s2, s3;
+          unpair(ls[0], s0, s1);
+          unpair(ls[1], s2, s3);
+          l += (s0 + s1) + (s2 + s3);
+        }
+        if (!ok) break;
+        if (n_mine > 0) {
+          ok = wait(&o_done[x], (count - 1) & 1u);
+          if (!ok) break;
+        }
+        tc_fence_after();
+        const bool row_ok = q0x + r < t.q_len;
+        const float inv = l > 0.f && row_ok ? flash_gate(p, t.q_begin + q0x + r, t.h) / l : 0.f;
+        __nv_bfloat16* orow = p.out + (long long)(t.q_begin + q0x + r) * p.ldo + t.h * D;
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t o[32];
+          if (n_mine > 0) {
             tmem_ld_32x32(tmem_o + c * 32, o);
             tmem_ld_wait();
+          } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32(tmem_o + c * 32, o);
+            for (int i = 0; i < 32; ++i) o[i] = 0u;
           }
-          tmem_st_wait();
-          l *= alpha;
-        }
-        if (need) m_used = m_new;
-      }
-      const float mref = m_used == -INFINITY ? 0.f : m_used;
-      float ls[4] = {0.f, 0.f, 0.f, 0.f};
+          if (row_ok) {
 #pragma unroll
-      for (int i = 0; i < FA_BN; i += 4) {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const float e = fast_exp2(fmaf(__uint_as_float(v[i + t]), p.scale_log2, -mref));
-          ls[t] += e;
-          v[i + t] = __float_as_uint(e);
-        }
-      }
-      l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
-      // P buffer is free once the previous P V of this tile has read it
-      ok = mbar_wait_backoff(smem_u32(&p_empty[x]), (uint32_t)((j & 1) ^ 1), abortp, p.status, ST_TIMEOUT_SMEM_EMPTY);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-#pragma unroll
-      for (int unit = 0; unit < FA_BN / 8; ++unit) {
-        uint4 w;
-        w.x = pack_bf16x2(__uint_as_float(v[unit * 8 + 0]), __uint_as_float(v[unit * 8 + 1]));
-        w.y = pack_bf16x2(__uint_as_float(v[unit * 8 + 2]), __uint_as_float(v[unit * 8 + 3]));
-        w.z = pack_bf16x2(__uint_as_float(v[unit * 8 + 4]), __uint_as_float(v[unit * 8 + 5]));
-        w.w = pack_bf16x2(__uint_as_float(v[unit * 8 + 6]), __uint_as_float(v[unit * 8 + 7]));
-        *reinterpret_cast<uint4*>(prow + (unit >> 3) * CHUNK_BYTES + (((unit & 7) ^ (r & 7)) << 4)) = w;
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&p_full[x]));
-    }
-    if (ok && n_mine > 0) {
-      ok = mbar_wait_backoff(smem_u32(&o_done[x]), (uint32_t)((n_mine - 1) & 1), abortp, p.status, ST_TIMEOUT_TMEM_FULL);
-      ok = __all_sync(0xffffffffu, ok);
-    }
-    if (ok && (x == 0 || has_b)) {
-      tc_fence_after();
-      const bool row_ok = q0x + r < q_len;
-      const float inv = l > 0.f && row_ok ? flash_gate(p, q_begin + q0x + r, h) / l : 0.f;
-      __nv_bfloat16* orow = p.out + (long long)(q_begin + q0x + r) * p.ldo + h * D;
-#pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t o[32];
-        if (n_mine > 0) {
-          tmem_ld_32x32(tmem_o + c * 32, o);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = 0u;
-        }
-        if (row_ok) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 w;
-            w.x = pack_bf16x2(__uint_as_float(o[u * 8 + 0]) * inv, __uint_as_float(o[u * 8 + 1]) * inv);
-            w.y = pack_bf16x2(__uint_as_float(o[u * 8 + 2]) * inv, __uint_as_float(o[u * 8 + 3]) * inv);
-            w.z = pack_bf16x2(__uint_as_float(o[u * 8 + 4]) * inv, __uint_as_float(o[u * 8 + 5]) * inv);
-            w.w = pack_bf16x2(__uint_as_float(o[u * 8 + 6]) * inv, __uint_as_float(o[u * 8 + 7]) * inv);
-            *reinterpret_cast<uint4*>(orow + c * 32 + u * 8) = w;
+            for (int u = 0; u < 4; ++u) {
+              uint4 w;
+              w.x = pack_bf16x2(__uint_as_float(o[u * 8 + 0]) * inv, __uint_as_float(o[u * 8 + 1]) * inv);
+              w.y = pack_bf16x2(__uint_as_float(o[u * 8 + 2]) * inv, __uint_as_float(o[u * 8 + 3]) * inv);
+              w.z = pack_bf16x2(__uint_as_float(o[u * 8 + 4]) * inv, __uint_as_float(o[u * 8 + 5]) * inv);
+              w.w = pack_bf16x2(__uint_as_float(o[u * 8 + 6]) * inv, __uint_as_float(o[u * 8 + 7]) * inv);
+              *reinterpret_cast<uint4*>(orow + c * 32 + u * 8) = w;
+            }
           }
         }
+        if (row_ok && p.lse != nullptr)
+          p.lse[(long long)t.h * p.Tq + t.q_begin + q0x + r] = l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
+        tc_fence_before();       // O has been read: the next item's first product may overwrite it
       }
-      if (row_ok && p.lse != nullptr)
-        p.lse[(long long)h * p.Tq + q_begin + q0x + r] = l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
-      tc_fence_before();
+      ++n;
+      if (!take_warp(n, t)) break;
     }
   }
   __syncthreads();
@@ -1788,12 +1953,19 @@ static int launch_flash_fwd(const FlashFwdParams& p, int max_seqlen_q, int B, cu
     if (cudaFuncSetAttribute(flash_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, FlashCfg<D>::kSmemBytes) != cudaSuccess ||
         cudaFuncSetAttribute(flash_fwd2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Flash2Cfg<D>::kSmemBytes) != cudaSuccess)
       return -10;
+    // the register shares of the roles have to add up to what a block is launched with
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, flash_fwd2_kernel<D>) != cudaSuccess || fa.numRegs < FA2_REGS_LAUNCH) return -13;
     attr = true;
   }
   static const bool one_tile = getenv("RB_FLASH_ONE_TILE") != nullptr;
-  if (max_seqlen_q > FA_BM && !one_tile) {   // two query tiles per CTA share every K/V tile
+  // Two query tiles per CTA share every K/V tile; a single tile's rows are better split over both warpgroups (flash_fwd_kernel).
+  // Causal, TFLOP/s, dense / paged keys (in brackets with P in shared memory and a CTA per tile pair): 4 x 8192 tokens, 32 / 8
+  // heads, D 128 1180 / 1011 (852 / 624); 8 x 2048 955 / 935 (470 / 416); 32 x 200 163 / 160 (67 / 66); 1 x 16384, 14 / 2 heads,
+  // D 64 703 / 697 (507 / 333); 16 x 512 179 / 175 (82 / 80).
+  if (max_seqlen_q > FA_BM && !one_tile) {
     dim3 grid((max_seqlen_q + 2 * FA_BM - 1) / (2 * FA_BM), p.Hq, B);
-    return launch_kernel(flash_fwd2_kernel<D>, grid, dim3(FA_THREADS), Flash2Cfg<D>::kSmemBytes, stream, p) == cudaSuccess ? 0 : -11;
+    return launch_kernel(flash_fwd2_kernel<D>, grid, dim3(FA2_THREADS), Flash2Cfg<D>::kSmemBytes, stream, p) == cudaSuccess ? 0 : -11;
   }
   dim3 grid((max_seqlen_q + FA_BM - 1) / FA_BM, p.Hq, B);
   return launch_kernel(flash_fwd_kernel<D>, grid, dim3(FA_THREADS), FlashCfg<D>::kSmemBytes, stream, p) == cudaSuccess ? 0 : -11;

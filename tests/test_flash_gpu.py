@@ -184,3 +184,41 @@ def test_flash_backward_head_split(cuda_device, monkeypatch, D, Hq, Hkv):
     assert flash.head_split_pays(1, 4096, 4096, 16, 2) and not flash.head_split_pays(1, 4096, 4096, 32, 8)
     assert not flash.head_split_pays(32, 512, 512, 14, 2) and not flash.head_split_pays(1, 4096, 4096, 8, 8)
     ops.check_status()
+
+
+@pytest.mark.parametrize("paged", [False, True])
+@pytest.mark.parametrize("D,H,Hkv,window", [(64, 14, 2, 0), (128, 8, 8, 0), (64, 6, 6, 200), (128, 4, 1, 129)])
+def test_flash_forward_tile_edges_many_items_a_block(D, H, Hkv, window, paged):
+    """More query tiles than the GPU has SMs, sequences around the tile sizes, empty ones and (paged) cached prefixes among them."""
+    lens = [1, 127, 128, 129, 255, 256, 257, 0, 640, 1000, 383, 384, 385]
+    prefix = [0, 5, 128, 0, 1, 130, 0, 7, 0, 16, 300, 0, 129] if paged else [0] * len(lens)
+    g = torch.Generator(device="cuda").manual_seed(D + H + window)
+    T, S = sum(lens), sum(lens) + sum(prefix)
+    q = torch.randn(T, H, D, device="cuda", generator=g).bfloat16()
+    k, v = (torch.randn(S, Hkv, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    cu_q = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device="cuda")
+    kv = [a + b for a, b in zip(lens, prefix)]
+    cu_k = torch.tensor([sum(kv[:i]) for i in range(len(kv) + 1)], dtype=torch.int32, device="cuda")
+    lse = torch.empty(H, T, device="cuda")
+    if paged:
+        blocks = [-(-n // 16) for n in kv]
+        order = torch.randperm(sum(blocks), generator=torch.Generator().manual_seed(1)).tolist()
+        bt = torch.zeros(len(kv), max(blocks), dtype=torch.int32)
+        kc, vc = (torch.zeros(sum(blocks), Hkv, 16, D, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        at = 0
+        for i, n in enumerate(kv):
+            for j in range(blocks[i]):
+                bt[i, j] = order[at]
+                m = min(16, n - 16 * j)
+                for cache, src in ((kc, k), (vc, v)):
+                    cache[order[at], :, :m] = src[int(cu_k[i]) + 16 * j:int(cu_k[i]) + 16 * j + m].transpose(0, 1)
+                at += 1
+        out = ops.flash_paged_prefill(q, kc, vc, bt.cuda(), cu_q, torch.tensor(kv, dtype=torch.int32, device="cuda"), max(lens), window=window, lse=lse)
+    else:
+        out, lse = ops.flash_attn_varlen(q, k, v, cu_q, cu_k, max(lens), window=window, return_lse=True)
+    ref, ref_lse = ops.flash_attn_varlen_reference(q.float(), k, v, cu_q, cu_k, window=window)
+    size, _ = ops.flash_attn_varlen_reference(q.float(), k, v.abs(), cu_q, cu_k, window=window)
+    # P and the output are rounded to bf16 (2^-9 each, relative); P's error meets every |v|
+    assert ((out.float() - ref).abs() <= 2.0 ** -8 * size + 2.0 ** -8 * ref.abs() + 1e-6).all()
+    assert ((lse - ref_lse).abs() <= 1e-4 * (1 + ref_lse.abs())).all()
+    ops.check_status(torch.device("cuda"))
