@@ -55,7 +55,10 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity
 }
 __device__ __forceinline__ bool mbar_wait_backoff(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
                                                   int code) {
-  if (mbar_try_wait(bar, parity)) return true;
+  // the timer is read only once the wait has become a long one: its read takes long enough to miss the flip by
+#pragma unroll 1
+  for (int i = 0; i < 16; ++i)
+    if (mbar_try_wait_hint(bar, parity, 2000u)) return true;
   const uint64_t t0 = globaltimer_ns();
   uint32_t spins = 0;
   while (true) {
@@ -1312,21 +1315,34 @@ static int launch_flash_latent(const FlashLatentParams& p, int max_q, int B, cud
 
 // ==========================================================================================
 // Backward. Three kernels, no atomics, deterministic:
-//   prep : delta[h,t] = sum_d dO*O and lse in log2 units
+//   prep : -lse (log2 units) and -delta, delta[h,t] = sum_d dO*O, per 128-query tile of every sequence
 //   dkdv : one CTA per (128-key tile, kv head); loops over the query heads of the group and their
-//          64-query tiles. S^T = K Q^T and dP^T = V dO^T land in TMEM (keys on the 128 lanes, so a
-//          thread owns a key row), P^T and dS^T go to shared memory as K-major A operands of
-//          dV += P^T dO and dK += dS^T Q, which accumulate in TMEM over the whole loop.
-//   dq   : one CTA per (128-query tile, head); loops over 64-key tiles. S = Q K^T, dP = dO V^T in
-//          TMEM, dS to shared memory, dQ += dS K accumulates in TMEM.
+//          128-query tiles. S^T = K Q^T and dP^T = V dO^T land in tensor memory (keys on the 128 lanes, so a
+//          thread owns a key row); P^T and dS^T go back there, packed to bf16, as A operands of
+//          dV += P^T dO and dK += dS^T Q, which accumulate in tensor memory over the whole loop.
+//   dq   : one CTA per (128-query tile, head); loops over 128-key tiles. S = Q K^T, dP = dO V^T, dS back to
+//          tensor memory, dQ += dS K accumulates there.
 // The same Q / dO / K / V shared-memory tile serves as a K-major operand of the score products and
 // as an MN-major operand of the gradient products: only the descriptor differs.
+//
+// What bounds it (D = 128, a 128 x 128 tile): 512 cycles of the tensor core for each of the four (dq: three) products and
+// 1024 of the special-function unit, while the way from a finished product through the softmax warps to the next one is
+// some 800 cycles long. Tensor memory has room for one S and one dP beside the accumulators, so the products are issued in
+// an order that always leaves two to run while the softmax warps work (dkdv; dq has one to run):
+//     dkdv:  dV(j)  S(j+1)  dK(j)  dP(j+1)      P(j+1) under dK(j), dP(j+1); dS(j) under dV(j), S(j+1)
+//     dq:    S(j+1)  dQ(j)  dP(j+1)             P(j+1) under dQ(j), dP(j+1); dS(j) under S(j+1)
+// P takes the columns of S and dS those of dP (products run in the order of their issue, so a new score tile never
+// overtakes the product that reads the old P). All 16 softmax warps work on one tile, 32 of its columns each. A 64-wide score
+// product would read 6 KB of shared memory for 32 cycles of work, one 128 wide 8 KB for 64: just what it delivers; dq
+// keeps Q and dO in tensor memory and reads half of that. The row statistics of a query tile arrive with its Q and dO.
+// Backward of causal attention, TFLOP/s by 2.5 x the forward's (in brackets with 64-wide tiles, P and dS through shared memory):
+// 4 x 8192 tokens, 32 / 8 heads, D 128 757 (442); 8 x 2048 650 (343); 32 x 200 125 (70); 1 x 16384, 14 / 2 heads, D 64 530 (212);
+// 16 x 512 159 (74).
 // ==========================================================================================
 struct FlashBwdParams {
-  CUtensorMap q64, do64, k128, v128;     // dkdv kernel boxes
-  CUtensorMap q128, do128, k64, v64;     // dq kernel boxes
-  const float* lse2;                     // [Hq, Tq]
-  const float* delta;                    // [Hq, Tq]
+  CUtensorMap q, dout, k, v;             // boxes of 64 columns x 128 rows
+  const float* stat;                     // [Hq][stat_tiles][2 (-lse2, -delta)][128]; the tiles of sequence b start at tile cu_q[b] / 128 + b
+  int stat_tiles;
   __nv_bfloat16 *dq, *dk, *dv;           // [Tq,Hq,D], [Tk,Hkv,D], [Tk,Hkv,D]
   const int* cu_q;
   const int* cu_k;
@@ -1341,78 +1357,122 @@ struct FlashBwdParams {
   float* dkv_part;
 };
 
-__global__ void flash_bwd_prep_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
-                                      const float* __restrict__ lse, float* __restrict__ delta,
-                                      float* __restrict__ lse2, int Tq, int Hq, int D) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= Tq * Hq) return;
-  const int t = warp / Hq, h = warp % Hq;
-  const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(dout + ((long long)t * Hq + h) * D);
-  const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(out + ((long long)t * Hq + h) * D);
-  float acc = 0.f;
-  for (int i = lane; i < D / 2; i += 32) {
-    const float2 x = __bfloat1622float2(a[i]), y = __bfloat1622float2(b[i]);
-    acc += x.x * y.x + x.y * y.y;
-  }
+// One warp per row, four rows in flight; block (tile of 128 queries, sequence, head).
+template <int D>
+__global__ void __launch_bounds__(256) flash_bwd_prep_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
+                                                             const float* __restrict__ lse, float* __restrict__ stat, const int* __restrict__ cu_q,
+                                                             int stat_tiles, int Tq, int Hq) {
+  const int b = blockIdx.y, h = blockIdx.z, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q_begin = cu_q[b], q_len = cu_q[b + 1] - q_begin, i0 = blockIdx.x * 128;
+  if (i0 >= q_len) return;
+  float* dst = stat + ((long long)h * stat_tiles + (q_begin >> 7) + b + blockIdx.x) * 256;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) {
-    delta[(long long)h * Tq + t] = acc;
-    lse2[(long long)h * Tq + t] = lse[(long long)h * Tq + t] * 1.4426950408889634f;
+  for (int r0 = 0; r0 < 16; r0 += 4) {
+    __nv_bfloat162 x[4][D / 64], y[4][D / 64];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + warp * 16 + r0 + u;
+      const long long at = ((long long)(q_begin + min(i, q_len - 1)) * Hq + h) * D;
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c) {
+        x[u][c] = reinterpret_cast<const __nv_bfloat162*>(dout + at)[c * 32 + lane];
+        y[u][c] = reinterpret_cast<const __nv_bfloat162*>(out + at)[c * 32 + lane];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int r = warp * 16 + r0 + u;
+      float acc = 0.f;
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c) {
+        const float2 f = __bfloat1622float2(x[u][c]), g = __bfloat1622float2(y[u][c]);
+        acc += f.x * g.x + f.y * g.y;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0) {
+        const bool in = i0 + r < q_len;      // past the end: P is exactly 0
+        dst[r] = in ? -(lse[(long long)h * Tq + q_begin + i0 + r] * 1.4426950408889634f) : -INFINITY;
+        dst[128 + r] = in ? -acc : 0.f;
+      }
+    }
   }
 }
 
 template <int D>
 struct FlashBwdCfg {
-  static constexpr int kQdoStages = D == 128 ? 2 : 4;       // dkdv: (Q, dO) 64-row tiles in flight
-  static constexpr int kKvStages = 3;                       // dq: (K, V) 64-row tiles in flight
-  static constexpr int kBig = 128 * D * 2;                  // a 128-row tile
-  static constexpr int kSmall = 64 * D * 2;                 // a 64-row tile
-  static constexpr int kPd = 128 * 64 * 2;                  // P^T / dS^T / dS tile
-  static constexpr int kSmemDkdv = 1024 + 2 * kBig + kQdoStages * 2 * kSmall + 4 * kPd;
-  static constexpr int kSmemDq = 1024 + 2 * kBig + kKvStages * 2 * kSmall + 2 * kPd;
+  static constexpr int kTile = 128 * D * 2;                 // a 128-row tile
+  static constexpr int kStat = 2 * 128 * 4;
+  static constexpr int kQdoStages = D == 128 ? 2 : 3;       // dkdv: (Q, dO, statistics) of 128 queries in flight
+  static constexpr int kKvStages = D == 128 ? 2 : 4;        // dq: (K, V) tiles in flight
+  static constexpr int kSmemDkdv = 1024 + 2 * kTile + kQdoStages * (2 * kTile + kStat);
+  static constexpr int kSmemDq = 1024 + 2 * kTile + kKvStages * 2 * kTile;
 };
 
-// 64 packed bf16 values of one row into a 128-byte swizzled row of a K-major tile
-__device__ __forceinline__ void store_row64_sw128(uint8_t* row_ptr, int r, const float (&x)[64]) {
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    uint4 w;
-    w.x = pack_bf16x2(x[u * 8 + 0], x[u * 8 + 1]);
-    w.y = pack_bf16x2(x[u * 8 + 2], x[u * 8 + 3]);
-    w.z = pack_bf16x2(x[u * 8 + 4], x[u * 8 + 5]);
-    w.w = pack_bf16x2(x[u * 8 + 6], x[u * 8 + 7]);
-    *reinterpret_cast<uint4*>(row_ptr + ((u ^ (r & 7)) << 4)) = w;
-  }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// contiguous copy global -> shared (both 16-byte aligned, whole 16-byte units)
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
 
-// 32 values (columns half*32 .. half*32+31) of one row into its 128-byte swizzled row
-__device__ __forceinline__ void store_row32_sw128(uint8_t* row_ptr, int r, int half, const float (&x)[32]) {
+// Warps 0 (TMA), 1 (products), 2 and 3 idle, then four softmax warpgroups, each with 32 of a tile's 128 columns.
+constexpr int FA_BWD_THREADS = 640;
+constexpr int FA_BWD_WARPS = 16;      // softmax warps
+
+// 32 columns of P: exp2(S * scale + statistic); `nl` holds one pair of -lse2 for each pair of columns, `dead` the masked ones
+template <typename Neg>
+__device__ __forceinline__ void bwd_probabilities(uint32_t (&v)[32], uint64_t scale_l2, Neg neg, uint32_t dead, uint32_t (&packed)[16]) {
 #pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    uint4 w;
-    w.x = pack_bf16x2(x[u * 8 + 0], x[u * 8 + 1]);
-    w.y = pack_bf16x2(x[u * 8 + 2], x[u * 8 + 3]);
-    w.z = pack_bf16x2(x[u * 8 + 4], x[u * 8 + 5]);
-    w.w = pack_bf16x2(x[u * 8 + 6], x[u * 8 + 7]);
-    *reinterpret_cast<uint4*>(row_ptr + (((half * 4 + u) ^ (r & 7)) << 4)) = w;
+  for (int c = 0; c < 32; c += 2) {
+    float x0, x1;
+    unpair(fma2(pair(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), scale_l2, neg(c)), x0, x1);
+    x0 = fast_exp2(x0);
+    x1 = fast_exp2(x1);
+    if (dead != 0) {
+      if (dead >> c & 1) x0 = 0.f;
+      if (dead >> (c + 1) & 1) x1 = 0.f;
+    }
+    v[c] = __float_as_uint(x0);
+    v[c + 1] = __float_as_uint(x1);
+    packed[c >> 1] = pack_bf16x2(x0, x1);
   }
 }
-
-// The backward kernels run two softmax warpgroups (warps 2-5 and 6-9): both see the same 128 TMEM
-// lanes and split the 64 columns of a tile, which puts two such warps on every scheduler.
-constexpr int FA_BWD_THREADS = 320;
+// dS = P * (dP - delta) * scale
+template <typename Neg>
+__device__ __forceinline__ void bwd_scores(const uint32_t (&prob)[32], const uint32_t (&dp)[32], uint64_t scale2, Neg neg, uint32_t (&packed)[16]) {
+#pragma unroll
+  for (int c = 0; c < 32; c += 2) {
+    float y0, y1;
+    unpair(mul2(mul2(pair(__uint_as_float(prob[c]), __uint_as_float(prob[c + 1])),
+                     add2(pair(__uint_as_float(dp[c]), __uint_as_float(dp[c + 1])), neg(c))), scale2), y0, y1);
+    packed[c >> 1] = pack_bf16x2(y0, y1);
+  }
+}
+// bit c: position first + c lies outside [lo, hi]
+__device__ __forceinline__ uint32_t outside_mask(int first, int lo, int hi) {
+  const int a = lo - first, z = hi - first;          // columns a .. z are inside
+  const uint32_t below = a <= 0 ? 0u : a >= 32 ? 0xffffffffu : (1u << a) - 1u;
+  const uint32_t upto = z < 0 ? 0u : z >= 31 ? 0xffffffffu : (2u << z) - 1u;
+  return below | ~upto;
+}
+// A operand of the gradient products: 128 columns = 8 k-steps of 8 packed columns, the quarters of a row 32 columns apart
+__device__ __forceinline__ uint32_t packed_column(int k) { return (k >> 1) * 32 + (k & 1) * 8; }
 
 template <int D>
 __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dkdv_kernel(const __grid_constant__ FlashBwdParams p) {
   using Cfg = FlashBwdCfg<D>;
   constexpr int DCH = D / 64;
   constexpr int ST = Cfg::kQdoStages;
-  constexpr int CH128 = 128 * 128, CH64 = 64 * 128;   // bytes of one 64-column chunk of a 128- / 64-row tile
+  constexpr int CH = 128 * 128;                    // bytes of one 64-column chunk of a tile
+  constexpr uint32_t TM_DP = 128, TM_DV = 256, TM_DK = 256 + D;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t kv_full, qdo_full[ST], qdo_empty[ST];
-  __shared__ __align__(8) uint64_t st_full[2], st_empty[2], pds_full[2], pds_empty[2], acc_done, stat_bar;
-  __shared__ __align__(16) float stat[2][2][64];
+  __shared__ __align__(8) uint64_t s_full, p_full, dp_full, ds_full, acc_done;
   __shared__ uint32_t tmem_base_smem;
   __shared__ int abort_flag;
 
@@ -1434,29 +1494,25 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dkdv_kernel(const
   int qi_lo = 0, qi_hi = q_len;
   if (p.causal) qi_lo = max(0, k0 - off);
   if (p.window > 0) qi_hi = min(q_len, kmax + p.window - off);
-  const int i_begin = qi_lo / 64;
-  const int n_qt = qi_hi > qi_lo ? (qi_hi + 63) / 64 - i_begin : 0;
+  const int i_begin = qi_lo / 128;
+  const int n_qt = qi_hi > qi_lo ? (qi_hi + 127) / 128 - i_begin : 0;
   const int n_iter = n_qt * (head_split ? 1 : G);
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t k_s = smem_base, v_s = k_s + Cfg::kBig;
-  const uint32_t qdo_s = v_s + Cfg::kBig;                       // stage: Q tile then dO tile
-  const uint32_t pds_off = 2 * Cfg::kBig + ST * 2 * Cfg::kSmall;   // buffer: P^T then dS^T
-  const uint32_t pds_s = smem_base + pds_off;
+  const uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
+  const uint32_t k_s = smem_base, v_s = k_s + Cfg::kTile;
+  const uint32_t qdo_s = v_s + Cfg::kTile;                       // stage: Q tile then dO tile
+  constexpr uint32_t stat_off = 2 * Cfg::kTile + ST * 2 * Cfg::kTile;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
     mbar_init(smem_u32(&kv_full), 1);
     for (int i = 0; i < ST; ++i) { mbar_init(smem_u32(&qdo_full[i]), 1); mbar_init(smem_u32(&qdo_empty[i]), 1); }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&st_full[i]), 1);
-      mbar_init(smem_u32(&st_empty[i]), 8);
-      mbar_init(smem_u32(&pds_full[i]), 8);
-      mbar_init(smem_u32(&pds_empty[i]), 1);
-    }
+    mbar_init(smem_u32(&s_full), 1);
+    mbar_init(smem_u32(&dp_full), 1);
+    mbar_init(smem_u32(&p_full), FA_BWD_WARPS);
+    mbar_init(smem_u32(&ds_full), FA_BWD_WARPS);
     mbar_init(smem_u32(&acc_done), 1);
-    mbar_init(smem_u32(&stat_bar), 256);
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -1467,17 +1523,16 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dkdv_kernel(const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
-  const uint32_t tm_dv = tmem_base + 256, tm_dk = tmem_base + 256 + D;
   volatile int* abortp = &abort_flag;
 
   if (warp == 0) {
     if (elect_one_sync()) {
       bool ok = true;
-      mbar_expect_tx(smem_u32(&kv_full), 2 * Cfg::kBig);
+      mbar_expect_tx(smem_u32(&kv_full), 2 * Cfg::kTile);
 #pragma unroll
       for (int c = 0; c < DCH; ++c) {
-        tma_load_2d(k_s + c * CH128, &p.k128, smem_u32(&kv_full), kvh * D + c * 64, k_begin + k0);
-        tma_load_2d(v_s + c * CH128, &p.v128, smem_u32(&kv_full), kvh * D + c * 64, k_begin + k0);
+        tma_load_2d(k_s + c * CH, &p.k, smem_u32(&kv_full), kvh * D + c * 64, k_begin + k0);
+        tma_load_2d(v_s + c * CH, &p.v, smem_u32(&kv_full), kvh * D + c * 64, k_begin + k0);
       }
       int it = 0;
       for (; it < n_iter; ++it) {
@@ -1486,184 +1541,153 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dkdv_kernel(const
         ok = mbar_wait_backoff(smem_u32(&qdo_empty[stage]), ((it / ST) & 1u) ^ 1u, abortp, p.status, ST_TIMEOUT_SMEM_EMPTY);
         if (!ok) break;
         const uint32_t fb = smem_u32(&qdo_full[stage]);
-        const uint32_t dst = qdo_s + stage * 2 * Cfg::kSmall;
-        mbar_expect_tx(fb, 2 * Cfg::kSmall);
+        const uint32_t dst = qdo_s + stage * 2 * Cfg::kTile;
+        mbar_expect_tx(fb, 2 * Cfg::kTile + Cfg::kStat);
 #pragma unroll
         for (int c = 0; c < DCH; ++c) {
-          tma_load_2d(dst + c * CH64, &p.q64, fb, h * D + c * 64, q_begin + i * 64);
-          tma_load_2d(dst + Cfg::kSmall + c * CH64, &p.do64, fb, h * D + c * 64, q_begin + i * 64);
+          tma_load_2d(dst + c * CH, &p.q, fb, h * D + c * 64, q_begin + i * 128);
+          tma_load_2d(dst + Cfg::kTile + c * CH, &p.dout, fb, h * D + c * 64, q_begin + i * 128);
         }
+        bulk_load(smem_base + stat_off + stage * Cfg::kStat, p.stat + ((long long)h * p.stat_tiles + (q_begin >> 7) + b + i) * 256, Cfg::kStat, fb);
       }
       if (!ok) {
-        for (int j = max(0, it - ST); j < it; ++j) {
+        auto drain = [&](uint64_t* bar, uint32_t parity) {
           const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(smem_u32(&qdo_full[j % ST]), (j / ST) & 1u))
+          while (!mbar_try_wait(smem_u32(bar), parity))
             if (globaltimer_ns() - t0 > 50000000ull) break;
-        }
+        };
+        drain(&kv_full, 0);
+        for (int j = max(0, it - ST); j < it; ++j) drain(&qdo_full[j % ST], (j / ST) & 1u);
       }
     }
   } else if (warp == 1) {
     if (elect_one_sync()) {
-      constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, 0, 0);
+      constexpr uint32_t idesc_st = make_idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, 0, 1);
-      bool ok = mbar_wait_backoff(smem_u32(&kv_full), 0, abortp, p.status, ST_TIMEOUT_SMEM_FULL);
-      auto issue_st = [&](int it) -> bool {
-        const int stage = it % ST;
-        if (!mbar_wait_backoff(smem_u32(&qdo_full[stage]), (it / ST) & 1u, abortp, p.status, ST_TIMEOUT_SMEM_FULL)) return false;
-        if (!mbar_wait_backoff(smem_u32(&st_empty[it & 1]), ((it >> 1) & 1u) ^ 1u, abortp, p.status, ST_TIMEOUT_TMEM_EMPTY)) return false;
-        tc_fence_after();
-        const uint32_t q_s = qdo_s + stage * 2 * Cfg::kSmall, do_s = q_s + Cfg::kSmall;
+      auto wait = [&](uint64_t* bar, uint32_t parity, int code) { return mbar_wait_backoff(smem_u32(bar), parity, abortp, p.status, code); };
+      bool ok = wait(&kv_full, 0, ST_TIMEOUT_SMEM_FULL);
+      // [128 keys x 128 queries] of K Q^T (which 0) or V dO^T (which 1)
+      auto issue_scores = [&](int it, int which) {
+        const uint32_t a_s = which ? v_s : k_s, b_s = qdo_s + (it % ST) * 2 * Cfg::kTile + which * Cfg::kTile;
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t a = make_smem_desc_sw128(k_s + (k >> 2) * CH128 + (k & 3) * 32, 16, 1024);
-          const uint64_t bq = make_smem_desc_sw128(q_s + (k >> 2) * CH64 + (k & 3) * 32, 16, 1024);
-          umma_bf16(tmem_base + (it & 1) * 64, a, bq, idesc_st, k > 0 ? 1u : 0u);
-        }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t a = make_smem_desc_sw128(v_s + (k >> 2) * CH128 + (k & 3) * 32, 16, 1024);
-          const uint64_t bd = make_smem_desc_sw128(do_s + (k >> 2) * CH64 + (k & 3) * 32, 16, 1024);
-          umma_bf16(tmem_base + 128 + (it & 1) * 64, a, bd, idesc_st, k > 0 ? 1u : 0u);
-        }
-        umma_commit(smem_u32(&st_full[it & 1]));
-        return true;
+        for (int k = 0; k < D / 16; ++k)
+          umma_bf16(tmem_base + which * TM_DP, make_smem_desc_sw128(a_s + (k >> 2) * CH + (k & 3) * 32, 16, 1024),
+                    make_smem_desc_sw128(b_s + (k >> 2) * CH + (k & 3) * 32, 16, 1024), idesc_st, k > 0 ? 1u : 0u);
+        umma_commit(smem_u32(which ? &dp_full : &s_full));
       };
-      if (ok && n_iter > 0) ok = issue_st(0);
+      // dV += P^T dO (which 0), dK += dS^T Q (which 1)
+      auto issue_grad = [&](int it, int which) {
+        const uint32_t b_s = qdo_s + (it % ST) * 2 * Cfg::kTile + (which ? 0 : Cfg::kTile);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          umma_bf16_ts(tmem_base + (which ? TM_DK : TM_DV), tmem_base + which * TM_DP + packed_column(k), make_smem_desc_sw128(b_s + k * 2048, CH, 1024),
+                       idesc_acc, (it > 0 || k > 0) ? 1u : 0u);
+      };
+      if (ok && n_iter > 0) {
+        ok = wait(&qdo_full[0], 0, ST_TIMEOUT_SMEM_FULL);
+        if (ok) {
+          tc_fence_after();
+          issue_scores(0, 0);
+          issue_scores(0, 1);
+        }
+      }
       for (int it = 0; it < n_iter && ok; ++it) {
-        if (it + 1 < n_iter) { ok = issue_st(it + 1); if (!ok) break; }
-        ok = mbar_wait_backoff(smem_u32(&pds_full[it & 1]), (it >> 1) & 1u, abortp, p.status, ST_TIMEOUT_TMEM_FULL);
+        const bool more = it + 1 < n_iter;
+        ok = wait(&p_full, it & 1u, ST_TIMEOUT_TMEM_FULL);
         if (!ok) break;
         tc_fence_after();
-        const int stage = it % ST;
-        const uint32_t q_s = qdo_s + stage * 2 * Cfg::kSmall, do_s = q_s + Cfg::kSmall;
-        const uint32_t pt_s = pds_s + (it & 1) * 2 * Cfg::kPd, dst_s = pt_s + Cfg::kPd;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {   // 64 queries = 4 k-steps
-          const uint64_t a = make_smem_desc_sw128(pt_s + k * 32, 16, 1024);
-          const uint64_t bd = make_smem_desc_sw128(do_s + k * 2048, CH64, 1024);
-          umma_bf16(tm_dv, a, bd, idesc_acc, (it > 0 || k > 0) ? 1u : 0u);
+        issue_grad(it, 0);
+        if (more) {
+          ok = wait(&qdo_full[(it + 1) % ST], ((it + 1) / ST) & 1u, ST_TIMEOUT_SMEM_FULL);
+          if (!ok) break;
+          tc_fence_after();
+          issue_scores(it + 1, 0);
         }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint64_t a = make_smem_desc_sw128(dst_s + k * 32, 16, 1024);
-          const uint64_t bq = make_smem_desc_sw128(q_s + k * 2048, CH64, 1024);
-          umma_bf16(tm_dk, a, bq, idesc_acc, (it > 0 || k > 0) ? 1u : 0u);
-        }
-        umma_commit(smem_u32(&qdo_empty[stage]));
-        umma_commit(smem_u32(&pds_empty[it & 1]));
+        ok = wait(&ds_full, it & 1u, ST_TIMEOUT_TMEM_FULL);
+        if (!ok) break;
+        tc_fence_after();
+        issue_grad(it, 1);
+        umma_commit(smem_u32(&qdo_empty[it % ST]));
+        if (more) issue_scores(it + 1, 1);
       }
       if (ok) umma_commit(smem_u32(&acc_done));
     }
-  } else {
+  } else if (warp >= 4) {
     const int qd = warp & 3;
     const int r = qd * 32 + lane;                  // key row of the tile
     const int kj = k0 + r;
     const uint32_t lane_addr = (uint32_t)(qd * 32) << 16;
-    const int half = (warp - 2) >> 2;              // which 32 of the 64 query columns
-    const int tid = threadIdx.x - 64;              // 0..255
+    const int wg = (warp >> 2) - 1;                // which 32 of the 128 query columns
+    const uint32_t tm_s = tmem_base + wg * 32 + lane_addr, tm_p = tm_s + TM_DP;
+    const uint64_t scale_l2 = pair(p.scale_log2, p.scale_log2), scale2 = pair(p.scale, p.scale);
+    // this key is seen from the query positions q_lo .. q_hi
+    const int q_lo = kj >= kv_len ? 1 << 30 : p.causal ? kj : -(1 << 30), q_hi = p.window > 0 ? kj + min(p.window, 1 << 29) - 1 : 1 << 30;
     bool ok = true;
-    // Row statistics of an iteration's 64 queries (thread t < 64 -> lse2, 64 <= t < 128 -> delta) are fetched one
-    // iteration ahead: the loads are issued at the top of iteration it for it + 1 and land in shared memory at its
-    // end, so their latency and the 256-thread barrier that publishes them are off the critical path.
-    auto load_stat = [&](int it2) -> float {
-      const int h2 = kvh * G + g_base + it2 / n_qt, qi = (i_begin + it2 % n_qt) * 64 + (tid & 63);
-      const int which = tid >> 6;
-      float val = which == 0 ? INFINITY : 0.f;      // lse2 = +inf makes P exactly 0 for rows past the end
-      if (qi < q_len) val = (which == 0 ? p.lse2 : p.delta)[(long long)h2 * p.Tq + q_begin + qi];
-      return val;
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+      return __all_sync(0xffffffffu, mbar_wait_backoff(smem_u32(bar), parity, abortp, p.status, ST_TIMEOUT_TMEM_FULL));
     };
-    if (n_iter > 0) {
-      if (tid < 128) stat[0][tid >> 6][tid & 63] = load_stat(0);
-      mbar_arrive(smem_u32(&stat_bar));
-      ok = mbar_wait_backoff(smem_u32(&stat_bar), 0u, abortp, p.status, ST_TIMEOUT_TMEM_FULL);
-      ok = __all_sync(0xffffffffu, ok);
-    }
-    for (int it = 0; it < n_iter && ok; ++it) {
-      const int qi0 = (i_begin + it % n_qt) * 64;
-      const bool have_next = it + 1 < n_iter;
-      float stat_next = 0.f;
-      if (have_next && tid < 128) stat_next = load_stat(it + 1);
-      ok = mbar_wait_backoff(smem_u32(&st_full[it & 1]), (it >> 1) & 1u, abortp, p.status, ST_TIMEOUT_TMEM_FULL);
-      ok = __all_sync(0xffffffffu, ok);
+    for (int it = 0; it < n_iter; ++it) {
+      const int qi0 = (i_begin + it % n_qt) * 128, stage = it % ST;
+      const uint64_t* stat = reinterpret_cast<const uint64_t*>(smem_al + stat_off + stage * Cfg::kStat) + wg * 16;
+      ok = wait(&qdo_full[stage], (it / ST) & 1u) && wait(&s_full, it & 1u);
       if (!ok) break;
       tc_fence_after();
-      uint32_t sv[32], dv[32];
-      tmem_ld_32x32(tmem_base + (it & 1) * 64 + half * 32 + lane_addr, sv);
-      tmem_ld_32x32(tmem_base + 128 + (it & 1) * 64 + half * 32 + lane_addr, dv);
+      uint32_t prob[32], packed[16];
+      tmem_ld_32x32(tm_s, prob);
       tmem_ld_wait();
+      const bool need_mask = (k0 + 127 >= kv_len) || (p.causal && k0 + 127 > off + qi0) ||
+                             (p.window > 0 && k0 <= off + qi0 + 127 - p.window);
+      const uint32_t dead = need_mask ? outside_mask(off + qi0 + wg * 32, q_lo, q_hi) : 0u;
+      bwd_probabilities(prob, scale_l2, [&](int c) { return stat[c >> 1]; }, dead, packed);
+      tmem_st_32x16(tm_s, packed);
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&st_empty[it & 1]));
-      const bool need_mask = (k0 + 127 >= kv_len) || (p.causal && k0 + 127 > off + qi0) ||
-                             (p.window > 0 && k0 <= off + qi0 + 63 - p.window);
-      const float* l2 = stat[it & 1][0] + half * 32;
-      const float* dl = stat[it & 1][1] + half * 32;
-      float pr[32], ds[32];
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        float pv = fast_exp2(fmaf(__uint_as_float(sv[c]), p.scale_log2, -l2[c]));
-        if (need_mask) {
-          const int qpos = off + qi0 + half * 32 + c;
-          if (kj >= kv_len || (p.causal && kj > qpos) || (p.window > 0 && kj <= qpos - p.window)) pv = 0.f;
-        }
-        pr[c] = pv;
-        ds[c] = pv * (__uint_as_float(dv[c]) - dl[c]) * p.scale;
-      }
-      ok = mbar_wait_backoff(smem_u32(&pds_empty[it & 1]), ((it >> 1) & 1u) ^ 1u, abortp, p.status, ST_TIMEOUT_SMEM_EMPTY);
-      ok = __all_sync(0xffffffffu, ok);
+      if (lane == 0) mbar_arrive(smem_u32(&p_full));
+      ok = wait(&dp_full, it & 1u);
       if (!ok) break;
-      uint8_t* pt_row = smem_al + pds_off + (it & 1) * 2 * Cfg::kPd + r * 128;
-      store_row32_sw128(pt_row, r, half, pr);
-      store_row32_sw128(pt_row + Cfg::kPd, r, half, ds);
-      fence_proxy_async_smem();
+      tc_fence_after();
+      uint32_t dv[32];
+      tmem_ld_32x32(tm_p, dv);
+      tmem_ld_wait();
+      bwd_scores(prob, dv, scale2, [&](int c) { return stat[64 + (c >> 1)]; }, packed);
+      tmem_st_32x16(tm_p, packed);
+      tmem_st_wait();
+      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&pds_full[it & 1]));
-      if (have_next) {
-        // every thread has read stat[(it + 1) & 1] for the last time in iteration it - 1, before that iteration's barrier
-        if (tid < 128) stat[(it + 1) & 1][tid >> 6][tid & 63] = stat_next;
-        mbar_arrive(smem_u32(&stat_bar));
-        ok = mbar_wait_backoff(smem_u32(&stat_bar), (uint32_t)((it + 1) & 1), abortp, p.status, ST_TIMEOUT_TMEM_FULL);
-        ok = __all_sync(0xffffffffu, ok);
-      }
+      if (lane == 0) mbar_arrive(smem_u32(&ds_full));
     }
-    if (ok && n_iter > 0) {
-      ok = mbar_wait_backoff(smem_u32(&acc_done), 0, abortp, p.status, ST_TIMEOUT_TMEM_FULL);
-      ok = __all_sync(0xffffffffu, ok);
-    }
+    if (ok && n_iter > 0) ok = wait(&acc_done, 0);
     if (ok) {
       tc_fence_after();
       const bool row_ok = kj < kv_len;
-      __nv_bfloat16* dv_row = p.dv + ((long long)(k_begin + kj) * p.Hkv + kvh) * D;
-      __nv_bfloat16* dk_row = p.dk + ((long long)(k_begin + kj) * p.Hkv + kvh) * D;
+      const int which = wg >> 1, half = wg & 1;    // warpgroups 0, 1: dV; 2, 3: dK; each half of the columns
+      __nv_bfloat16* row = (which == 0 ? p.dv : p.dk) + ((long long)(k_begin + kj) * p.Hkv + kvh) * D;
 #pragma unroll 1
-      for (int which = 0; which < 2; ++which) {
-#pragma unroll 1
-        for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {   // each warpgroup stores half the columns
-          uint32_t v[32];
-          if (n_iter > 0) {
-            tmem_ld_32x32((which == 0 ? tm_dv : tm_dk) + lane_addr + c * 32, v);
-            tmem_ld_wait();
-          } else {
+      for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
+        uint32_t v[32];
+        if (n_iter > 0) {
+          tmem_ld_32x32(tmem_base + (which == 0 ? TM_DV : TM_DK) + lane_addr + c * 32, v);
+          tmem_ld_wait();
+        } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0u;
-          }
-          if (row_ok && head_split) {
-            float* dst = p.dkv_part + (((long long)(which * G + g_base) * p.Tk + k_begin + kj) * p.Hkv + kvh) * D + c * 32;
+          for (int i = 0; i < 32; ++i) v[i] = 0u;
+        }
+        if (row_ok && head_split) {
+          float* dst = p.dkv_part + (((long long)(which * G + g_base) * p.Tk + k_begin + kj) * p.Hkv + kvh) * D + c * 32;
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-              *reinterpret_cast<float4*>(dst + u * 4) = make_float4(__uint_as_float(v[u * 4]), __uint_as_float(v[u * 4 + 1]),
-                                                                    __uint_as_float(v[u * 4 + 2]), __uint_as_float(v[u * 4 + 3]));
-          } else if (row_ok) {
-            __nv_bfloat16* dst = (which == 0 ? dv_row : dk_row) + c * 32;
+          for (int u = 0; u < 8; ++u)
+            *reinterpret_cast<float4*>(dst + u * 4) = make_float4(__uint_as_float(v[u * 4]), __uint_as_float(v[u * 4 + 1]),
+                                                                  __uint_as_float(v[u * 4 + 2]), __uint_as_float(v[u * 4 + 3]));
+        } else if (row_ok) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              uint4 w;
-              w.x = pack_bf16x2(__uint_as_float(v[u * 8 + 0]), __uint_as_float(v[u * 8 + 1]));
-              w.y = pack_bf16x2(__uint_as_float(v[u * 8 + 2]), __uint_as_float(v[u * 8 + 3]));
-              w.z = pack_bf16x2(__uint_as_float(v[u * 8 + 4]), __uint_as_float(v[u * 8 + 5]));
-              w.w = pack_bf16x2(__uint_as_float(v[u * 8 + 6]), __uint_as_float(v[u * 8 + 7]));
-              *reinterpret_cast<uint4*>(dst + u * 8) = w;
-            }
+          for (int u = 0; u < 4; ++u) {
+            uint4 w;
+            w.x = pack_bf16x2(__uint_as_float(v[u * 8 + 0]), __uint_as_float(v[u * 8 + 1]));
+            w.y = pack_bf16x2(__uint_as_float(v[u * 8 + 2]), __uint_as_float(v[u * 8 + 3]));
+            w.z = pack_bf16x2(__uint_as_float(v[u * 8 + 4]), __uint_as_float(v[u * 8 + 5]));
+            w.w = pack_bf16x2(__uint_as_float(v[u * 8 + 6]), __uint_as_float(v[u * 8 + 7]));
+            *reinterpret_cast<uint4*>(row + c * 32 + u * 8) = w;
           }
         }
       }
@@ -1682,10 +1706,11 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dq_kernel(const _
   using Cfg = FlashBwdCfg<D>;
   constexpr int DCH = D / 64;
   constexpr int ST = Cfg::kKvStages;
-  constexpr int CH128 = 128 * 128, CH64 = 64 * 128;
+  constexpr int CH = 128 * 128;
+  constexpr uint32_t TM_DP = 128, TM_DQ = 256, TM_Q = 384, TM_DO = 448;      // Q, dO: packed bf16, D / 2 columns
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t qdo_full, kv_full[ST], kv_empty[ST];
-  __shared__ __align__(8) uint64_t s_full[2], s_empty[2], ds_full[2], ds_empty[2], acc_done;
+  __shared__ __align__(8) uint64_t qdo_full, qdo_ready, kv_full[ST], kv_empty[ST];
+  __shared__ __align__(8) uint64_t s_full, s_read, dp_full, ds_full, acc_done;
   __shared__ uint32_t tmem_base_smem;
   __shared__ int abort_flag;
 
@@ -1700,26 +1725,23 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dq_kernel(const _
   const int kvh = h / (p.Hq / p.Hkv);
   const int hi = p.causal ? min(kv_len, off + q0 + 128) : kv_len;
   const int lo = p.window > 0 ? max(0, off + q0 - p.window + 1) : 0;
-  const int t_begin = lo / 64;
-  const int n_iter = max((hi + 63) / 64 - t_begin, 0);
+  const int t_begin = lo / 128;
+  const int n_iter = max((hi + 127) / 128 - t_begin, 0);
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t q_s = smem_base, do_s = q_s + Cfg::kBig;
-  const uint32_t kv_s = do_s + Cfg::kBig;                        // stage: K tile then V tile (64 rows each)
-  const uint32_t ds_off = 2 * Cfg::kBig + ST * 2 * Cfg::kSmall;
-  const uint32_t ds_s = smem_base + ds_off;
+  const uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
+  const uint32_t q_s = smem_base, do_s = q_s + Cfg::kTile;
+  const uint32_t kv_s = do_s + Cfg::kTile;                       // stage: K tile then V tile
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
     mbar_init(smem_u32(&qdo_full), 1);
+    mbar_init(smem_u32(&qdo_ready), 8 * DCH);
     for (int i = 0; i < ST; ++i) { mbar_init(smem_u32(&kv_full[i]), 1); mbar_init(smem_u32(&kv_empty[i]), 1); }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&s_full[i]), 1);
-      mbar_init(smem_u32(&s_empty[i]), 8);
-      mbar_init(smem_u32(&ds_full[i]), 8);
-      mbar_init(smem_u32(&ds_empty[i]), 1);
-    }
+    mbar_init(smem_u32(&s_full), 1);
+    mbar_init(smem_u32(&dp_full), 1);
+    mbar_init(smem_u32(&s_read), FA_BWD_WARPS);
+    mbar_init(smem_u32(&ds_full), FA_BWD_WARPS);
     mbar_init(smem_u32(&acc_done), 1);
     fence_mbar_init();
   }
@@ -1731,17 +1753,16 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dq_kernel(const _
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem;
-  const uint32_t tm_dq = tmem_base + 256;
   volatile int* abortp = &abort_flag;
 
   if (warp == 0) {
     if (elect_one_sync()) {
       bool ok = true;
-      mbar_expect_tx(smem_u32(&qdo_full), 2 * Cfg::kBig);
+      mbar_expect_tx(smem_u32(&qdo_full), 2 * Cfg::kTile);
 #pragma unroll
       for (int c = 0; c < DCH; ++c) {
-        tma_load_2d(q_s + c * CH128, &p.q128, smem_u32(&qdo_full), h * D + c * 64, q_begin + q0);
-        tma_load_2d(do_s + c * CH128, &p.do128, smem_u32(&qdo_full), h * D + c * 64, q_begin + q0);
+        tma_load_2d(q_s + c * CH, &p.q, smem_u32(&qdo_full), h * D + c * 64, q_begin + q0);
+        tma_load_2d(do_s + c * CH, &p.dout, smem_u32(&qdo_full), h * D + c * 64, q_begin + q0);
       }
       int it = 0;
       for (; it < n_iter; ++it) {
@@ -1749,141 +1770,157 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dq_kernel(const _
         ok = mbar_wait_backoff(smem_u32(&kv_empty[stage]), ((it / ST) & 1u) ^ 1u, abortp, p.status, ST_TIMEOUT_SMEM_EMPTY);
         if (!ok) break;
         const uint32_t fb = smem_u32(&kv_full[stage]);
-        const uint32_t dst = kv_s + stage * 2 * Cfg::kSmall;
-        const int y = k_begin + (t_begin + it) * 64;
-        mbar_expect_tx(fb, 2 * Cfg::kSmall);
+        const uint32_t dst = kv_s + stage * 2 * Cfg::kTile;
+        const int y = k_begin + (t_begin + it) * 128;
+        mbar_expect_tx(fb, 2 * Cfg::kTile);
 #pragma unroll
         for (int c = 0; c < DCH; ++c) {
-          tma_load_2d(dst + c * CH64, &p.k64, fb, kvh * D + c * 64, y);
-          tma_load_2d(dst + Cfg::kSmall + c * CH64, &p.v64, fb, kvh * D + c * 64, y);
+          tma_load_2d(dst + c * CH, &p.k, fb, kvh * D + c * 64, y);
+          tma_load_2d(dst + Cfg::kTile + c * CH, &p.v, fb, kvh * D + c * 64, y);
         }
       }
       if (!ok) {
-        for (int j = max(0, it - ST); j < it; ++j) {
+        auto drain = [&](uint64_t* bar, uint32_t parity) {
           const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(smem_u32(&kv_full[j % ST]), (j / ST) & 1u))
+          while (!mbar_try_wait(smem_u32(bar), parity))
             if (globaltimer_ns() - t0 > 50000000ull) break;
-        }
+        };
+        drain(&qdo_full, 0);
+        for (int j = max(0, it - ST); j < it; ++j) drain(&kv_full[j % ST], (j / ST) & 1u);
       }
     }
   } else if (warp == 1) {
     if (elect_one_sync()) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);
+      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t idesc_acc = make_idesc_bf16(128, D, 0, 1);
-      bool ok = mbar_wait_backoff(smem_u32(&qdo_full), 0, abortp, p.status, ST_TIMEOUT_SMEM_FULL);
-      auto issue_s = [&](int it) -> bool {
-        const int stage = it % ST;
-        if (!mbar_wait_backoff(smem_u32(&kv_full[stage]), (it / ST) & 1u, abortp, p.status, ST_TIMEOUT_SMEM_FULL)) return false;
-        if (!mbar_wait_backoff(smem_u32(&s_empty[it & 1]), ((it >> 1) & 1u) ^ 1u, abortp, p.status, ST_TIMEOUT_TMEM_EMPTY)) return false;
-        tc_fence_after();
-        const uint32_t k_s = kv_s + stage * 2 * Cfg::kSmall, v_s = k_s + Cfg::kSmall;
+      auto wait = [&](uint64_t* bar, uint32_t parity, int code) { return mbar_wait_backoff(smem_u32(bar), parity, abortp, p.status, code); };
+      bool ok = wait(&qdo_ready, 0, ST_TIMEOUT_SMEM_FULL);
+      // Q K^T (which 0) or dO V^T (which 1)
+      auto issue_scores = [&](int it, int which) {
+        const uint32_t b_s = kv_s + (it % ST) * 2 * Cfg::kTile + which * Cfg::kTile;
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t a = make_smem_desc_sw128(q_s + (k >> 2) * CH128 + (k & 3) * 32, 16, 1024);
-          const uint64_t bk = make_smem_desc_sw128(k_s + (k >> 2) * CH64 + (k & 3) * 32, 16, 1024);
-          umma_bf16(tmem_base + (it & 1) * 64, a, bk, idesc_s, k > 0 ? 1u : 0u);
-        }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t a = make_smem_desc_sw128(do_s + (k >> 2) * CH128 + (k & 3) * 32, 16, 1024);
-          const uint64_t bv = make_smem_desc_sw128(v_s + (k >> 2) * CH64 + (k & 3) * 32, 16, 1024);
-          umma_bf16(tmem_base + 128 + (it & 1) * 64, a, bv, idesc_s, k > 0 ? 1u : 0u);
-        }
-        umma_commit(smem_u32(&s_full[it & 1]));
-        return true;
+        for (int k = 0; k < D / 16; ++k)
+          umma_bf16_ts(tmem_base + which * TM_DP, tmem_base + (which ? TM_DO : TM_Q) + k * 8,
+                       make_smem_desc_sw128(b_s + (k >> 2) * CH + (k & 3) * 32, 16, 1024), idesc_s, k > 0 ? 1u : 0u);
+        umma_commit(smem_u32(which ? &dp_full : &s_full));
       };
-      if (ok && n_iter > 0) ok = issue_s(0);
+      if (ok && n_iter > 0) {
+        ok = wait(&kv_full[0], 0, ST_TIMEOUT_SMEM_FULL);
+        if (ok) {
+          tc_fence_after();
+          issue_scores(0, 0);
+          issue_scores(0, 1);
+        }
+      }
       for (int it = 0; it < n_iter && ok; ++it) {
-        if (it + 1 < n_iter) { ok = issue_s(it + 1); if (!ok) break; }
-        ok = mbar_wait_backoff(smem_u32(&ds_full[it & 1]), (it >> 1) & 1u, abortp, p.status, ST_TIMEOUT_TMEM_FULL);
+        const bool more = it + 1 < n_iter;
+        if (more) {
+          ok = wait(&kv_full[(it + 1) % ST], ((it + 1) / ST) & 1u, ST_TIMEOUT_SMEM_FULL) && wait(&s_read, it & 1u, ST_TIMEOUT_TMEM_EMPTY);
+          if (!ok) break;
+          tc_fence_after();
+          issue_scores(it + 1, 0);
+        }
+        ok = wait(&ds_full, it & 1u, ST_TIMEOUT_TMEM_FULL);
         if (!ok) break;
         tc_fence_after();
-        const int stage = it % ST;
-        const uint32_t k_s = kv_s + stage * 2 * Cfg::kSmall;
-        const uint32_t dsb = ds_s + (it & 1) * Cfg::kPd;
+        const uint32_t k_s = kv_s + (it % ST) * 2 * Cfg::kTile;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {   // 64 keys = 4 k-steps
-          const uint64_t a = make_smem_desc_sw128(dsb + k * 32, 16, 1024);
-          const uint64_t bk = make_smem_desc_sw128(k_s + k * 2048, CH64, 1024);
-          umma_bf16(tm_dq, a, bk, idesc_acc, (it > 0 || k > 0) ? 1u : 0u);
-        }
-        umma_commit(smem_u32(&kv_empty[stage]));
-        umma_commit(smem_u32(&ds_empty[it & 1]));
+        for (int k = 0; k < 8; ++k)   // 128 keys = 8 k-steps
+          umma_bf16_ts(tmem_base + TM_DQ, tmem_base + TM_DP + packed_column(k), make_smem_desc_sw128(k_s + k * 2048, CH, 1024), idesc_acc,
+                       (it > 0 || k > 0) ? 1u : 0u);
+        umma_commit(smem_u32(&kv_empty[it % ST]));
+        if (more) issue_scores(it + 1, 1);
       }
       if (ok) umma_commit(smem_u32(&acc_done));
     }
-  } else {
+  } else if (warp >= 4) {
     const int qd = warp & 3;
     const int r = qd * 32 + lane;                  // query row of the tile
-    const int half = (warp - 2) >> 2;              // which 32 of the 64 key columns
+    const int wg = (warp >> 2) - 1;                // which 32 of the 128 key columns
     const int qi = q0 + r, qpos = off + qi;
     const uint32_t lane_addr = (uint32_t)(qd * 32) << 16;
-    float l2 = INFINITY, dl = 0.f;                 // a row past the end gets P = 0 everywhere
+    const uint32_t tm_s = tmem_base + wg * 32 + lane_addr, tm_p = tm_s + TM_DP;
+    const uint64_t scale_l2 = pair(p.scale_log2, p.scale_log2), scale2 = pair(p.scale, p.scale);
+    float nl = -INFINITY, nd = 0.f;                // a row past the end gets P = 0 everywhere
     if (qi < q_len) {
-      l2 = p.lse2[(long long)h * p.Tq + q_begin + qi];
-      dl = p.delta[(long long)h * p.Tq + q_begin + qi];
+      const float* st = p.stat + ((long long)h * p.stat_tiles + (q_begin >> 7) + b + q_tile) * 256 + r;
+      nl = st[0];
+      nd = st[128];
     }
+    const uint64_t nl2 = pair(nl, nl), nd2 = pair(nd, nd);
+    // keys k_lo .. k_hi are seen from this query
+    const int k_lo = p.window > 0 ? qpos - p.window + 1 : 0, k_hi = p.causal ? min(qpos, kv_len - 1) : kv_len - 1;
     bool ok = true;
-    for (int it = 0; it < n_iter; ++it) {
-      const int k0 = (t_begin + it) * 64;
-      ok = mbar_wait_backoff(smem_u32(&s_full[it & 1]), (it >> 1) & 1u, abortp, p.status, ST_TIMEOUT_TMEM_FULL);
-      ok = __all_sync(0xffffffffu, ok);
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+      return __all_sync(0xffffffffu, mbar_wait_backoff(smem_u32(bar), parity, abortp, p.status, ST_TIMEOUT_TMEM_FULL));
+    };
+    if (wg < 2 * DCH) {      // Q and dO to tensor memory, one 64-column chunk a warpgroup
+      ok = wait(&qdo_full, 0);
+      if (ok) {
+        const int which = wg / DCH, c = wg % DCH;
+        const uint8_t* src = smem_al + which * Cfg::kTile + c * CH + r * 128;
+        uint32_t v[32];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) *reinterpret_cast<uint4*>(&v[u * 4]) = *reinterpret_cast<const uint4*>(src + ((u ^ (r & 7)) << 4));
+        tmem_st_32x32(tmem_base + (which ? TM_DO : TM_Q) + c * 32 + lane_addr, v);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&qdo_ready));
+      }
+    }
+    for (int it = 0; it < n_iter && ok; ++it) {
+      const int k0 = (t_begin + it) * 128;
+      ok = wait(&s_full, it & 1u);
       if (!ok) break;
       tc_fence_after();
-      uint32_t sv[32], dv[32];
-      tmem_ld_32x32(tmem_base + (it & 1) * 64 + half * 32 + lane_addr, sv);
-      tmem_ld_32x32(tmem_base + 128 + (it & 1) * 64 + half * 32 + lane_addr, dv);
+      uint32_t prob[32], packed[16];
+      tmem_ld_32x32(tm_s, prob);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&s_empty[it & 1]));
-      const bool need_mask = (k0 + 63 >= kv_len) || (p.causal && k0 + 63 > off + q0) ||
+      if (lane == 0) mbar_arrive(smem_u32(&s_read));
+      const bool need_mask = (k0 + 127 >= kv_len) || (p.causal && k0 + 127 > off + q0) ||
                              (p.window > 0 && k0 <= off + q0 + 127 - p.window);
-      float ds[32];
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        float pv = fast_exp2(fmaf(__uint_as_float(sv[c]), p.scale_log2, -l2));
-        if (need_mask) {
-          const int kj = k0 + half * 32 + c;
-          if (kj >= kv_len || (p.causal && kj > qpos) || (p.window > 0 && kj <= qpos - p.window)) pv = 0.f;
-        }
-        ds[c] = pv * (__uint_as_float(dv[c]) - dl) * p.scale;
-      }
-      ok = mbar_wait_backoff(smem_u32(&ds_empty[it & 1]), ((it >> 1) & 1u) ^ 1u, abortp, p.status, ST_TIMEOUT_SMEM_EMPTY);
-      ok = __all_sync(0xffffffffu, ok);
+      const uint32_t dead = need_mask ? outside_mask(k0 + wg * 32, k_lo, k_hi) : 0u;
+      bwd_probabilities(prob, scale_l2, [&](int) { return nl2; }, dead, packed);
+      ok = wait(&dp_full, it & 1u);
       if (!ok) break;
-      store_row32_sw128(smem_al + ds_off + (it & 1) * Cfg::kPd + r * 128, r, half, ds);
-      fence_proxy_async_smem();
+      tc_fence_after();
+      uint32_t dv[32];
+      tmem_ld_32x32(tm_p, dv);
+      tmem_ld_wait();
+      bwd_scores(prob, dv, scale2, [&](int) { return nd2; }, packed);
+      tmem_st_32x16(tm_p, packed);
+      tmem_st_wait();
+      tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&ds_full[it & 1]));
+      if (lane == 0) mbar_arrive(smem_u32(&ds_full));
     }
-    if (ok && n_iter > 0) {
-      ok = mbar_wait_backoff(smem_u32(&acc_done), 0, abortp, p.status, ST_TIMEOUT_TMEM_FULL);
-      ok = __all_sync(0xffffffffu, ok);
-    }
+    if (ok && n_iter > 0) ok = wait(&acc_done, 0);
     if (ok) {
       tc_fence_after();
       const bool row_ok = qi < q_len;
       __nv_bfloat16* dq_row = p.dq + ((long long)(q_begin + qi) * p.Hq + h) * D;
 #pragma unroll 1
-      for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {   // each warpgroup stores half the columns
-        uint32_t v[32];
+      for (int c = wg * (D / 64); c < (wg + 1) * (D / 64); ++c) {       // 16 columns at a time, a quarter of them a warpgroup
+        uint32_t v[16];
         if (n_iter > 0) {
-          tmem_ld_32x32(tm_dq + lane_addr + c * 32, v);
+          tmem_ld_32x16(tmem_base + TM_DQ + lane_addr + c * 16, v);
           tmem_ld_wait();
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = 0u;
+          for (int i = 0; i < 16; ++i) v[i] = 0u;
         }
         if (row_ok) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
+          for (int u = 0; u < 2; ++u) {
             uint4 w;
             w.x = pack_bf16x2(__uint_as_float(v[u * 8 + 0]), __uint_as_float(v[u * 8 + 1]));
             w.y = pack_bf16x2(__uint_as_float(v[u * 8 + 2]), __uint_as_float(v[u * 8 + 3]));
             w.z = pack_bf16x2(__uint_as_float(v[u * 8 + 4]), __uint_as_float(v[u * 8 + 5]));
             w.w = pack_bf16x2(__uint_as_float(v[u * 8 + 6]), __uint_as_float(v[u * 8 + 7]));
-            *reinterpret_cast<uint4*>(dq_row + c * 32 + u * 8) = w;
+            *reinterpret_cast<uint4*>(dq_row + c * 16 + u * 8) = w;
           }
         }
       }
@@ -2063,7 +2100,7 @@ int rb_flash_latent(const void* q, const void* k, const void* rot, const void* v
 }
 
 // Backward of rb_flash_fwd in dense mode. out, dout, dq are contiguous [Tq,Hq,D]; dk, dv contiguous
-// [Tk,Hkv,D]; workspace holds 2*Hq*Tq floats (delta, lse in log2 units). dkv_part (may be null): 2*(Hq/Hkv)*Tk*Hkv*D
+// [Tk,Hkv,D]; workspace (16-byte aligned) holds Hq * (Tq / 128 + B + 1) * 256 floats (row statistics by tiles of 128 queries). dkv_part (may be null): 2*(Hq/Hkv)*Tk*Hkv*D
 // floats; when given, dK/dV run with one CTA per (key tile, query head) and are reduced over each group afterwards
 // (few long sequences: the per-kv-head grid is too coarse to fill the SMs).
 int rb_flash_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
@@ -2075,14 +2112,13 @@ int rb_flash_bwd(const void* q, const void* k, const void* v, const void* out, c
   if ((D != 64 && D != 128) || Hq % Hkv != 0) return -1;
   FlashBwdParams p;
   const unsigned long long qc = (unsigned long long)Hq * D, kc = (unsigned long long)Hkv * D;
-  if (tma_map_2d_bf16(&p.q64, q, Tq, qc, ldq, 64) != 0 || tma_map_2d_bf16(&p.q128, q, Tq, qc, ldq, 128) != 0) return -20;
-  if (tma_map_2d_bf16(&p.do64, dout, Tq, qc, qc, 64) != 0 || tma_map_2d_bf16(&p.do128, dout, Tq, qc, qc, 128) != 0) return -21;
-  if (tma_map_2d_bf16(&p.k64, k, Tk, kc, ldk, 64) != 0 || tma_map_2d_bf16(&p.k128, k, Tk, kc, ldk, 128) != 0) return -22;
-  if (tma_map_2d_bf16(&p.v64, v, Tk, kc, ldv, 64) != 0 || tma_map_2d_bf16(&p.v128, v, Tk, kc, ldv, 128) != 0) return -23;
-  float* delta = workspace;
-  float* lse2 = workspace + (long long)Hq * Tq;
-  p.lse2 = lse2;
-  p.delta = delta;
+  if (tma_map_2d_bf16(&p.q, q, Tq, qc, ldq, 128) != 0) return -20;
+  if (tma_map_2d_bf16(&p.dout, dout, Tq, qc, qc, 128) != 0) return -21;
+  if (tma_map_2d_bf16(&p.k, k, Tk, kc, ldk, 128) != 0) return -22;
+  if (tma_map_2d_bf16(&p.v, v, Tk, kc, ldv, 128) != 0) return -23;
+  if (((unsigned long long)workspace & 15) != 0) return -1;
+  p.stat = workspace;
+  p.stat_tiles = Tq / 128 + B + 1;
   p.dkv_part = (Hq > Hkv) ? dkv_part : nullptr;
   p.dq = (__nv_bfloat16*)dq;
   p.dk = (__nv_bfloat16*)dk;
@@ -2094,9 +2130,11 @@ int rb_flash_bwd(const void* q, const void* k, const void* v, const void* out, c
   p.scale = scale;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.status = status;
-  const long long warps = (long long)Tq * Hq;
-  launch_kernel(flash_bwd_prep_kernel, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256), 0, stream,
-                (const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, lse, delta, lse2, Tq, Hq, D);
+  const dim3 prep_grid((max_seqlen_q + 127) / 128, B, Hq);
+  const auto prep = D == 64 ? flash_bwd_prep_kernel<64> : flash_bwd_prep_kernel<128>;
+  if (launch_kernel(prep, prep_grid, dim3(256), 0, stream, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, lse, workspace, cu_q, p.stat_tiles, Tq, Hq) !=
+      cudaSuccess)
+    return -11;
   dim3 grid_kv((max_seqlen_k + 127) / 128, p.dkv_part != nullptr ? Hq : Hkv, B), grid_q((max_seqlen_q + 127) / 128, Hq, B);
   int rc = D == 64 ? launch_flash_bwd<64>(p, grid_kv, grid_q, stream) : launch_flash_bwd<128>(p, grid_kv, grid_q, stream);
   if (rc != 0) return rc;

@@ -134,8 +134,8 @@ def flash_attn_varlen_backward(q, k, v, out, dout, lse, cu_q, cu_k, max_seqlen_q
     dq = torch.empty(Tq, Hq, D, dtype=torch.bfloat16, device=q.device)
     dk = torch.empty(Tk, Hkv, D, dtype=torch.bfloat16, device=q.device)
     dv = torch.empty(Tk, Hkv, D, dtype=torch.bfloat16, device=q.device)
-    ws = torch.empty(2 * Hq * Tq, dtype=torch.float32, device=q.device)
     B = cu_q.shape[0] - 1
+    ws = torch.empty(Hq * (Tq // 128 + B + 1) * 256, dtype=torch.float32, device=q.device)
     part = None
     if head_split_pays(B, max_seqlen_q, max_seqlen_k, Hq, Hkv):
         part = torch.empty(2 * (Hq // Hkv) * Tk * Hkv * D, dtype=torch.float32, device=q.device)

@@ -222,3 +222,44 @@ def test_flash_forward_tile_edges_many_items_a_block(D, H, Hkv, window, paged):
     assert ((out.float() - ref).abs() <= 2.0 ** -8 * size + 2.0 ** -8 * ref.abs() + 1e-6).all()
     assert ((lse - ref_lse).abs() <= 1e-4 * (1 + ref_lse.abs())).all()
     ops.check_status(torch.device("cuda"))
+
+
+@pytest.mark.parametrize("causal,window", [(True, 0), (True, 100), (True, 129), (False, 0)])
+@pytest.mark.parametrize("D,H,Hkv", [(64, 4, 2), (128, 2, 2)])
+def test_flash_backward_tile_edges(D, H, Hkv, causal, window):
+    """Sequences around the 128-row tiles, an empty one, and one with more keys than queries, against 64 bits."""
+    q_lens = [1, 127, 128, 129, 0, 255, 256, 257, 60, 383]
+    k_lens = [1, 127, 128, 129, 0, 255, 256, 257, 200, 383]
+    g = torch.Generator(device="cuda").manual_seed(D + window)
+    q, do = (torch.randn(sum(q_lens), H, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(sum(k_lens), Hkv, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    cu_q, cu_k = _cu(q_lens, "cuda"), _cu(k_lens, "cuda")
+    out, lse = flash.flash_attn_varlen(q, k, v, cu_q, cu_k, max(q_lens), causal=causal, window=window, return_lse=True)
+    got = flash.flash_attn_varlen_backward(q, k, v, out, do, lse, cu_q, cu_k, max(q_lens), max(k_lens), causal=causal, window=window)
+    u = 2.0 ** -8        # two roundings to bf16, each at most 2^-9 of the value
+    at_q = at_k = 0
+    for nq, nk in zip(q_lens, k_lens):
+        want = [torch.zeros(n, h, D, device="cuda", dtype=torch.float64) for n, h in ((nq, H), (nk, Hkv), (nk, Hkv))]
+        room = [torch.zeros_like(w) for w in want]
+        for h in range(H):
+            kv = h // (H // Hkv)
+            qh, oh, dh = (t[at_q:at_q + nq, h].double() for t in (q, out, do))
+            kh, vh = k[at_k:at_k + nk, kv].double(), v[at_k:at_k + nk, kv].double()
+            i, j = torch.arange(nq, device="cuda")[:, None] + nk - nq, torch.arange(nk, device="cuda")[None]
+            dead = (j > i) if causal else torch.zeros(nq, nk, dtype=torch.bool, device="cuda")
+            dead = dead | (j <= i - window) if window else dead
+            p = (qh @ kh.T * D ** -0.5).masked_fill(dead, -math.inf).softmax(-1)
+            exact_o = p @ vh
+            ds = p * (dh @ vh.T - (dh * exact_o).sum(-1, keepdim=True)) * D ** -0.5
+            # dS is rounded; its delta is taken from the rounded output
+            slack = u * ds.abs() + p * D ** -0.5 * (u * (dh.abs() * (p @ vh.abs())).sum(-1, keepdim=True) + 1e-5)
+            want[0][:, h] = ds @ kh
+            want[1][:, kv] += ds.T @ qh
+            want[2][:, kv] += p.T @ dh
+            room[0][:, h] = slack @ kh.abs()
+            room[1][:, kv] += slack.T @ qh.abs()
+            room[2][:, kv] += u * p.T @ dh.abs()
+        for x, w, m, (lo, n) in zip(got, want, room, ((at_q, nq), (at_k, nk), (at_k, nk))):
+            assert ((x[lo:lo + n].double() - w).abs() <= m + u * w.abs() + 1e-5).all()
+        at_q, at_k = at_q + nq, at_k + nk
+    ops.check_status(torch.device("cuda"))
