@@ -16,11 +16,17 @@
 //     "empty" mbarrier of the stage in both CTAs and, after the last k-block, to the "accumulator full" mbarrier
 //     of both CTAs;
 //   * each CTA's four epilogue warps drain its own 128 TMEM lanes (all BN columns of its 128 rows) and arrive on
-//     the leader's "accumulator empty" mbarrier; the accumulator is double buffered (2 x BN columns).
+//     the leader's "accumulator empty" mbarrier; the accumulator is double buffered (2 x BN columns). A warp collects
+//     32 rows x 128 bytes in swizzled shared memory and sends them off as one TMA store, two boxes in flight: a thread
+//     has a row of the accumulator, and storing it directly makes every 16-byte store of a warp touch 32 lines, 8000
+//     cycles a tile of fp32 output, more than the main loop of K = 896 has (7000). Microseconds before / with
+//     boxes: 2048 x 151936 x 896 fp32 698 / 478, 8192 x 9728 x 896 135 / 112, 8192 x 4096 x 4096 with residual 230 / 190,
+//     weight gradient 9728 x 896 x 8192 190 / 154, 4096 x 28672 x 4096 604 / 591.
 // Operand majorness is a descriptor flag as in the one-CTA kernel, so forward (K-major, K-major), dgrad
 // (K-major, MN-major) and wgrad (MN-major, MN-major) run on the same code. Every wait is bounded; a CTA that gives
 // up drains its copies, meets its peer at the cluster barrier and frees its TMEM before it returns.
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 #include "tma_host.h"
 
 #include <string.h>
@@ -39,15 +45,14 @@ struct G2Cfg {
   static constexpr int kBBytes = (BN / 2) * G2_BK * 2;         // this CTA's half of the B tile
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kStages = (BN == 256) ? 6 : 8;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024;
+  static constexpr int kOutBytes = G2_EPI_WARPS * 2 * 4096;    // two boxes of 32 rows x 128 bytes a warp
+  static constexpr int kSmemBytes = kStages * kStageBytes + kOutBytes + 1024;
   static constexpr int kTmemCols = G2_ACC * BN;               // 512 or 256
 };
 
 struct G2Params {
-  CUtensorMap a_map, b_map;
+  CUtensorMap a_map, b_map, c_map;
   int M, N, K;
-  void* C;
-  long long ldc;
   const __nv_bfloat16* residual;
   long long ldr;
   const __nv_bfloat16* bias;
@@ -56,6 +61,9 @@ struct G2Params {
   float* tail;
   long long tail_ld;
   int* status;
+  // Vocabulary epilogue (G2_DLOGITS): a tile's fp32 logits become their gradient and never leave the tensor memory.
+  const int* targets;                 // [M]
+  const float *lse, *entropy, *g_logprob, *g_entropy;      // [M]; entropy and g_entropy may be null
   // Fused all-gather of a row-sharded matrix (GATHER instantiations; same contract as the one-CTA kernel): part r is
   // gather_part_bytes at gather_src[r] (rank r's shard, peer memory); the gather warps of every CTA copy an
   // interleaved share of each part to gather_dst + r * bytes, own part first, and the last CTA to finish a part
@@ -73,6 +81,7 @@ struct G2Params {
   int gather_chunks, gather_chunk_tiles;
   long long gather_chunk_bytes;
 };
+constexpr int G2_STORE = 0, G2_DLOGITS = 1;      // epilogues
 constexpr int G2_GATHER_WARPS = 4;      // measured with 2: the copy (159 GB/s over NVLink) set the launch's time
 constexpr int G2_THREADS_GATHER = G2_THREADS + 32 * G2_GATHER_WARPS;
 
@@ -103,7 +112,7 @@ __device__ __forceinline__ void umma2_commit(uint32_t bar_cluster_addr) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 
-template <int BN, bool A_MN, bool B_MN, bool GATHER = false>
+template <int BN, bool A_MN, bool B_MN, bool GATHER = false, int EPI = G2_STORE>
 __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) gemm2cta_kernel(const __grid_constant__ G2Params p) {
   using Cfg = G2Cfg<BN>;
   constexpr int STAGES = Cfg::kStages;
@@ -295,6 +304,9 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
     const int q = warp & 3;                       // TMEM lane quarter this warp may access
     uint32_t tile_iter = 0;
     bool ok = true;
+    const uint32_t out_s = smem_base + STAGES * Cfg::kStageBytes + (warp - 2) * 8192;
+    uint8_t* out_ptr = smem_raw + (out_s - smem_u32(smem_raw));
+    int out_buf = 0;
     const uint32_t leader_empty0 = mapa_cluster(smem_u32(&tmem_empty_bar[0]), 0);
     const uint32_t leader_empty1 = mapa_cluster(smem_u32(&tmem_empty_bar[1]), 0);
     for (int t = pair; t < num_tiles && ok; t += num_pairs, ++tile_iter) {
@@ -309,18 +321,37 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
       const bool row_ok = row < p.M;
       const int n_base = nt * BN;
       const int n_valid = min(BN, p.N - n_base);
+      // what the vocabulary epilogue needs of this row
+      int target = -1;
+      float glp = 0.f, gent = 0.f, l = 0.f, H = 0.f;
+      if constexpr (EPI == G2_DLOGITS) {
+        if (row_ok) {
+          const int t = p.targets[row];
+          target = t - n_base;
+          glp = t >= 0 && t < p.N ? p.g_logprob[row] : 0.f;
+          l = p.lse[row];
+          if (p.g_entropy != nullptr) gent = p.g_entropy[row];
+          if (p.entropy != nullptr) H = p.entropy[row];
+        }
+      }
+      const int row0 = mt * 256 + (int)cta * G2_BM + q * 32;
+      const bool f32 = EPI == G2_STORE && p.out_f32;
+      bool pending = false;                       // the first 32 bf16 columns of a box are collected
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      for (int c0 = 0; c0 < n_valid && row0 < p.M; c0 += 32) {
         uint32_t r[32];
         tmem_ld_32x32(tmem_base + acc * BN + c0 + ((uint32_t)(q * 32) << 16), r);
         tmem_ld_wait();
         const int ncols = min(32, n_valid - c0);
-        if (row_ok && ncols > 0) {
-          float v[32];
+        float v[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-          const int col = n_base + c0;
-          if (p.bias != nullptr) {
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        const int col = n_base + c0;
+        if constexpr (EPI == G2_DLOGITS) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = dlogit_epi(v[j], l, glp, gent, H, c0 + j == target);
+        } else {
+          if (row_ok && p.bias != nullptr) {
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               if (j < ncols) {
@@ -333,7 +364,7 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
               }
             }
           }
-          if (p.residual != nullptr) {
+          if (row_ok && p.residual != nullptr) {
             const __nv_bfloat16* rp = p.residual + row * p.ldr + col;
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
@@ -347,36 +378,50 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
               }
             }
           }
-          if (p.tail != nullptr && col >= p.tail_col) {
-            float* dst = p.tail + row * p.tail_ld + (col - p.tail_col);
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-              if (j < ncols) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-            continue;
-          }
           if (col < p.silu_cols) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = silu_fast(v[j]);
           }
-          if (p.out_f32) {
-            float* dst = reinterpret_cast<float*>(p.C) + row * p.ldc + col;
+        }
+        const bool tail = EPI == G2_STORE && p.tail != nullptr && col >= p.tail_col;
+        const bool second = !f32 && (c0 & 32);
+        if (tail) {
+          if (row_ok) {
+            float* dst = p.tail + row * p.tail_ld + (col - p.tail_col);
 #pragma unroll
             for (int j = 0; j < 32; j += 4)
               if (j < ncols) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-          } else {
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + row * p.ldc + col;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (j < ncols) {
-                uint4 o;
-                o.x = pack_bf16x2(v[j], v[j + 1]);
-                o.y = pack_bf16x2(v[j + 2], v[j + 3]);
-                o.z = pack_bf16x2(v[j + 4], v[j + 5]);
-                o.w = pack_bf16x2(v[j + 6], v[j + 7]);
-                *reinterpret_cast<uint4*>(dst + j) = o;
-              }
-            }
           }
+        } else {
+          if (!second) {                          // a new box: the store of the box before the last has read its buffer
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            __syncwarp();
+          }
+          uint8_t* dst = out_ptr + out_buf * 4096 + lane * 128;
+          if (f32) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              *reinterpret_cast<float4*>(dst + ((u ^ (lane & 7)) << 4)) = make_float4(v[u * 4], v[u * 4 + 1], v[u * 4 + 2], v[u * 4 + 3]);
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              *reinterpret_cast<uint4*>(dst + (((u + (second ? 4 : 0)) ^ (lane & 7)) << 4)) =
+                  make_uint4(pack_bf16x2(v[u * 8], v[u * 8 + 1]), pack_bf16x2(v[u * 8 + 2], v[u * 8 + 3]),
+                             pack_bf16x2(v[u * 8 + 4], v[u * 8 + 5]), pack_bf16x2(v[u * 8 + 6], v[u * 8 + 7]));
+          }
+          pending = true;
+        }
+        // the box is full, or nothing more comes for it; rows and columns past the matrix are cut off by the copy
+        if (pending && (f32 || second || c0 + 32 >= n_valid)) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(&p.c_map)),
+                         "r"(out_s + out_buf * 4096), "r"(second ? col - 32 : col), "r"(row0) : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+          out_buf ^= 1;
+          pending = false;
         }
       }
       // accumulator drained in this CTA: tell the leader's MMA thread
@@ -384,6 +429,7 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(acc == 0 ? leader_empty0 : leader_empty1);
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");       // no store still reads this CTA's memory
   }
 
   // ------------------------------ teardown ------------------------------------------------------
@@ -397,10 +443,10 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
 }
 
 // ---------------------------------- host side ------------------------------------------------
-template <int BN, bool A_MN, bool B_MN, bool GATHER = false>
+template <int BN, bool A_MN, bool B_MN, bool GATHER = false, int EPI = G2_STORE>
 static int g2_launch(const G2Params& p, int tiles, cudaStream_t stream) {
   using Cfg = G2Cfg<BN>;
-  auto kern = gemm2cta_kernel<BN, A_MN, B_MN, GATHER>;
+  auto kern = gemm2cta_kernel<BN, A_MN, B_MN, GATHER, EPI>;
   constexpr int THREADS = GATHER ? G2_THREADS_GATHER : G2_THREADS;
   static bool attr_set[64] = {};
   static int max_pairs[64] = {};
@@ -461,7 +507,6 @@ extern "C" int rb_gemm2_bf16(const void* A, const void* B, void* C, const void* 
   G2Params p;
   memset(&p, 0, sizeof(p));
   p.M = M; p.N = N; p.K = K;
-  p.C = C; p.ldc = ldc;
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual); p.ldr = ldr;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.out_f32 = out_f32;
@@ -472,6 +517,10 @@ extern "C" int rb_gemm2_bf16(const void* A, const void* B, void* C, const void* 
   if (rc != 0) return -20 + rc;
   rc = b_mn_major ? tma_map_2d_bf16(&p.b_map, B, K, N, ldb, G2_BK) : tma_map_2d_bf16(&p.b_map, B, N, K, ldb, bn / 2);
   if (rc != 0) return -30 + rc;
+  if (tail == nullptr || tail_col > 0) {
+    rc = tma_map_2d_out(&p.c_map, C, M, tail != nullptr ? tail_col : N, ldc, out_f32, 32);
+    if (rc != 0) return -40 + rc;
+  }
   const int tiles = m_tiles * ((N + bn - 1) / bn);
   if (bn == 256) {
     if (!a_mn_major && !b_mn_major) return g2_launch<256, false, false>(p, tiles, stream);
@@ -502,7 +551,6 @@ extern "C" int rb_gemm2_bf16_gather(const void* A, const void* B, void* C, const
   G2Params p;
   memset(&p, 0, sizeof(p));
   p.M = M; p.N = N; p.K = K;
-  p.C = C; p.ldc = ldc;
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual); p.ldr = ldr;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.out_f32 = out_f32;
@@ -525,7 +573,32 @@ extern "C" int rb_gemm2_bf16_gather(const void* A, const void* B, void* C, const
   if (rc != 0) return -20 + rc;
   rc = b_mn_major ? tma_map_2d_bf16(&p.b_map, B, K, N, ldb, G2_BK) : tma_map_2d_bf16(&p.b_map, B, N, K, ldb, 128);
   if (rc != 0) return -30 + rc;
+  rc = tma_map_2d_out(&p.c_map, C, M, N, ldc, out_f32, 32);
+  if (rc != 0) return -40 + rc;
   const int tiles = ((M + 255) / 256) * ((N + 255) / 256);
   if (!a_mn_major) return g2_launch<256, false, false, true>(p, tiles, stream);
   return g2_launch<256, true, true, true>(p, tiles, stream);
+}
+
+// The gradient of log-probabilities to logits, from the product that recomputes the logits A[M,K] B[N,K]^T: bit for bit what
+// rb_logprob_entropy_bwd makes of the fp32 output of rb_gemm2_bf16 (2048 x 151936 x 896: 700 + 343 us for the two, which write, read
+// and convert 2.5 GB; 453 us here).
+// dlogits bf16 [M, N] (rows ldd apart, a multiple of 8). entropy and g_entropy may be null.
+extern "C" int rb_gemm2_dlogits(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, const int* targets,
+                                const float* lse, const float* entropy, const float* g_logprob, const float* g_entropy, void* dlogits,
+                                long long ldd, int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || N % 8 != 0 || K % 8 != 0) return -1;
+  if (ldd % 8 != 0 || ((unsigned long long)dlogits & 15) != 0) return -1;
+  G2Params p;
+  memset(&p, 0, sizeof(p));
+  p.M = M; p.N = N; p.K = K;
+  p.status = status;
+  int rc = tma_map_2d_bf16(&p.a_map, A, M, K, lda, G2_BM);
+  if (rc != 0) return -20 + rc;
+  rc = tma_map_2d_bf16(&p.b_map, B, N, K, ldb, 128);
+  if (rc != 0) return -30 + rc;
+  p.targets = targets; p.lse = lse; p.entropy = entropy; p.g_logprob = g_logprob; p.g_entropy = g_entropy;
+  rc = tma_map_2d_out(&p.c_map, dlogits, M, N, ldd, 0, 32);
+  if (rc != 0) return -40 + rc;
+  return g2_launch<256, false, false, false, G2_DLOGITS>(p, ((M + 255) / 256) * ((N + 255) / 256), stream);
 }

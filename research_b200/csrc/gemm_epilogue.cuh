@@ -16,4 +16,12 @@ __device__ __forceinline__ float swiglu_epi(float gate, float up) {
   return __bfloat162float(__float2bfloat16_rn(g / (1.f + __expf(-g)))) * u;
 }
 
+// Gradient to a logit x of a row with log-sum-exp l: of the target's log-probability (upstream gradient glp) and of the row's entropy H
+// (gent).
+__device__ __forceinline__ float dlogit_epi(float x, float l, float glp, float gent, float H, bool is_target) {
+  const float lp = x - l;
+  const float p = __expf(lp);
+  return glp * ((is_target ? 1.f : 0.f) - p) - gent * p * (lp + H);
+}
+
 }  // namespace rb

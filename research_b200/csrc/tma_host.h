@@ -41,4 +41,21 @@ inline int tma_map_2d_bf16(CUtensorMap* out, const void* base, unsigned long lon
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
+// Output matrix, bf16 or fp32: boxes of box_rows x 128 bytes (64 or 32 columns).
+inline int tma_map_2d_out(CUtensorMap* out, void* base, unsigned long long rows, unsigned long long cols, unsigned long long ld, int f32,
+                          unsigned box_rows) {
+  EncodeTiledFnT fn = tma_encode_fn();
+  if (fn == nullptr) return -1;
+  const unsigned es = f32 ? 4 : 2;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (ld * es) % 16 != 0) return -2;
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {ld * es};
+  cuuint32_t box[2] = {128 / es, box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -3;
+}
+
 }  // namespace rb

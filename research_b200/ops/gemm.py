@@ -123,6 +123,8 @@ def _lib2() -> ctypes.CDLL:
         lib.rb_gemm2_bf16_gather.argtypes = ([vp] * 5 + [i, i, i, ll, ll, ll, ll, i, i, i] +
                                              [ctypes.POINTER(vp), vp, ll, vp, vp, i, i, i, i, i, vp, vp])
         lib.rb_gemm2_bf16_gather.restype = i
+        lib.rb_gemm2_dlogits.argtypes = [vp] * 2 + [i] * 3 + [ll] * 2 + [vp] * 6 + [ll, vp, vp]
+        lib.rb_gemm2_dlogits.restype = i
         lib._rb_typed = True
     return lib
 
@@ -198,6 +200,24 @@ def gemm2(a: torch.Tensor, b: torch.Tensor, bias=None, residual=None, out=None, 
                                int(b_mn_major), int(out_f32), bn, silu_cols, tail.data_ptr() if tail is not None else None,
                                N - tail.shape[1] if tail is not None else 0, tail.stride(0) if tail is not None else 0, status_tensor(a.device).data_ptr(), stream_handle(a.device))
     check_rc(rc, "rb_gemm2_bf16")
+    return out
+
+
+def vocabulary_takes(h: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether ``vocabulary_dlogits`` runs on these operands: where the product alone would run on the kernel whose epilogue it is, so that both
+    see the same logits."""
+    return (h.is_cuda and h.dtype == w.dtype == torch.bfloat16 and h.dim() == w.dim() == 2 and h.stride(1) == w.stride(1) == 1
+            and w.shape[0] > 128 and _use_pair_kernel(h.shape[0], w.shape[0], h.shape[1], False, False))
+
+
+def vocabulary_dlogits(h, w, targets, lse, entropy, g_logprob, g_entropy) -> torch.Tensor:
+    """``logprob_entropy_bwd(h @ w.T, ...)`` (bf16) as one product whose epilogue turns its tiles into their gradient."""
+    M, N = h.shape[0], w.shape[0]
+    assert targets.dtype == torch.int32 and all(t is None or (t.dtype == torch.float32 and t.is_contiguous()) for t in (lse, entropy, g_logprob, g_entropy))
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=h.device)
+    rc = _lib2().rb_gemm2_dlogits(h.data_ptr(), w.data_ptr(), M, N, h.shape[1], h.stride(0), w.stride(0), targets.data_ptr(), lse.data_ptr(), ptr(entropy),
+                                  g_logprob.data_ptr(), ptr(g_entropy), out.data_ptr(), N, status_tensor(h.device).data_ptr(), stream_handle(h.device))
+    check_rc(rc, "rb_gemm2_dlogits")
     return out
 
 

@@ -274,9 +274,11 @@ class _FusedLogprob(torch.autograd.Function):
         g_ent = g_ent.contiguous().float() if ctx.need_entropy else None
         for s in range(0, N, _FusedLogprob.CHUNK):
             e = min(N, s + _FusedLogprob.CHUNK)
-            logits = ops.gemm(h[s:e], w, out_f32=True)
-            dl = T.logprob_entropy_bwd(logits, targets[s:e], lse[s:e], ent[s:e] if ctx.need_entropy else None,
-                                       g_lp[s:e], g_ent[s:e] if g_ent is not None else None)
+            rows = (targets[s:e], lse[s:e], ent[s:e] if ctx.need_entropy else None, g_lp[s:e], g_ent[s:e] if g_ent is not None else None)
+            if ops.gemm_mod.vocabulary_takes(h[s:e], w):     # the same values, without the logits in memory
+                dl = ops.gemm_mod.vocabulary_dlogits(h[s:e], w, *rows)
+            else:
+                dl = T.logprob_entropy_bwd(ops.gemm(h[s:e], w, out_f32=True), *rows)
             dl = dl.to(h.dtype) if dl.dtype != h.dtype else dl
             ops.gemm(dl, w, out=dh[s:e], b_mn_major=True)
             acc = ctx.sink.accumulate_into(ctx.gw)
