@@ -57,6 +57,8 @@ struct G2Params {
   long long ldr;
   const __nv_bfloat16* bias;
   int out_f32;
+  int glu_kind;                       // G2_GLU: columns are 128 gate, 128 up, alternating; as in RbGemmArgs
+  float glu_limit;
   int silu_cols, tail_col;            // as in RbGemmArgs
   float* tail;
   long long tail_ld;
@@ -81,7 +83,7 @@ struct G2Params {
   int gather_chunks, gather_chunk_tiles;
   long long gather_chunk_bytes;
 };
-constexpr int G2_STORE = 0, G2_DLOGITS = 1;      // epilogues
+constexpr int G2_STORE = 0, G2_DLOGITS = 1, G2_GLU = 2;      // epilogues
 constexpr int G2_GATHER_WARPS = 4;      // measured with 2: the copy (159 GB/s over NVLink) set the launch's time
 constexpr int G2_THREADS_GATHER = G2_THREADS + 32 * G2_GATHER_WARPS;
 
@@ -336,21 +338,35 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
       }
       const int row0 = mt * 256 + (int)cta * G2_BM + q * 32;
       const bool f32 = EPI == G2_STORE && p.out_f32;
+      const int n_store = EPI == G2_GLU ? BN / 2 : n_valid;        // columns that leave
       bool pending = false;                       // the first 32 bf16 columns of a box are collected
 #pragma unroll 1
-      for (int c0 = 0; c0 < n_valid && row0 < p.M; c0 += 32) {
+      for (int c0 = 0; c0 < n_store && row0 < p.M; c0 += 32) {
         uint32_t r[32];
         tmem_ld_32x32(tmem_base + acc * BN + c0 + ((uint32_t)(q * 32) << 16), r);
-        tmem_ld_wait();
-        const int ncols = min(32, n_valid - c0);
         float v[32];
+        if constexpr (EPI == G2_GLU) {
+          uint32_t up[32];
+          tmem_ld_32x32(tmem_base + acc * BN + BN / 2 + c0 + ((uint32_t)(q * 32) << 16), up);
+          tmem_ld_wait();
+          if (p.glu_kind == 1) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-        const int col = n_base + c0;
+            for (int j = 0; j < 32; ++j) v[j] = clamped_glu_epi(__uint_as_float(r[j]), __uint_as_float(up[j]), p.glu_limit);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = swiglu_epi(__uint_as_float(r[j]), __uint_as_float(up[j]));
+          }
+        } else {
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        }
+        const int ncols = min(32, n_store - c0);
+        const int col = (EPI == G2_GLU ? nt * (BN / 2) : n_base) + c0;
         if constexpr (EPI == G2_DLOGITS) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = dlogit_epi(v[j], l, glp, gent, H, c0 + j == target);
-        } else {
+        } else if constexpr (EPI == G2_STORE) {
           if (row_ok && p.bias != nullptr) {
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
@@ -412,7 +428,7 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
           pending = true;
         }
         // the box is full, or nothing more comes for it; rows and columns past the matrix are cut off by the copy
-        if (pending && (f32 || second || c0 + 32 >= n_valid)) {
+        if (pending && (f32 || second || c0 + 32 >= n_store)) {
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
@@ -490,10 +506,12 @@ extern "C" int rb_gemm2_pairs() {
 
 // C[M,N] = op(A) op(B)^T (+bias) (+residual). K-major operands are [rows, K] with K contiguous, MN-major operands
 // [K, rows] with rows contiguous (as in rb_gemm_bf16). bn: 256 or 128 output columns per tile (0 = choose).
+// glu: 0, or 1 silu(gate) * up / 2 the clamped unit, of B's rows in blocks of 128 gate and 128 up (K-major
+// operands, N a multiple of 256, bf16 output [M, N / 2], nothing added).
 extern "C" int rb_gemm2_bf16(const void* A, const void* B, void* C, const void* bias, const void* residual, int M, int N,
                              int K, long long lda, long long ldb, long long ldc, long long ldr, int a_mn_major,
                              int b_mn_major, int out_f32, int bn, int silu_cols, float* tail, int tail_col, long long tail_ld,
-                             int* status, cudaStream_t stream) {
+                             int glu, float glu_limit, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0 || N % 8 != 0) return -1;
   if ((!a_mn_major || !b_mn_major) && K % 8 != 0) return -1;
   if (a_mn_major && !b_mn_major) return -12;         // not used by forward, dgrad or wgrad
@@ -510,6 +528,8 @@ extern "C" int rb_gemm2_bf16(const void* A, const void* B, void* C, const void* 
   p.residual = reinterpret_cast<const __nv_bfloat16*>(residual); p.ldr = ldr;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.out_f32 = out_f32;
+  if (glu != 0 && (N % 256 != 0 || (bn != 0 && bn != 256) || a_mn_major || b_mn_major || out_f32 || bias || residual || silu_cols || tail)) return -1;
+  p.glu_kind = glu == 2; p.glu_limit = glu_limit;
   p.silu_cols = silu_cols; p.tail = tail; p.tail_col = tail_col; p.tail_ld = tail_ld;
   if (silu_cols % 32 != 0 || (tail != nullptr && (tail_col % 32 != 0 || tail_ld % 4 != 0))) return -1;
   p.status = status;
@@ -518,10 +538,11 @@ extern "C" int rb_gemm2_bf16(const void* A, const void* B, void* C, const void* 
   rc = b_mn_major ? tma_map_2d_bf16(&p.b_map, B, K, N, ldb, G2_BK) : tma_map_2d_bf16(&p.b_map, B, N, K, ldb, bn / 2);
   if (rc != 0) return -30 + rc;
   if (tail == nullptr || tail_col > 0) {
-    rc = tma_map_2d_out(&p.c_map, C, M, tail != nullptr ? tail_col : N, ldc, out_f32, 32);
+    rc = tma_map_2d_out(&p.c_map, C, M, tail != nullptr ? tail_col : glu ? N / 2 : N, ldc, out_f32, 32);
     if (rc != 0) return -40 + rc;
   }
   const int tiles = m_tiles * ((N + bn - 1) / bn);
+  if (glu != 0) return g2_launch<256, false, false, false, G2_GLU>(p, tiles, stream);
   if (bn == 256) {
     if (!a_mn_major && !b_mn_major) return g2_launch<256, false, false>(p, tiles, stream);
     if (!a_mn_major && b_mn_major) return g2_launch<256, false, true>(p, tiles, stream);

@@ -117,7 +117,7 @@ def _lib2() -> ctypes.CDLL:
     lib = _native.load("rb_gemm2")
     if not getattr(lib, "_rb_typed", False):
         vp, i, ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
-        lib.rb_gemm2_bf16.argtypes = [vp] * 5 + [i, i, i, ll, ll, ll, ll, i, i, i, i, i, vp, i, ll, vp, vp]
+        lib.rb_gemm2_bf16.argtypes = [vp] * 5 + [i, i, i, ll, ll, ll, ll, i, i, i, i, i, vp, i, ll, i, ctypes.c_float, vp, vp]
         lib.rb_gemm2_bf16.restype = i
         lib.rb_gemm2_pairs.restype = i
         lib.rb_gemm2_bf16_gather.argtypes = ([vp] * 5 + [i, i, i, ll, ll, ll, ll, i, i, i] +
@@ -182,23 +182,35 @@ def _use_pair_kernel(M: int, N: int, K: int, a_mn_major: bool, b_mn_major: bool)
     return -(-M // 256) * -(-N // 128) >= _GEMM2_PAIRS
 
 
+def _pair_glu_takes(N: int, bn: int, bias, residual, out_f32: bool, silu_cols: int, tail) -> bool:
+    """The gated unit in the two-CTA kernel's epilogue: its tile is 256 columns, so are the blocks of gate and up rows. Microseconds, one-CTA
+    kernel / this one: 8192 x 28672 x 4096 1490 / 1272, 1500 x 28672 x 4096 350 / 280, 5210 x 16384 x 2048 328 / 263, 600 x 16384 x 2048
+    76 / 67. With a folded norm, whose row sums the one-CTA kernel takes from its operand tiles, the two are equal at 10000 rows
+    (a launch more here), so it stays there."""
+    return bn == 256 and N % 256 == 0 and bias is None and residual is None and not out_f32 and not silu_cols and tail is None
+
+
 def gemm2(a: torch.Tensor, b: torch.Tensor, bias=None, residual=None, out=None, *, a_mn_major=False, b_mn_major=False,
-          out_f32=False, bn: int = 0, silu_cols: int = 0, tail: torch.Tensor | None = None) -> torch.Tensor:
+          out_f32=False, bn: int = 0, silu_cols: int = 0, tail: torch.Tensor | None = None,
+          swiglu: bool = False, glu_limit: float | None = None) -> torch.Tensor:
     """``C = op(A) @ op(B)^T (+bias) (+residual)`` on the two-CTA (``cta_group::2``) kernel; same operand conventions
-    as ``gemm`` (``silu_cols`` and ``tail`` too). ``bn``: 256 or 128 output columns per tile (0 = fewest waves)."""
+    as ``gemm`` (``silu_cols``, ``tail`` and, for ``bn`` 256, ``swiglu`` too). ``bn``: 256 or 128 output columns per
+    tile (0 = fewest waves)."""
     assert a.is_cuda and a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.dim() == 2 and b.dim() == 2
     assert a.stride(1) == 1 and b.stride(1) == 1
     K, M = a.shape if a_mn_major else a.shape[::-1]
     Kb, N = b.shape if b_mn_major else b.shape[::-1]
     assert K == Kb, f"K mismatch: {K} vs {Kb}"
     if out is None:
-        out = torch.empty(M, N - (tail.shape[1] if tail is not None else 0), dtype=torch.float32 if out_f32 else torch.bfloat16, device=a.device)
+        out = torch.empty(M, N // 2 if swiglu else N - (tail.shape[1] if tail is not None else 0), dtype=torch.float32 if out_f32 else torch.bfloat16, device=a.device)
     assert out.stride(1) == 1 and (residual is None or residual.stride(1) == 1)
     rc = _lib2().rb_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), bias.data_ptr() if bias is not None else None,
                                residual.data_ptr() if residual is not None else None, M, N, K, a.stride(0), b.stride(0),
                                out.stride(0), residual.stride(0) if residual is not None else 0, int(a_mn_major),
                                int(b_mn_major), int(out_f32), bn, silu_cols, tail.data_ptr() if tail is not None else None,
-                               N - tail.shape[1] if tail is not None else 0, tail.stride(0) if tail is not None else 0, status_tensor(a.device).data_ptr(), stream_handle(a.device))
+                               N - tail.shape[1] if tail is not None else 0, tail.stride(0) if tail is not None else 0,
+                               (2 if glu_limit is not None else 1) if swiglu else 0, glu_limit or 0.0, status_tensor(a.device).data_ptr(),
+                               stream_handle(a.device))
     check_rc(rc, "rb_gemm2_bf16")
     return out
 
@@ -396,9 +408,11 @@ def gemm(
     if softcap > 0:
         assert not swiglu and split_k in (0, 1), "the soft cap belongs to a plain store"
         split_k, cluster_split = 1, False
-    if (gather is None and softcap == 0 and wait_flag is None and not swiglu and norm_eps is None and alpha == 1.0 and beta == 1.0 and bn == 0 and max_ctas == 0 and split_k in (0, 1)
-            and not cluster_split and _use_pair_kernel(M, N, K, a_mn_major, b_mn_major)):
-        return gemm2(a, b, bias, residual, out, a_mn_major=a_mn_major, b_mn_major=b_mn_major, out_f32=out_f32, silu_cols=silu_cols, tail=tail)
+    if (gather is None and softcap == 0 and wait_flag is None and norm_eps is None and alpha == 1.0 and beta == 1.0 and max_ctas == 0 and split_k in (0, 1)
+            and not cluster_split and _use_pair_kernel(M, N, K, a_mn_major, b_mn_major)
+            and (_pair_glu_takes(N, bn, bias, residual, out_f32, silu_cols, tail) if swiglu else bn == 0)):
+        return gemm2(a, b, bias, residual, out, a_mn_major=a_mn_major, b_mn_major=b_mn_major, out_f32=out_f32, silu_cols=silu_cols, tail=tail,
+                     swiglu=swiglu, glu_limit=glu_limit)
     if silu_cols or tail is not None:
         assert gather is None and wait_flag is None and not swiglu and norm_eps is None and alpha == beta == 1.0 and not out_f32 and softcap == 0, \
             "silu_cols and tail belong to a plain store"

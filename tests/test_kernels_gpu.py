@@ -507,3 +507,20 @@ def test_gemm_waits_for_a_flag_inside_the_launch(cuda_device):
         want = a.float() @ w.float().t()
         assert (out.float() - want).abs().max().item() < 0.02 * K ** 0.5
     ops.check_status()
+
+
+@pytest.mark.parametrize("limit", [None, 1.5])
+@pytest.mark.parametrize("M,N,K", [(512, 9728, 256), (513, 9728, 264), (1000, 4864 * 2, 896), (2049, 2560, 512)])
+def test_gated_unit_on_the_pair_kernel(cuda_device, M, N, K, limit):
+    """The two-CTA kernel's gated unit equals the one-CTA kernel's (same sums, same epilogue): partial row tiles, a K remainder, strided rows."""
+    from research_b200.ops import gemm_mod
+
+    g = torch.Generator(device=cuda_device).manual_seed(M + N)
+    a = torch.randn(M, K + 8, device=cuda_device, generator=g).bfloat16()[:, :K]
+    b = (torch.randn(N, K, device=cuda_device, generator=g) * 2 * K ** -0.5).bfloat16()
+    out = torch.full((M, N // 2 + 8), 7.0, device=cuda_device, dtype=torch.bfloat16)
+    assert gemm_mod._use_pair_kernel(M, N, K, False, False)
+    got = ops.gemm(a, b, out=out[:, :N // 2], bn=256, swiglu=True, glu_limit=limit)
+    want = ops.gemm(a, b, bn=256, swiglu=True, glu_limit=limit, max_ctas=148)
+    assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs() + 1e-6).all()
+    assert (out[:, N // 2:] == 7.0).all()
