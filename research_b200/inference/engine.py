@@ -249,6 +249,10 @@ class InferenceEngine:
 
     def _run_decode(self, n: int) -> None:
         """Stage the scheduled decode rows, run one decode step and wait for it."""
+        self._launch_decode(n)
+        self._sync()
+
+    def _launch_decode(self, n: int) -> None:
         r = self.runner
         mb, o = r.max_batch, r._pf_offsets()
         base, pf = r.meta_host.data_ptr(), r.pf_host.data_ptr()
@@ -256,11 +260,11 @@ class InferenceEngine:
             self._core, 1, base, base + 4 * mb, base + 8 * mb, pf + 4 * o["cu_q"], base + 12 * mb, r.bt_host.data_ptr(),
             r.max_blocks_per_seq, base + 16 * mb, base + 20 * mb, pf + 4 * o["sample_rows"], mb, mb)
         assert T == n, T
-        self._lib.rbe_batch_slots(self._core, 1, base + 28 * mb)
-        max_blocks = self._max_blocks_in(r.meta_host[3 * mb:3 * mb + n])
+        if self.state_slots:      # (nothing else reads them)
+            self._lib.rbe_batch_slots(self._core, 1, base + 28 * mb)
+        max_blocks = -(-int(r.meta_rows[3 * mb:3 * mb + n].max()) // BLOCK)
         r.stage_decode_padding(n)
         r.decode(n, max_blocks)
-        self._sync()
 
     def _build_packed(self, which: int, n_rows: int) -> tuple[int, int, int, int]:
         """Stage the scheduled prefill (2) or decode + prefill (3) rows; returns the arguments of a packed pass."""
@@ -293,6 +297,18 @@ class InferenceEngine:
         if rc < 0:
             raise RuntimeError({-1: "feed: unknown stream or an entry without tokens", -2: "feed: the KV cache is full",
                                 -3: "feed: more tokens than the engine was made for", -4: "feed: every state slot is taken"}[rc])
+        if lib.rbe_get_scheduled(core, None, None, None) == n:
+            # single tokens only: rows in the order of the entries; their logits are taken before the step is waited for
+            self._launch_decode(n)
+            wanted = [i + w for i, (_, _, places) in enumerate(entries) for w in places]
+            out = None
+            if wanted == list(range(n)):
+                out = r.a_logits[:n].clone(memory_format=torch.contiguous_format)
+            elif wanted:
+                out = r.a_logits[:n].index_select(0, torch.tensor(wanted, device=self.device))
+            self._sync()
+            lib.rbe_commit_fed(core)
+            return out
         pre, dec = (_LL * n)(), (_LL * n)()
         n_dec = lib.rbe_get_scheduled(core, pre, dec, None)
         order = list(dec[:n_dec]) + list(pre[:n - n_dec])
@@ -302,12 +318,8 @@ class InferenceEngine:
             first[s] = at
             at += count[s]
         wanted = [first[s] + w for s, _, places in entries for w in places]
-        if n_dec == n:
-            self._run_decode(n)
-            out = r.a_logits[:n].index_select(0, torch.tensor(wanted, device=self.device)) if wanted else None
-        else:
-            out = r.packed_logits(*self._build_packed(3, n), wanted)
-            self._sync()
+        out = r.packed_logits(*self._build_packed(3, n), wanted)
+        self._sync()
         lib.rbe_commit_fed(core)
         return out
 

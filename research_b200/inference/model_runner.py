@@ -89,6 +89,7 @@ class RunnerBase:
         self.meta_fields = 8
         self.meta_dev = torch.zeros(self.meta_fields * mb, dtype=torch.int32, device=device)
         self.meta_host = self._pinned(torch.zeros(self.meta_fields * mb, dtype=torch.int32))
+        self.meta_rows = self.meta_host.numpy()          # the same memory: a few numbers a step are cheaper to read and write there
         self.bt_dev = torch.zeros(mb, self.max_blocks_per_seq, dtype=torch.int32, device=device)
         self.bt_host = self._pinned(torch.zeros(mb, self.max_blocks_per_seq, dtype=torch.int32))
         self.out_dev = torch.zeros(2 * mb, dtype=torch.int32, device=device)
@@ -206,15 +207,10 @@ class RunnerBase:
     def stage_decode_padding(self, n: int) -> None:
         """Mark rows n..bucket as padding (no KV write, empty context)."""
         bk = self.bucket(n) if (self.use_cuda_graphs or self.row_align > 1) else max(n, 1)
-        mb = self.max_batch
-        mh = self.meta_host
         if bk > n:
-            mh[0 * mb + n:0 * mb + bk] = 0
-            mh[1 * mb + n:1 * mb + bk] = 0
-            mh[2 * mb + n:2 * mb + bk] = -1
-            mh[3 * mb + n:3 * mb + bk] = 0
-            mh[4 * mb + n:4 * mb + bk] = 0
-            mh[7 * mb + n:7 * mb + bk] = -1
+            mb, mh = self.max_batch, self.meta_rows
+            for field, fill in ((0, 0), (1, 0), (2, -1), (3, 0), (4, 0), (7, -1)):
+                mh[field * mb + n:field * mb + bk] = fill
 
     # ------------------------------------------------------------------ packed batches
     def _stage_packed(self, rows: int, T: int, max_new: int, max_blocks: int) -> "PackedBatch":
@@ -255,10 +251,10 @@ class RunnerBase:
 
     def packed_logits(self, rows: int, T: int, max_new: int, max_blocks: int, wanted: list[int]) -> torch.Tensor | None:
         """The same pass without sampling: fp32 logits ``[len(wanted), V]`` of the packed rows ``wanted``."""
-        x = self._packed_forward(self._stage_packed(rows, T, max_new, max_blocks))
-        if not wanted:
-            return None
-        return self._row_logits(x, torch.tensor(wanted, dtype=torch.int32).to(self.device))
+        b = self._stage_packed(rows, T, max_new, max_blocks)
+        at = torch.tensor(wanted, dtype=torch.int32).to(self.device) if wanted else None      # before the pass: the copy waits for what is queued
+        x = self._packed_forward(b)
+        return self._row_logits(x, at) if wanted else None
 
     # ------------------------------------------------------------------ teacher forcing
     def score(self, token_ids: torch.Tensor) -> torch.Tensor:
