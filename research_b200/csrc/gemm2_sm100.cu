@@ -59,6 +59,10 @@ struct G2Params {
   int out_f32;
   int glu_kind;                       // G2_GLU: columns are 128 gate, 128 up, alternating; as in RbGemmArgs
   float glu_limit;
+  // G2_GROUPS: group g is C rows [g M, (g + 1) M) = A[k rows of g]^T B[k rows of g], both MN-major, with the contraction over the rows
+  // group_offsets[g] .. group_offsets[g + 1] (multiples of 64, at least 64 rows each)
+  const int* group_offsets;
+  int groups;
   int silu_cols, tail_col;            // as in RbGemmArgs
   float* tail;
   long long tail_ld;
@@ -83,7 +87,7 @@ struct G2Params {
   int gather_chunks, gather_chunk_tiles;
   long long gather_chunk_bytes;
 };
-constexpr int G2_STORE = 0, G2_DLOGITS = 1, G2_GLU = 2;      // epilogues
+constexpr int G2_STORE = 0, G2_DLOGITS = 1, G2_GLU = 2, G2_GROUPS = 3;      // epilogues; the last: plain, of a product per group
 constexpr int G2_GATHER_WARPS = 4;      // measured with 2: the copy (159 GB/s over NVLink) set the launch's time
 constexpr int G2_THREADS_GATHER = G2_THREADS + 32 * G2_GATHER_WARPS;
 
@@ -133,14 +137,24 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int m_tiles = (p.M + 255) / 256, n_tiles = (p.N + BN - 1) / BN;
-  const int num_tiles = m_tiles * n_tiles;
-  const int num_kb = (p.K + G2_BK - 1) / G2_BK;
+  const int num_tiles = m_tiles * n_tiles * (EPI == G2_GROUPS ? p.groups : 1);
   // tile t -> (row tile, column tile); a launch that consumes its own gather starts at the local part's columns
   const int nt_rot = (GATHER && p.consume) ? p.rank * p.n_tiles_per_part : 0;
   auto tile_mn = [&](int t, int& mt, int& nt) {
+    if (EPI == G2_GROUPS) t %= m_tiles * n_tiles;
     mt = t % m_tiles;
     nt = t / m_tiles + nt_rot;
     if (nt >= n_tiles) nt -= n_tiles;
+  };
+  // first row of the contraction and its 64-row blocks
+  auto tile_k = [&](int t, int& k_first, int& num_kb) {
+    k_first = 0;
+    num_kb = (p.K + G2_BK - 1) / G2_BK;
+    if (EPI == G2_GROUPS) {
+      const int g = t / (m_tiles * n_tiles);
+      k_first = p.group_offsets[g];
+      num_kb = (p.group_offsets[g + 1] - k_first) / G2_BK;
+    }
   };
 
   if (threadIdx.x == 0) {
@@ -174,8 +188,9 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
       bool ok = true;
       unsigned long long chunks_seen = 0;
       for (int t = pair; t < num_tiles && ok; t += num_pairs) {
-        int mt, nt;
+        int mt, nt, k_first, num_kb;
         tile_mn(t, mt, nt);
+        tile_k(t, k_first, num_kb);
         const int m0 = mt * 256 + (int)cta * G2_BM;        // this CTA's rows of A
         const int n0 = nt * BN + (int)cta * HALF_N;        // this CTA's rows of B
         if (GATHER && p.consume) {
@@ -199,13 +214,13 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
             tma_load_2d_pair(sa, &p.a_map, fb, kb * G2_BK, m0);
           } else {
 #pragma unroll
-            for (int c = 0; c < G2_BM / 64; ++c) tma_load_2d_pair(sa + c * (G2_BK * 128), &p.a_map, fb, m0 + c * 64, kb * G2_BK);
+            for (int c = 0; c < G2_BM / 64; ++c) tma_load_2d_pair(sa + c * (G2_BK * 128), &p.a_map, fb, m0 + c * 64, k_first + kb * G2_BK);
           }
           if (!B_MN) {
             tma_load_2d_pair(sb, &p.b_map, fb, kb * G2_BK, n0);
           } else {
 #pragma unroll
-            for (int c = 0; c < HALF_N / 64; ++c) tma_load_2d_pair(sb + c * (G2_BK * 128), &p.b_map, fb, n0 + c * 64, kb * G2_BK);
+            for (int c = 0; c < HALF_N / 64; ++c) tma_load_2d_pair(sb + c * (G2_BK * 128), &p.b_map, fb, n0 + c * 64, k_first + kb * G2_BK);
           }
           if (++s == STAGES) { s = 0; ph ^= 1u; }
         }
@@ -233,6 +248,8 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
         if (!ok) break;
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * BN;
+        int k_first, num_kb;
+        tile_k(t, k_first, num_kb);
         for (int kb = 0; kb < num_kb; ++kb) {
           ok = mbar_wait_bounded_cluster(smem_u32(&full_bar[s]), ph, abortp, p.status, ST_TIMEOUT_SMEM_FULL);
           if (!ok) break;
@@ -319,8 +336,10 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
       ok = mbar_wait_bounded_cluster(smem_u32(&tmem_full_bar[acc]), acc_ph, abortp, p.status, ST_TIMEOUT_TMEM_FULL);
       if (!ok) break;
       tc_fence_after();
-      const long long row = (long long)mt * 256 + (long long)cta * G2_BM + q * 32 + lane;
-      const bool row_ok = row < p.M;
+      const int row0 = mt * 256 + (int)cta * G2_BM + q * 32;       // of the group's M rows; whole boxes of 32 belong to it
+      const bool row_ok = row0 + lane < p.M;
+      const int group_row = EPI == G2_GROUPS ? t / (m_tiles * n_tiles) * p.M : 0;
+      const long long row = (long long)group_row + row0 + lane;
       const int n_base = nt * BN;
       const int n_valid = min(BN, p.N - n_base);
       // what the vocabulary epilogue needs of this row
@@ -336,7 +355,6 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
           if (p.entropy != nullptr) H = p.entropy[row];
         }
       }
-      const int row0 = mt * 256 + (int)cta * G2_BM + q * 32;
       const bool f32 = EPI == G2_STORE && p.out_f32;
       const int n_store = EPI == G2_GLU ? BN / 2 : n_valid;        // columns that leave
       bool pending = false;                       // the first 32 bf16 columns of a box are collected
@@ -366,7 +384,7 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
         if constexpr (EPI == G2_DLOGITS) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = dlogit_epi(v[j], l, glp, gent, H, c0 + j == target);
-        } else if constexpr (EPI == G2_STORE) {
+        } else if constexpr (EPI == G2_STORE || EPI == G2_GROUPS) {
           if (row_ok && p.bias != nullptr) {
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
@@ -433,7 +451,7 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
           __syncwarp();
           if (lane == 0) {
             asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(&p.c_map)),
-                         "r"(out_s + out_buf * 4096), "r"(second ? col - 32 : col), "r"(row0) : "memory");
+                         "r"(out_s + out_buf * 4096), "r"(second ? col - 32 : col), "r"(group_row + row0) : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
           out_buf ^= 1;
@@ -622,4 +640,27 @@ extern "C" int rb_gemm2_dlogits(const void* A, const void* B, int M, int N, int 
   rc = tma_map_2d_out(&p.c_map, dlogits, M, N, ldd, 0, 32);
   if (rc != 0) return -40 + rc;
   return g2_launch<256, false, false, false, G2_DLOGITS>(p, ((M + 255) / 256) * ((N + 255) / 256), stream);
+}
+
+// C[g M .. , N] = A[rows of g, M]^T B[rows of g, N] (+ residual at the same places) for every group of rows of A [rows, M] and B [rows, N]:
+// the weight gradients of all experts. offsets [groups + 1] on the device: multiples of 64, every group at least 64 rows. M a
+// multiple of 32. One 256 x 256 tile per pair of CTAs loads a third less than the one-CTA kernel's 128 x 256 tiles, whose loads at a
+// contraction of 256 rows bounded it: 128 experts, 37000 rows, 1536 x 2048 and 2048 x 768 635 us together, 464 here.
+extern "C" int rb_gemm2_groups(const void* A, const void* B, void* C, const void* residual, int groups, int M, int N, int rows, long long lda,
+                               long long ldb, long long ldc, long long ldr, const int* offsets, int* status, cudaStream_t stream) {
+  if (groups <= 0 || M <= 0 || N <= 0 || rows <= 0 || M % 32 != 0 || N % 8 != 0 || offsets == nullptr) return -1;
+  if ((long long)groups * ((M + 255) / 256) * ((N + 255) / 256) > 0x7fffffff || (long long)groups * M > 0x7fffffff) return -1;
+  G2Params p;
+  memset(&p, 0, sizeof(p));
+  p.M = M; p.N = N; p.K = rows;
+  p.residual = reinterpret_cast<const __nv_bfloat16*>(residual); p.ldr = ldr;
+  p.group_offsets = offsets; p.groups = groups;
+  p.status = status;
+  int rc = tma_map_2d_bf16(&p.a_map, A, rows, M, lda, G2_BK);
+  if (rc != 0) return -20 + rc;
+  rc = tma_map_2d_bf16(&p.b_map, B, rows, N, ldb, G2_BK);
+  if (rc != 0) return -30 + rc;
+  rc = tma_map_2d_out(&p.c_map, C, (unsigned long long)groups * M, N, ldc, 0, 32);
+  if (rc != 0) return -40 + rc;
+  return g2_launch<256, true, true, false, G2_GROUPS>(p, groups * ((M + 255) / 256) * ((N + 255) / 256), stream);
 }

@@ -2,7 +2,7 @@
 experts of a layer run as six grouped launches over expert-sorted rows, with no host synchronisation.
 
 The (token, slot) pairs are sorted by expert on the device; every expert's row range is padded with zero rows to a
-multiple of 64, so the weight gradient ``dW_e = dY_e^T X_e`` is one grouped launch whose contraction runs over the
+multiple of 64, so the weight gradient ``dW_e = dY_e^T X_e`` is one grouped launch (csrc/gemm2_sm100.cu) whose contraction runs over the
 expert's row range (a 64-row k-block never straddles two experts). Rows keep the token order inside an expert, so the
 result does not depend on scheduling.
 
@@ -20,7 +20,7 @@ import torch
 from .. import _native
 from . import elementwise as _ew
 from ._util import check_rc, status_tensor, stream_handle
-from .gemm import EPI_STORE, RbGemmArgs, _lib as _gemm_lib
+from .gemm import EPI_STORE, RbGemmArgs, _lib as _gemm_lib, _lib2 as _gemm2_lib
 
 _LIB = None
 _I, _VP = ctypes.c_int, ctypes.c_void_p
@@ -43,7 +43,7 @@ def _lib():
 
 
 MAX_EXPERTS = 256
-FWD_GU, FWD_DN, DGRAD_DN, DGRAD_GU, WGRAD_DN, WGRAD_GU = range(6)
+FWD_GU, FWD_DN, DGRAD_DN, DGRAD_GU = range(4)
 
 
 def _tile_width(n: int) -> int:
@@ -71,23 +71,18 @@ class GroupedPlan:
         st = status_tensor(dev).data_ptr()
         self.counts = torch.zeros(E, dtype=torch.int32, device=dev)
         check_rc(lib.rb_moe_count(idx.data_ptr(), n, E, self.counts.data_ptr(), s), "rb_moe_count")
-        # (mode, output columns per expert, tile width, rows of the stacked B per expert | output rows per expert)
-        self.desc = [(0, 2 * F, _tile_width(2 * F), 2 * F), (0, d, _tile_width(d), d),
-                     (1, F, _tile_width(F), d), (1, d, _tile_width(d), 2 * F),
-                     (2, F, _tile_width(F), d), (2, d, _tile_width(d), 2 * F)]
+        # (mode, output columns per expert, tile width, rows of the stacked B per expert)
+        self.desc = [(0, 2 * F, _tile_width(2 * F), 2 * F), (0, d, _tile_width(d), d), (1, F, _tile_width(F), d), (1, d, _tile_width(d), 2 * F)]
         m_tiles = self.cap // 128 + E
-        sizes = []
-        for mode, n_total, bn, bs in self.desc:
-            nt = -(-n_total // bn)
-            sizes.append((E * -(-bs // 128) if mode == 2 else m_tiles) * nt)
-        self.max_tiles = max(sizes)
-        self.tiles = torch.empty(6, self.max_tiles, 4, dtype=torch.int32, device=dev)
-        self.ntiles = torch.zeros(6, dtype=torch.int32, device=dev)
+        self.max_tiles = max(m_tiles * -(-n_total // bn) for _, n_total, bn, _ in self.desc)
+        tables = len(self.desc)
+        self.tiles = torch.empty(tables, self.max_tiles, 4, dtype=torch.int32, device=dev)
+        self.ntiles = torch.zeros(tables, dtype=torch.int32, device=dev)
         self.offsets = torch.empty(E + 1, dtype=torch.int32, device=dev)
-        flat = (_I * 24)(*[v for dsc in self.desc for v in dsc])
-        tptr = (_VP * 6)(*[self.tiles[i].data_ptr() for i in range(6)])
-        nptr = (_VP * 6)(*[self.ntiles.data_ptr() + 4 * i for i in range(6)])
-        check_rc(lib.rb_moe_train_plan(self.counts.data_ptr(), E, self.offsets.data_ptr(), flat, tptr, nptr, 6, self.max_tiles,
+        flat = (_I * (4 * tables))(*[v for dsc in self.desc for v in dsc])
+        tptr = (_VP * tables)(*[self.tiles[i].data_ptr() for i in range(tables)])
+        nptr = (_VP * tables)(*[self.ntiles.data_ptr() + 4 * i for i in range(tables)])
+        check_rc(lib.rb_moe_train_plan(self.counts.data_ptr(), E, self.offsets.data_ptr(), flat, tptr, nptr, tables, self.max_tiles,
                                        self.cap, st, s), "rb_moe_train_plan")
         self.row_of = torch.empty(n, dtype=torch.int32, device=dev)
         self.src_of = torch.empty(self.cap, dtype=torch.int32, device=dev)
@@ -164,12 +159,14 @@ class GroupedPlan:
         self._launch(which, dy, w, out, M=self.cap, N=n, K=kd, group_n=n, a_mn=False, b_mn=True, group_mode=1, group_b_rows=self.E * kd)
         return out
 
-    def wgrad(self, which: int, dy: torch.Tensor, x: torch.Tensor, gw: torch.Tensor, accumulate: bool) -> None:
+    def wgrad(self, dy: torch.Tensor, x: torch.Tensor, gw: torch.Tensor, accumulate: bool) -> None:
         """``gw_e (+)= dy[rows of e]^T @ x[rows of e]`` for every expert; ``gw`` is ``[E * m, n]``."""
-        n, m = self.desc[which][1], self.desc[which][3]
-        assert dy.shape == (self.cap, m) and x.shape == (self.cap, n) and gw.shape == (self.E * m, n)
-        self._launch(which, dy, x, gw, M=m, N=n, K=self.cap, group_n=n, a_mn=True, b_mn=True, group_mode=2,
-                     residual=gw if accumulate else None)
+        m, n = dy.shape[1], x.shape[1]
+        assert dy.shape[0] == x.shape[0] == self.cap and gw.shape == (self.E * m, n) and gw.stride(1) == 1
+        rc = _gemm2_lib().rb_gemm2_groups(dy.data_ptr(), x.data_ptr(), gw.data_ptr(), gw.data_ptr() if accumulate else None, self.E, m, n, self.cap,
+                                          dy.stride(0), x.stride(0), gw.stride(0), gw.stride(0), self.offsets.data_ptr(),
+                                          status_tensor(self.device).data_ptr(), stream_handle(self.device))
+        check_rc(rc, "rb_gemm2_groups")
 
 
 class GroupedExperts(torch.autograd.Function):
@@ -198,11 +195,11 @@ class GroupedExperts(torch.autograd.Function):
         dwt = plan.dot(dout, y) if ctx.needs_input_grad[1] else None
         dy = plan.gather(dout, wt)
         act = _ew.swiglu(gu)                                  # recomputed: cheaper than keeping [rows, F] alive
-        plan.wgrad(WGRAD_DN, dy, act, ctx.gd, ctx.sink.accumulate_into(ctx.gd))
+        plan.wgrad(dy, act, ctx.gd, ctx.sink.accumulate_into(ctx.gd))
         dact = plan.dgrad(DGRAD_DN, dy, wd)
         del act, dy
         dgu = _ew.swiglu_backward(gu, dact)
-        plan.wgrad(WGRAD_GU, dgu, xs, ctx.ggu, ctx.sink.accumulate_into(ctx.ggu))
+        plan.wgrad(dgu, xs, ctx.ggu, ctx.sink.accumulate_into(ctx.ggu))
         dh = None
         if ctx.needs_input_grad[0]:
             dh = plan.combine(plan.dgrad(DGRAD_GU, dgu, wgu))
