@@ -135,27 +135,44 @@ def _lib_skinny() -> ctypes.CDLL:
     if not getattr(lib, "_rb_typed", False):
         vp, i, ll, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
         lib.rb_skinny.argtypes = [vp] * 5 + [i] * 3 + [ll] * 4 + [i, i, i, f, i, f, f, i, vp, i, ll, i, vp]
-        lib.rb_skinny.restype = i
+        lib.rb_stream.argtypes = lib.rb_skinny.argtypes[:-1] + [vp, vp]
+        lib.rb_skinny.restype = lib.rb_stream.restype = i
         lib._rb_typed = True
     return lib
 
 
 # rows -> most elements of B, for csrc/skinny_sm100.cu
-_SKINNY = ((8, 1 << 62), (16, 120_000_000), (32, 17_000_000))
+_SKINNY = ((8, 1 << 62), (16, 60_000_000))
+# fewest and most rows, most 128-column tiles of the output, for its rb_stream
+_STREAM = (9, 64, 296)
 
 
 def _skinny_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail) -> bool:
-    """Few rows (csrc/skinny_sm100.cu): weights streamed by every warp on its own. Each 8 rows cost it another pass of activations
-    through L1 beside the weights, so past 8 rows the tcgen05 kernel is the better one where the matrix is large enough for its tiles
-    to fill the machine. Microseconds of a chain of captured launches over weights that are not in L2, tcgen05 kernel / this one:
-    2 rows: 896 x 896 8.2 / 2.5, 4096 x 4096 17.5 / 7.5, 28672 x 4096 71 / 46, 151936 x 896 59.5 / 54; 16 rows: 28672 x 4096
-    54.1 / 50.5, 151936 x 896 61.5 / 71.8; 32 rows: 896 x 896 8.2 / 6.1, 4096 x 4096 17.2 / 14.6, 6144 x 4096 21.5 / 23.6. What it
-    does not take (a layout the vector loads need, what the other kernel refuses or leaves unsaid) is left to the other kernel."""
-    if M > 32 or N * K > next(most for rows, most in _SKINNY if M <= rows):
+    """Up to 16 rows (``rb_skinny``): weights streamed by every warp on its own. Each 8 rows cost it another pass of activations through L1 beside
+    the weights, so past 8 rows other kernels are better for large matrices. Microseconds of a chain of captured launches over weights that
+    are not in L2, one-CTA kernel / this one: 2 rows: 896 x 896 8.2 / 2.5, 4096 x 4096 17.5 / 7.5, 28672 x 4096 71 / 46,
+    151936 x 896 59.5 / 54; 16 rows: 896 x 896 8.2 / 4.2, 4096 x 4096 16.7 / 10.0, 151936 x 896 61.5 / 71.8; 28672 x 4096 50.5, rb_stream
+    42.4. What it does not take (a layout the vector loads need, what the one-CTA kernel refuses or leaves unsaid) is left to the others."""
+    if M > _SKINNY[-1][0] or N * K > next(most for rows, most in _SKINNY if M <= rows):
         return False
-    if N % 8 or K % 16 or a.stride(0) % 16 or b.stride(0) % 16 or a.data_ptr() % 32 or b.data_ptr() % 32:
+    return K % 16 == 0 and a.stride(0) % 16 == 0 and b.stride(0) % 16 == 0 and a.data_ptr() % 32 == 0 and b.data_ptr() % 32 == 0 and _few_rows_form(
+        a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail)
+
+
+def _stream_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail) -> bool:
+    """Up to 64 rows (``rb_stream``): weights as the 128-row side of tcgen05, K over clusters. Microseconds as above,
+    one-CTA kernel / this one: 32 rows: 896 x 896 8.2 / 5.6, 4096 x 4096 17.2 / 11.8, 6144 x 4096 21.6 / 16.2, 28672 x 4096 48.8 / 43.2,
+    4096 x 14336 31.0 / 27.7, 2048 x 8192 33.4 / 11.2; 64 rows: 896 x 896 8.1 / 7.0, 4096 x 4096 16.9 / 14.0, 28672 x 4096 49.8 / 46.0; 128 rows:
+    8.1 / 10.1, 17.8 / 18.4, 49.9 / 51.0, which stay where they are, as do outputs of more than two tiles an SM."""
+    if not _STREAM[0] <= M <= _STREAM[1] or -(-N // 128) > _STREAM[2] or K < 64:
         return False
-    if residual is not None and (residual.stride(1) != 1 or residual.dtype != torch.bfloat16):
+    return (K % 8 == 0 and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0
+            and (not swiglu or bn >= 128) and _few_rows_form(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail))
+
+
+def _few_rows_form(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail) -> bool:
+    """The forms of a product whose epilogue both kernels for few rows have."""
+    if N % 8 or (residual is not None and (residual.stride(1) != 1 or residual.dtype != torch.bfloat16)):
         return False
     if bias is not None and (bias.dtype != torch.bfloat16 or not bias.is_contiguous()):
         return False
@@ -425,15 +442,20 @@ def gemm(
     if out is None:
         out = torch.empty(M, N // 2 if swiglu else N - (tail.shape[1] if tail is not None else 0), dtype=torch.float32 if out_f32 else torch.bfloat16, device=a.device)
     assert out.stride(1) == 1
-    if (gather is None and wait_flag is None and not (a_mn_major or b_mn_major) and alpha == 1.0 and beta == 1.0 and max_ctas == 0 and split_k in (0, 1)
-            and not cluster_split and _skinny_takes(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail)):
-        rc = _lib_skinny().rb_skinny(
-            a.data_ptr(), b.data_ptr(), out.data_ptr(), ptr(bias), ptr(residual), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-            residual.stride(0) if residual is not None else 0, int(out_f32), bn // 2 if swiglu else 0, int(glu_limit is not None), glu_limit or 0.0,
-            int(norm_eps is not None), norm_eps or 0.0, softcap, silu_cols, ptr(tail), N - tail.shape[1] if tail is not None else 0,
-            tail.stride(0) if tail is not None else 0, int(constant_b), stream_handle(a.device))
-        check_rc(rc, "rb_skinny")
-        return out
+    if M <= 128 and gather is None and wait_flag is None and not (a_mn_major or b_mn_major) and alpha == 1.0 and beta == 1.0 and max_ctas == 0 \
+            and split_k in (0, 1) and not cluster_split:
+        form = (a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail)
+        skinny, stream = _skinny_takes(*form), _stream_takes(*form)
+        if skinny or stream:
+            call = (a.data_ptr(), b.data_ptr(), out.data_ptr(), ptr(bias), ptr(residual), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                    residual.stride(0) if residual is not None else 0, int(out_f32), bn // 2 if swiglu else 0, int(glu_limit is not None),
+                    glu_limit or 0.0, int(norm_eps is not None), norm_eps or 0.0, softcap, silu_cols, ptr(tail),
+                    N - tail.shape[1] if tail is not None else 0, tail.stride(0) if tail is not None else 0, int(constant_b))
+            if skinny:
+                check_rc(_lib_skinny().rb_skinny(*call, stream_handle(a.device)), "rb_skinny")
+            else:
+                check_rc(_lib_skinny().rb_stream(*call, status_tensor(a.device).data_ptr(), stream_handle(a.device)), "rb_stream")
+            return out
     args = RbGemmArgs()
     args.A[0] = a.data_ptr()
     args.B[0] = b.data_ptr()

@@ -56,7 +56,7 @@ FORMS = {
 
 
 @pytest.mark.parametrize("form", FORMS)
-@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16])
 @pytest.mark.parametrize("N,K", [(8, 16), (72, 48), (136, 1040), (896, 4864), (4096, 64)])
 def test_few_rows(form, M, N, K, monkeypatch):
     kw = dict(FORMS[form])
@@ -87,9 +87,42 @@ def test_few_rows(form, M, N, K, monkeypatch):
     assert ((out.double() - y[:, :n]).abs() <= room[:, :n]).all()
     if tails[0] is not None:
         assert ((tails[0].double() - y[:, n:]).abs() <= (spread + 1e-6)[:, n:]).all()
-    monkeypatch.setattr(gemm_mod, "_SKINNY", ((32, 0),))
+    monkeypatch.setattr(gemm_mod, "_SKINNY", ((16, 0),))
+    monkeypatch.setattr(gemm_mod, "_STREAM", (1, 0, 0))
     other = run(tails[1])
     assert ((out.double() - other.double()).abs() <= 2 * room[:, :n]).all()
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("M", [1, 17, 33, 64, 100, 128])
+@pytest.mark.parametrize("N,K", [(8, 64), (136, 72), (896, 4864), (4096, 264)])
+def test_up_to_128_rows(form, M, N, K, monkeypatch):
+    """``rb_stream``: token counts around its steps of 16, K remainders and cuts, N below and above a tile."""
+    kw = dict(FORMS[form])
+    if kw.get("swiglu"):
+        kw["bn"] = max(kw["bn"], 128)
+        N = -(-N // kw["bn"]) * kw["bn"]
+    if kw.get("tail"):
+        N += 64 - N % 32 + kw["tail"]
+    gen = torch.Generator(device="cuda").manual_seed(M * 1000 + N + K)
+    a, b = _strided(M, K, 8, gen), _strided(N, K, 24, gen, K ** -0.5)
+    if kw.pop("bias", False):
+        kw["bias"] = torch.randn(N, device="cuda", generator=gen).bfloat16()
+    if kw.pop("residual", False):
+        kw["residual"] = _strided(M, N, 8, gen)
+    tail = torch.empty(M, kw["tail"] + 8, device="cuda")[:, :kw["tail"]] if kw.get("tail") else None
+    monkeypatch.setattr(gemm_mod, "_SKINNY", ((16, 0),))
+    monkeypatch.setattr(gemm_mod, "_STREAM", (1, 128, 296))
+    assert gemm_mod._stream_takes(a, b, kw.get("bias"), kw.get("residual"), M, N, K, kw.get("bn", 0), kw.get("swiglu", False),
+                                  kw.get("out_f32", False), kw.get("softcap", 0.0), kw.get("silu_cols", 0), tail)
+    out = ops.gemm(a, b, tail=tail, **{k: v for k, v in kw.items() if k != "tail"})
+    y, spread = _reference(a, b, **{k: v for k, v in kw.items() if k != "tail"})
+    n = N - kw["tail"] if kw.get("tail") else y.shape[1]
+    room = spread + (0.0 if kw.get("out_f32") else 2.0 ** -8) * y.abs() + 1e-6 * (1 + y.abs())
+    assert ((out.double() - y[:, :n]).abs() <= room[:, :n]).all()
+    if tail is not None:
+        assert ((tail.double() - y[:, n:]).abs() <= (spread + 1e-6)[:, n:]).all()
+    ops.check_status(torch.device("cuda"))
 
 
 def test_few_rows_under_capture_with_constant_weights():
