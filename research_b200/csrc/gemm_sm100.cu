@@ -27,11 +27,11 @@
 // write the result (all-reduce: to every peer). This is the GEMM -> reduce-scatter path.
 #include "common.cuh"
 #include "gemm_epilogue.cuh"
+#include "tma_host.h"
 #include "gemm_sm100.h"
 
 #include <stdlib.h>
 
-#include <mutex>
 #include <stdio.h>
 
 namespace rb {
@@ -1136,42 +1136,6 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
 }
 
 // ---------------------------------- host side ------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess) {
-      fn = reinterpret_cast<EncodeTiledFn>(f);
-    }
-  });
-  return fn;
-}
-
-// 2-D bf16 tensor map over `rows` x `cols` (cols contiguous, leading dimension ld elements),
-// box = box_rows x 64 columns, 128-byte swizzle.
-static int make_map_2d(CUtensorMap* out, const void* base, long long rows, long long cols,
-                       long long ld, int box_rows) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (fn == nullptr) return -1;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (ld * 2) % 16 != 0) return -2;
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box,
-                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : -3;
-}
-
 static int num_sms() {
   static int n = 0;
   if (n == 0) {
@@ -1438,14 +1402,14 @@ extern "C" int rb_gemm_bf16_ex(const RbGemmArgs* a, cudaStream_t stream) {
   // tensor maps: one per slab
   for (int i = 0; i < p.a_parts; ++i) {
     int rc = a->a_mn_major
-                 ? make_map_2d(&p.a_map[i], a->A[i], a->K, p.a_rows_per_part, a->lda, BK)
-                 : make_map_2d(&p.a_map[i], a->A[i], p.a_rows_per_part, a->K, a->lda, BM);
+                 ? tma_map_2d_bf16(&p.a_map[i], a->A[i], a->K, p.a_rows_per_part, a->lda, BK)
+                 : tma_map_2d_bf16(&p.a_map[i], a->A[i], p.a_rows_per_part, a->K, a->lda, BM);
     if (rc != 0) return -20 + rc;
   }
   for (int i = 0; i < p.b_parts; ++i) {
     int rc = a->b_mn_major
-                 ? make_map_2d(&p.b_map[i], a->B[i], a->group_mode == 1 ? a->group_b_rows : a->K, total_b_rows, a->ldb, BK)
-                 : make_map_2d(&p.b_map[i], a->B[i], total_b_rows, a->K, a->ldb, bn);
+                 ? tma_map_2d_bf16(&p.b_map[i], a->B[i], a->group_mode == 1 ? a->group_b_rows : a->K, total_b_rows, a->ldb, BK)
+                 : tma_map_2d_bf16(&p.b_map[i], a->B[i], total_b_rows, a->K, a->ldb, bn);
     if (rc != 0) return -30 + rc;
   }
   switch (bn) {

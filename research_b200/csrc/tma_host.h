@@ -25,6 +25,19 @@ inline EncodeTiledFnT tma_encode_fn() {
   return fn;
 }
 
+// The encoder needs the device's context to be current in the calling thread, which a thread that has made no runtime call of its own
+// yet does not have (autograd's, whose allocations may all come from the cache): selecting the thread's device makes it so.
+inline CUresult tma_encode_2d(EncodeTiledFnT fn, CUtensorMap* out, CUtensorMapDataType type, void* base, const cuuint64_t* dims,
+                              const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapL2promotion promotion) {
+  const cuuint32_t estr[2] = {1, 1};
+  for (int attempt = 0;; ++attempt) {
+    const CUresult r = fn(out, type, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, promotion,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    int device = 0;
+    if (r == CUDA_SUCCESS || attempt > 0 || cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return r;
+  }
+}
+
 // rows x cols matrix, cols contiguous, leading dimension ld (elements); box = box_rows x 64 columns.
 inline int tma_map_2d_bf16(CUtensorMap* out, const void* base, unsigned long long rows, unsigned long long cols,
                            unsigned long long ld, unsigned box_rows) {
@@ -34,10 +47,8 @@ inline int tma_map_2d_bf16(CUtensorMap* out, const void* base, unsigned long lon
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld * 2};
   cuuint32_t box[2] = {64, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = tma_encode_2d(fn, out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, const_cast<void*>(base), dims, strides, box,
+                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
@@ -51,10 +62,8 @@ inline int tma_map_2d_out(CUtensorMap* out, void* base, unsigned long long rows,
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld * es};
   cuuint32_t box[2] = {128 / es, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = tma_encode_2d(fn, out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, dims, strides, box,
+                                   CU_TENSOR_MAP_L2_PROMOTION_NONE);
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 

@@ -263,3 +263,26 @@ def test_flash_backward_tile_edges(D, H, Hkv, causal, window):
             assert ((x[lo:lo + n].double() - w).abs() <= m + u * w.abs() + 1e-5).all()
         at_q, at_k = at_q + nq, at_k + nk
     ops.check_status(torch.device("cuda"))
+
+
+def test_flash_in_a_thread_without_context(cuda_device):
+    """A thread whose first CUDA call is the kernel's (autograd's may be one: its memory can all come from the cache)."""
+    import threading
+
+    q, k, v, do = (torch.randn(183, h, 128, device=cuda_device).bfloat16() for h in (4, 2, 2, 4))
+    cu = torch.tensor([0, 183], dtype=torch.int32, device=cuda_device)
+    out, lse = flash.flash_attn_varlen(q, k, v, cu, cu, 183, return_lse=True)
+    want = flash.flash_attn_varlen_backward(q, k, v, out, do, lse, cu, cu, 183, 183)
+    del want
+    got = []
+
+    def work():
+        try:
+            got.append(flash.flash_attn_varlen_backward(q, k, v, out, do, lse, cu, cu, 183, 183))
+        except RuntimeError as e:
+            got.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert isinstance(got[0], tuple), got[0]

@@ -125,12 +125,13 @@ def test_up_to_128_rows(form, M, N, K, monkeypatch):
     ops.check_status(torch.device("cuda"))
 
 
-def test_few_rows_under_capture_with_constant_weights():
+@pytest.mark.parametrize("M", [4, 40])
+def test_few_rows_under_capture_with_constant_weights(M):
     """First loads of the weights before the launch dependency is waited for: a chain in which every product reads the one before."""
     gen = torch.Generator(device="cuda").manual_seed(1)
     ws = [(torch.randn(512, 512, device="cuda", generator=gen) / 512 ** 0.5).bfloat16() for _ in range(6)]
-    x = torch.randn(4, 512, device="cuda", generator=gen).bfloat16()
-    bufs = [torch.empty(4, 512, device="cuda", dtype=torch.bfloat16) for _ in ws]
+    x = torch.randn(M, 512, device="cuda", generator=gen).bfloat16()
+    bufs = [torch.empty(M, 512, device="cuda", dtype=torch.bfloat16) for _ in ws]
 
     def body():
         h = x
