@@ -377,7 +377,9 @@ __device__ __forceinline__ bool wait_flag_ge(const int* p, int want, int* status
 #ifdef __CUDACC__
 #include <utility>
 namespace rb {
-inline bool& pdl_enabled() {
+// The switch of one library. Hidden: the static of an inline function is otherwise one object for all libraries of a process,
+// and turning it on for one would give the attribute to kernels of others that never wait for the launch before them.
+__attribute__((visibility("hidden"))) inline bool& pdl_enabled() {
   static bool on = false;
   return on;
 }

@@ -129,6 +129,8 @@ static int launch_gemv(const void* a, const void* b, const void* sfa, const void
 
 extern "C" {
 
+void rb_quant_set_pdl(int on) { rb::pdl_enabled() = on != 0; }
+
 // a [L, M, K/2], b [L, K/2], sfa [L, M, K/16], sfb [L, K/16] bytes; c [L, M] fp16. K % 32 == 0.
 int rb_nvfp4_gemv(const void* a, const void* b, const void* sfa, const void* sfb, void* c, int L, int M, int K,
                   cudaStream_t stream) {

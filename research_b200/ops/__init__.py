@@ -67,12 +67,13 @@ from .sampling import sample_with_logprobs, sample_with_logprobs_reference, toke
 
 def set_pdl(on: bool) -> None:
     """Enable programmatic dependent launch for the decode-path kernels (GEMM, norms, RoPE,
-    attention, SwiGLU, embedding, sampling): consecutive kernels overlap prologue and tail."""
+    attention, SwiGLU, embedding, sampling): consecutive kernels overlap prologue and tail. The libraries not listed
+    (two-CTA GEMM, flash attention, training, collectives) have kernels that do not wait for the launch before them."""
     from .. import _native
 
     for lib, fn in (("rb_gemm", "rb_gemm_set_pdl"), ("rb_skinny", "rb_skinny_set_pdl"), ("rb_ops", "rb_ops_set_pdl"), ("rb_attn", "rb_attn_set_pdl"),
                     ("rb_latent", "rb_latent_set_pdl"), ("rb_gemm_f32", "rb_gemm_f32_set_pdl"),
-                    ("rb_recurrent", "rb_recurrent_set_pdl"), ("rb_moe", "rb_moe_set_pdl")):
+                    ("rb_recurrent", "rb_recurrent_set_pdl"), ("rb_moe", "rb_moe_set_pdl"), ("rb_quant", "rb_quant_set_pdl")):
         if _native.available(lib):      # a partial build has only the libraries its models need
             getattr(_native.load(lib), fn)(int(on))
 
