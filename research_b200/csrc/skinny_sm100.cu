@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
   const uint32_t tmem_base = tmem_base_smem;
   volatile int* abortp = &abort_flag;
   pdl_launch_dependents();
+  int issued = 0;      // stages filled by this thread (the elected one of warp 0)
 
   if (warp == 0) {
     if (elect_one_sync()) {
@@ -369,18 +370,13 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
         load_w(i);
         load_x(i);
       }
-      if (i < n_kb) {      // given up: no copy may land in memory that has another use
-        for (int j = i > sp.stages ? i - sp.stages : 0; j < i; ++j) {
-          const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(smem_u32(&full[j % sp.stages]), (j / sp.stages) & 1u))
-            if (globaltimer_ns() - t0 > 50000000ull) break;
-        }
-      }
+      issued = i;
     }
   } else if (warp == 1) {
     if (elect_one_sync()) {
       const uint32_t idesc = make_idesc_bf16(ST_ROWS, T, 0, 0);
       bool ok = true;
+      pdl_wait();      // no stage is full before: the budget of the first wait is not spent on the kernel before this one
       for (int i = 0; i < n_kb; ++i) {
         const int s = i % sp.stages;
         ok = mbar_wait_bounded(smem_u32(&full[s]), (i / sp.stages) & 1u, abortp, status, ST_TIMEOUT_SMEM_FULL);
@@ -392,7 +388,8 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
           umma_bf16(tmem_base, make_smem_desc_sw128(w_s + k * 32, 16, 1024), make_smem_desc_sw128(x_s + k * 32, 16, 1024), idesc, (i > 0 || k > 0) ? 1u : 0u);
         umma_commit(smem_u32(&empty[s]));
       }
-      umma_commit(smem_u32(&acc_full));      // (a wait that ran out is seen by its flag)
+      __threadfence_block();
+      umma_commit(smem_u32(&acc_full));      // a wait that ran out has set the flag before
     }
   } else {
     const int tid = threadIdx.x - 64, q = warp & 3;
@@ -422,7 +419,8 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
       }
       ssq[tid] = sum;
     }
-    const bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&acc_full), 0, abortp, status, ST_TIMEOUT_TMEM_FULL));
+    bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&acc_full), 0, abortp, status, ST_TIMEOUT_TMEM_FULL));
+    if (__any_sync(0xffffffffu, *abortp != 0)) ok = false;       // copies may still land in the ring
     // every warp has left the ring before one of them writes over it
     asm volatile("bar.sync 1, 128;" ::: "memory");
     if (ok) {
@@ -438,6 +436,15 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
     }
   }
   __syncthreads();
+  if (*abortp != 0 && issued > 0) {      // given up: no copy may land in memory, no product read memory that has another use
+    auto drain = [&](uint64_t* bar, uint32_t parity) {
+      const uint64_t t0 = globaltimer_ns();
+      while (!mbar_try_wait(smem_u32(bar), parity))
+        if (globaltimer_ns() - t0 > 50000000ull) break;
+    };
+    for (int j = max(issued - sp.stages, 0); j < issued; ++j) drain(&full[j % sp.stages], (j / sp.stages) & 1u);
+    drain(&acc_full, 0);
+  }
   if (S > 1) cluster_sync_all();
   if (warp == 0) pdl_wait();
   if (p.norm_fold) {

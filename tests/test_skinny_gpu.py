@@ -152,3 +152,29 @@ def test_few_rows_under_capture_with_constant_weights(M):
             o.zero_()
         graph.replay()
         assert torch.equal(bufs[-1], want)
+
+
+def test_waits_do_not_count_the_kernels_before():
+    """Two products whose own bounded wait runs out (a flag that nothing sets) hold the stream for longer than the budget of one wait. The
+    product behind them, which has started under them, still computes: its waits begin where theirs end."""
+    from research_b200.ops._util import KernelStatusError
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    a, slow_w = torch.randn(64, 128, device="cuda", generator=gen).bfloat16(), torch.randn(256, 128, device="cuda", generator=gen).bfloat16()
+    x, w = torch.randn(32, 896, device="cuda", generator=gen).bfloat16(), torch.randn(896, 896, device="cuda", generator=gen).bfloat16()
+    assert gemm_mod._stream_takes(x, w, None, None, 32, 896, 896, 0, False, False, 0.0, 0, None)
+    want = ops.gemm(x, w)
+    got, slow = torch.zeros_like(want), [torch.zeros(64, 256, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    flag = torch.tensor([0, 1], dtype=torch.int32, device="cuda")      # [0] the flag, [1] what it would have to reach
+    torch.cuda.synchronize()
+    ops.set_pdl(True)
+    try:
+        for o in slow:
+            ops.gemm(a, slow_w, out=o, split_k=1, wait_flag=(flag.data_ptr(), flag.data_ptr() + 4))
+        ops.gemm(x, w, out=got, constant_b=True)
+    finally:
+        ops.set_pdl(False)
+    with pytest.raises(KernelStatusError):
+        ops.check_status(torch.device("cuda"))
+    assert torch.equal(got, want)
+    ops.check_status(torch.device("cuda"))
