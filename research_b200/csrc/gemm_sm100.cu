@@ -250,16 +250,13 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  pdl_launch_dependents();  // the next kernel may begin its own prologue now
 
   const int m_tiles_per_part = (p.a_rows_per_part + BM - 1) / BM;
   const int n_tiles_per_part = (p.b_rows_per_part + BN - 1) / BN;
   const int num_m_tiles = m_tiles_per_part * p.a_parts;
   const int num_n_tiles = n_tiles_per_part * p.b_parts;
   const bool grouped = p.tile_table != nullptr;
-  if (grouped) pdl_wait();  // the tile count itself is produced by the previous kernel
   const int split_k = p.split_k;
-  const int num_tiles = (grouped ? *p.num_tiles_ptr : num_m_tiles * num_n_tiles) * split_k;  // work units
   const int num_kb = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -287,8 +284,12 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // The next kernel may begin its own prologue now, and not before this CTA has its tensor memory: a kernel that took columns first and
+  // then waits for this one would never give them back.
+  pdl_launch_dependents();
   if (p.cluster_k) cluster_sync_all();   // no peer may signal a barrier that is not initialised yet
   pdl_wait();  // barriers and TMEM are set up; from here on we read what the previous kernel wrote
+  const int num_tiles = (grouped ? *p.num_tiles_ptr : num_m_tiles * num_n_tiles) * split_k;  // work units (grouped: counted by the previous kernel)
   RB_TS(0);
   const uint32_t tmem_base = tmem_base_smem;
   volatile int* abortp = &abort_flag;

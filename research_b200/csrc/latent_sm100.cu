@@ -278,12 +278,24 @@ __global__ void __launch_bounds__(LAT_THREADS, 1) latent_attn_kernel(const __gri
   __shared__ int abort_flag, u_shared;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nch = (p.CW + 63) / 64, nblk = (p.RW + 127) / 128, tile_bytes = max(nch, 2 * nblk) * CHUNK;
+  // before the next kernel may start: one that took columns first and then waits for this one would never give them back
+  const uint32_t tmem_cols = O_COL + (nblk * NH + 31) / 32 * 32 <= 256 ? 256 : 512;
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&tmem_base_smem), tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
   pdl_launch_dependents();
   pdl_wait();
   const int units = p.B * p.row_tiles, total = p.plan[units];
   const int share = latent_share(total, gridDim.x);
   const int t_begin = min((int)blockIdx.x * share, total), t_end = min(t_begin + share, total);
-  if (t_begin >= t_end) return;                  // uniform per CTA, before any set-up
+  if (t_begin >= t_end) {                        // uniform per CTA
+    if (warp == 1) tmem_dealloc(tmem_base_smem, tmem_cols);
+    return;
+  }
   const int u_first = latent_find_cta(p.plan, units, t_begin, &u_shared);
 
   const uint32_t q_s = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -307,14 +319,7 @@ __global__ void __launch_bounds__(LAT_THREADS, 1) latent_attn_kernel(const __gri
     mbar_init(smem_u32(&o_free), 4);
     fence_mbar_init();
   }
-  const uint32_t tmem_cols = O_COL + (nblk * NH + 31) / 32 * 32 <= 256 ? 256 : 512;
-  if (warp == 1) {
-    tmem_alloc(smem_u32(&tmem_base_smem), tmem_cols);
-    tmem_relinquish();
-  }
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
   const uint32_t tmem_base = tmem_base_smem, tmem_o = tmem_base + O_COL;
   volatile int* abortp = &abort_flag;
 

@@ -18,6 +18,18 @@ def test_every_library_has_a_switch_of_its_own():
             ctypes.c_bool.in_dll(_native.load(name), "_ZZN2rb11pdl_enabledEvE2on")
 
 
+def test_tensor_memory_is_taken_before_dependents_start():
+    """A kernel that releases its dependents first can find its columns taken by one that then waits for it. (Read from the sources: the hang
+    itself would need the GPU.)"""
+    found = 0
+    for path in sorted([*_native.SRC_DIR.glob("*.cu"), *_native.SRC_DIR.glob("*.cuh")]):
+        for body in path.read_text().split("__global__")[1:]:
+            if "tmem_alloc(" in body and "pdl_launch_dependents()" in body:
+                assert body.index("tmem_alloc(") < body.index("pdl_launch_dependents()"), (path.name, body[:80])
+                found += 1
+    assert found >= 8
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("M", [512, 1024])
 def test_two_cta_products_in_a_captured_chain(M):
