@@ -381,6 +381,7 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
         }
         const int ncols = min(32, n_store - c0);
         const int col = (EPI == G2_GLU ? nt * (BN / 2) : n_base) + c0;
+        const bool tail = EPI == G2_STORE && p.tail != nullptr && col >= p.tail_col;
         if constexpr (EPI == G2_DLOGITS) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = dlogit_epi(v[j], l, glp, gent, H, c0 + j == target);
@@ -412,12 +413,11 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
               }
             }
           }
-          if (col < p.silu_cols) {
+          if (col < p.silu_cols && !tail) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = silu_fast(v[j]);
           }
         }
-        const bool tail = EPI == G2_STORE && p.tail != nullptr && col >= p.tail_col;
         const bool second = !f32 && (c0 & 32);
         if (tail) {
           if (row_ok) {

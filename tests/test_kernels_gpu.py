@@ -524,3 +524,27 @@ def test_gated_unit_on_the_pair_kernel(cuda_device, M, N, K, limit):
     want = ops.gemm(a, b, bn=256, swiglu=True, glu_limit=limit, max_ctas=148)
     assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs() + 1e-6).all()
     assert (out[:, N // 2:] == 7.0).all()
+
+
+@pytest.mark.parametrize("n,silu", [(4864, 0), (4896, 64), (4896, 1 << 13), (5152, 4896)])
+@pytest.mark.parametrize("M", [512, 1001])
+def test_tail_behind_whole_and_half_boxes_of_the_pair_kernel(cuda_device, M, n, silu):
+    """The bf16 columns end in the middle of a 64-column box or with one; ``silu_cols`` never reaches the tail; nothing is written past either."""
+    K, t, N = 264, 40, n + 40
+    g = torch.Generator(device=cuda_device).manual_seed(M + n)
+    a = torch.randn(M, K, device=cuda_device, generator=g).bfloat16()
+    b = (torch.randn(N, K, device=cuda_device, generator=g) * K ** -0.5).bfloat16()
+    out = torch.full((M, n + 16), 7.0, device=cuda_device, dtype=torch.bfloat16)
+    tail = torch.full((M, t + 8), 7.0, device=cuda_device)
+    assert ops.gemm_mod._use_pair_kernel(M, N, K, False, False)
+    ops.gemm(a, b, out=out[:, :n], tail=tail[:, :t], silu_cols=silu)
+    y = a.double() @ b.double().T
+    room = (a.double().abs() @ b.double().abs().T) * 2 * K * 2.0 ** -24          # fp32 sums in the worst order
+    assert ((tail[:, :t].double() - y[:, n:]).abs() <= room[:, n:]).all()
+    y = y[:, :n]
+    c = min(silu, n)
+    y[:, :c] = torch.nn.functional.silu(y[:, :c])
+    # one rounding to bf16 (2^-9, doubled for its half unit at a power of two), silu at most 1.1 times its argument's error
+    assert ((out[:, :n].double() - y).abs() <= 1.1 * room[:, :n] + 2.0 ** -8 * y.abs() + 1e-6).all()
+    assert (out[:, n:] == 7.0).all() and (tail[:, t:] == 7.0).all()
+    ops.check_status(cuda_device)
