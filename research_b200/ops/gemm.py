@@ -172,7 +172,7 @@ def _stream_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu:
 
 def _few_rows_form(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail) -> bool:
     """The forms of a product whose epilogue both kernels for few rows have."""
-    if N % 8 or (residual is not None and (residual.stride(1) != 1 or residual.dtype != torch.bfloat16)):
+    if N % 8 or (residual is not None and (residual.dim() != 2 or residual.stride(1) != 1 or residual.dtype != torch.bfloat16)):
         return False
     if bias is not None and (bias.dtype != torch.bfloat16 or not bias.is_contiguous()):
         return False

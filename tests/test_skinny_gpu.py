@@ -5,7 +5,6 @@ import torch
 
 from research_b200 import ops
 
-pytestmark = pytest.mark.gpu
 gemm_mod = ops.gemm_mod
 
 
@@ -55,6 +54,15 @@ FORMS = {
 }
 
 
+@pytest.mark.parametrize("K", [64, 896])
+def test_a_row_as_residual_is_left_to_the_general_path(K):
+    """The general path takes the residual of a single row as a vector."""
+    a, b = torch.zeros(1, K, dtype=torch.bfloat16), torch.zeros(128, K, dtype=torch.bfloat16)
+    for residual, taken in ((torch.zeros(128, dtype=torch.bfloat16), False), (torch.zeros(1, 128, dtype=torch.bfloat16), True)):
+        assert gemm_mod._few_rows_form(a, b, None, residual, 1, 128, K, 0, False, False, 0.0, 0, None) == taken
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("M", [1, 7, 8, 9, 16])
 @pytest.mark.parametrize("N,K", [(8, 16), (72, 48), (136, 1040), (896, 4864), (4096, 64)])
@@ -93,6 +101,7 @@ def test_few_rows(form, M, N, K, monkeypatch):
     assert ((out.double() - other.double()).abs() <= 2 * room[:, :n]).all()
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("M", [1, 17, 33, 64, 100, 128])
 @pytest.mark.parametrize("N,K", [(8, 64), (136, 72), (896, 4864), (4096, 264)])
@@ -125,6 +134,7 @@ def test_up_to_128_rows(form, M, N, K, monkeypatch):
     ops.check_status(torch.device("cuda"))
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("M", [4, 40])
 def test_few_rows_under_capture_with_constant_weights(M):
     """First loads of the weights before the launch dependency is waited for: a chain in which every product reads the one before."""
@@ -154,6 +164,7 @@ def test_few_rows_under_capture_with_constant_weights(M):
         assert torch.equal(bufs[-1], want)
 
 
+@pytest.mark.gpu
 def test_waits_do_not_count_the_kernels_before():
     """Two products whose own bounded wait runs out (a flag that nothing sets) hold the stream for longer than the budget of one wait. The
     product behind them, which has started under them, still computes: its waits begin where theirs end."""
