@@ -14,6 +14,8 @@
 #include "common.cuh"
 #include "gemm_epilogue.cuh"
 
+#include <type_traits>
+
 namespace rb {
 
 constexpr int ROW_THREADS = 512;
@@ -61,23 +63,29 @@ logprob_entropy_fwd_kernel(const float* __restrict__ logits, long long ld, int V
                            float* __restrict__ logprob, float* __restrict__ lse_out, float* __restrict__ entropy) {
   const long long row = blockIdx.x;
   const float* x = logits + row * ld;
-  // Eight loads in flight; a value that is no new maximum costs one exponential (the other factor of the merge is exactly 1).
-  // 2048 x 151936: 293 us with a merge and a load at a time, 261 us.
+  // Eight loads in flight, and one exponential a value without a branch: of the two factors of a merge the one of the larger maximum
+  // is exactly 1.
   Lse v = {-INFINITY, 0.f};
   auto take = [&](float y) {
-    if (y <= v.m && v.m != -INFINITY) v.s += __expf(y - v.m);
-    else v = lse_merge(v, {y, 1.f});
+    const float m = fmaxf(v.m, y);
+    const float e = m == -INFINITY ? 0.f : __expf((y - m) + (v.m - m));     // one of the differences is 0, or neither is finite
+    v.s = y > v.m ? fmaf(v.s, e, 1.f) : v.s + e;
+    v.m = m;
   };
-  constexpr int U = 8;
   int at = threadIdx.x;
-  for (; at + (U - 1) * ROW_THREADS < V; at += U * ROW_THREADS) {
-    float y[U];
+  auto rounds = [&](auto count) {
+    constexpr int U = decltype(count)::value;
+    for (; at + (U - 1) * ROW_THREADS < V; at += U * ROW_THREADS) {
+      float y[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) y[u] = x[at + u * ROW_THREADS];
+      for (int u = 0; u < U; ++u) y[u] = x[at + u * ROW_THREADS];
 #pragma unroll
-    for (int u = 0; u < U; ++u) take(y[u]);
-  }
-  for (; at < V; at += ROW_THREADS) take(x[at]);
+      for (int u = 0; u < U; ++u) take(y[u]);
+    }
+  };
+  rounds(std::integral_constant<int, 8>{});
+  rounds(std::integral_constant<int, 3>{});
+  rounds(std::integral_constant<int, 1>{});
   v = block_lse(v);
   const float lse = v.m + __logf(v.s);
   float ent = 0.f;
