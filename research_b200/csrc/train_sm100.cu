@@ -64,7 +64,8 @@ logprob_entropy_fwd_kernel(const float* __restrict__ logits, long long ld, int V
   const long long row = blockIdx.x;
   const float* x = logits + row * ld;
   // Eight loads in flight, and one exponential a value without a branch: of the two factors of a merge the one of the larger maximum
-  // is exactly 1.
+  // is exactly 1. 2048 x 151936: 289 us with a merge and a load at a time, 218; 2048 x 32000 74 / 59, 100 x 151936 28 / 26 (a branch in place of the
+  // select: 240, 80, 32).
   Lse v = {-INFINITY, 0.f};
   auto take = [&](float y) {
     const float m = fmaxf(v.m, y);
