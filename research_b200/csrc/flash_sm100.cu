@@ -55,10 +55,7 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint32_t bar, uint32_t parity
 }
 __device__ __forceinline__ bool mbar_wait_backoff(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
                                                   int code) {
-  // the timer is read only once the wait has become a long one: its read takes long enough to miss the flip by
-#pragma unroll 1
-  for (int i = 0; i < 16; ++i)
-    if (mbar_try_wait_hint(bar, parity, 2000u)) return true;
+  if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
   uint32_t spins = 0;
   while (true) {
