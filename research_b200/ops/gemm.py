@@ -141,33 +141,65 @@ def _lib_skinny() -> ctypes.CDLL:
     return lib
 
 
-# rows -> most elements of B, for csrc/skinny_sm100.cu
-_SKINNY = ((8, 1 << 62), (16, 60_000_000))
-# fewest and most rows, most 128-column tiles of the output, for its rb_stream
-_STREAM = (9, 64, 296)
+def _skinny_pays(M: int, N: int, K: int, swiglu: bool) -> bool:
+    """Up to 16 rows (``rb_skinny``): weights streamed by every warp on its own. Microseconds of a chain of captured launches over weights
+    that are not in L2, one-CTA kernel / this one: 2 rows: 896 x 896 8.2 / 2.5, 4096 x 4096 17.5 / 7.5, 28672 x 4096 71 / 46, 151936 x 896
+    59.5 / 54; 16 rows: 896 x 896 8.2 / 4.2, 4096 x 4096 16.7 / 10.0. Each 8 rows cost it another pass of activations through L1 beside
+    the weights: 8 rows with 151936 x 896 are 54 / 60, 16 rows 61.5 / 71.8, and 16 rows with 28672 x 4096 50.5 / 55 (rb_stream 42.4). With
+    one or two 64-column blocks of K the partial sums are what takes the time past 8 rows (2048 x 128 with residual, 16 rows: 1.24 times
+    the one-CTA kernel); the one-CTA kernel's gated unit is so much slower there that this one stays better."""
+    if M <= 6:
+        return True
+    if M <= 8:
+        return N <= 1 << 17
+    return M <= 16 and N * K <= 60_000_000 and (K >= 256 or swiglu)
 
 
-def _skinny_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail) -> bool:
-    """Up to 16 rows (``rb_skinny``): weights streamed by every warp on its own. Each 8 rows cost it another pass of activations through L1 beside
-    the weights, so past 8 rows other kernels are better for large matrices. Microseconds of a chain of captured launches over weights that
-    are not in L2, one-CTA kernel / this one: 2 rows: 896 x 896 8.2 / 2.5, 4096 x 4096 17.5 / 7.5, 28672 x 4096 71 / 46,
-    151936 x 896 59.5 / 54; 16 rows: 896 x 896 8.2 / 4.2, 4096 x 4096 16.7 / 10.0, 151936 x 896 61.5 / 71.8; 28672 x 4096 50.5, rb_stream
-    42.4. What it does not take (a layout the vector loads need, what the one-CTA kernel refuses or leaves unsaid) is left to the others."""
-    if M > _SKINNY[-1][0] or N * K > next(most for rows, most in _SKINNY if M <= rows):
-        return False
-    return K % 16 == 0 and a.stride(0) % 16 == 0 and b.stride(0) % 16 == 0 and a.data_ptr() % 32 == 0 and b.data_ptr() % 32 == 0 and _few_rows_form(
-        a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail)
+def _stream_most_rows(N: int, K: int, swiglu: bool, norm: bool) -> int:
+    """Most rows for ``rb_stream`` (weights as the 128-row side of tcgen05, K over clusters), of 9 to 64. Time by the one-CTA kernel's
+    in brackets, plain products unless said:
+    * outputs of more than two tiles of 128 columns an SM, or less than one block of K: never.
+    * gated units always (0.2-0.95; 64 rows with 28672 x 4096 0.95, 9728 x 896 with a norm 0.86).
+    * K below 256: 12 rows (2048 x 128: 12 rows 0.94, 24 1.16, 64 1.94), below 512 16 (2048 x 256: 16 rows 0.97, 24 1.09, 64 1.52): a CTA's
+      partial tile costs more than its few blocks of weights. Two CTAs an SM cover that better: 48 rows (32768 x 256 0.96, 64 rows 1.10).
+    * K below 896: 40 rows for a few tiles (64 x 512 0.95, 48 rows 1.05), 32 (8192 x 512 0.89, 40 rows 1.02 eager), past 64 tiles 24 (16384 x 512
+      0.82-0.93, 32 rows 1.01).
+    * 75 to 148 tiles leave one CTA an SM with all of K, half the loads in flight: 24 rows (9728 x 2048 0.89, 32 rows 1.11; 16384 x 2048 0.80 and 1.07),
+      with a folded norm below 100 tiles 16 (9728 x 2048 24 rows 1.05). 49 to 74 tiles: 40 (8192 x 2048 0.98, 48 rows 1.03).
+    * more than 148 tiles: 48 (28672 x 4096 1.00, 64 rows 1.02-1.05; 37888 x 1024 0.94 and 1.07).
+    * the rest up to 64 (4096 x 4096 0.86, 6144 x 4096 0.88, 896 x 4864 0.79), 56 where K is short (3072 x 1024 0.84, 64 rows 1.01)."""
+    tiles, blocks = -(-N // 128), -(-K // 64)
+    if tiles > 296 or K < 64:
+        return 0
+    if swiglu:
+        return 64
+    if blocks < 4:
+        return 12
+    if tiles > 148:
+        return 48
+    if blocks < 8:
+        return 16
+    if blocks < 14:
+        return 40 if tiles <= 32 else 32 if tiles <= 64 else 24
+    if tiles > 74:
+        return 16 if norm and tiles < 100 else 24
+    if tiles > 48:
+        return 40
+    return 56 if tiles > 16 and blocks < 32 else 64
 
 
-def _stream_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail) -> bool:
-    """Up to 64 rows (``rb_stream``): weights as the 128-row side of tcgen05, K over clusters. Microseconds as above,
-    one-CTA kernel / this one: 32 rows: 896 x 896 8.2 / 5.6, 4096 x 4096 17.2 / 11.8, 6144 x 4096 21.6 / 16.2, 28672 x 4096 48.8 / 43.2,
-    4096 x 14336 31.0 / 27.7, 2048 x 8192 33.4 / 11.2; 64 rows: 896 x 896 8.1 / 7.0, 4096 x 4096 16.9 / 14.0, 28672 x 4096 49.8 / 46.0; 128 rows:
-    8.1 / 10.1, 17.8 / 18.4, 49.9 / 51.0, which stay where they are, as do outputs of more than two tiles an SM."""
-    if not _STREAM[0] <= M <= _STREAM[1] or -(-N // 128) > _STREAM[2] or K < 64:
-        return False
-    return (K % 8 == 0 and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0
-            and (not swiglu or bn >= 128) and _few_rows_form(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail))
+def _skinny_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail,
+                  norm: bool = False) -> bool:
+    """What it does not take (a layout the vector loads need, what the one-CTA kernel refuses or leaves unsaid) is left to the others."""
+    return (_skinny_pays(M, N, K, swiglu) and K % 16 == 0 and a.stride(0) % 16 == 0 and b.stride(0) % 16 == 0 and a.data_ptr() % 32 == 0
+            and b.data_ptr() % 32 == 0 and _few_rows_form(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail))
+
+
+def _stream_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail,
+                  norm: bool = False) -> bool:
+    return (9 <= M <= _stream_most_rows(N, K, swiglu, norm) and K % 8 == 0 and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0
+            and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and (not swiglu or bn >= 128)
+            and _few_rows_form(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail))
 
 
 def _few_rows_form(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail) -> bool:
@@ -444,7 +476,7 @@ def gemm(
     assert out.stride(1) == 1
     if M <= 128 and gather is None and wait_flag is None and not (a_mn_major or b_mn_major) and alpha == 1.0 and beta == 1.0 and max_ctas == 0 \
             and split_k in (0, 1) and not cluster_split:
-        form = (a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail)
+        form = (a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail, norm_eps is not None)
         skinny, stream = _skinny_takes(*form), _stream_takes(*form)
         if skinny or stream:
             call = (a.data_ptr(), b.data_ptr(), out.data_ptr(), ptr(bias), ptr(residual), M, N, K, a.stride(0), b.stride(0), out.stride(0),

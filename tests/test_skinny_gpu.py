@@ -62,6 +62,20 @@ def test_a_row_as_residual_is_left_to_the_general_path(K):
         assert gemm_mod._few_rows_form(a, b, None, residual, 1, 128, K, 0, False, False, 0.0, 0, None) == taken
 
 
+def test_sizes_at_which_few_row_kernels_pay():
+    """The measured sides of every line of the rules: (M, N, K, gated unit, folded norm) -> kernel."""
+    rows = lambda M, N, K, glu=False, norm=False: "skinny" if gemm_mod._skinny_pays(M, N, K, glu) else (
+        "stream" if 9 <= M <= gemm_mod._stream_most_rows(N, K, glu, norm) else "one-CTA")
+    for want, *sizes in (
+            ("skinny", (1, 64, 64), (6, 151936, 896), (8, 128256, 4096), (16, 896, 4864), (16, 4096, 4096, False, True), (16, 2048, 128, True)),
+            ("stream", (9, 28672, 4096), (9, 2048, 128), (12, 64, 64), (48, 32768, 256), (32, 2048, 512), (24, 16384, 512),
+             (24, 9728, 2048), (40, 8192, 2048), (48, 37888, 1024), (64, 4096, 4096), (64, 896, 4864), (64, 28672, 4096, True), (64, 2048, 64, True)),
+            ("one-CTA", (8, 151936, 896), (16, 2048, 128), (17, 2048, 256), (32, 64, 64), (64, 2048, 256), (64, 32768, 256), (48, 64, 512),
+             (32, 16384, 512), (32, 9728, 896), (64, 9728, 896, False, True), (24, 9728, 2048, False, True), (32, 16384, 2048), (64, 28672, 4096), (64, 3072, 1024), (12, 151936, 896), (40, 128256, 4096, True))):
+        for s in sizes:
+            assert rows(*s) == want, (want, s, rows(*s))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("M", [1, 7, 8, 9, 16])
@@ -84,6 +98,7 @@ def test_few_rows(form, M, N, K, monkeypatch):
         args = {k: v for k, v in kw.items() if k != "tail"}
         return ops.gemm(a, b, tail=tail, **args)
 
+    monkeypatch.setattr(gemm_mod, "_skinny_pays", lambda *_: True)
     assert gemm_mod._skinny_takes(a, b, kw.get("bias"), kw.get("residual"), M, N, K, kw.get("bn", 0), kw.get("swiglu", False),
                                   kw.get("out_f32", False), kw.get("softcap", 0.0), kw.get("silu_cols", 0), tails[0])
     y, spread = _reference(a, b, **{k: v for k, v in kw.items() if k != "tail"})
@@ -95,15 +110,15 @@ def test_few_rows(form, M, N, K, monkeypatch):
     assert ((out.double() - y[:, :n]).abs() <= room[:, :n]).all()
     if tails[0] is not None:
         assert ((tails[0].double() - y[:, n:]).abs() <= (spread + 1e-6)[:, n:]).all()
-    monkeypatch.setattr(gemm_mod, "_SKINNY", ((16, 0),))
-    monkeypatch.setattr(gemm_mod, "_STREAM", (1, 0, 0))
+    monkeypatch.setattr(gemm_mod, "_skinny_pays", lambda *_: False)
+    monkeypatch.setattr(gemm_mod, "_stream_most_rows", lambda *_: 0)
     other = run(tails[1])
     assert ((out.double() - other.double()).abs() <= 2 * room[:, :n]).all()
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("form", FORMS)
-@pytest.mark.parametrize("M", [1, 17, 33, 64, 100, 128])
+@pytest.mark.parametrize("M", [9, 17, 33, 64, 100, 128])
 @pytest.mark.parametrize("N,K", [(8, 64), (136, 72), (896, 4864), (4096, 264)])
 def test_up_to_128_rows(form, M, N, K, monkeypatch):
     """``rb_stream``: token counts around its steps of 16, K remainders and cuts, N below and above a tile."""
@@ -120,8 +135,8 @@ def test_up_to_128_rows(form, M, N, K, monkeypatch):
     if kw.pop("residual", False):
         kw["residual"] = _strided(M, N, 8, gen)
     tail = torch.empty(M, kw["tail"] + 8, device="cuda")[:, :kw["tail"]] if kw.get("tail") else None
-    monkeypatch.setattr(gemm_mod, "_SKINNY", ((16, 0),))
-    monkeypatch.setattr(gemm_mod, "_STREAM", (1, 128, 296))
+    monkeypatch.setattr(gemm_mod, "_skinny_pays", lambda *_: False)
+    monkeypatch.setattr(gemm_mod, "_stream_most_rows", lambda *_: 128)
     assert gemm_mod._stream_takes(a, b, kw.get("bias"), kw.get("residual"), M, N, K, kw.get("bn", 0), kw.get("swiglu", False),
                                   kw.get("out_f32", False), kw.get("softcap", 0.0), kw.get("silu_cols", 0), tail)
     out = ops.gemm(a, b, tail=tail, **{k: v for k, v in kw.items() if k != "tail"})
