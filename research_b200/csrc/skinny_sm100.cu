@@ -11,7 +11,7 @@
 // at k = 16 t of row g and feeds four to each of four instructions, so 32-byte loads need no shuffles (a load of 8 rows x 64 bytes
 // occupies the load unit as long as one of 8 rows x 128 bytes: 16-byte loads were a fifth slower). Split of the work: a CTA's 8 warps cover `wr` row tiles x `wk` slices of K, and a cluster of S CTAs splits
 // K further; slices meet in shared memory, the cluster's through distributed shared memory, always summed in the same
-// order. K is cut until about 16 warps an SM have work or a slice is three loads long.
+// order. K is cut until about 16 warps an SM have work or a slice is less than three loads long.
 //
 // With b_static the weights are known not to be written by the kernels before this one on the stream: their first loads
 // are issued before the programmatic-launch wait and overlap the producer of A.
@@ -284,13 +284,14 @@ static int launch_skinny(const SkinnyParams& p, int blocks, cudaStream_t stream)
 }
 
 // ------------------------------------------------------------------------------------------
-// The same products for up to 64 rows (the code takes 128): the weights are the 128-row side of tcgen05.mma (a CTA has 128 rows of B and all
+// The same products for up to 64 rows: the weights are the 128-row side of tcgen05.mma (a CTA has 128 rows of B and all
 // tokens), so no accumulator row is spent on padding and an output of a few hundred columns still gives work to many CTAs: K is cut
 // over a cluster, whose fp32 partial tiles meet in distributed shared memory, four columns a load, always in the same order.
 // What bounds it is reading B once: 16 KB boxes of weights in a ring, two CTAs an SM; with b_static the first of them are on
 // their way before the kernel before this one has ended. The epilogue sums four groups of four columns a thread at a time: with one
 // group, whose loads from the other CTAs and of the residual wait for each other, 4096 x 4096 at 64 rows took 17.3 us, not 14.0.
-// Past 64 rows the partial tiles are what takes the time, and the one-CTA kernel is the better one. Warp 0 TMA, warp 1 products, warps 2-5 row sums of squares (a folded
+// Past 64 rows the partial tiles are what takes the time, and the one-CTA kernel is the better one (128 rows: 896 x 896 8.1 us there, 10.1
+// here, 28672 x 4096 49.9 / 51.0). Warp 0 TMA, warp 1 products, warps 2-5 row sums of squares (a folded
 // norm) while the ring turns, then all warps the epilogue.
 // ------------------------------------------------------------------------------------------
 struct StreamParams {
@@ -299,7 +300,7 @@ struct StreamParams {
   int tokens, stages;            // M rounded up to 16; ring depth
   int quads;                     // output, residual and bias take four columns at a time
 };
-constexpr int ST_THREADS = 192, ST_ROWS = 128, ST_LD = ST_ROWS + 4, ST_MAX_STAGES = 8;
+constexpr int ST_THREADS = 192, ST_MAX_TOKENS = 64, ST_ROWS = 128, ST_LD = ST_ROWS + 4, ST_MAX_STAGES = 8;
 
 // S: CTAs of a cluster
 template <int S>
@@ -307,7 +308,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
   const SkinnyParams& p = sp.e;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full[ST_MAX_STAGES], empty[ST_MAX_STAGES], acc_full;
-  __shared__ float ssq[128], rstd[128];
+  __shared__ float ssq[ST_MAX_TOKENS], rstd[ST_MAX_TOKENS];
   __shared__ uint32_t tmem_base_smem;
   __shared__ int abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
   float* red = reinterpret_cast<float*>(smem_al);        // over the ring once it has run: [tokens][ST_LD]
-  const uint32_t tmem_cols = T <= 32 ? 32u : T <= 64 ? 64u : 128u;
+  const uint32_t tmem_cols = T <= 32 ? 32u : 64u;
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&empty[s]));
       }
-      ssq[tid] = sum;
+      if (tid < T) ssq[tid] = sum;
     }
     bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&acc_full), 0, abortp, status, ST_TIMEOUT_TMEM_FULL));
     if (__any_sync(0xffffffffu, *abortp != 0)) ok = false;       // copies may still land in the ring
@@ -541,7 +542,7 @@ int rb_skinny(const void* A, const void* B, void* C, const void* bias, const voi
   if (glu_half > 0 && (glu_half % 16 || N % (2 * glu_half) || bias || residual || out_f32 || tail || silu_cols || softcap > 0.f)) return -1;
   if ((silu_cols || tail) && out_f32) return -1;
   // A CTA's row tiles share the T tokens that come through L1, so more tokens want more of them. K is cut in powers of two
-  // while the whole grid fits the SMs at once (16 warps each) and a slice keeps three steps.
+  // while the whole grid fits the SMs at once (16 warps each) and what is cut has three 64-column steps: no slice is below one and a half.
   const int tiles = glu_half > 0 ? N / 16 : (N + 15) / 16, steps = (K + 63) / 64, nt = (M + 7) / 8;
   const int min_wr = nt > 1 || glu_half > 0 ? 2 : 1;
   int parts = 1;
@@ -562,14 +563,13 @@ int rb_skinny(const void* A, const void* B, void* C, const void* bias, const voi
   return nt == 1 ? launch_skinny<1>(p, blocks, stream) : launch_skinny<2>(p, blocks, stream);
 }
 
-// The same for M <= 128 on the tensor cores (stream_kernel): glu_half a multiple of 64, rows 16-byte aligned. Returns -2 where the grid would
-// not fit the SMs at once.
+// The same for M <= 64 on the tensor cores (stream_kernel): K a multiple of 8, glu_half of 64, rows 16-byte aligned.
 int rb_stream(const void* A, const void* B, void* C, const void* bias, const void* residual, int M, int N, int K, long long lda,
               long long ldb, long long ldc, long long ldr, int out_f32, int glu_half, int glu_kind, float glu_limit, int norm_fold,
               float norm_eps, float softcap, int silu_cols, float* tail, int tail_col, long long tail_ld, int b_static, int* status,
               cudaStream_t stream) {
   using namespace rb;
-  if (M <= 0 || M > 128 || N <= 0 || K <= 0 || N % 8 || K % 8) return -1;
+  if (M <= 0 || M > ST_MAX_TOKENS || N <= 0 || K <= 0 || N % 8 || K % 8) return -1;
   if (glu_half > 0 && (glu_half % 64 || N % (2 * glu_half) || bias || residual || out_f32 || tail || silu_cols || softcap > 0.f)) return -1;
   if ((silu_cols || tail) && out_f32) return -1;
   const int tiles = glu_half > 0 ? N / 128 : (N + 127) / 128, num_kb = (K + 63) / 64;
@@ -589,7 +589,6 @@ int rb_stream(const void* A, const void* B, void* C, const void* bias, const voi
   int splits = 1;
   while (splits < 8 && tiles * splits * 2 <= 148 && num_kb >= splits * 4) splits *= 2;
   p.splits = splits;
-  if (tiles * splits > 296) return -2;
   const int stage = (ST_ROWS + sp.tokens) * 128, per = (num_kb + splits - 1) / splits;
   int stages = (108 * 1024) / stage;
   if (stages > ST_MAX_STAGES) stages = ST_MAX_STAGES;

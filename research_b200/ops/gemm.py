@@ -474,7 +474,7 @@ def gemm(
     if out is None:
         out = torch.empty(M, N // 2 if swiglu else N - (tail.shape[1] if tail is not None else 0), dtype=torch.float32 if out_f32 else torch.bfloat16, device=a.device)
     assert out.stride(1) == 1
-    if M <= 128 and gather is None and wait_flag is None and not (a_mn_major or b_mn_major) and alpha == 1.0 and beta == 1.0 and max_ctas == 0 \
+    if M <= 64 and gather is None and wait_flag is None and not (a_mn_major or b_mn_major) and alpha == 1.0 and beta == 1.0 and max_ctas == 0 \
             and split_k in (0, 1) and not cluster_split:
         form = (a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail, norm_eps is not None)
         skinny, stream = _skinny_takes(*form), _stream_takes(*form)

@@ -118,9 +118,9 @@ def test_few_rows(form, M, N, K, monkeypatch):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("form", FORMS)
-@pytest.mark.parametrize("M", [9, 17, 33, 64, 100, 128])
+@pytest.mark.parametrize("M", [9, 16, 17, 32, 33, 64])
 @pytest.mark.parametrize("N,K", [(8, 64), (136, 72), (896, 4864), (4096, 264)])
-def test_up_to_128_rows(form, M, N, K, monkeypatch):
+def test_up_to_64_rows(form, M, N, K, monkeypatch):
     """``rb_stream``: token counts around its steps of 16, K remainders and cuts, N below and above a tile."""
     kw = dict(FORMS[form])
     if kw.get("swiglu"):
@@ -136,7 +136,7 @@ def test_up_to_128_rows(form, M, N, K, monkeypatch):
         kw["residual"] = _strided(M, N, 8, gen)
     tail = torch.empty(M, kw["tail"] + 8, device="cuda")[:, :kw["tail"]] if kw.get("tail") else None
     monkeypatch.setattr(gemm_mod, "_skinny_pays", lambda *_: False)
-    monkeypatch.setattr(gemm_mod, "_stream_most_rows", lambda *_: 128)
+    monkeypatch.setattr(gemm_mod, "_stream_most_rows", lambda *_: 64)
     assert gemm_mod._stream_takes(a, b, kw.get("bias"), kw.get("residual"), M, N, K, kw.get("bn", 0), kw.get("swiglu", False),
                                   kw.get("out_f32", False), kw.get("softcap", 0.0), kw.get("silu_cols", 0), tail)
     out = ops.gemm(a, b, tail=tail, **{k: v for k, v in kw.items() if k != "tail"})
