@@ -645,7 +645,8 @@ extern "C" int rb_gemm2_dlogits(const void* A, const void* B, int M, int N, int 
 // C[g M .. , N] = A[rows of g, M]^T B[rows of g, N] (+ residual at the same places) for every group of rows of A [rows, M] and B [rows, N]:
 // the weight gradients of all experts. offsets [groups + 1] on the device: multiples of 64, every group at least 64 rows. M a
 // multiple of 32. One 256 x 256 tile per pair of CTAs loads a third less than the one-CTA kernel's 128 x 256 tiles, whose loads at a
-// contraction of 256 rows bounded it: 128 experts, 37000 rows, 1536 x 2048 and 2048 x 768 635 us together, 464 here.
+// contraction of 256 rows bounded it: 128 experts, 37000 rows, 1536 x 2048 and 2048 x 768 635 us together, 464 here. Tiles of 128 columns where
+// that is all there is (8 experts of 1024 rows, 64 x 64: 10.1 us with 256, 8.2).
 extern "C" int rb_gemm2_groups(const void* A, const void* B, void* C, const void* residual, int groups, int M, int N, int rows, long long lda,
                                long long ldb, long long ldc, long long ldr, const int* offsets, int* status, cudaStream_t stream) {
   if (groups <= 0 || M <= 0 || N <= 0 || rows <= 0 || M % 32 != 0 || N % 8 != 0 || offsets == nullptr) return -1;
@@ -662,5 +663,6 @@ extern "C" int rb_gemm2_groups(const void* A, const void* B, void* C, const void
   if (rc != 0) return -30 + rc;
   rc = tma_map_2d_out(&p.c_map, C, (unsigned long long)groups * M, N, ldc, 0, 32);
   if (rc != 0) return -40 + rc;
+  if (N <= 128) return g2_launch<128, true, true, false, G2_GROUPS>(p, groups * ((M + 255) / 256), stream);
   return g2_launch<256, true, true, false, G2_GROUPS>(p, groups * ((M + 255) / 256) * ((N + 255) / 256), stream);
 }

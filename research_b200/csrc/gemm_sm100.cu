@@ -104,6 +104,7 @@ struct GemmParams {
   long long stage_parity_bytes, flag_parity_bytes;
   const int4* tile_table;
   const int* num_tiles_ptr;
+  int group_k;            // grouped weight gradient: tiles carry their own K range and output group (see RbGemmArgs::group_mode)
   const unsigned long long* row_dst;
   int swiglu;
   int glu_kind;           // see RbGemmArgs
@@ -256,6 +257,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
   const int num_m_tiles = m_tiles_per_part * p.a_parts;
   const int num_n_tiles = n_tiles_per_part * p.b_parts;
   const bool grouped = p.tile_table != nullptr;
+  const bool grp = grouped && !p.group_k;   // tiles address rows of A directly (forward and data-gradient forms)
   const int split_k = p.split_k;
   const int num_kb = (p.K + BK - 1) / BK;
 
@@ -306,13 +308,18 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
   // own slab last so that every owner finds its partials early.
   // grouped tiles: m_in = first A row, n_part = first B row, n_in = first output column,
   // m_part carries the number of valid rows
-  // kb_lo / kb_hi: the k-blocks of the work unit (a split-K slice)
+  // kb_lo / kb_hi: the k-blocks of the work unit (a split-K slice, or a group's row range in the grouped weight gradient)
   auto tile_coords = [&](int t, int& m_part, int& m_in, int& n_part, int& n_in, int& kb_lo, int& kb_hi) {
     kb_lo = (t % split_k) * p.kb_per_split;
     kb_hi = split_k > 1 ? min(num_kb, kb_lo + p.kb_per_split) : num_kb;
     t /= split_k;
     if (grouped) {
       const int4 e = p.tile_table[t];
+      if (p.group_k) {
+        kb_lo = e.x / BK; kb_hi = kb_lo + e.y / BK;
+        m_part = e.z; m_in = (e.w >> 16) * BM; n_part = 0; n_in = (e.w & 0xffff) * BN;
+        return;
+      }
       m_in = e.x; m_part = e.y; n_part = e.z; n_in = e.w;
       return;
     }
@@ -366,8 +373,8 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
         }
         const CUtensorMap* amap = &p.a_map[grouped ? 0 : m_part];
         const CUtensorMap* bmap = &p.b_map[grouped ? 0 : n_part];
-        const int b_row = (grouped && !B_MN) ? n_part : n_in;   // first B row (K-major) or column (MN-major) of the tile
-        const int b_k0 = (grouped && B_MN) ? n_part : 0;        // grouped data gradient: the group's first row of the stacked B
+        const int b_row = (grp && !B_MN) ? n_part : n_in;   // first B row (K-major) or column (MN-major) of the tile
+        const int b_k0 = (grp && B_MN) ? n_part : 0;        // grouped data gradient: the group's first row of the stacked B
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           // ring slot and phase advance incrementally: the depth is a run-time value, and a division per k-block sat
           // on the single-thread critical path of this role
@@ -427,6 +434,10 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
         const uint32_t tmem_d = tmem_base + acc * BN;
         int kb0 = (t % split_k) * p.kb_per_split;
         int kb1 = split_k > 1 ? min(num_kb, kb0 + p.kb_per_split) : num_kb;
+        if (p.group_k) {
+          const int4 e = p.tile_table[t];
+          kb0 = e.x / BK; kb1 = kb0 + e.y / BK;
+        }
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           // ring slot and phase advance incrementally: the depth is a run-time value, and a division per k-block sat
           // on the single-thread critical path of this role
@@ -590,9 +601,9 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
         rscale = rs_smem[acc][q * 32 + lane];
       }
       const int row_in = m_in + q * 32 + lane;                 // row inside the A slab
-      const bool row_ok = grouped ? (q * 32 + lane < m_part) : (row_in < p.a_rows_per_part);
-      const long long row = grouped ? (long long)row_in : (long long)m_part * p.a_rows_per_part + row_in;
-      const int n_base = grouped ? n_in : n_part * p.b_rows_per_part + n_in;    // global column
+      const bool row_ok = grp ? (q * 32 + lane < m_part) : (row_in < p.a_rows_per_part);
+      const long long row = grp ? (long long)row_in : (long long)m_part * p.a_rows_per_part + row_in;
+      const int n_base = grp ? n_in : n_part * p.b_rows_per_part + n_in;    // global column
       const int n_valid = min(BN, p.b_rows_per_part - n_in);   // columns valid in this tile
       if (p.cluster_k) {
         // ---- cluster split-K: the split_k CTAs of a cluster each hold the fp32 partial tile of one K slice.
@@ -919,7 +930,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
       if (p.epi_mode != RB_EPI_STORE) {
         // rows of this warp: q*32 .. q*32+31 of the tile; each row holds n_valid columns
         const int units_per_row = n_valid >> 3;                      // 16-byte units
-        const int rows_here = min(32, (grouped ? m_part : p.a_rows_per_part - m_in) - q * 32);
+        const int rows_here = min(32, (grp ? m_part : p.a_rows_per_part - m_in) - q * 32);
         const int n_dst = p.epi_mode == RB_EPI_ALL_REDUCE_ONESHOT ? p.world : 1;
         for (int u = lane; u < rows_here * units_per_row; u += 32) {
           const int rr = u / units_per_row, cu = u - rr * units_per_row;
@@ -1374,8 +1385,10 @@ extern "C" int rb_gemm_bf16_ex(const RbGemmArgs* a, cudaStream_t stream) {
     const int gm = a->group_mode;
     if (gm == 0 ? (a->a_mn_major || a->b_mn_major)
         : gm == 1 ? (a->a_mn_major || !a->b_mn_major || a->group_b_rows <= 0 || a->K % BK != 0 || a->row_dst || a->swiglu)
+        : gm == 2 ? (!a->a_mn_major || !a->b_mn_major || a->K % BK != 0 || a->row_dst || a->swiglu || a->bn < 64)
                   : true)
       return -1;
+    p.group_k = gm == 2;
   } else if (a->group_mode != 0) {
     return -1;
   }

@@ -391,14 +391,15 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const fl
 // the row order inside an expert is the token order, so results do not depend on scheduling.
 
 struct TrainTableDesc {
-  int mode;        // 0 forward {a_row0, valid_rows, e * b_stride + n0, n0}; 1 data gradient {a_row0, valid_rows, e * b_stride, n0}
+  int mode;        // 0 forward {a_row0, valid_rows, e * b_stride + n0, n0}; 1 data gradient {a_row0, valid_rows, e * b_stride, n0};
+                   // 2 weight gradient {row0, rows, e, (m tile << 16) | n tile}
   int n_total;     // output columns per expert
   int bn;          // tile width
-  int b_stride;    // rows of the stacked B matrix per expert
+  int b_stride;    // rows of the stacked B matrix per expert (modes 0, 1); output rows per expert M (mode 2)
   int4* tiles;
   int* ntiles;
 };
-constexpr int MAX_TRAIN_TABLES = 4;
+constexpr int MAX_TRAIN_TABLES = 6;
 struct TrainTables { TrainTableDesc t[MAX_TRAIN_TABLES]; int n; };
 
 // One CTA per table (blockIdx.x) plus every CTA's own copy of the offsets. offsets[e] = first row of expert e,
@@ -422,7 +423,7 @@ __global__ void moe_train_plan_kernel(const int* __restrict__ counts, int E, int
     for (int e = 0; e < E; ++e) {
       const int rows = off_s[e + 1];
       base_s[e] = b;
-      b += (rows + 127) / 128 * nt;
+      b += (d.mode == 2 ? (d.b_stride + 127) / 128 : (rows + 127) / 128) * nt;
       o += rows;
       off_s[e + 1] = o;
     }
@@ -445,11 +446,17 @@ __global__ void moe_train_plan_kernel(const int* __restrict__ counts, int E, int
     }
     const int e = lo, j = t - base_s[e];
     const int rows = off_s[e + 1] - off_s[e];
-    const int mt = (rows + 127) / 128;
-    // consecutive tiles share the B tile
+    const int mt = d.mode == 2 ? (d.b_stride + 127) / 128 : (rows + 127) / 128;
+    // consecutive tiles share the B tile (modes 0, 1) or the A tile's k range (mode 2)
     const int in = j / mt, im = j % mt;
-    const int r0 = off_s[e] + im * 128;
-    d.tiles[t] = make_int4(r0, min(128, off_s[e + 1] - r0), d.mode == 0 ? e * d.b_stride + in * d.bn : e * d.b_stride, in * d.bn);
+    int4 v;
+    if (d.mode == 2) {
+      v = make_int4(off_s[e], rows, e, (im << 16) | in);
+    } else {
+      const int r0 = off_s[e] + im * 128;
+      v = make_int4(r0, min(128, off_s[e + 1] - r0), d.mode == 0 ? e * d.b_stride + in * d.bn : e * d.b_stride, in * d.bn);
+    }
+    d.tiles[t] = v;
   }
 }
 
@@ -709,9 +716,10 @@ extern "C" int rb_moe_train_plan(const int* counts, int E, int* offsets, const i
   for (int i = 0; i < n_tables; ++i) {
     tabs.t[i].mode = desc[4 * i]; tabs.t[i].n_total = desc[4 * i + 1]; tabs.t[i].bn = desc[4 * i + 2]; tabs.t[i].b_stride = desc[4 * i + 3];
     tabs.t[i].tiles = reinterpret_cast<int4*>(tiles[i]); tabs.t[i].ntiles = ntiles[i];
-    if (tabs.t[i].mode < 0 || tabs.t[i].mode > 1 || tabs.t[i].bn <= 0 || tabs.t[i].n_total <= 0 || tabs.t[i].tiles == nullptr ||
+    if (tabs.t[i].mode < 0 || tabs.t[i].mode > 2 || tabs.t[i].bn <= 0 || tabs.t[i].n_total <= 0 || tabs.t[i].tiles == nullptr ||
         tabs.t[i].ntiles == nullptr)
       return -1;
+    if (tabs.t[i].mode == 2 && ((tabs.t[i].b_stride + 127) / 128 > 0xffff || (tabs.t[i].n_total + tabs.t[i].bn - 1) / tabs.t[i].bn > 0xffff)) return -1;
   }
   if (n_tables == 0) return -1;
   moe_train_plan_kernel<<<n_tables, 256, 0, s>>>(counts, E, offsets, tabs, max_tiles, cap_rows, status);

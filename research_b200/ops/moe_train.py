@@ -2,7 +2,7 @@
 experts of a layer run as six grouped launches over expert-sorted rows, with no host synchronisation.
 
 The (token, slot) pairs are sorted by expert on the device; every expert's row range is padded with zero rows to a
-multiple of 64, so the weight gradient ``dW_e = dY_e^T X_e`` is one grouped launch (csrc/gemm2_sm100.cu) whose contraction runs over the
+multiple of 64, so the weight gradient ``dW_e = dY_e^T X_e`` is one grouped launch whose contraction runs over the
 expert's row range (a 64-row k-block never straddles two experts). Rows keep the token order inside an expert, so the
 result does not depend on scheduling.
 
@@ -43,11 +43,28 @@ def _lib():
 
 
 MAX_EXPERTS = 256
-FWD_GU, FWD_DN, DGRAD_DN, DGRAD_GU = range(4)
+FWD_GU, FWD_DN, DGRAD_DN, DGRAD_GU, WGRAD_DN, WGRAD_GU = range(6)
 
 
 def _tile_width(n: int) -> int:
     return 256 if n >= 256 else 128 if n >= 128 else 64
+
+
+def _pair_wgrad_pays(E: int, m: int, n: int, accumulate: bool) -> bool:
+    """Weight gradients ``[m, n]`` of ``E`` experts on the two-CTA kernel's 256-row tiles (csrc/gemm2_sm100.cu) or on the one-CTA kernel's 128 rows.
+    Microseconds, one-CTA / two-CTA. The two-CTA kernel reads less per product: E 128, 1536 x 2048 and 2048 x 768 508 / 385 at 64 rows an
+    expert, E 256, 512 x 96 .75 of the time. Rows of a tile that the matrix does not have leave one CTA of the pair without an epilogue,
+    which is what bounds short contractions: E 256, 128 x 1024 at 64 rows 30 / 46, adding 68 / 120; 384 x 1024 81 / 87, adding 211 / 240; 1024 x 32 19 / 23.
+    Up to two waves of tiles that does not show (E 128, 64 x 256 .92; E 8, 64 x 64 .87). A single 128-column tile that is only written:
+    E 256, 2048 x 128 at 192 rows 80 / 96, adding .91."""
+    def up(x: int, step: int) -> int:
+        return -(-x // step) * step
+
+    columns = 128 if n <= 128 else 256
+    pair = up(m, 256) * up(n, columns)
+    if E * pair <= 148 * 256 * columns:
+        return True
+    return pair <= 1.25 * up(m, 128) * up(n, _tile_width(n)) and (accumulate or n != 128)
 
 
 class GroupedPlan:
@@ -71,15 +88,21 @@ class GroupedPlan:
         st = status_tensor(dev).data_ptr()
         self.counts = torch.zeros(E, dtype=torch.int32, device=dev)
         check_rc(lib.rb_moe_count(idx.data_ptr(), n, E, self.counts.data_ptr(), s), "rb_moe_count")
-        # (mode, output columns per expert, tile width, rows of the stacked B per expert)
-        self.desc = [(0, 2 * F, _tile_width(2 * F), 2 * F), (0, d, _tile_width(d), d), (1, F, _tile_width(F), d), (1, d, _tile_width(d), 2 * F)]
+        # (mode, output columns per expert, tile width, rows of the stacked B per expert | output rows per expert)
+        self.desc = [(0, 2 * F, _tile_width(2 * F), 2 * F), (0, d, _tile_width(d), d),
+                     (1, F, _tile_width(F), d), (1, d, _tile_width(d), 2 * F),
+                     (2, F, _tile_width(F), d), (2, d, _tile_width(d), 2 * F)]
         m_tiles = self.cap // 128 + E
-        self.max_tiles = max(m_tiles * -(-n_total // bn) for _, n_total, bn, _ in self.desc)
-        tables = len(self.desc)
+        # tables are written for the launches that read one
+        used = [w for w in range(6) if w < WGRAD_DN or not _pair_wgrad_pays(E, self.desc[w][3], self.desc[w][1], False)]
+        self.table_of = {which: table for table, which in enumerate(used)}
+        written = [self.desc[which] for which in self.table_of]
+        self.max_tiles = max((E * -(-bs // 128) if mode == 2 else m_tiles) * -(-n_total // bn) for mode, n_total, bn, bs in written)
+        tables = len(written)
         self.tiles = torch.empty(tables, self.max_tiles, 4, dtype=torch.int32, device=dev)
         self.ntiles = torch.zeros(tables, dtype=torch.int32, device=dev)
         self.offsets = torch.empty(E + 1, dtype=torch.int32, device=dev)
-        flat = (_I * (4 * tables))(*[v for dsc in self.desc for v in dsc])
+        flat = (_I * (4 * tables))(*[v for dsc in written for v in dsc])
         tptr = (_VP * tables)(*[self.tiles[i].data_ptr() for i in range(tables)])
         nptr = (_VP * tables)(*[self.ntiles.data_ptr() + 4 * i for i in range(tables)])
         check_rc(lib.rb_moe_train_plan(self.counts.data_ptr(), E, self.offsets.data_ptr(), flat, tptr, nptr, tables, self.max_tiles,
@@ -136,7 +159,8 @@ class GroupedPlan:
         args.epi_mode = EPI_STORE
         args.rank, args.world = 0, 1
         args.status = status_tensor(self.device).data_ptr()
-        args.tile_table, args.num_tiles_ptr = self.tiles[which].data_ptr(), self.ntiles.data_ptr() + 4 * which
+        table = self.table_of[which]
+        args.tile_table, args.num_tiles_ptr = self.tiles[table].data_ptr(), self.ntiles.data_ptr() + 4 * table
         args.group_n, args.max_tiles = group_n, self.max_tiles
         args.group_mode, args.group_b_rows = group_mode, group_b_rows
         if residual is not None:
@@ -159,10 +183,15 @@ class GroupedPlan:
         self._launch(which, dy, w, out, M=self.cap, N=n, K=kd, group_n=n, a_mn=False, b_mn=True, group_mode=1, group_b_rows=self.E * kd)
         return out
 
-    def wgrad(self, dy: torch.Tensor, x: torch.Tensor, gw: torch.Tensor, accumulate: bool) -> None:
+    def wgrad(self, which: int, dy: torch.Tensor, x: torch.Tensor, gw: torch.Tensor, accumulate: bool) -> None:
         """``gw_e (+)= dy[rows of e]^T @ x[rows of e]`` for every expert; ``gw`` is ``[E * m, n]``."""
-        m, n = dy.shape[1], x.shape[1]
-        assert dy.shape[0] == x.shape[0] == self.cap and gw.shape == (self.E * m, n) and gw.stride(1) == 1
+        n, m = self.desc[which][1], self.desc[which][3]
+        assert dy.shape == (self.cap, m) and x.shape == (self.cap, n) and gw.shape == (self.E * m, n)
+        if not _pair_wgrad_pays(self.E, m, n, accumulate):
+            self._launch(which, dy, x, gw, M=m, N=n, K=self.cap, group_n=n, a_mn=True, b_mn=True, group_mode=2,
+                         residual=gw if accumulate else None)
+            return
+        assert gw.stride(1) == 1
         rc = _gemm2_lib().rb_gemm2_groups(dy.data_ptr(), x.data_ptr(), gw.data_ptr(), gw.data_ptr() if accumulate else None, self.E, m, n, self.cap,
                                           dy.stride(0), x.stride(0), gw.stride(0), gw.stride(0), self.offsets.data_ptr(),
                                           status_tensor(self.device).data_ptr(), stream_handle(self.device))
@@ -195,11 +224,11 @@ class GroupedExperts(torch.autograd.Function):
         dwt = plan.dot(dout, y) if ctx.needs_input_grad[1] else None
         dy = plan.gather(dout, wt)
         act = _ew.swiglu(gu)                                  # recomputed: cheaper than keeping [rows, F] alive
-        plan.wgrad(dy, act, ctx.gd, ctx.sink.accumulate_into(ctx.gd))
+        plan.wgrad(WGRAD_DN, dy, act, ctx.gd, ctx.sink.accumulate_into(ctx.gd))
         dact = plan.dgrad(DGRAD_DN, dy, wd)
         del act, dy
         dgu = _ew.swiglu_backward(gu, dact)
-        plan.wgrad(dgu, xs, ctx.ggu, ctx.sink.accumulate_into(ctx.ggu))
+        plan.wgrad(WGRAD_GU, dgu, xs, ctx.ggu, ctx.sink.accumulate_into(ctx.ggu))
         dh = None
         if ctx.needs_input_grad[0]:
             dh = plan.combine(plan.dgrad(DGRAD_GU, dgu, wgu))

@@ -155,3 +155,30 @@ def test_grouped_experts_training_vs_reference(cuda_device, T, k, E, d, F):
     out2.backward(dout)
     assert rel(ggu, 2 * wgur.grad) < 3e-2 and rel(gd, 2 * wdr.grad) < 3e-2
     ops.check_status()
+
+
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("E,d,F", [(160, 256, 32), (160, 256, 128), (160, 64, 288), (5, 64, 32), (3, 320, 160), (150, 192, 96)])
+def test_weight_gradients_of_all_experts(cuda_device, E, d, F, accumulate):
+    """Both matrices through the launch that the sizes choose, against 64 bits; experts without rows, ragged tiles of 128 and 256."""
+    from research_b200.ops import check_status
+    from research_b200.ops.moe_train import WGRAD_DN, WGRAD_GU, GroupedPlan
+
+    g = torch.Generator(device=cuda_device).manual_seed(E + d + F)
+    T, k = 700, 2
+    idx = torch.randint(0, E, (T, k), device=cuda_device, generator=g, dtype=torch.int32)
+    idx[idx == E // 2] = 0
+    plan = GroupedPlan(idx.contiguous(), E, d, F)
+    off = plan.offsets.tolist()
+    for which, m, n in ((WGRAD_GU, 2 * F, d), (WGRAD_DN, d, F)):
+        dy, x = (plan.gather(torch.randn(T, c, device=cuda_device, generator=g).bfloat16()) for c in (m, n))
+        dy[off[-1]:], x[off[-1]:] = 7.0, 7.0                     # rows past those in use
+        gw = torch.randn(E * m, n, device=cuda_device, generator=g).bfloat16()
+        start = gw.double().view(E, m, n) if accumulate else torch.zeros(E, m, n, device=cuda_device, dtype=torch.float64)
+        plan.wgrad(which, dy, x, gw, accumulate)
+        for e in range(E):
+            p, q = dy[off[e]:off[e + 1]].double(), x[off[e]:off[e + 1]].double()
+            want = start[e] + p.T @ q
+            room = (p.abs().T @ q.abs()) * 2 * len(p) * 2.0 ** -24 + 2.0 ** -8 * want.abs() + 1e-6      # fp32 sums in the worst order, one rounding to bf16
+            assert ((gw.view(E, m, n)[e].double() - want).abs() <= room).all(), (which, e)
+    check_status(cuda_device)

@@ -475,3 +475,14 @@ def test_vocab_parallel_logprob_matches_log_softmax_and_tp_backend_runs_alone():
     assert be.forward_backward({"input_ids": ids, "labels": ids}).wait()["loss"] < first and be.tp_size == 1 and be.current_step == 6
     with pytest.raises(AssertionError, match="expert parallelism"):
         TensorParallelTrainingBackend(get_preset("tiny-moe"))
+
+
+def test_weight_gradient_kernel_by_size():
+    """The measured sides of the rule: (experts, rows, columns of a gradient, adding) -> two-CTA kernel."""
+    from research_b200.ops.moe_train import _pair_wgrad_pays as pays
+
+    for E, m, n in ((128, 1536, 2048), (128, 2048, 768), (8, 64, 64), (8, 128, 64), (128, 64, 256), (256, 192, 512), (256, 512, 96), (64, 576, 192), (256, 1024, 192)):
+        assert pays(E, m, n, False) and pays(E, m, n, True), (E, m, n)
+    for E, m, n in ((256, 128, 1024), (256, 64, 1024), (256, 1024, 64), (256, 1024, 32), (256, 384, 1024), (128, 2048, 64), (64, 4096, 64)):
+        assert not pays(E, m, n, False) and not pays(E, m, n, True), (E, m, n)
+    assert pays(256, 2048, 128, True) and not pays(256, 2048, 128, False)
