@@ -257,8 +257,10 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
   const int num_m_tiles = m_tiles_per_part * p.a_parts;
   const int num_n_tiles = n_tiles_per_part * p.b_parts;
   const bool grouped = p.tile_table != nullptr;
-  const bool grp = grouped && !p.group_k;   // tiles address rows of A directly (forward and data-gradient forms)
+  const bool group_k = A_MN && B_MN && p.group_k;   // the other instantiations stay without its branches
+  const bool grp = grouped && !group_k;   // tiles address rows of A directly (forward and data-gradient forms)
   const int split_k = p.split_k;
+  int num_tiles = num_m_tiles * num_n_tiles * split_k;   // work units
   const int num_kb = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -291,7 +293,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
   pdl_launch_dependents();
   if (p.cluster_k) cluster_sync_all();   // no peer may signal a barrier that is not initialised yet
   pdl_wait();  // barriers and TMEM are set up; from here on we read what the previous kernel wrote
-  const int num_tiles = (grouped ? *p.num_tiles_ptr : num_m_tiles * num_n_tiles) * split_k;  // work units (grouped: counted by the previous kernel)
+  if (grouped) num_tiles = *p.num_tiles_ptr * split_k;   // counted by the previous kernel
   RB_TS(0);
   const uint32_t tmem_base = tmem_base_smem;
   volatile int* abortp = &abort_flag;
@@ -315,7 +317,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
     t /= split_k;
     if (grouped) {
       const int4 e = p.tile_table[t];
-      if (p.group_k) {
+      if (group_k) {
         kb_lo = e.x / BK; kb_hi = kb_lo + e.y / BK;
         m_part = e.z; m_in = (e.w >> 16) * BM; n_part = 0; n_in = (e.w & 0xffff) * BN;
         return;
@@ -434,7 +436,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
         const uint32_t tmem_d = tmem_base + acc * BN;
         int kb0 = (t % split_k) * p.kb_per_split;
         int kb1 = split_k > 1 ? min(num_kb, kb0 + p.kb_per_split) : num_kb;
-        if (p.group_k) {
+        if (group_k) {
           const int4 e = p.tile_table[t];
           kb0 = e.x / BK; kb1 = kb0 + e.y / BK;
         }
