@@ -811,22 +811,20 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
             tmem_ld_wait();
             if (row_ok) {
               __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + row * p.ldc + out_col0 + c0;
+              // the branch on the kind outside the loops, whose elements then overlap
+              if (p.glu_kind == 1) {
 #pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                uint32_t o[4];
+                for (int j = 0; j < 32; ++j)
+                  g[j] = __float_as_uint(clamped_glu_epi(__uint_as_float(g[j]) * rscale, __uint_as_float(u[j]) * rscale, p.glu_limit));
+              } else {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  if (p.glu_kind == 1) {
-                    o[e] = pack_bf16x2(
-                        clamped_glu_epi(__uint_as_float(g[j + 2 * e]) * rscale, __uint_as_float(u[j + 2 * e]) * rscale, p.glu_limit),
-                        clamped_glu_epi(__uint_as_float(g[j + 2 * e + 1]) * rscale, __uint_as_float(u[j + 2 * e + 1]) * rscale, p.glu_limit));
-                    continue;
-                  }
-                  o[e] = pack_bf16x2(swiglu_epi(__uint_as_float(g[j + 2 * e]) * rscale, __uint_as_float(u[j + 2 * e]) * rscale),
-                                     swiglu_epi(__uint_as_float(g[j + 2 * e + 1]) * rscale, __uint_as_float(u[j + 2 * e + 1]) * rscale));
-                }
-                *reinterpret_cast<uint4*>(dst + j) = make_uint4(o[0], o[1], o[2], o[3]);
+                for (int j = 0; j < 32; ++j) g[j] = __float_as_uint(swiglu_epi(__uint_as_float(g[j]) * rscale, __uint_as_float(u[j]) * rscale));
               }
+#pragma unroll
+              for (int j = 0; j < 32; j += 8)
+                *reinterpret_cast<uint4*>(dst + j) =
+                    make_uint4(pack_bf16x2(__uint_as_float(g[j]), __uint_as_float(g[j + 1])), pack_bf16x2(__uint_as_float(g[j + 2]), __uint_as_float(g[j + 3])),
+                               pack_bf16x2(__uint_as_float(g[j + 4]), __uint_as_float(g[j + 5])), pack_bf16x2(__uint_as_float(g[j + 6]), __uint_as_float(g[j + 7])));
             }
           }
         }

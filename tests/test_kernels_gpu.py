@@ -512,7 +512,8 @@ def test_gemm_waits_for_a_flag_inside_the_launch(cuda_device):
 @pytest.mark.parametrize("limit", [None, 1.5])
 @pytest.mark.parametrize("M,N,K", [(512, 9728, 256), (513, 9728, 264), (1000, 4864 * 2, 896), (2049, 2560, 512)])
 def test_gated_unit_on_the_pair_kernel(cuda_device, M, N, K, limit):
-    """The two-CTA kernel's gated unit equals the one-CTA kernel's (same sums, same epilogue): partial row tiles, a K remainder, strided rows."""
+    """The two-CTA kernel's gated unit is the one-CTA kernel's in every bit (same sums, same epilogue), and both are within their roundings of
+    64 bits: partial row tiles, a K remainder, strided rows."""
     from research_b200.ops import gemm_mod
 
     g = torch.Generator(device=cuda_device).manual_seed(M + N)
@@ -521,9 +522,44 @@ def test_gated_unit_on_the_pair_kernel(cuda_device, M, N, K, limit):
     out = torch.full((M, N // 2 + 8), 7.0, device=cuda_device, dtype=torch.bfloat16)
     assert gemm_mod._use_pair_kernel(M, N, K, False, False)
     got = ops.gemm(a, b, out=out[:, :N // 2], bn=256, swiglu=True, glu_limit=limit)
-    want = ops.gemm(a, b, bn=256, swiglu=True, glu_limit=limit, max_ctas=148)
-    assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * want.float().abs() + 1e-6).all()
+    assert torch.equal(got, ops.gemm(a, b, bn=256, swiglu=True, glu_limit=limit, max_ctas=148))
     assert (out[:, N // 2:] == 7.0).all()
+    gate, up = (a.double() @ b.double().T).view(M, -1, 2, 128).unbind(2)
+    sums = ((a.double().abs() @ b.double().abs().T) * 2 * K * 2.0 ** -24).view(M, -1, 2, 128)      # fp32 sums in the worst order
+    if limit is None:
+        want, roundings, slope = torch.nn.functional.silu(gate) * up, 4, 1.1
+    else:
+        gate, up = gate.clamp(max=limit), up.clamp(-limit, limit)
+        want, roundings, slope = gate * torch.sigmoid(1.702 * gate) * (up + 1), 1, 1.2
+    # gate, silu, up and the product are rounded to bf16 (2^-8 each); the activation passes an error of its argument on at most `slope` times
+    size = (gate.abs() + 0.3) * (up.abs() + 1)
+    room = roundings * 2.0 ** -8 * slope * size + slope * (sums[:, :, 0] * (up.abs() + 1) + sums[:, :, 1] * (gate.abs() + 0.3)) + 1e-6
+    assert ((got.double() - want.reshape(M, -1)).abs() <= room.reshape(M, -1)).all()
+
+
+@pytest.mark.parametrize("limit", [None, 7.0])
+@pytest.mark.parametrize("M", [16, 64, 128, 512])
+def test_gated_units_over_the_range_of_the_quotient(cuda_device, M, limit):
+    """Gates down to where the exponential overflows, met exactly (one-hot rows) on each of the kernels with a gated epilogue. A reciprocal that
+    gives up above 2^126 turns the last of them into zeros, which large up values show."""
+    N, inner = 4864, 88.5 if limit is None else 52.0
+    g = torch.Generator(device=cuda_device).manual_seed(M)
+    a = torch.eye(M, device=cuda_device).bfloat16()
+    b = torch.randn(N, M, device=cuda_device, generator=g).view(-1, 2, 128, M)
+    b[:, 0] = torch.rand(N // 256, 128, M, device=cuda_device, generator=g) * (inner + 5) - inner
+    b[:, 0, :8] = -inner + torch.rand(N // 256, 8, M, device=cuda_device, generator=g) * 1.3
+    b[:, 1, :64] *= 1e30
+    b = b.bfloat16().view(N, M).contiguous()
+    got = ops.gemm(a, b, bn=256, swiglu=True, glu_limit=limit).double()
+    gate, up = b.double().T.reshape(M, -1, 2, 128).unbind(2)
+    if limit is None:
+        want = gate / (1 + torch.exp(-gate)) * up
+    else:
+        gate, up = gate.clamp(max=limit), up.clamp(-limit, limit)
+        want = gate / (1 + torch.exp(-1.702 * gate)) * (up + 1)
+    want = want.reshape(M, -1)
+    # two roundings to bf16 (2^-8 each), and 2^-14 for their product and for an fp32 exponential whose argument of up to 128 (base 2) is rounded; half a step of bf16 below its normal numbers
+    assert ((got - want).abs() <= (2.0 ** -7 + 2.0 ** -14) * want.abs() + 1e-40).all()
 
 
 @pytest.mark.parametrize("n,silu", [(4864, 0), (4896, 64), (4896, 1 << 13), (5152, 4896)])
@@ -544,7 +580,7 @@ def test_tail_behind_whole_and_half_boxes_of_the_pair_kernel(cuda_device, M, n, 
     y = y[:, :n]
     c = min(silu, n)
     y[:, :c] = torch.nn.functional.silu(y[:, :c])
-    # one rounding to bf16 (2^-9, doubled for its half unit at a power of two), silu at most 1.1 times its argument's error
+    # one rounding to bf16 (2^-8), silu passes at most 1.1 times its argument's error on
     assert ((out[:, :n].double() - y).abs() <= 1.1 * room[:, :n] + 2.0 ** -8 * y.abs() + 1e-6).all()
     assert (out[:, n:] == 7.0).all() and (tail[:, t:] == 7.0).all()
     ops.check_status(cuda_device)
