@@ -1,11 +1,11 @@
 // Flash attention for sm_100a on the 5th-generation tensor cores.
 //
-// Forward: one CTA owns 128 query rows of one head. S = Q K^T and O += P V are tcgen05.mma
-// instructions issued by one thread; S (two buffers) and O live in tensor memory, Q/K/V tiles are
-// brought into 128-byte-swizzled shared memory by TMA, P goes back to shared memory as the A operand
-// of the second product. Warp roles: warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2-9
-// softmax (two threads per query row, each reading half of it from TMEM with tcgen05.ld). The running maximum is only
-// refreshed when it grew by more than 2^8, so the O accumulator is rescaled rarely.
+// S = Q K^T and O += P V are tcgen05.mma instructions issued by one thread; S and O live in tensor memory, Q/K/V tiles are
+// brought into 128-byte-swizzled shared memory by TMA. The running maximum is only refreshed when it grew by more than 2^8, so
+// the O accumulator is rescaled rarely. Forward of more than 128 query rows: flash_fwd2_kernel, two query tiles a CTA, P in tensor
+// memory. Up to 128 rows: flash_fwd_kernel, one tile a CTA, two S buffers, P through shared memory as the A operand of the second
+// product; warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warps 2-9 softmax (two threads per query row, each reading half of it
+// from TMEM with tcgen05.ld).
 //
 // Inputs are packed variable-length batches (`cu_seqlens`), grouped-query heads, causal and
 // sliding-window masks; K/V come either from dense [T, Hkv, D] tensors (training) or from the paged
@@ -1979,7 +1979,7 @@ static int launch_flash_bwd(const FlashBwdParams& p, dim3 grid_kv, dim3 grid_q, 
 
 template <int D>
 static int launch_flash_fwd(const FlashFwdParams& p, int max_seqlen_q, int B, cudaStream_t stream) {
-  static bool attr_dev[64] = {};       // the shared-memory opt-in is a per-device function attribute
+  static bool attr_dev[64] = {}, two_tiles[64] = {};       // the shared-memory opt-in is a per-device function attribute
   int dev_i = 0;
   if (cudaGetDevice(&dev_i) != cudaSuccess || dev_i < 0 || dev_i >= 64) return -10;
   bool& attr = attr_dev[dev_i];
@@ -1987,9 +1987,11 @@ static int launch_flash_fwd(const FlashFwdParams& p, int max_seqlen_q, int B, cu
     if (cudaFuncSetAttribute(flash_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, FlashCfg<D>::kSmemBytes) != cudaSuccess ||
         cudaFuncSetAttribute(flash_fwd2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Flash2Cfg<D>::kSmemBytes) != cudaSuccess)
       return -10;
-    // the register shares of the roles have to add up to what a block is launched with
+    // The register shares of the roles have to add up to what a block is launched with. A compiler that gives the kernel fewer leaves all
+    // sizes to the one-tile kernel.
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, flash_fwd2_kernel<D>) != cudaSuccess || fa.numRegs < FA2_REGS_LAUNCH) return -13;
+    if (cudaFuncGetAttributes(&fa, flash_fwd2_kernel<D>) != cudaSuccess) return -13;
+    two_tiles[dev_i] = fa.numRegs >= FA2_REGS_LAUNCH;
     attr = true;
   }
   static const bool one_tile = getenv("RB_FLASH_ONE_TILE") != nullptr;
@@ -1997,7 +1999,7 @@ static int launch_flash_fwd(const FlashFwdParams& p, int max_seqlen_q, int B, cu
   // Causal, TFLOP/s, dense / paged keys (in brackets with P in shared memory and a CTA per tile pair): 4 x 8192 tokens, 32 / 8
   // heads, D 128 1180 / 1011 (852 / 624); 8 x 2048 955 / 935 (470 / 416); 32 x 200 163 / 160 (67 / 66); 1 x 16384, 14 / 2 heads,
   // D 64 703 / 697 (507 / 333); 16 x 512 179 / 175 (82 / 80).
-  if (max_seqlen_q > FA_BM && !one_tile) {
+  if (max_seqlen_q > FA_BM && two_tiles[dev_i] && !one_tile) {
     dim3 grid((max_seqlen_q + 2 * FA_BM - 1) / (2 * FA_BM), p.Hq, B);
     return launch_kernel(flash_fwd2_kernel<D>, grid, dim3(FA2_THREADS), Flash2Cfg<D>::kSmemBytes, stream, p) == cudaSuccess ? 0 : -11;
   }
