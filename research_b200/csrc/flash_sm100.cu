@@ -1333,8 +1333,8 @@ static int launch_flash_latent(const FlashLatentParams& p, int max_q, int B, cud
 // product would read 6 KB of shared memory for 32 cycles of work, one 128 wide 8 KB for 64: just what it delivers; dq
 // keeps Q and dO in tensor memory and reads half of that. The row statistics of a query tile arrive with its Q and dO.
 // Backward of causal attention, TFLOP/s by 2.5 x the forward's (in brackets with 64-wide tiles, P and dS through shared memory):
-// 4 x 8192 tokens, 32 / 8 heads, D 128 757 (442); 8 x 2048 650 (343); 32 x 200 125 (70); 1 x 16384, 14 / 2 heads, D 64 530 (212);
-// 16 x 512 159 (74).
+// 4 x 8192 tokens, 32 / 8 heads, D 128 772 (443); 8 x 2048 664 (343); 32 x 200 126 (70); 1 x 16384, 14 / 2 heads, D 64 549 (212);
+// 16 x 512 163 (74).
 // ==========================================================================================
 struct FlashBwdParams {
   CUtensorMap q, dout, k, v;             // boxes of 64 columns x 128 rows
@@ -1997,8 +1997,8 @@ static int launch_flash_fwd(const FlashFwdParams& p, int max_seqlen_q, int B, cu
   static const bool one_tile = getenv("RB_FLASH_ONE_TILE") != nullptr;
   // Two query tiles per CTA share every K/V tile; a single tile's rows are better split over both warpgroups (flash_fwd_kernel).
   // Causal, TFLOP/s, dense / paged keys (in brackets with P in shared memory and a CTA per tile pair): 4 x 8192 tokens, 32 / 8
-  // heads, D 128 1180 / 1011 (852 / 624); 8 x 2048 955 / 935 (470 / 416); 32 x 200 163 / 160 (67 / 66); 1 x 16384, 14 / 2 heads,
-  // D 64 703 / 697 (507 / 333); 16 x 512 179 / 175 (82 / 80).
+  // heads, D 128 1215 / 1000 (854 / 619); 8 x 2048 952 / 932 (475 / 417); 32 x 200 160 / 160 (67 / 66); 1 x 16384, 14 / 2 heads,
+  // D 64 633 / 656 (506 / 333); 16 x 512 193 / 193 (82 / 80).
   if (max_seqlen_q > FA_BM && two_tiles[dev_i] && !one_tile) {
     dim3 grid((max_seqlen_q + 2 * FA_BM - 1) / (2 * FA_BM), p.Hq, B);
     return launch_kernel(flash_fwd2_kernel<D>, grid, dim3(FA2_THREADS), Flash2Cfg<D>::kSmemBytes, stream, p) == cudaSuccess ? 0 : -11;

@@ -620,8 +620,8 @@ extern "C" int rb_gemm2_bf16_gather(const void* A, const void* B, void* C, const
 }
 
 // The gradient of log-probabilities to logits, from the product that recomputes the logits A[M,K] B[N,K]^T: bit for bit what
-// rb_logprob_entropy_bwd makes of the fp32 output of rb_gemm2_bf16 (2048 x 151936 x 896: 700 + 343 us for the two, which write, read
-// and convert 2.5 GB; 453 us here).
+// rb_logprob_entropy_bwd makes of the fp32 output of rb_gemm2_bf16 (2048 x 151936 x 896: 476 + 343 us for the two, 802 in a row, which
+// write, read and convert 2.5 GB; 442 us here).
 // dlogits bf16 [M, N] (rows ldd apart, a multiple of 8). entropy and g_entropy may be null.
 extern "C" int rb_gemm2_dlogits(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb, const int* targets,
                                 const float* lse, const float* entropy, const float* g_logprob, const float* g_entropy, void* dlogits,

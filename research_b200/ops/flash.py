@@ -152,11 +152,13 @@ _HEAD_SPLIT = os.environ.get("RB_FLASH_BWD_HEAD_SPLIT", "auto")     # auto | 0 |
 
 def head_split_pays(B: int, max_seqlen_q: int, max_seqlen_k: int, Hq: int, Hkv: int) -> bool:
     """dK/dV as one CTA per (key tile, QUERY head) + a reduction over each group, instead of one CTA per (key tile,
-    key/value head) looping over its G query heads. It pays only where the coarse grid has fewer CTAs than the GPU has
-    SMs (one long sequence with two kv heads: 64 CTAs). Measured on the Llama-3-8B step (one 4096-token sequence, 8 kv
-    heads: 256 CTAs, the longest 256 iterations against 228 per SM on average) the split changes nothing: 255.2 ms per
-    step with it, 253.5 without; the kernel is bound by its 3.7 us per iteration, not by balance. The split costs
-    2 * G * Tk * Hkv * D floats of workspace and one pass over them."""
+    key/value head) looping over its G query heads and 128-query tiles. The split costs 2 * G * Tk * Hkv * D floats of
+    workspace and one pass over them; it pays where the longest of the whole loops is well above the average per SM.
+    The rule asks for fewer CTAs than the GPU has SMs and a longest loop of at least 32 iterations (counted as 64
+    half tiles). Backward in microseconds, whole / split. Taken: 1 x 4096 tokens, 14 / 2 heads, D 64 414 / 189; 1 x 2048, 32 / 8, D 128
+    200 / 194; 1 x 8192, 16 / 2 1284 / 901. Refused: 1 x 4096, 32 / 8 (256 CTAs, the longest 128 iterations against 114 per SM) 469 / 546;
+    16 x 512, 14 / 2 104 / 131. The line is not sharp: below it 1 x 512, 14 / 2 would gain (60 / 30), above it several
+    sequences lose where their average comes near the longest loop (2 x 1024, 32 / 8 121 / 141; 16 x 512, 16 / 2 174 / 254)."""
     G = Hq // Hkv
     if _HEAD_SPLIT in ("0", "1"):
         return G > 1 and _HEAD_SPLIT == "1"
