@@ -141,18 +141,19 @@ def _lib_skinny() -> ctypes.CDLL:
     return lib
 
 
-def _skinny_pays(M: int, N: int, K: int, swiglu: bool) -> bool:
+def _skinny_pays(M: int, N: int, K: int, swiglu: bool, bn: int = 0) -> bool:
     """Up to 16 rows (``rb_skinny``): weights streamed by every warp on its own. Microseconds of a chain of captured launches over weights
     that are not in L2, one-CTA kernel / this one: 2 rows: 896 x 896 8.2 / 2.5, 4096 x 4096 17.5 / 7.5, 28672 x 4096 71 / 46, 151936 x 896
     59.5 / 54; 16 rows: 896 x 896 8.2 / 4.2, 4096 x 4096 16.7 / 10.0. Each 8 rows cost it another pass of activations through L1 beside
     the weights: 8 rows with 151936 x 896 are 54 / 60, 16 rows 61.5 / 71.8, and 16 rows with 28672 x 4096 50.5 / 55 (rb_stream 42.4). With
     one or two 64-column blocks of K the partial sums are what takes the time past 8 rows (2048 x 128 with residual, 16 rows: 1.24 times
-    the one-CTA kernel); the one-CTA kernel's gated unit is so much slower there that this one stays better."""
+    the one-CTA kernel); the one-CTA kernel's gated unit is so much slower there that this one stays better. Gated units in blocks of 64, which
+    rb_stream does not take, are better here at any size (12 rows of 28672 x 4096 95 / 53, 16 rows 66 / 51)."""
     if M <= 6:
         return True
     if M <= 8:
         return N <= 1 << 17
-    return M <= 16 and N * K <= 60_000_000 and (K >= 256 or swiglu)
+    return M <= 16 and (N * K <= 60_000_000 or (swiglu and bn < 128)) and (K >= 256 or swiglu)
 
 
 def _stream_most_rows(N: int, K: int, swiglu: bool, norm: bool) -> int:
@@ -191,7 +192,7 @@ def _stream_most_rows(N: int, K: int, swiglu: bool, norm: bool) -> int:
 def _skinny_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail,
                   norm: bool = False) -> bool:
     """What it does not take (a layout the vector loads need, what the one-CTA kernel refuses or leaves unsaid) is left to the others."""
-    return (_skinny_pays(M, N, K, swiglu) and K % 16 == 0 and a.stride(0) % 16 == 0 and b.stride(0) % 16 == 0 and a.data_ptr() % 32 == 0
+    return (_skinny_pays(M, N, K, swiglu, bn) and K % 16 == 0 and a.stride(0) % 16 == 0 and b.stride(0) % 16 == 0 and a.data_ptr() % 32 == 0
             and b.data_ptr() % 32 == 0 and _few_rows_form(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail))
 
 

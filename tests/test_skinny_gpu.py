@@ -74,6 +74,8 @@ def test_sizes_at_which_few_row_kernels_pay():
              (32, 16384, 512), (32, 9728, 896), (64, 9728, 896, False, True), (24, 9728, 2048, False, True), (32, 16384, 2048), (64, 28672, 4096), (64, 3072, 1024), (12, 151936, 896), (40, 128256, 4096, True))):
         for s in sizes:
             assert rows(*s) == want, (want, s, rows(*s))
+    # gated units in blocks of 64, which the stream kernel does not take
+    assert gemm_mod._skinny_pays(12, 28672, 4096, True, 64) and not gemm_mod._skinny_pays(12, 28672, 4096, True, 256)
 
 
 @pytest.mark.gpu
