@@ -148,7 +148,7 @@ def _skinny_pays(M: int, N: int, K: int, swiglu: bool, bn: int = 0) -> bool:
     the weights: 8 rows with 151936 x 896 are 54 / 60, 16 rows 61.5 / 71.8, and 16 rows with 28672 x 4096 50.5 / 55 (rb_stream 42.4). With
     one or two 64-column blocks of K the partial sums are what takes the time past 8 rows (2048 x 128 with residual, 16 rows: 1.24 times
     the one-CTA kernel); the one-CTA kernel's gated unit is so much slower there that this one stays better. Gated units in blocks of 64, which
-    rb_stream does not take, are better here at any size (12 rows of 28672 x 4096 95 / 53, 16 rows 66 / 51)."""
+    rb_stream does not take, are better here at any size (12 rows of 28672 x 4096 91 / 51, 16 rows 67 / 51, 16 rows of 128256 x 4096 218 / 199)."""
     if M <= 6:
         return True
     if M <= 8:
