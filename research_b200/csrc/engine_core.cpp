@@ -710,6 +710,42 @@ int rbe_build_batch(void* h, int which, int* tokens, int* positions, int* slots,
   return t;
 }
 
+// Stages the scheduled decode rows for a captured step: `meta` holds fields of `mb` ints (tokens, positions, slots, lengths,
+// temperatures, seeds in two, state slots), rows behind the batch up to `padded` are marked as padding. Returns the number of rows and, in
+// *max_blocks, the longest block list; -1 if a buffer is too small.
+int rbe_stage_decode(void* h, int* meta, int mb, int padded, int* block_tables, int bt_stride, int with_slots, int* max_blocks) {
+  auto* e = static_cast<EngineCore*>(h);
+  const int bs = e->kv.pool.block_size, n = (int)e->sched_decode.size();
+  if (n > mb || padded > mb) return -1;
+  int* const tokens = meta, * const positions = meta + mb, * const slots = meta + 2 * mb, * const lens = meta + 3 * mb;
+  float* const temps = reinterpret_cast<float*>(meta + 4 * mb);
+  char* const seeds = reinterpret_cast<char*>(meta + 5 * mb);        // 64 bits a row; an odd mb leaves them on 4 bytes
+  int* const state = meta + 7 * mb;
+  int longest = 0;
+  for (int row = 0; row < n; ++row) {
+    const Seq* s = e->get(e->sched_decode[row]);
+    const int p = s->n_computed, blocks = (int)s->blocks.size();
+    if (blocks > bt_stride || s->n_target != p + 1) return -1;
+    tokens[row] = s->tokens[p];
+    positions[row] = p;
+    slots[row] = s->blocks[p / bs] * bs + p % bs;
+    lens[row] = s->n_target;
+    temps[row] = s->temperature;
+    const unsigned long long seed = s->seed + 0x9E3779B97F4A7C15ull * (unsigned long long)(s->n_target - s->n_prompt);
+    std::memcpy(seeds + 8 * (size_t)row, &seed, 8);
+    if (with_slots) state[row] = s->slot;
+    std::copy(s->blocks.begin(), s->blocks.end(), block_tables + (size_t)row * bt_stride);
+    longest = std::max(longest, (s->n_target + bs - 1) / bs);
+  }
+  for (int row = n; row < padded; ++row) {
+    tokens[row] = positions[row] = lens[row] = 0;
+    slots[row] = state[row] = -1;
+    temps[row] = 0.f;
+  }
+  *max_blocks = longest;
+  return n;
+}
+
 // State slots of the rows of a batch, in the order of rbe_build_batch (-1: the model keeps no state).
 void rbe_batch_slots(void* h, int which, int* out) {
   auto* e = static_cast<EngineCore*>(h);

@@ -233,6 +233,26 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 }
 
 // ------------------------------------------------------------------------------------------
+// Inputs of a step out of pinned host memory: `n` ints and the used part (rows x cols) of a block table with rows of `stride` ints.
+// What bounds it is a trip over PCIe (about 1.5 us). It stands before a captured step, not in it: kernels of a step read lengths and tables
+// before they wait for the launch before them.
+// ------------------------------------------------------------------------------------------
+__global__ void stage_step_kernel(const int* host, int* dev, int n, const int* host_table, int* dev_table, int stride, int rows, int cols) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int at = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  const int4* from = reinterpret_cast<const int4*>(host);      // allocations: 16-byte aligned
+  for (int i = at; i < n >> 2; i += step) reinterpret_cast<int4*>(dev)[i] = __ldcv(from + i);
+  if (at < (n & 3)) dev[(n & ~3) + at] = __ldcv(host + (n & ~3) + at);
+  const int cells = rows * cols;
+  for (int i = at; i < cells; i += step) {
+    const int r = i / cols;
+    const long long o = (long long)r * stride + (i - r * cols);
+    dev_table[o] = __ldcv(host_table + o);
+  }
+}
+
+// ------------------------------------------------------------------------------------------
 // Embedding gather: out[t, :] = table[ids[t], :]
 // ------------------------------------------------------------------------------------------
 __global__ void embedding_kernel(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
@@ -677,9 +697,11 @@ sample_logprob_kernel(const float* __restrict__ logits, long long ld, int V,
                       const float* __restrict__ temperature, const unsigned long long* __restrict__ seeds,
                       const unsigned long long* __restrict__ step_ptr, unsigned long long step_add,
                       int* __restrict__ out_tokens, float* __restrict__ out_logprobs,
-                      float4* __restrict__ partials /*[rows][splits], splits > 1 only*/, int* __restrict__ tickets /*[rows]*/) {
+                      float4* __restrict__ partials /*[rows][splits], splits > 1 only*/, int* __restrict__ tickets /*[rows]*/,
+                      const int* __restrict__ skip) {
   pdl_launch_dependents();
   pdl_wait();
+  if (skip != nullptr && *skip != 0) return;      // a captured step whose tokens are given: nobody reads what it would draw
   // grid (splits, rows): with few rows the vocabulary of a row is cut into `splits` contiguous chunks so that all
   // SMs share the transcendental work (three per element); the last CTA of a row merges the chunk records in
   // chunk order
@@ -915,6 +937,18 @@ extern "C" int rb_swiglu_bwd(const void* gu, const void* dout, void* dgu, long l
   return RB_CHECK_LAUNCH();
 }
 
+// Pointers of the host side are pinned memory; all buffers 16-byte aligned.
+extern "C" int rb_stage_step(const int* host, int* dev, int n, const int* host_table, int* dev_table, int stride, int rows, int cols,
+                             cudaStream_t stream) {
+  if (n < 0 || rows < 0 || cols < 0 || cols > stride || (long long)rows * cols > 0x7fffffffll) return -1;
+  if (((reinterpret_cast<uintptr_t>(host) | reinterpret_cast<uintptr_t>(dev)) & 15) != 0) return -1;
+  long long work = (n + 3) / 4;
+  if ((long long)rows * cols > work) work = (long long)rows * cols;
+  const long long want = (work + 255) / 256;
+  return launch_kernel(stage_step_kernel, dim3((unsigned)(want < 1 ? 1 : want > 148 ? 148 : want)), dim3(256), 0, stream, host, dev, n, host_table,
+                       dev_table, stride, rows, cols) == cudaSuccess ? 0 : -11;
+}
+
 extern "C" int rb_embedding(const int* ids, const void* table, void* out, int T, int d, int vocab,
                             int* status, cudaStream_t stream) {
   if (d % 8 != 0 || T <= 0) return -1;
@@ -928,21 +962,21 @@ extern "C" int rb_sample_logprob(const float* logits, long long ld, int B, int V
                                  cudaStream_t stream) {
   if (B <= 0) return 0;
   return launch_kernel(sample_logprob_kernel, dim3(1, B), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V, temperature,
-                       seeds, step_ptr, step_add, out_tokens, out_logprobs, (float4*)nullptr, (int*)nullptr) == cudaSuccess ? 0 : -11;
+                       seeds, step_ptr, step_add, out_tokens, out_logprobs, (float4*)nullptr, (int*)nullptr, (const int*)nullptr) == cudaSuccess ? 0 : -11;
 }
 // Same with every row's vocabulary cut into `splits` chunks (grid splits x B). `partials` holds B * splits float4
 // records, `tickets` B zero-initialised counters (they reset themselves). splits <= 0 picks about four CTAs per SM.
 extern "C" int rb_sample_logprob_split(const float* logits, long long ld, int B, int V, const float* temperature,
                                        const unsigned long long* seeds, const unsigned long long* step_ptr,
                                        unsigned long long step_add, int* out_tokens, float* out_logprobs, void* partials,
-                                       int* tickets, int splits, cudaStream_t stream) {
+                                       int* tickets, int splits, const int* skip, cudaStream_t stream) {
   if (B <= 0) return 0;
   if (splits <= 0) splits = (4 * 148 + B - 1) / B;
   if (splits > 8) splits = 8;
   while (splits > 1 && V / splits < 4096) --splits;
   if (splits > 1 && (partials == nullptr || tickets == nullptr)) return -1;
   return launch_kernel(sample_logprob_kernel, dim3(splits, B), dim3(SAMPLE_THREADS), 0, stream, logits, ld, V, temperature,
-                       seeds, step_ptr, step_add, out_tokens, out_logprobs, (float4*)partials, tickets) == cudaSuccess ? 0 : -11;
+                       seeds, step_ptr, step_add, out_tokens, out_logprobs, (float4*)partials, tickets, skip) == cudaSuccess ? 0 : -11;
 }
 
 extern "C" int rb_token_logprob(const float* logits, long long ld, int B, int V, const int* tokens,

@@ -14,6 +14,7 @@ tokens and log-probabilities -> commit (stop rules, block publication).
 from __future__ import annotations
 
 import ctypes
+from array import array
 from pathlib import Path
 
 import torch
@@ -46,6 +47,7 @@ def _core_lib():
         lib.rbe_open.argtypes = [_VP]
         lib.rbe_feed.argtypes = [_VP, _VP, _VP, _I, _VP]
         lib.rbe_commit_fed.argtypes = [_VP]
+        lib.rbe_stage_decode.argtypes = [_VP, _VP, _I, _I, _VP, _I, _I, _VP]
         for f in ("rbe_num_waiting", "rbe_num_running", "rbe_num_free_blocks", "rbe_num_finished", "rbe_check_invariants"):
             getattr(lib, f).argtypes = [_VP]
         lib.rbe_schedule.argtypes = [_VP, _VP]
@@ -120,6 +122,7 @@ class InferenceEngine:
         self.steps = 0
         self._counts = (_I * 6)()
         self._info = (_I * 5)()
+        self._longest = _I()
         self._seed_counter = config.seed * 1000003 + 12345
         self.eos_token_id = -1
         if not config.ignore_eos:
@@ -252,32 +255,25 @@ class InferenceEngine:
         self._launch_decode(n)
         self._sync()
 
-    def _launch_decode(self, n: int) -> None:
+    def _launch_decode(self, n: int, sample: bool = True) -> None:
         r = self.runner
-        mb, o = r.max_batch, r._pf_offsets()
-        base, pf = r.meta_host.data_ptr(), r.pf_host.data_ptr()
-        T = self._lib.rbe_build_batch(
-            self._core, 1, base, base + 4 * mb, base + 8 * mb, pf + 4 * o["cu_q"], base + 12 * mb, r.bt_host.data_ptr(),
-            r.max_blocks_per_seq, base + 16 * mb, base + 20 * mb, pf + 4 * o["sample_rows"], mb, mb)
-        assert T == n, T
-        if self.state_slots:      # (nothing else reads them)
-            self._lib.rbe_batch_slots(self._core, 1, base + 28 * mb)
-        max_blocks = -(-int(r.meta_rows[3 * mb:3 * mb + n].max()) // BLOCK)
-        r.stage_decode_padding(n)
-        r.decode(n, max_blocks)
+        rows = self._lib.rbe_stage_decode(self._core, r.meta_host.data_ptr(), r.max_batch, r.step_rows(n), r.bt_host.data_ptr(), r.max_blocks_per_seq,
+                                          int(self.state_slots > 0), ctypes.byref(self._longest))
+        assert rows == n, rows
+        r.decode(n, self._longest.value, sample)
 
     def _build_packed(self, which: int, n_rows: int) -> tuple[int, int, int, int]:
         """Stage the scheduled prefill (2) or decode + prefill (3) rows; returns the arguments of a packed pass."""
         r = self.runner
-        o, base = r._pf_offsets(), r.pf_host.data_ptr()
+        o, base = r.pf_at, r.pf_host.data_ptr()
         T = self._lib.rbe_build_batch(
             self._core, which, base + 4 * o["tokens"], base + 4 * o["positions"], base + 4 * o["slots"], base + 4 * o["cu_q"],
             base + 4 * o["seq_lens"], r.bt_host.data_ptr(), r.max_blocks_per_seq, base + 4 * o["temps"],
             base + 4 * o["seeds"], base + 4 * o["sample_rows"], r.max_prefill_tokens, r.max_batch)
         self._lib.rbe_batch_slots(self._core, which, base + 4 * o["state_slots"])
         assert T > 0, f"packed batch does not fit the staging buffers ({T})"
-        cu = r.pf_host[o["cu_q"]:o["cu_q"] + n_rows + 1]
-        return n_rows, T, int((cu[1:] - cu[:-1]).max()), self._max_blocks_in(r.pf_host[o["seq_lens"]:o["seq_lens"] + n_rows])
+        cu = r.pf_rows[o["cu_q"]:o["cu_q"] + n_rows + 1]
+        return n_rows, T, int((cu[1:] - cu[:-1]).max()), self._max_blocks_in(r.pf_rows[o["seq_lens"]:o["seq_lens"] + n_rows])
 
     # ---------------------------------------------------------------- given tokens instead of sampled ones
     def open_stream(self) -> int:
@@ -292,22 +288,27 @@ class InferenceEngine:
         assert entries and len({e[0] for e in entries}) == len(entries), "one entry per stream"
         lib, core, r = self._lib, self._core, self.runner
         n = len(entries)
+        streams, counts = array("q", [e[0] for e in entries]), array("i", [len(e[1]) for e in entries])
         flat = [t for _, toks, _ in entries for t in toks]
-        rc = lib.rbe_feed(core, (_LL * n)(*[e[0] for e in entries]), (_I * n)(*[len(e[1]) for e in entries]), n, (_I * len(flat))(*flat))
+        try:
+            flat = array("i", flat)
+        except OverflowError:              # no token: the kernels report it, as any other bad index
+            flat = array("i", (_I * len(flat))(*flat))
+        rc = lib.rbe_feed(core, streams.buffer_info()[0], counts.buffer_info()[0], n, flat.buffer_info()[0])
         if rc < 0:
             raise RuntimeError({-1: "feed: unknown stream or an entry without tokens", -2: "feed: the KV cache is full",
                                 -3: "feed: more tokens than the engine was made for", -4: "feed: every state slot is taken"}[rc])
         if lib.rbe_get_scheduled(core, None, None, None) == n:
             # single tokens only: rows in the order of the entries; their logits are taken before the step is waited for
-            self._launch_decode(n)
+            self._launch_decode(n, sample=False)
             wanted = [i + w for i, (_, _, places) in enumerate(entries) for w in places]
             out = None
             if wanted == list(range(n)):
                 out = r.a_logits[:n].clone(memory_format=torch.contiguous_format)
             elif wanted:
                 out = r.a_logits[:n].index_select(0, torch.tensor(wanted, device=self.device))
-            self._sync()
             lib.rbe_commit_fed(core)
+            self._sync()
             return out
         pre, dec = (_LL * n)(), (_LL * n)()
         n_dec = lib.rbe_get_scheduled(core, pre, dec, None)
@@ -345,7 +346,7 @@ class InferenceEngine:
         return self.has_pending() or (self.ep is not None and self.peers_pending)
 
     @staticmethod
-    def _max_blocks_in(seq_lens: torch.Tensor) -> int:
+    def _max_blocks_in(seq_lens) -> int:
         return int(-(-int(seq_lens.max()) // BLOCK))
 
     def _sync(self) -> None:

@@ -85,10 +85,11 @@ class RunnerBase:
 
     def _init_step_buffers(self, vocab_padded: int) -> None:
         device, mb = self.device, self.max_batch
-        # one int32 staging vector: tokens | positions | slots | seq_lens | temps | seeds(lo,hi) | state slots
+        # one int32 staging vector: tokens | positions | slots | seq_lens | temps | seeds(lo,hi) | state slots | 1 where nothing
+        # is to be sampled
         self.meta_fields = 8
-        self.meta_dev = torch.zeros(self.meta_fields * mb, dtype=torch.int32, device=device)
-        self.meta_host = self._pinned(torch.zeros(self.meta_fields * mb, dtype=torch.int32))
+        self.meta_dev = torch.zeros(self.meta_fields * mb + 1, dtype=torch.int32, device=device)
+        self.meta_host = self._pinned(torch.zeros(self.meta_fields * mb + 1, dtype=torch.int32))
         self.meta_rows = self.meta_host.numpy()          # the same memory: a few numbers a step are cheaper to read and write there
         self.bt_dev = torch.zeros(mb, self.max_blocks_per_seq, dtype=torch.int32, device=device)
         self.bt_host = self._pinned(torch.zeros(mb, self.max_blocks_per_seq, dtype=torch.int32))
@@ -99,6 +100,7 @@ class RunnerBase:
         self.d_temps = m[4 * mb:5 * mb].view(torch.float32)
         self.d_seeds = m[5 * mb:7 * mb].view(torch.int64)
         self.d_state_slots = m[7 * mb:8 * mb]
+        self.d_skip = m[8 * mb:8 * mb + 1]
         self.d_out_tokens = self.out_dev[0:mb]
         self.d_out_logprobs = self.out_dev[mb:2 * mb].view(torch.float32)
         self.logits_padded = torch.empty(mb, vocab_padded, dtype=torch.float32, device=device)
@@ -110,6 +112,8 @@ class RunnerBase:
         T = self.max_prefill_tokens
         self.pf_host = self._pinned(torch.zeros(3 * T + 7 * (mb + 1), dtype=torch.int32))
         self.pf_dev = torch.zeros_like(self.pf_host, device=device)
+        self.pf_rows = self.pf_host.numpy()
+        self.pf_at = self._pf_offsets()
 
     def _init_geometry(self, cfg, *, device, num_kv_blocks: int, max_batch: int, max_model_len: int, max_prefill_tokens: int,
                        use_cuda_graphs: bool, graph_batch_sizes: tuple[int, ...], dtype: torch.dtype) -> None:
@@ -136,9 +140,11 @@ class RunnerBase:
     def _pinned(self, t: torch.Tensor) -> torch.Tensor:
         return t.pin_memory() if self.on_gpu else t
 
-    def _sample(self, logits, temps, seeds, n: int) -> None:
+    def _sample(self, logits, temps, seeds, n: int, skip=None) -> None:
         if self.on_gpu:
-            ops.sample_with_logprobs(logits, temps, seeds, 0, None, self.d_out_tokens[:n], self.d_out_logprobs[:n])
+            ops.sample_with_logprobs(logits, temps, seeds, 0, None, self.d_out_tokens[:n], self.d_out_logprobs[:n], skip=skip)
+            return
+        if skip is not None and int(skip):
             return
         # CPU twin: one seeded generator per row so a request reproduces in any batch slot
         for r in range(n):
@@ -187,43 +193,43 @@ class RunnerBase:
         torch.cuda.synchronize(self.device)
         ops.check_status(self.device)
 
-    def decode(self, n: int, max_blocks: int) -> None:
+    def step_rows(self, n: int) -> int:
+        """Rows that a decode step of ``n`` sequences runs over."""
+        return self.bucket(n) if (self.use_cuda_graphs or self.row_align > 1) else max(n, 1)
+
+    def decode(self, n: int, max_blocks: int, sample: bool = True) -> None:
         """Run one decode step for the ``n`` rows staged in ``meta_host`` / ``bt_host``.
 
-        Host->device: one copy of the packed metadata vector and one 2-D copy of the used
-        block-table columns. Device->host: one copy of tokens|logprobs into ``out_host``.
-        The caller synchronises before reading ``out_host``.
+        Host->device: one kernel reads the metadata vector and the used block-table columns out of the pinned memory. Device->host: one copy of tokens|logprobs into ``out_host``, unless ``sample`` is off.
+        The caller synchronises before reading ``out_host`` or staging the next step.
         """
-        bk = self.bucket(n) if (self.use_cuda_graphs or self.row_align > 1) else max(n, 1)
-        self.meta_dev.copy_(self.meta_host, non_blocking=True)
-        self.bt_dev[:n, :max_blocks].copy_(self.bt_host[:n, :max_blocks], non_blocking=True)
+        bk = self.step_rows(n)
+        self.meta_rows[-1] = not sample
+        ops.stage_step(self.meta_host, self.meta_dev, self.bt_host, self.bt_dev, n, max_blocks)
         g = self.graphs.get(bk)
         if g is not None:
             g.replay()
         else:
             self._decode_body(bk)
-        self.out_host.copy_(self.out_dev, non_blocking=True)
+        if sample:
+            self.out_host.copy_(self.out_dev, non_blocking=True)
 
     def stage_decode_padding(self, n: int) -> None:
-        """Mark rows n..bucket as padding (no KV write, empty context)."""
-        bk = self.bucket(n) if (self.use_cuda_graphs or self.row_align > 1) else max(n, 1)
-        if bk > n:
-            mb, mh = self.max_batch, self.meta_rows
-            for field, fill in ((0, 0), (1, 0), (2, -1), (3, 0), (4, 0), (7, -1)):
-                mh[field * mb + n:field * mb + bk] = fill
+        """Mark the rows from n on as padding (no KV write, empty context)."""
+        mb, mh = self.max_batch, self.meta_rows
+        for field, fill in ((0, 0), (1, 0), (2, -1), (3, 0), (4, 0), (7, -1)):
+            mh[field * mb + n:(field + 1) * mb] = fill
 
     # ------------------------------------------------------------------ packed batches
     def _stage_packed(self, rows: int, T: int, max_new: int, max_blocks: int) -> "PackedBatch":
         """Copy the batch staged in ``pf_host`` / ``bt_host`` (filled by the engine core) to the device."""
-        o = self._pf_offsets()
-        ph = self.pf_host
+        o, ph = self.pf_at, self.pf_rows
         Tp = -(-T // self.row_align) * self.row_align  # padded row count (tensor parallel only)
         if Tp > T:
             ph[o["tokens"] + T:o["tokens"] + Tp] = 0
             ph[o["positions"] + T:o["positions"] + Tp] = 0
             ph[o["slots"] + T:o["slots"] + Tp] = -1   # padding rows never touch the KV cache
-        self.pf_dev.copy_(ph, non_blocking=True)
-        self.bt_dev[:rows, :max_blocks].copy_(self.bt_host[:rows, :max_blocks], non_blocking=True)
+        ops.stage_step(self.pf_host, self.pf_dev, self.bt_host, self.bt_dev, rows, max_blocks)
         pd = self.pf_dev
         cu = ph[o["cu_q"]:o["cu_q"] + rows + 1].tolist()
         return PackedBatch(
@@ -251,10 +257,14 @@ class RunnerBase:
 
     def packed_logits(self, rows: int, T: int, max_new: int, max_blocks: int, wanted: list[int]) -> torch.Tensor | None:
         """The same pass without sampling: fp32 logits ``[len(wanted), V]`` of the packed rows ``wanted``."""
-        b = self._stage_packed(rows, T, max_new, max_blocks)
-        at = torch.tensor(wanted, dtype=torch.int32).to(self.device) if wanted else None      # before the pass: the copy waits for what is queued
-        x = self._packed_forward(b)
-        return self._row_logits(x, at) if wanted else None
+        n, o = len(wanted), self.pf_at["sample_rows"]
+        if n <= self.max_batch:        # they travel in the place of the rows to sample
+            self.pf_rows[o:o + n] = wanted
+            at = self.pf_dev[o:o + n]
+        else:                          # before the pass: the copy waits for what is queued
+            at = torch.tensor(wanted, dtype=torch.int32).to(self.device)
+        x = self._packed_forward(self._stage_packed(rows, T, max_new, max_blocks))
+        return self._row_logits(x, at) if n else None
 
     # ------------------------------------------------------------------ teacher forcing
     def score(self, token_ids: torch.Tensor) -> torch.Tensor:
@@ -547,7 +557,7 @@ class ModelRunner(RunnerBase):
             tp.gemm_reduce_scatter(act, lw.wd, xs, residual=xs)
         ops.rmsnorm(xs, self.final_norm, eps, out=hs)
         logits = gathered(self.lm_head, self.a_logits[:bk], out_f32=True)
-        self._sample(logits, self.d_temps[:bk], self.d_seeds[:bk], bk)
+        self._sample(logits, self.d_temps[:bk], self.d_seeds[:bk], bk, self.d_skip)
         tp.comm.barrier(self._sp_slot)     # every peer has read hs: the next step may overwrite it
 
     def _decode_body(self, bk: int) -> None:
@@ -569,9 +579,9 @@ class ModelRunner(RunnerBase):
 
         self._forward_layers(x, h, bk, self.d_pos[:bk], self.d_slots[:bk], attn_fn, static=True)
         ops.rmsnorm(x[:bk], self.final_norm, cfg.rms_norm_eps, out=h[:bk])
-        self._lm_head_sample(h[:bk], self.d_temps[:bk], self.d_seeds[:bk], bk)
+        self._lm_head_sample(h[:bk], self.d_temps[:bk], self.d_seeds[:bk], bk, self.d_skip)
 
-    def _lm_head_sample(self, h, temps, seeds, n: int) -> None:
+    def _lm_head_sample(self, h, temps, seeds, n: int, skip=None) -> None:
         """Final projection + sampling. On the GPU one GEMM whose epilogue reduces each tile to a sampling record
         (no [n, vocab] fp32 logits are written), then a merge kernel (RB_FUSED_SAMPLE=1); default is the GEMM followed by
         the sampling kernel, which measured faster."""
@@ -580,7 +590,7 @@ class ModelRunner(RunnerBase):
                                workspace=self.sample_ws)
             return
         logits = ops.gemm(h, self.lm_head, out=self.a_logits[:n], out_f32=True, constant_b=True)
-        self._sample(logits, temps, seeds, n)
+        self._sample(logits, temps, seeds, n, skip)
 
     # ------------------------------------------------------------------ packed batches
     def _packed_forward(self, b: PackedBatch) -> torch.Tensor:

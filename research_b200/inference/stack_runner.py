@@ -374,7 +374,7 @@ class StackRunner(RunnerBase):
         self._layers(self._decode_batch(bk))
         self._final_rows(self.x[:bk], self.hl)
         logits = self._head(self.hl[:bk], self.logits_padded[:bk])
-        self._sample(logits, self.d_temps[:bk], self.d_seeds[:bk], bk)
+        self._sample(logits, self.d_temps[:bk], self.d_seeds[:bk], bk, self.d_skip)
 
     def capture_graphs(self) -> None:
         super().capture_graphs()

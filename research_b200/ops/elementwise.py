@@ -28,6 +28,8 @@ def _lib() -> ctypes.CDLL:
         lib.rb_swiglu_bounded.argtypes = [c_vp, c_vp, c_ll, c_int, c_vp, c_vp]
         lib.rb_swiglu_bounded.restype = c_int
         lib.rb_embedding.argtypes = [c_vp, c_vp, c_vp, c_int, c_int, c_int, c_vp, c_vp]
+        lib.rb_stage_step.argtypes = [c_vp, c_vp, c_int, c_vp, c_vp, c_int, c_int, c_int, c_vp]
+        lib.rb_stage_step.restype = c_int
         lib.rb_transpose_bf16.argtypes = [c_vp, c_vp, c_int, c_int, c_vp]
         lib.rb_layernorm.argtypes = [c_vp, c_ll, c_vp, c_ll] + [c_vp] * 4 + [c_ll, c_int, c_int, c_int, c_float, c_int, c_vp, c_vp]
         lib.rb_clamped_glu.argtypes = [c_vp, c_vp, c_int, c_ll, c_int, c_float, c_vp]
@@ -42,6 +44,23 @@ def _lib() -> ctypes.CDLL:
             getattr(lib, f).restype = c_int
         lib._rb_typed = True
     return lib
+
+
+# ------------------------------------------------------------------------------- inputs of a step
+def stage_step(host: torch.Tensor, dev: torch.Tensor, host_table: torch.Tensor, dev_table: torch.Tensor, rows: int,
+               cols: int) -> None:
+    """Copy the int32 vector ``host`` and the first ``rows x cols`` of ``host_table``, both pinned, to the device in one launch."""
+    if not dev.is_cuda:
+        dev.copy_(host)
+        dev_table[:rows, :cols].copy_(host_table[:rows, :cols])
+        return
+    if not all(t.dtype == torch.int32 and t.is_contiguous() for t in (host, host_table, dev, dev_table)) or not (host.is_pinned() and host_table.is_pinned()):
+        raise ValueError("stage_step: contiguous int32 tensors, those of the host pinned")
+    if host.numel() != dev.numel() or host_table.shape != dev_table.shape or rows > dev_table.shape[0] or cols > dev_table.shape[1]:
+        raise ValueError("stage_step: sizes of host and device differ")
+    rc = _lib().rb_stage_step(ptr(host), ptr(dev), host.numel(), ptr(host_table), ptr(dev_table), dev_table.shape[1], rows, cols,
+                              stream_handle(dev.device))
+    check_rc(rc, "rb_stage_step")
 
 
 # ------------------------------------------------------------------------------- RMSNorm

@@ -22,7 +22,7 @@ def _lib() -> ctypes.CDLL:
     if not getattr(lib, "_rb_typed_s", False):
         lib.rb_sample_logprob.argtypes = [c_vp, c_ll, c_int, c_int, c_vp, c_vp, c_vp, c_ull, c_vp, c_vp, c_vp]
         lib.rb_sample_logprob.restype = c_int
-        lib.rb_sample_logprob_split.argtypes = [c_vp, c_ll, c_int, c_int, c_vp, c_vp, c_vp, c_ull, c_vp, c_vp, c_vp, c_vp, c_int, c_vp]
+        lib.rb_sample_logprob_split.argtypes = [c_vp, c_ll, c_int, c_int, c_vp, c_vp, c_vp, c_ull, c_vp, c_vp, c_vp, c_vp, c_int, c_vp, c_vp]
         lib.rb_sample_logprob_split.restype = c_int
         lib.rb_token_logprob.argtypes = [c_vp, c_ll, c_int, c_int, c_vp, c_vp, c_vp]
         lib.rb_token_logprob.restype = c_int
@@ -43,17 +43,19 @@ def sample_with_logprobs_reference(logits: torch.Tensor, temperatures: torch.Ten
 
 
 def sample_with_logprobs(logits, temperatures, seeds=None, step: int = 0, step_tensor=None, out_tokens=None,
-                         out_logprobs=None):
+                         out_logprobs=None, skip=None):
     """Sample one token per row of fp32 ``logits [B, V]``.
 
     ``seeds`` (uint64 per row, stored as int64) and ``step`` select the random stream, so a
-    request reproduces its samples regardless of which batch slot it occupies.
+    request reproduces its samples regardless of which batch slot it occupies. A non-zero int32 in the device tensor ``skip``
+    leaves both outputs as they are (a captured step whose tokens the caller gives).
     """
     if not logits.is_cuda:
         g = None
         if seeds is not None:
             g = torch.Generator().manual_seed(int(seeds[0].item()) * 1000003 + step)
         return sample_with_logprobs_reference(logits, temperatures, g)
+    assert skip is None or (skip.is_cuda and skip.dtype == torch.int32)
     assert logits.dtype == torch.float32 and logits.stride(1) == 1
     B, V = logits.shape
     if seeds is None:
@@ -65,7 +67,7 @@ def sample_with_logprobs(logits, temperatures, seeds=None, step: int = 0, step_t
     part, tickets = _split_scratch(logits.device, B)
     rc = _lib().rb_sample_logprob_split(ptr(logits), logits.stride(0), B, V, ptr(temperatures), ptr(seeds), ptr(step_tensor),
                                         step, ptr(out_tokens), ptr(out_logprobs), ptr(part), ptr(tickets), 0,
-                                        stream_handle(logits.device))
+                                        ptr(skip), stream_handle(logits.device))
     check_rc(rc, "rb_sample_logprob_split")
     return out_tokens, out_logprobs
 
