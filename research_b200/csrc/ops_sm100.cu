@@ -8,77 +8,90 @@
 namespace rb {
 
 // ------------------------------------------------------------------------------------------
-// RMSNorm: y = bf16( bf16(x * rsqrt(mean(x^2)+eps)) * w ). One warp per row.
+// RMSNorm: y = bf16( bf16(x * rsqrt(mean(x^2)+eps)) * w ).
 // Reference math: rollouts/tools/functional_extractor/qwen_functional.py:46-65.
 // ------------------------------------------------------------------------------------------
-// The row is read from global memory once: up to 8 vectors of 8 bf16 per lane stay in
-// registers (d <= 2048); longer rows fall back to a second read that hits L1/L2.
+__device__ __forceinline__ float square_sum8(uint4 u, float ss) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = unpack_bf16x2(w[j]);
+    ss += f.x * f.x + f.y * f.y;
+  }
+  return ss;
+}
+__device__ __forceinline__ uint4 rms_scaled(uint4 u, uint4 ww, float rstd) {
+  const uint32_t xi[4] = {u.x, u.y, u.z, u.w}, wi[4] = {ww.x, ww.y, ww.z, ww.w};
+  uint32_t oi[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = unpack_bf16x2(xi[j]), g = unpack_bf16x2(wi[j]);
+    // round the normalised value to bf16 before the weight multiply, like the HF module
+    const float a = __bfloat162float(__float2bfloat16_rn(f.x * rstd)), b = __bfloat162float(__float2bfloat16_rn(f.y * rstd));
+    oi[j] = pack_bf16x2(a * g.x, b * g.y);
+  }
+  return make_uint4(oi[0], oi[1], oi[2], oi[3]);
+}
+
+// blockDim.x threads a row (blockDim.y rows where that is a warp), V vectors of 8 a thread in registers: the row is read once, and all of its loads and those of the weight are in flight
+// together. Few rows are a chain of latencies (V = 1 spreads a row over as many threads as it has vectors): 32 rows of 4096 took 4.8 us
+// with a warp a row, now 2.1. Many rows are bound by bytes: 8192 of 4096 took 29.9 us, now 24.8.
+template <int V>
+__global__ void __launch_bounds__(V == 4 ? 512 : 1024) rmsnorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                   __nv_bfloat16* __restrict__ y, long long rows, int d, long long ldx, long long ldy, float eps) {
+  __shared__ float red[32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long row = (long long)blockIdx.x * blockDim.y + threadIdx.y;
+  if (row >= rows) return;
+  const __nv_bfloat16* xr = x + row * ldx;
+  __nv_bfloat16* yr = y + row * ldy;
+  const int nvec = d >> 3;
+  uint4 keep[V], ww[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    keep[i] = v < nvec ? *reinterpret_cast<const uint4*>(xr + v * 8) : make_uint4(0, 0, 0, 0);
+    ww[i] = v < nvec ? *reinterpret_cast<const uint4*>(w + v * 8) : make_uint4(0, 0, 0, 0);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i) ss = square_sum8(keep[i], ss);
+  ss = warp_sum(ss);
+  const int warps = blockDim.x >> 5;
+  if (warps > 1) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();
+    ss = warp_sum(lane < warps ? red[lane] : 0.f);
+  }
+  const float rstd = rsqrtf(ss / (float)d + eps);
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int v = threadIdx.x + i * blockDim.x;
+    if (v < nvec) *reinterpret_cast<uint4*>(yr + v * 8) = rms_scaled(keep[i], ww[i], rstd);
+  }
+}
+
+// Rows of any length, one warp each, read twice.
 __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                __nv_bfloat16* __restrict__ y, long long rows, int d, long long ldx,
                                long long ldy, float eps) {
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int MAXV = 8;
   const int lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const __nv_bfloat16* xr = x + row * ldx;
   __nv_bfloat16* yr = y + row * ldy;
   const int nvec = d >> 3;
-  const bool in_regs = nvec <= MAXV * 32;
-  uint4 keep[MAXV];
   float ss = 0.f;
-  if (in_regs) {
-#pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int v = lane + 32 * i;
-      keep[i] = v < nvec ? *reinterpret_cast<const uint4*>(xr + v * 8) : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      float2 f;
-      f = unpack_bf16x2(keep[i].x); ss += f.x * f.x + f.y * f.y;
-      f = unpack_bf16x2(keep[i].y); ss += f.x * f.x + f.y * f.y;
-      f = unpack_bf16x2(keep[i].z); ss += f.x * f.x + f.y * f.y;
-      f = unpack_bf16x2(keep[i].w); ss += f.x * f.x + f.y * f.y;
-    }
-  } else {
-    for (int v = lane; v < nvec; v += 32) {
-      uint4 u = *reinterpret_cast<const uint4*>(xr + v * 8);
-      float2 f;
-      f = unpack_bf16x2(u.x); ss += f.x * f.x + f.y * f.y;
-      f = unpack_bf16x2(u.y); ss += f.x * f.x + f.y * f.y;
-      f = unpack_bf16x2(u.z); ss += f.x * f.x + f.y * f.y;
-      f = unpack_bf16x2(u.w); ss += f.x * f.x + f.y * f.y;
-    }
-  }
+  for (int v = lane; v < nvec; v += 32) ss = square_sum8(*reinterpret_cast<const uint4*>(xr + v * 8), ss);
   ss = warp_sum(ss);
   const float rstd = rsqrtf(ss / (float)d + eps);
-  auto emit = [&](int v, uint4 u) {
-    uint4 ww = *reinterpret_cast<const uint4*>(w + v * 8);
-    uint32_t xi[4] = {u.x, u.y, u.z, u.w};
-    uint32_t wi[4] = {ww.x, ww.y, ww.z, ww.w};
-    uint32_t oi[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 f = unpack_bf16x2(xi[j]);
-      float2 g = unpack_bf16x2(wi[j]);
-      // round the normalised value to bf16 before the weight multiply, like the HF module
-      float a = __bfloat162float(__float2bfloat16_rn(f.x * rstd));
-      float b = __bfloat162float(__float2bfloat16_rn(f.y * rstd));
-      oi[j] = pack_bf16x2(a * g.x, b * g.y);
-    }
-    *reinterpret_cast<uint4*>(yr + v * 8) = make_uint4(oi[0], oi[1], oi[2], oi[3]);
-  };
-  if (in_regs) {
-#pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int v = lane + 32 * i;
-      if (v < nvec) emit(v, keep[i]);
-    }
-  } else {
-    for (int v = lane; v < nvec; v += 32) emit(v, *reinterpret_cast<const uint4*>(xr + v * 8));
-  }
+  for (int v = lane; v < nvec; v += 32)
+    *reinterpret_cast<uint4*>(yr + v * 8) =
+        rms_scaled(*reinterpret_cast<const uint4*>(xr + v * 8), *reinterpret_cast<const uint4*>(w + v * 8), rstd);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -87,85 +100,165 @@ __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
 //   q_out : [T, Hq * D] bf16 (rotated)
 //   k_cache / v_cache : [num_blocks, Hkv, block_size, D] bf16, slot = block*block_size + off
 //   cos_sin : [max_pos, D/2] float2
-// One warp per (token, head). Slots < 0 are skipped (padding rows of a captured graph).
+// A thread takes E elements of a head's first half and the E that rotate with them. Many tokens are bound by moving qkv once: E = 8, 16-byte
+// accesses (WIDE: all pointers are 16-byte aligned). With a warp a head and 2-byte accesses 16384 tokens of 14 + 2 + 2 heads of 64 took
+// 48 us, 8192 of 32 + 8 + 8 of 128 84 us; now 21 and 57. Few tokens are a chain of latencies, which E = 2 keeps shorter
+// (128 tokens of 14 + 2 + 2 heads: 1.85 us, E = 8 2.18).
+// Slots < 0 are skipped (padding rows of a captured graph).
 // Reference math: qwen_functional.py:68-150; cache store: inference/attention/flex_backend.py:116-142.
 // ------------------------------------------------------------------------------------------
-template <int D>
+template <int E> struct Pairs { uint32_t w[E / 2]; };
+template <int E, bool WIDE> __device__ __forceinline__ Pairs<E> load_pairs(const __nv_bfloat16* p) {
+  Pairs<E> r;
+  if constexpr (WIDE && E == 8) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    r.w[0] = v.x; r.w[1] = v.y; r.w[2] = v.z; r.w[3] = v.w;
+  } else if constexpr (WIDE) {
+#pragma unroll
+    for (int i = 0; i < E / 2; ++i) r.w[i] = reinterpret_cast<const uint32_t*>(p)[i];
+  } else {
+    const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
+#pragma unroll
+    for (int i = 0; i < E / 2; ++i) r.w[i] = h[2 * i] | ((uint32_t)h[2 * i + 1] << 16);
+  }
+  return r;
+}
+template <int E, bool WIDE> __device__ __forceinline__ void store_pairs(__nv_bfloat16* p, const Pairs<E>& v) {
+  if constexpr (WIDE && E == 8) {
+    *reinterpret_cast<uint4*>(p) = make_uint4(v.w[0], v.w[1], v.w[2], v.w[3]);
+  } else if constexpr (WIDE) {
+#pragma unroll
+    for (int i = 0; i < E / 2; ++i) reinterpret_cast<uint32_t*>(p)[i] = v.w[i];
+  } else {
+    unsigned short* h = reinterpret_cast<unsigned short*>(p);
+#pragma unroll
+    for (int i = 0; i < E / 2; ++i) {
+      h[2 * i] = (unsigned short)v.w[i];
+      h[2 * i + 1] = (unsigned short)(v.w[i] >> 16);
+    }
+  }
+}
+template <int E> __device__ __forceinline__ void to_floats(const Pairs<E>& v, float (&f)[E]) {
+#pragma unroll
+  for (int i = 0; i < E / 2; ++i) {
+    const float2 x = unpack_bf16x2(v.w[i]);
+    f[2 * i] = x.x;
+    f[2 * i + 1] = x.y;
+  }
+}
+
+// blockDim.x: a multiple of 32; items of `tokens` tokens a CTA
+template <int D, int E, bool WIDE>
 __global__ void rope_kv_append_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ q_out,
                                       __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
                                       const int* __restrict__ positions, const int* __restrict__ slots,
                                       const float2* __restrict__ cos_sin, const __nv_bfloat16* __restrict__ q_norm_w,
                                       const __nv_bfloat16* __restrict__ k_norm_w, float norm_eps, int T, int Hq,
-                                      int Hkv, int block_size, long long num_slots, int max_pos, int* status) {
-  constexpr int HALF = D / 2;
-  constexpr int PER_LANE = HALF / 32;  // pairs handled per lane: D=64 -> 1, D=128 -> 2
+                                      int Hkv, int block_size, long long num_slots, int max_pos, int tokens, int* status) {
+  constexpr int HALF = D / 2, G = HALF / E;       // G threads a head
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31;
-  const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int heads = Hq + 2 * Hkv;
-  if (gw >= (long long)T * heads) return;
-  const int t = (int)(gw / heads);
-  const int h = (int)(gw % heads);
-  const __nv_bfloat16* src = qkv + (long long)t * heads * D + (long long)h * D;
-  int pos = positions[t];
-  const int slot = slots[t];
-  if (pos < 0) pos = 0;
-  if (pos >= max_pos) { set_status(status, ST_BAD_INDEX); pos = max_pos - 1; }
-
-  float lo[PER_LANE], hi[PER_LANE];
-#pragma unroll
-  for (int j = 0; j < PER_LANE; ++j) {
-    lo[j] = __bfloat162float(src[lane + 32 * j]);
-    hi[j] = __bfloat162float(src[lane + 32 * j + HALF]);
-  }
-  __nv_bfloat16* dst;
-  bool is_v = h >= Hq + Hkv;
-  if (h < Hq) {
-    dst = q_out + (long long)t * Hq * D + (long long)h * D;
-  } else {
-    if (slot < 0) return;
-    if (slot >= num_slots) { set_status(status, ST_BAD_INDEX); return; }
-    const int kvh = is_v ? h - Hq - Hkv : h - Hq;
-    const long long blk = slot / block_size, off = slot % block_size;
-    __nv_bfloat16* cache = is_v ? v_cache : k_cache;
-    dst = cache + ((blk * Hkv + kvh) * block_size + off) * D;
-  }
-  if (is_v) {
-#pragma unroll
-    for (int j = 0; j < PER_LANE; ++j) {
-      dst[lane + 32 * j] = __float2bfloat16_rn(lo[j]);
-      dst[lane + 32 * j + HALF] = __float2bfloat16_rn(hi[j]);
+  const int heads = Hq + 2 * Hkv, per = heads * G;
+  const long long t0 = (long long)blockIdx.x * tokens;
+  const int items = (int)min((long long)tokens, T - t0) * per;
+  for (int base = 0; base < items; base += blockDim.x) {
+    const int item = base + threadIdx.x;
+    const bool in = item < items;              // a head's threads are in one warp and agree; the shuffles want the whole warp
+    const int tl = in ? item / per : 0, rest = in ? item - tl * per : 0, h = rest / G, c = (rest - h * G) * E;
+    const long long t = t0 + tl;
+    const __nv_bfloat16* src = qkv + (t * heads + h) * D + c;
+    const Pairs<E> raw_lo = load_pairs<E, WIDE>(src), raw_hi = load_pairs<E, WIDE>(src + HALF);
+    int pos = positions[t];
+    const int slot = slots[t];
+    const bool is_v = h >= Hq + Hkv;
+    if (pos < 0) pos = 0;
+    if (pos >= max_pos) {
+      if (in) set_status(status, ST_BAD_INDEX);
+      pos = max_pos - 1;
     }
-    return;
-  }
-  const __nv_bfloat16* nw = (h < Hq) ? q_norm_w : k_norm_w;
-  if (nw != nullptr) {
-    float ss = 0.f;
-#pragma unroll
-    for (int j = 0; j < PER_LANE; ++j) ss += lo[j] * lo[j] + hi[j] * hi[j];
-    ss = warp_sum(ss);
-    const float rstd = rsqrtf(ss / (float)D + norm_eps);
-#pragma unroll
-    for (int j = 0; j < PER_LANE; ++j) {
-      float a = __bfloat162float(__float2bfloat16_rn(lo[j] * rstd));
-      float b = __bfloat162float(__float2bfloat16_rn(hi[j] * rstd));
-      lo[j] = __bfloat162float(__float2bfloat16_rn(a * __bfloat162float(nw[lane + 32 * j])));
-      hi[j] = __bfloat162float(__float2bfloat16_rn(b * __bfloat162float(nw[lane + 32 * j + HALF])));
+    bool write = in;
+    __nv_bfloat16* dst = q_out + (t * Hq + h) * D + c;
+    if (h >= Hq) {
+      if (slot < 0) {
+        write = false;
+      } else if (slot >= num_slots) {
+        if (in) set_status(status, ST_BAD_INDEX);
+        write = false;
+      } else {
+        const int kvh = is_v ? h - Hq - Hkv : h - Hq;
+        const long long blk = slot / block_size, off = slot % block_size;
+        dst = (is_v ? v_cache : k_cache) + ((blk * Hkv + kvh) * block_size + off) * D + c;
+      }
     }
-  }
+    if (q_norm_w == nullptr && k_norm_w == nullptr) {
+      if (!write) continue;
+      if (is_v) {
+        store_pairs<E, WIDE>(dst, raw_lo);
+        store_pairs<E, WIDE>(dst + HALF, raw_hi);
+        continue;
+      }
+    }
+    float lo[E], hi[E];
+    to_floats(raw_lo, lo);
+    to_floats(raw_hi, hi);
+    const __nv_bfloat16* nw = (h < Hq) ? q_norm_w : k_norm_w;
+    if (q_norm_w != nullptr || k_norm_w != nullptr) {
+      float ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < PER_LANE; ++j) {
-    const float2 cs = cos_sin[(long long)pos * HALF + lane + 32 * j];
-    // bf16 rounding of cos/sin and of each product mirrors q*cos + rotate_half(q)*sin in bf16
-    const float c = __bfloat162float(__float2bfloat16_rn(cs.x));
-    const float s = __bfloat162float(__float2bfloat16_rn(cs.y));
-    const float a = __bfloat162float(__float2bfloat16_rn(lo[j] * c));
-    const float b = __bfloat162float(__float2bfloat16_rn(-hi[j] * s));
-    const float e = __bfloat162float(__float2bfloat16_rn(hi[j] * c));
-    const float f = __bfloat162float(__float2bfloat16_rn(lo[j] * s));
-    dst[lane + 32 * j] = __float2bfloat16_rn(a + b);
-    dst[lane + 32 * j + HALF] = __float2bfloat16_rn(e + f);
+      for (int j = 0; j < E; ++j) ss += lo[j] * lo[j] + hi[j] * hi[j];
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (!write) continue;
+      if (is_v) {
+        store_pairs<E, WIDE>(dst, raw_lo);
+        store_pairs<E, WIDE>(dst + HALF, raw_hi);
+        continue;
+      }
+      if (nw != nullptr) {
+        const float rstd = rsqrtf(ss / (float)D + norm_eps);
+        float wl[E], wh[E];
+        to_floats(load_pairs<E, WIDE>(nw + c), wl);
+        to_floats(load_pairs<E, WIDE>(nw + c + HALF), wh);
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+          const float a = __bfloat162float(__float2bfloat16_rn(lo[j] * rstd));
+          const float b = __bfloat162float(__float2bfloat16_rn(hi[j] * rstd));
+          lo[j] = __bfloat162float(__float2bfloat16_rn(a * wl[j]));
+          hi[j] = __bfloat162float(__float2bfloat16_rn(b * wh[j]));
+        }
+      }
+    }
+    const float2* cs_row = cos_sin + (long long)pos * HALF + c;
+    Pairs<E> ol, oh;
+#pragma unroll
+    for (int j = 0; j < E; j += 2) {
+      float2 cs[2];
+      if (WIDE) {
+        const float4 v = *reinterpret_cast<const float4*>(cs_row + j);
+        cs[0] = make_float2(v.x, v.y);
+        cs[1] = make_float2(v.z, v.w);
+      } else {
+        cs[0] = cs_row[j];
+        cs[1] = cs_row[j + 1];
+      }
+      float first[2], second[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        // bf16 rounding of cos/sin and of each product mirrors q*cos + rotate_half(q)*sin in bf16
+        const float co = __bfloat162float(__float2bfloat16_rn(cs[i].x));
+        const float si = __bfloat162float(__float2bfloat16_rn(cs[i].y));
+        const float a = __bfloat162float(__float2bfloat16_rn(lo[j + i] * co));
+        const float b = __bfloat162float(__float2bfloat16_rn(-hi[j + i] * si));
+        const float e = __bfloat162float(__float2bfloat16_rn(hi[j + i] * co));
+        const float f = __bfloat162float(__float2bfloat16_rn(lo[j + i] * si));
+        first[i] = a + b;
+        second[i] = e + f;
+      }
+      ol.w[j / 2] = pack_bf16x2(first[0], first[1]);
+      oh.w[j / 2] = pack_bf16x2(second[0], second[1]);
+    }
+    store_pairs<E, WIDE>(dst, ol);
+    store_pairs<E, WIDE>(dst + HALF, oh);
   }
 }
 
@@ -578,7 +671,7 @@ __global__ void __launch_bounds__(256) poly_norm_kernel(const TA* __restrict__ z
   }
 }
 
-// Layer norm of fp32 rows with a two-pass variance; the row is kept in shared memory.
+// Layer norm of fp32 rows with a two-pass variance; the row is kept in registers (layernorm_row_kernel, below) or in shared memory.
 //   y == nullptr : out = LN(x[rows[i]]) * w + b                     (rows == nullptr: row i)
 //   otherwise    : x += LN(y) * w + b, out = x                      (norm on the sublayer's output, residual add)
 // The caller folds a layer scale into w and b.
@@ -618,6 +711,71 @@ __global__ void layernorm_kernel(const float* __restrict__ y, long long ldy, flo
       x[r * ldx + c] = v;
     }
     out[r * ldo + c] = to_act<TA>(v);
+  }
+}
+
+// The same for rows of 4 V blockDim.x elements at most whose pointers and strides are multiples of four elements: every load of the row, the
+// weights and the residual is in flight before the first sum. 4 rows of 2048 took 5.0 us from shared memory, now 2.3; 5210 rows
+// 50.6 us, now 26.1 (bytes).
+template <typename TA> __device__ __forceinline__ void store_four(TA* p, float4 v);
+template <> __device__ __forceinline__ void store_four<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+template <> __device__ __forceinline__ void store_four<__nv_bfloat16>(__nv_bfloat16* p, float4 v) {
+  *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+}
+template <typename TA, int V>
+__global__ void __launch_bounds__(1024) layernorm_row_kernel(const float* __restrict__ y, long long ldy, float* __restrict__ x, long long ldx,
+                                     const int* __restrict__ rows, const float* __restrict__ w, const float* __restrict__ b,
+                                     TA* __restrict__ out, long long ldo, int d, float eps, int num_src_rows, int* status) {
+  __shared__ float red[2][32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long r = blockIdx.x;
+  long long xr = r;
+  if (rows != nullptr) {
+    xr = rows[r];
+    if (xr < 0 || xr >= num_src_rows) { if (threadIdx.x == 0) set_status(status, ST_BAD_INDEX); xr = 0; }
+  }
+  const float* src = y != nullptr ? y + r * ldy : x + xr * ldx;
+  float4 v[V], ww[V], bb[V], res[V];
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int c = 4 * (threadIdx.x + i * blockDim.x);
+    const bool in = c < d;
+    v[i] = in ? *reinterpret_cast<const float4*>(src + c) : zero;
+    ww[i] = in ? *reinterpret_cast<const float4*>(w + c) : zero;
+    bb[i] = in ? *reinterpret_cast<const float4*>(b + c) : zero;
+    res[i] = in && y != nullptr ? *reinterpret_cast<const float4*>(x + r * ldx + c) : zero;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  auto total = [&](float s, float* at) {
+    s = warp_sum(s);
+    if (lane == 0) at[warp] = s;
+    __syncthreads();
+    return warp_sum(lane < warps ? at[lane] : 0.f);
+  };
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+  const float mean = total(s, red[0]) / (float)d;
+  float q = 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    v[i] = make_float4(v[i].x - mean, v[i].y - mean, v[i].z - mean, v[i].w - mean);
+    if (4 * (threadIdx.x + i * blockDim.x) < d) q += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+  }
+  const float rstd = 1.f / sqrtf(total(q, red[1]) / (float)d + eps);
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int c = 4 * (threadIdx.x + i * blockDim.x);
+    if (c >= d) continue;
+    float4 o = make_float4(fmaf(v[i].x * rstd, ww[i].x, bb[i].x), fmaf(v[i].y * rstd, ww[i].y, bb[i].y), fmaf(v[i].z * rstd, ww[i].z, bb[i].z),
+                           fmaf(v[i].w * rstd, ww[i].w, bb[i].w));
+    if (y != nullptr) {
+      o = make_float4(o.x + res[i].x, o.y + res[i].y, o.z + res[i].z, o.w + res[i].w);
+      *reinterpret_cast<float4*>(x + r * ldx + c) = o;
+    }
+    store_four(out + r * ldo + c, o);
   }
 }
 
@@ -882,7 +1040,19 @@ extern "C" void rb_ops_set_pdl(int on) { rb::pdl_enabled() = on != 0; }
 extern "C" int rb_rmsnorm(const void* x, const void* w, void* y, long long rows, int d, long long ldx,
                           long long ldy, float eps, cudaStream_t stream) {
   if (d % 8 != 0 || rows <= 0) return -1;
-  const int warps = rows >= 148 * 8 * 4 ? 8 : 2;   // few rows: spread them over more SMs
+  const int nvec = d >> 3;
+  // few rows: one vector a thread; many: about four, which leaves enough CTAs an SM to hide the reduction
+  const int v = rows <= 148 && nvec <= 1024 ? 1 : 4;
+  if (nvec <= (v == 4 ? 2048 : 1024) && rows <= 0x7fffffffll) {
+    const unsigned a_row = (unsigned)(((nvec + v - 1) / v + 31) / 32 * 32);
+    const dim3 threads(a_row, a_row == 32 && v > 1 ? 8 : 1);
+#define RB_RMSNORM(VV) launch_kernel(rmsnorm_row_kernel<VV>, dim3((unsigned)((rows + threads.y - 1) / threads.y)), threads, 0, stream, (const __nv_bfloat16*)x, \
+                                     (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rows, d, ldx, ldy, eps)
+    const cudaError_t e = v == 1 ? RB_RMSNORM(1) : RB_RMSNORM(4);
+#undef RB_RMSNORM
+    return e == cudaSuccess ? 0 : -11;
+  }
+  const int warps = 8;
   const long long grid = (rows + warps - 1) / warps;
   return launch_kernel(rmsnorm_kernel, dim3((unsigned)grid), dim3(warps * 32), 0, stream, (const __nv_bfloat16*)x,
                        (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rows, d, ldx, ldy, eps) == cudaSuccess ? 0 : -11;
@@ -894,18 +1064,26 @@ extern "C" int rb_rope_kv_append(const void* qkv, void* q_out, void* k_cache, vo
                                  int Hkv, int D, int block_size, long long num_slots, int max_pos,
                                  int* status, cudaStream_t stream) {
   if (T <= 0) return 0;
-  const long long warps_total = (long long)T * (Hq + 2 * Hkv);
-  const int warps = 8;
-  const unsigned grid = (unsigned)((warps_total + warps - 1) / warps);
-#define LAUNCH_ROPE(DD)                                                                              \
-  launch_kernel(rope_kv_append_kernel<DD>, dim3(grid), dim3(warps * 32), 0, stream,                   \
+  if (D != 64 && D != 128) return -1;
+  // about 256 threads a CTA, whole tokens; narrow accesses while they leave an SM no more than a CTA
+  const bool few = (long long)T * (Hq + 2 * Hkv) * (D / 4) <= 148 * 256;
+  const int per = (Hq + 2 * Hkv) * (few ? D / 4 : D / 16);
+  const int tokens = per >= 256 ? 1 : 256 / per;
+  const int threads = min((tokens * per + 31) / 32 * 32, 512);
+  const unsigned grid = (unsigned)(((long long)T + tokens - 1) / tokens);
+  bool wide = true;
+  for (const void* q : {qkv, (const void*)q_out, (const void*)k_cache, (const void*)v_cache, cos_sin, q_norm_w, k_norm_w})
+    wide = wide && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+#define LAUNCH_ROPE(DD, EE, WW)                                                                      \
+  launch_kernel(rope_kv_append_kernel<DD, EE, WW>, dim3(grid), dim3(threads), 0, stream,              \
       (const __nv_bfloat16*)qkv, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, \
       positions, slots, (const float2*)cos_sin, (const __nv_bfloat16*)q_norm_w,                       \
-      (const __nv_bfloat16*)k_norm_w, norm_eps, T, Hq, Hkv, block_size, num_slots, max_pos, status)
+      (const __nv_bfloat16*)k_norm_w, norm_eps, T, Hq, Hkv, block_size, num_slots, max_pos, tokens, status)
+#define LAUNCH_ROPE_WIDE(DD, EE) (wide ? LAUNCH_ROPE(DD, EE, true) : LAUNCH_ROPE(DD, EE, false))
   cudaError_t e;
-  if (D == 64) { e = LAUNCH_ROPE(64); }
-  else if (D == 128) { e = LAUNCH_ROPE(128); }
-  else return -1;
+  if (D == 64) e = few ? LAUNCH_ROPE_WIDE(64, 2) : LAUNCH_ROPE_WIDE(64, 8);
+  else e = few ? LAUNCH_ROPE_WIDE(128, 2) : LAUNCH_ROPE_WIDE(128, 8);
+#undef LAUNCH_ROPE_WIDE
 #undef LAUNCH_ROPE
   return e == cudaSuccess ? 0 : -11;
 }
@@ -1075,8 +1253,21 @@ extern "C" int rb_token_side(const float* z, long long ldz, const int* ids, cons
 extern "C" int rb_layernorm(const float* y, long long ldy, float* x, long long ldx, const int* rows, const float* w, const float* b, void* out,
                             long long ldo, int dtype, int n, int d, float eps, int num_src_rows, int* status, cudaStream_t stream) {
   if (n <= 0 || d <= 0 || d > 12288 || ldo < d || (y != nullptr && rows != nullptr)) return -1;
-  const int threads = d <= 512 ? 128 : 256;
   cudaError_t e;
+  const int elem = dtype == 1 ? 4 : 2;
+  const uintptr_t floats = reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(b);
+  if (d % 4 == 0 && d <= 8192 && (y == nullptr || ldy % 4 == 0) && ldx % 4 == 0 && ldo % 4 == 0 && (floats & 15) == 0 &&
+      reinterpret_cast<uintptr_t>(out) % (4 * elem) == 0) {
+    // few rows: a row over up to 1024 threads; many: two vectors a thread
+    const int quads = d / 4, v = n <= 148 && quads <= 1024 ? 1 : 2;
+    const dim3 threads((unsigned)(((quads + v - 1) / v + 31) / 32 * 32));
+    RB_ACT_DISPATCH(dtype, e = v == 1 ? launch_kernel(layernorm_row_kernel<TA, 1>, dim3(n), threads, 0, stream, y, ldy, x, ldx, rows, w, b, (TA*)out, ldo,
+                                                      d, eps, num_src_rows, status)
+                                      : launch_kernel(layernorm_row_kernel<TA, 2>, dim3(n), threads, 0, stream, y, ldy, x, ldx, rows, w, b, (TA*)out, ldo,
+                                                      d, eps, num_src_rows, status);)
+    return e == cudaSuccess ? 0 : -11;
+  }
+  const int threads = d <= 512 ? 128 : 256;
   RB_ACT_DISPATCH(dtype, e = launch_kernel(layernorm_kernel<TA>, dim3(n), dim3(threads), (size_t)d * 4, stream, y, ldy, x, ldx, rows, w, b,
                                            (TA*)out, ldo, d, eps, num_src_rows, status);)
   return e == cudaSuccess ? 0 : -11;
