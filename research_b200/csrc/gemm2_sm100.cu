@@ -66,6 +66,12 @@ struct G2Params {
   int silu_cols, tail_col;            // as in RbGemmArgs
   float* tail;
   long long tail_ld;
+  // Folded RMS norm of A's rows: the sum of norm_sq[i M + row] over norm_parts parts i is a row's sum of squares. sq_out (bf16 output of plain
+  // products): the sums of squares of the stored rows, part i from column tile i.
+  const float* norm_sq;
+  int norm_parts;
+  float norm_eps;
+  float* sq_out;
   int* status;
   // Vocabulary epilogue (G2_DLOGITS): a tile's fp32 logits become their gradient and never leave the tensor memory.
   const int* targets;                 // [M]
@@ -333,11 +339,19 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
       tile_mn(t, mt, nt);
       const int acc = tile_iter % G2_ACC;
       const uint32_t acc_ph = (tile_iter / G2_ACC) & 1u;
+      const int row0 = mt * 256 + (int)cta * G2_BM + q * 32;       // of the group's M rows; whole boxes of 32 belong to it
+      const bool row_ok = row0 + lane < p.M;
+      float norm = 1.f, squares = 0.f;
+      if constexpr (EPI == G2_STORE || EPI == G2_GLU) {
+        if (p.norm_sq != nullptr && row_ok) {     // loaded while the main loop runs
+          float s = 0.f;
+          for (int i = 0; i < p.norm_parts; ++i) s += p.norm_sq[(long long)i * p.M + row0 + lane];
+          norm = rsqrtf(s / (float)p.K + p.norm_eps);
+        }
+      }
       ok = mbar_wait_bounded_cluster(smem_u32(&tmem_full_bar[acc]), acc_ph, abortp, p.status, ST_TIMEOUT_TMEM_FULL);
       if (!ok) break;
       tc_fence_after();
-      const int row0 = mt * 256 + (int)cta * G2_BM + q * 32;       // of the group's M rows; whole boxes of 32 belong to it
-      const bool row_ok = row0 + lane < p.M;
       const int group_row = EPI == G2_GROUPS ? t / (m_tiles * n_tiles) * p.M : 0;
       const long long row = (long long)group_row + row0 + lane;
       const int n_base = nt * BN;
@@ -367,6 +381,13 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
           uint32_t up[32];
           tmem_ld_32x32(tmem_base + acc * BN + BN / 2 + c0 + ((uint32_t)(q * 32) << 16), up);
           tmem_ld_wait();
+          if (p.norm_sq != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              r[j] = __float_as_uint(__uint_as_float(r[j]) * norm);
+              up[j] = __float_as_uint(__uint_as_float(up[j]) * norm);
+            }
+          }
           if (p.glu_kind == 1) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = clamped_glu_epi(__uint_as_float(r[j]), __uint_as_float(up[j]), p.glu_limit);
@@ -386,6 +407,10 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = dlogit_epi(v[j], l, glp, gent, H, c0 + j == target);
         } else if constexpr (EPI == G2_STORE || EPI == G2_GROUPS) {
+          if (EPI == G2_STORE && p.norm_sq != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] *= norm;
+          }
           if (row_ok && p.bias != nullptr) {
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
@@ -416,6 +441,13 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
           if (col < p.silu_cols && !tail) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = silu_fast(v[j]);
+          }
+          if (EPI == G2_STORE && p.sq_out != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const float f = j < ncols ? __bfloat162float(__float2bfloat16_rn(v[j])) : 0.f;
+              squares = fmaf(f, f, squares);
+            }
           }
         }
         const bool second = !f32 && (c0 & 32);
@@ -458,6 +490,7 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
           pending = false;
         }
       }
+      if (EPI == G2_STORE && p.sq_out != nullptr && row_ok) p.sq_out[(long long)nt * p.M + row0 + lane] = squares;
       // accumulator drained in this CTA: tell the leader's MMA thread
       tc_fence_before();
       __syncwarp();
@@ -526,10 +559,13 @@ extern "C" int rb_gemm2_pairs() {
 // [K, rows] with rows contiguous (as in rb_gemm_bf16). bn: 256 or 128 output columns per tile (0 = choose).
 // glu: 0, or 1 silu(gate) * up / 2 the clamped unit, of B's rows in blocks of 128 gate and 128 up (K-major
 // operands, N a multiple of 256, bf16 output [M, N / 2], nothing added).
+// norm_sq [norm_parts, M] (K-major operands): C's sums are scaled by the RMS norm of A's rows, whose squares these parts add up to.
+// sq_out [column tiles of bn, M]: the squares of the bf16 rows as they are stored (no unit, tail or fp32 output).
 extern "C" int rb_gemm2_bf16(const void* A, const void* B, void* C, const void* bias, const void* residual, int M, int N,
                              int K, long long lda, long long ldb, long long ldc, long long ldr, int a_mn_major,
                              int b_mn_major, int out_f32, int bn, int silu_cols, float* tail, int tail_col, long long tail_ld,
-                             int glu, float glu_limit, int* status, cudaStream_t stream) {
+                             int glu, float glu_limit, const float* norm_sq, int norm_parts, float norm_eps, float* sq_out, int* status,
+                             cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0 || N % 8 != 0) return -1;
   if ((!a_mn_major || !b_mn_major) && K % 8 != 0) return -1;
   if (a_mn_major && !b_mn_major) return -12;         // not used by forward, dgrad or wgrad
@@ -550,6 +586,9 @@ extern "C" int rb_gemm2_bf16(const void* A, const void* B, void* C, const void* 
   p.glu_kind = glu == 2; p.glu_limit = glu_limit;
   p.silu_cols = silu_cols; p.tail = tail; p.tail_col = tail_col; p.tail_ld = tail_ld;
   if (silu_cols % 32 != 0 || (tail != nullptr && (tail_col % 32 != 0 || tail_ld % 4 != 0))) return -1;
+  if (norm_sq != nullptr && (a_mn_major || norm_parts < 1)) return -1;
+  if (sq_out != nullptr && (glu != 0 || tail != nullptr || out_f32)) return -1;
+  p.norm_sq = norm_sq; p.norm_parts = norm_parts; p.norm_eps = norm_eps; p.sq_out = sq_out;
   p.status = status;
   int rc = a_mn_major ? tma_map_2d_bf16(&p.a_map, A, K, M, lda, G2_BK) : tma_map_2d_bf16(&p.a_map, A, M, K, lda, G2_BM);
   if (rc != 0) return -20 + rc;

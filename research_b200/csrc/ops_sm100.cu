@@ -94,6 +94,20 @@ __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
         rms_scaled(*reinterpret_cast<const uint4*>(xr + v * 8), *reinterpret_cast<const uint4*>(w + v * 8), rstd);
 }
 
+// out[row] = sum of squares of a row, a warp each: for the folded norm of a product whose input no product left with its squares.
+__global__ void row_squares_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ out, int rows, int d, long long ldx) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const __nv_bfloat16* xr = x + row * ldx;
+  float ss = 0.f;
+#pragma unroll 4
+  for (int v = lane; v < d >> 3; v += 32) ss = square_sum8(*reinterpret_cast<const uint4*>(xr + v * 8), ss);
+  ss = warp_sum(ss);
+  if (lane == 0) out[row] = ss;
+}
+
 // ------------------------------------------------------------------------------------------
 // RoPE (rotate_half convention) + optional per-head QK RMSNorm + paged KV append.
 //   qkv   : [T, (Hq + 2*Hkv) * D] bf16  (q heads, then k heads, then v heads)
@@ -1056,6 +1070,12 @@ extern "C" int rb_rmsnorm(const void* x, const void* w, void* y, long long rows,
   const long long grid = (rows + warps - 1) / warps;
   return launch_kernel(rmsnorm_kernel, dim3((unsigned)grid), dim3(warps * 32), 0, stream, (const __nv_bfloat16*)x,
                        (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rows, d, ldx, ldy, eps) == cudaSuccess ? 0 : -11;
+}
+
+extern "C" int rb_row_squares(const void* x, float* out, int rows, int d, long long ldx, cudaStream_t stream) {
+  if (rows <= 0 || d % 8 != 0 || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0) return -1;
+  return launch_kernel(row_squares_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, stream, (const __nv_bfloat16*)x, out, rows, d, ldx) ==
+                 cudaSuccess ? 0 : -11;
 }
 
 extern "C" int rb_rope_kv_append(const void* qkv, void* q_out, void* k_cache, void* v_cache,

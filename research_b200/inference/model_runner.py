@@ -480,12 +480,14 @@ class ModelRunner(RunnerBase):
                 lw.wgu.mul_(lw.ln2[None, :])
 
     # ------------------------------------------------------------------ layer math
-    def _mlp(self, lw: LayerWeights, h: torch.Tensor, x: torch.Tensor, n: int, static: bool) -> None:
-        """x += MLP(post-attention norm of x) for the first n rows; ``h`` is scratch for the normalised rows."""
+    def _mlp(self, lw: LayerWeights, h: torch.Tensor, x: torch.Tensor, n: int, static: bool, squares=None) -> None:
+        """x += MLP(post-attention norm of x) for the first n rows; ``h`` is scratch for the normalised rows, ``squares`` goes with x."""
         cfg = self.cfg
         if lw.moe is not None:
             ops.rmsnorm(x[:n], lw.ln2, cfg.rms_norm_eps, out=h[:n])
             lw.moe.forward(h[:n], x[:n])
+            if squares is not None:
+                squares.n = 0
             return
         if self.fold_norm:
             src, eps = x, cfg.rms_norm_eps
@@ -495,24 +497,28 @@ class ModelRunner(RunnerBase):
         gu = self.a_gu[:n] if static else None
         act = self.a_act[:n] if static else None
         if self.fuse_swiglu:
-            act = ops.gemm(src[:n], lw.wgu, out=act, bn=self.swiglu_bn, swiglu=True, norm_eps=eps, constant_b=True)
+            act = ops.gemm(src[:n], lw.wgu, out=act, bn=self.swiglu_bn, swiglu=True, norm_eps=eps, constant_b=True, squares=squares)
         else:
-            gu = ops.gemm(src[:n], lw.wgu, out=gu, norm_eps=eps, constant_b=True)
+            gu = ops.gemm(src[:n], lw.wgu, out=gu, norm_eps=eps, constant_b=True, squares=squares)
             act = ops.swiglu(gu, out=act)
-        self._row_parallel(act, lw.wd, x[:n])
+        self._row_parallel(act, lw.wd, x[:n], squares)
 
-    def _row_parallel(self, a: torch.Tensor, w: torch.Tensor, x: torch.Tensor) -> None:
+    def _row_parallel(self, a: torch.Tensor, w: torch.Tensor, x: torch.Tensor, squares=None) -> None:
         """x += a @ w.T, summed over tensor-parallel ranks when sharded."""
         if self.tp is None or self.tp_size == 1:
-            ops.gemm(a, w, residual=x, out=x, constant_b=True)
-        else:
-            self.tp.gemm_all_reduce(a, w, x)
+            ops.gemm(a, w, residual=x, out=x, constant_b=True, leave_squares=squares)
+            return
+        self.tp.gemm_all_reduce(a, w, x)
+        if squares is not None:
+            squares.n = 0
 
     def _forward_layers(self, x, h, n, positions, slots, attn_fn, static: bool):
         cfg = self.cfg
+        squares = ops.RowSquares(n, cfg.hidden_size, x.device) if self.fold_norm and self.on_gpu and n >= 512 else None
         for li, lw in enumerate(self.layers):
             if self.fold_norm:
-                qkv = ops.gemm(x[:n], lw.wqkv, bias=lw.bqkv, out=self.a_qkv[:n] if static else None, norm_eps=cfg.rms_norm_eps, constant_b=True)
+                qkv = ops.gemm(x[:n], lw.wqkv, bias=lw.bqkv, out=self.a_qkv[:n] if static else None, norm_eps=cfg.rms_norm_eps, constant_b=True,
+                               squares=squares)
             else:
                 ops.rmsnorm(x[:n], lw.ln1, cfg.rms_norm_eps, out=h[:n])
                 qkv = ops.gemm(h[:n], lw.wqkv, bias=lw.bqkv, out=self.a_qkv[:n] if static else None, constant_b=True)
@@ -520,8 +526,8 @@ class ModelRunner(RunnerBase):
                                    self.Hkv, self.D, lw.q_norm, lw.k_norm, cfg.rms_norm_eps,
                                    q_out=self.a_q[:n] if static else None)
             attn = attn_fn(li, q.view(n, self.Hq, self.D))
-            self._row_parallel(attn.view(n, self.Hq * self.D), lw.wo, x[:n])
-            self._mlp(lw, h, x, n, static)
+            self._row_parallel(attn.view(n, self.Hq * self.D), lw.wo, x[:n], squares)
+            self._mlp(lw, h, x, n, static, squares)
 
     # ------------------------------------------------------------------ decode
     def _decode_body_sp(self, bk: int) -> None:

@@ -17,6 +17,7 @@ from .elementwise import (
     layernorm_reference,
     layernorm_residual,
     layernorm_rows,
+    RowSquares,
     rmsnorm,
     rmsnorm_reference,
     rope_kv_append,
@@ -84,7 +85,7 @@ __all__ = [
     "paged_decode_reference", "paged_prefill", "paged_prefill_reference", "embedding", "rmsnorm",
     "rmsnorm_reference", "rope_kv_append", "rope_kv_append_reference", "rope_table", "swiglu", "swiglu_backward",
     "swiglu_reference", "transpose", "gemm", "gemm_reference", "linear", "sample_with_logprobs",
-    "sample_with_logprobs_reference", "token_logprobs", "set_pdl", "interleave_gate_up", "gemm_mod", "gemm_symmetric", "gemm_fp8", "quantize_fp8", "lm_head_sample", "lm_head_sample_workspace", "stage_step", "flash_attention", "flash_attn_varlen",
+    "sample_with_logprobs_reference", "token_logprobs", "set_pdl", "interleave_gate_up", "gemm_mod", "gemm_symmetric", "gemm_fp8", "quantize_fp8", "lm_head_sample", "lm_head_sample_workspace", "stage_step", "RowSquares", "flash_attention", "flash_attn_varlen",
     "flash_attn_varlen_backward", "flash_attn_varlen_reference", "flash_paged_prefill", "flash_latent_prefill", "flash_latent_supported", "clamped_glu", "clamped_glu_reference",
     "layernorm_reference", "layernorm_residual", "layernorm_rows", "softcap", "gemm_f32", "LatentGeometry",
     "head_gemm_absorb", "head_gemm_expand", "latent_append", "latent_attention", "latent_gather", "latent_plan", "latent_query", "latent_units", "latent_workspace",

@@ -28,6 +28,8 @@ def _lib() -> ctypes.CDLL:
         lib.rb_swiglu_bounded.argtypes = [c_vp, c_vp, c_ll, c_int, c_vp, c_vp]
         lib.rb_swiglu_bounded.restype = c_int
         lib.rb_embedding.argtypes = [c_vp, c_vp, c_vp, c_int, c_int, c_int, c_vp, c_vp]
+        lib.rb_row_squares.argtypes = [c_vp, c_vp, c_int, c_int, c_ll, c_vp]
+        lib.rb_row_squares.restype = c_int
         lib.rb_stage_step.argtypes = [c_vp, c_vp, c_int, c_vp, c_vp, c_int, c_int, c_int, c_vp]
         lib.rb_stage_step.restype = c_int
         lib.rb_transpose_bf16.argtypes = [c_vp, c_vp, c_int, c_int, c_vp]
@@ -88,6 +90,21 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6, out: torch.Tens
     rc = _lib().rb_rmsnorm(ptr(x2), ptr(w), ptr(o2), x2.shape[0], d, x2.stride(0), o2.stride(0), eps, stream_handle(x.device))
     check_rc(rc, "rb_rmsnorm")
     return out.reshape(x.shape)
+
+
+class RowSquares:
+    """Sums of squares of the rows of a bf16 matrix ``[rows, cols]`` in ``n`` parts that add up to them (``n`` 0: not known). A product leaves them
+    with the matrix it writes (``gemm(leave_squares=)``); the product that reads the matrix through a folded norm takes them (``squares=``)."""
+
+    def __init__(self, rows: int, cols: int, device) -> None:
+        self.parts = torch.empty(max(1, -(-cols // 256)), rows, dtype=torch.float32, device=device)
+        self.n = 0
+
+    def measure(self, x: torch.Tensor) -> None:
+        """From the matrix itself, in a launch of its own."""
+        rc = _lib().rb_row_squares(ptr(x), ptr(self.parts), x.shape[0], x.shape[1], x.stride(0), stream_handle(x.device))
+        check_rc(rc, "rb_row_squares")
+        self.n = 1
 
 
 # ------------------------------------------------------------------------------- RoPE tables

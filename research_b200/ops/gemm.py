@@ -13,6 +13,7 @@ import os
 import torch
 
 from .. import _native
+from .elementwise import RowSquares
 from ._util import check_rc, ptr, status_tensor, stream_handle
 
 RB_MAX_PARTS = 8
@@ -117,7 +118,7 @@ def _lib2() -> ctypes.CDLL:
     lib = _native.load("rb_gemm2")
     if not getattr(lib, "_rb_typed", False):
         vp, i, ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
-        lib.rb_gemm2_bf16.argtypes = [vp] * 5 + [i, i, i, ll, ll, ll, ll, i, i, i, i, i, vp, i, ll, i, ctypes.c_float, vp, vp]
+        lib.rb_gemm2_bf16.argtypes = [vp] * 5 + [i, i, i, ll, ll, ll, ll, i, i, i, i, i, vp, i, ll, i, ctypes.c_float, vp, i, ctypes.c_float, vp, vp, vp]
         lib.rb_gemm2_bf16.restype = i
         lib.rb_gemm2_pairs.restype = i
         lib.rb_gemm2_bf16_gather.argtypes = ([vp] * 5 + [i, i, i, ll, ll, ll, ll, i, i, i] +
@@ -236,14 +237,24 @@ def _use_pair_kernel(M: int, N: int, K: int, a_mn_major: bool, b_mn_major: bool)
 def _pair_glu_takes(N: int, bn: int, bias, residual, out_f32: bool, silu_cols: int, tail) -> bool:
     """The gated unit in the two-CTA kernel's epilogue: its tile is 256 columns, so are the blocks of gate and up rows. Microseconds, one-CTA
     kernel / this one: 8192 x 28672 x 4096 1490 / 1272, 1500 x 28672 x 4096 350 / 280, 5210 x 16384 x 2048 328 / 263, 600 x 16384 x 2048
-    76 / 67. With a folded norm, whose row sums the one-CTA kernel takes from its operand tiles, the two are equal at 10000 rows
-    (a launch more here), so it stays there."""
+    76 / 67."""
     return bn == 256 and N % 256 == 0 and bias is None and residual is None and not out_f32 and not silu_cols and tail is None
+
+
+def _pair_norm_takes(a: torch.Tensor, squares: RowSquares | None, silu_cols: int, tail) -> bool:
+    """A folded norm on the two-CTA kernel, whose epilogue scales by the rows' squares that the product before it left or a short launch
+    measures. Microseconds (L2 flushed), one-CTA kernel with four warps that square its operand tiles / this one with squares left / measured:
+    gated 9820 x 9728 x 896 162 / 152 / 161, 3000 66 / 60 / 68, 512 27 / 26 / 34; 9820 x 1152 x 896 44 / 34 / 42, 3000 25 / 21 / 29; gated 9820 x 16384 x
+    2048 536 / 407 / 413, 512 47 / 39 / 44; 1500 x 3072 x 2048 44 / 36 / 40, 1024 40 / 34 / 40."""
+    if (squares is None or squares.n == 0) and a.shape[1] < 2048 and a.shape[0] < 8192:
+        return False
+    return a.shape[1] % 8 == 0 and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and not silu_cols and tail is None
 
 
 def gemm2(a: torch.Tensor, b: torch.Tensor, bias=None, residual=None, out=None, *, a_mn_major=False, b_mn_major=False,
           out_f32=False, bn: int = 0, silu_cols: int = 0, tail: torch.Tensor | None = None,
-          swiglu: bool = False, glu_limit: float | None = None) -> torch.Tensor:
+          swiglu: bool = False, glu_limit: float | None = None, norm_eps: float | None = None, squares: RowSquares | None = None,
+          leave_squares: RowSquares | None = None) -> torch.Tensor:
     """``C = op(A) @ op(B)^T (+bias) (+residual)`` on the two-CTA (``cta_group::2``) kernel; same operand conventions
     as ``gemm`` (``silu_cols``, ``tail`` and, for ``bn`` 256, ``swiglu`` too). ``bn``: 256 or 128 output columns per
     tile (0 = fewest waves)."""
@@ -260,9 +271,13 @@ def gemm2(a: torch.Tensor, b: torch.Tensor, bias=None, residual=None, out=None, 
                                out.stride(0), residual.stride(0) if residual is not None else 0, int(a_mn_major),
                                int(b_mn_major), int(out_f32), bn, silu_cols, tail.data_ptr() if tail is not None else None,
                                N - tail.shape[1] if tail is not None else 0, tail.stride(0) if tail is not None else 0,
-                               (2 if glu_limit is not None else 1) if swiglu else 0, glu_limit or 0.0, status_tensor(a.device).data_ptr(),
+                               (2 if glu_limit is not None else 1) if swiglu else 0, glu_limit or 0.0,
+                               ptr(squares.parts) if norm_eps is not None else None, squares.n if norm_eps is not None else 0, norm_eps or 0.0,
+                               ptr(leave_squares.parts) if leave_squares is not None else None, status_tensor(a.device).data_ptr(),
                                stream_handle(a.device))
     check_rc(rc, "rb_gemm2_bf16")
+    if leave_squares is not None:
+        leave_squares.n = -(-N // (bn or (256 if N > 128 else 128)))
     return out
 
 
@@ -369,6 +384,8 @@ def gemm(
     silu_cols: int = 0,
     tail: torch.Tensor | None = None,
     constant_b: bool = False,
+    squares: RowSquares | None = None,
+    leave_squares: RowSquares | None = None,
 ) -> torch.Tensor:
     """``C[M,N] = alpha * op(A) @ op(B)^T (+bias) (+ beta * residual)``.
 
@@ -384,7 +401,9 @@ def gemm(
 
     ``norm_eps`` folds an RMSNorm of A's rows into the launch: ``C = rstd(row) * (A @ B^T) (+bias)`` with
     ``rstd = rsqrt(mean(A[row]^2) + norm_eps)``; together with the norm weight multiplied into B's columns
-    beforehand this equals ``rmsnorm(A) @ B^T`` without a separate normalisation pass.
+    beforehand this equals ``rmsnorm(A) @ B^T`` without a separate normalisation pass. ``squares``: what is known of the squares of A's rows (large
+    products measure them first where nothing is known, others take them from their operand tiles). ``leave_squares``, of the shape of the output, receives
+    those of the stored rows, or is marked as unknown.
 
     ``glu_limit`` makes the fused gate|up epilogue (``swiglu=True``) the clamped unit of ``elementwise.clamped_glu``;
     ``softcap`` stores ``softcap * tanh(C / softcap)``. ``silu_cols``: the first so many columns are stored as ``silu(C)``.
@@ -459,11 +478,19 @@ def gemm(
     if softcap > 0:
         assert not swiglu and split_k in (0, 1), "the soft cap belongs to a plain store"
         split_k, cluster_split = 1, False
-    if (gather is None and softcap == 0 and wait_flag is None and norm_eps is None and alpha == 1.0 and beta == 1.0 and max_ctas == 0 and split_k in (0, 1)
-            and not cluster_split and _use_pair_kernel(M, N, K, a_mn_major, b_mn_major)
+    if leave_squares is not None:
+        leave_squares.n = 0
+    if (gather is None and softcap == 0 and wait_flag is None and alpha == 1.0 and beta == 1.0 and max_ctas == 0 and split_k in (0, 1)
+            and not cluster_split and _use_pair_kernel(M, N, K, a_mn_major, b_mn_major) and (norm_eps is None or _pair_norm_takes(a, squares, silu_cols, tail))
             and (_pair_glu_takes(N, bn, bias, residual, out_f32, silu_cols, tail) if swiglu else bn == 0)):
+        if norm_eps is not None:
+            squares = squares if squares is not None else RowSquares(M, 1, a.device)
+            if squares.n == 0:
+                squares.measure(a)
+        if out_f32 or tail is not None or swiglu:
+            leave_squares = None
         return gemm2(a, b, bias, residual, out, a_mn_major=a_mn_major, b_mn_major=b_mn_major, out_f32=out_f32, silu_cols=silu_cols, tail=tail,
-                     swiglu=swiglu, glu_limit=glu_limit)
+                     swiglu=swiglu, glu_limit=glu_limit, norm_eps=norm_eps, squares=squares, leave_squares=leave_squares)
     if silu_cols or tail is not None:
         assert gather is None and wait_flag is None and not swiglu and norm_eps is None and alpha == beta == 1.0 and not out_f32 and softcap == 0, \
             "silu_cols and tail belong to a plain store"
