@@ -106,7 +106,9 @@ logprob_entropy_fwd_kernel(const float* __restrict__ logits, long long ld, int V
   }
 }
 
-// dlogits[j] = g_lp * (1[j == t] - p_j) - g_ent * p_j * (log p_j + H)
+// dlogits[j] = g_lp * (1[j == t] - p_j) - g_ent * p_j * (log p_j + H). WIDE: V and both row strides are multiples of 8, both bases 16-byte aligned.
+// What bounds it is six bytes an element: with pairs of elements a thread 2048 x 151936 took 343 us, with eight (two loads, one store) 296.
+template <bool WIDE>
 __global__ void __launch_bounds__(ROW_THREADS)
 logprob_entropy_bwd_kernel(const float* __restrict__ logits, long long ld, int V, const int* __restrict__ targets,
                            const float* __restrict__ lse, const float* __restrict__ entropy,
@@ -120,6 +122,19 @@ logprob_entropy_bwd_kernel(const float* __restrict__ logits, long long ld, int V
   const float gent = g_entropy != nullptr ? g_entropy[row] : 0.f;
   const float H = entropy != nullptr ? entropy[row] : 0.f;
   const float l = lse[row];
+  if (WIDE) {
+#pragma unroll 2
+    for (int i = threadIdx.x * 8; i < V; i += ROW_THREADS * 8) {
+      const float4 a = __ldcs(reinterpret_cast<const float4*>(x + i)), b = __ldcs(reinterpret_cast<const float4*>(x + i + 4));
+      const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 8; j += 2)
+        o[j / 2] = pack_bf16x2(dlogit_epi(v[j], l, glp, gent, H, i + j == t), dlogit_epi(v[j + 1], l, glp, gent, H, i + j + 1 == t));
+      *reinterpret_cast<uint4*>(d + i) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    return;
+  }
   for (int i = threadIdx.x * 2; i < V; i += ROW_THREADS * 2) {
     float o[2];
 #pragma unroll
@@ -468,8 +483,9 @@ extern "C" int rb_logprob_entropy_bwd(const float* logits, long long ld, int row
                                       const float* lse, const float* entropy, const float* g_logprob,
                                       const float* g_entropy, void* dlogits, long long ldd, cudaStream_t s) {
   if (rows <= 0) return 0;
-  logprob_entropy_bwd_kernel<<<rows, ROW_THREADS, 0, s>>>(logits, ld, V, targets, lse, entropy, g_logprob, g_entropy,
-                                                         (__nv_bfloat16*)dlogits, ldd);
+  const bool wide = V % 8 == 0 && ld % 8 == 0 && ldd % 8 == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(dlogits)) & 15) == 0;
+  (wide ? logprob_entropy_bwd_kernel<true> : logprob_entropy_bwd_kernel<false>)<<<rows, ROW_THREADS, 0, s>>>(
+      logits, ld, V, targets, lse, entropy, g_logprob, g_entropy, (__nv_bfloat16*)dlogits, ldd);
   return RB_OK();
 }
 extern "C" int rb_rmsnorm_bwd_num_partials() { return 148 * 2; }

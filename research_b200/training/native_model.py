@@ -243,31 +243,45 @@ class _Embedding(torch.autograd.Function):
 
 
 class _FusedLogprob(torch.autograd.Function):
-    """(h [N,d], W [V,d]) -> per-token log-prob of ``targets`` and entropy, chunked over rows."""
+    """(h [N,d], W [V,d]) -> per-token log-prob of ``targets`` and entropy, chunked over rows.
+
+    ``keep``: the fp32 logits stay until backward, which then reads six bytes a logit instead of multiplying them out again. Microseconds for 2048
+    rows, product with the gradient in its epilogue / gradient of kept logits: V 151936, K 896 455 / 296; V 128256, K 4096 1514 / 255. The values are
+    the same."""
 
     CHUNK = 2048
 
     @staticmethod
-    def forward(ctx, h, w, gw, targets, need_entropy, sink):
+    def keeps(h: torch.Tensor, vocabulary: int) -> bool:
+        """Whether the logits of ``h`` may stay until backward: they take at most a quarter of the memory that is free."""
+        if not h.is_cuda or not torch.is_grad_enabled() or not h.requires_grad:
+            return False
+        stats = torch.cuda.memory.memory_stats_as_nested_dict(h.device)
+        pooled = stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
+        return 16 * h.shape[0] * vocabulary <= torch.cuda.mem_get_info(h.device)[0] + pooled
+
+    @staticmethod
+    def forward(ctx, h, w, gw, targets, need_entropy, sink, keep=False):
         N = h.shape[0]
         lp = torch.empty(N, dtype=torch.float32, device=h.device)
         lse = torch.empty_like(lp)
         ent = torch.empty_like(lp) if need_entropy else None
+        kept = torch.empty(N, w.shape[0], dtype=torch.float32, device=h.device) if keep else None
         for s in range(0, N, _FusedLogprob.CHUNK):
             e = min(N, s + _FusedLogprob.CHUNK)
-            logits = ops.gemm(h[s:e], w, out_f32=True)
+            logits = ops.gemm(h[s:e], w, out=kept[s:e] if keep else None, out_f32=True)
             a, b, c = T.logprob_entropy_fwd(logits, targets[s:e], need_entropy)
             lp[s:e], lse[s:e] = a, b
             if need_entropy:
                 ent[s:e] = c
-        ctx.save_for_backward(h, w, targets, lse, ent if need_entropy else lse)
+        ctx.save_for_backward(h, w, targets, lse, ent if need_entropy else lse, kept)
         ctx.gw, ctx.need_entropy, ctx.sink = gw, need_entropy, sink
         ctx.mark_non_differentiable(lse)
         return lp, (ent if need_entropy else lse.new_zeros(N)), lse
 
     @staticmethod
     def backward(ctx, g_lp, g_ent, _g_lse):
-        h, w, targets, lse, ent = ctx.saved_tensors
+        h, w, targets, lse, ent, kept = ctx.saved_tensors
         N = h.shape[0]
         dh = torch.empty_like(h)
         g_lp = g_lp.contiguous().float()
@@ -275,7 +289,9 @@ class _FusedLogprob(torch.autograd.Function):
         for s in range(0, N, _FusedLogprob.CHUNK):
             e = min(N, s + _FusedLogprob.CHUNK)
             rows = (targets[s:e], lse[s:e], ent[s:e] if ctx.need_entropy else None, g_lp[s:e], g_ent[s:e] if g_ent is not None else None)
-            if ops.gemm_mod.vocabulary_takes(h[s:e], w):     # the same values, without the logits in memory
+            if kept is not None:
+                dl = T.logprob_entropy_bwd(kept[s:e], *rows)
+            elif ops.gemm_mod.vocabulary_takes(h[s:e], w):     # the same values, without the logits in memory
                 dl = ops.gemm_mod.vocabulary_dlogits(h[s:e], w, *rows)
             else:
                 dl = T.logprob_entropy_bwd(ops.gemm(h[s:e], w, out_f32=True), *rows)
@@ -283,7 +299,7 @@ class _FusedLogprob(torch.autograd.Function):
             ops.gemm(dl, w, out=dh[s:e], b_mn_major=True)
             acc = ctx.sink.accumulate_into(ctx.gw)
             ops.gemm(dl, h[s:e], residual=ctx.gw if acc else None, out=ctx.gw, a_mn_major=True, b_mn_major=True)
-        return dh, None, None, None, None, None
+        return dh, None, None, None, None, None, None
 
 
 # ------------------------------------------------------------------------------ the model
@@ -671,5 +687,6 @@ class NativeCausalLM:
         if trace is not None:
             trace["final_norm"] = h.detach().view(B, Tn, -1)
         tg = targets.reshape(-1).to(torch.int32).contiguous()
-        lp, ent, _ = _FusedLogprob.apply(h, self.p(head), self.g(head), tg, need_entropy, sink)
+        w = self.p(head)
+        lp, ent, _ = _FusedLogprob.apply(h, w, self.g(head), tg, need_entropy, sink, _FusedLogprob.keeps(h, w.shape[0]))
         return lp.view(B, Tn), (ent.view(B, Tn) if need_entropy else None)
