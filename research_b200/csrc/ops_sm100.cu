@@ -4,6 +4,9 @@
 // bf16 Hugging Face modules (see the functional oracles in research_b200/models/functional.py)
 // so that greedy decoding matches the fp32/bf16 reference token for token.
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
+
+#include <type_traits>
 
 namespace rb {
 
@@ -11,14 +14,12 @@ namespace rb {
 // RMSNorm: y = bf16( bf16(x * rsqrt(mean(x^2)+eps)) * w ).
 // Reference math: rollouts/tools/functional_extractor/qwen_functional.py:46-65.
 // ------------------------------------------------------------------------------------------
+__device__ __forceinline__ float pair_square(uint32_t w) {
+  const float2 f = unpack_bf16x2(w);
+  return fmaf(f.x, f.x, f.y * f.y);
+}
 __device__ __forceinline__ float square_sum8(uint4 u, float ss) {
-  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 f = unpack_bf16x2(w[j]);
-    ss += f.x * f.x + f.y * f.y;
-  }
-  return ss;
+  return (((ss + pair_square(u.x)) + pair_square(u.y)) + pair_square(u.z)) + pair_square(u.w);
 }
 __device__ __forceinline__ uint4 rms_scaled(uint4 u, uint4 ww, float rstd) {
   const uint32_t xi[4] = {u.x, u.y, u.z, u.w}, wi[4] = {ww.x, ww.y, ww.z, ww.w};
@@ -33,48 +34,42 @@ __device__ __forceinline__ uint4 rms_scaled(uint4 u, uint4 ww, float rstd) {
   return make_uint4(oi[0], oi[1], oi[2], oi[3]);
 }
 
-// blockDim.x threads a row (blockDim.y rows where that is a warp), V vectors of 8 a thread in registers: the row is read once, and all of its loads and those of the weight are in flight
-// together. Few rows are a chain of latencies (V = 1 spreads a row over as many threads as it has vectors): 32 rows of 4096 took 4.8 us
-// with a warp a row, now 2.1. Many rows are bound by bytes: 8192 of 4096 took 29.9 us, now 24.8.
-template <int V>
-__global__ void __launch_bounds__(V == 4 ? 512 : 1024) rmsnorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                                   __nv_bfloat16* __restrict__ y, long long rows, int d, long long ldx, long long ldy, float eps) {
-  __shared__ float red[32];
+// Few rows are a chain of latencies: a CTA a row, a vector a thread, so that all loads of the row and the weight are in flight together. The
+// squares meet in shared memory, where one warp adds them up in the order of the kernel below, so that a row's norm does not depend on how many
+// rows there are. 32 rows of 4096 took 4.8 us with a warp a row, now 2.4.
+__global__ void __launch_bounds__(1024) rmsnorm_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                           __nv_bfloat16* __restrict__ y, int d, long long ldx, long long ldy, float eps) {
+  extern __shared__ __align__(16) float4 squares[];      // of a vector's four pairs
+  __shared__ float rstd_s;
   pdl_launch_dependents();
   pdl_wait();
-  const long long row = (long long)blockIdx.x * blockDim.y + threadIdx.y;
-  if (row >= rows) return;
-  const __nv_bfloat16* xr = x + row * ldx;
-  __nv_bfloat16* yr = y + row * ldy;
-  const int nvec = d >> 3;
-  uint4 keep[V], ww[V];
-#pragma unroll
-  for (int i = 0; i < V; ++i) {
-    const int v = threadIdx.x + i * blockDim.x;
-    keep[i] = v < nvec ? *reinterpret_cast<const uint4*>(xr + v * 8) : make_uint4(0, 0, 0, 0);
-    ww[i] = v < nvec ? *reinterpret_cast<const uint4*>(w + v * 8) : make_uint4(0, 0, 0, 0);
+  const int v = threadIdx.x, nvec = d >> 3;
+  uint4 keep = make_uint4(0, 0, 0, 0), ww = keep;
+  if (v < nvec) {
+    keep = *reinterpret_cast<const uint4*>(x + blockIdx.x * ldx + v * 8);
+    ww = *reinterpret_cast<const uint4*>(w + v * 8);
+    squares[v] = make_float4(pair_square(keep.x), pair_square(keep.y), pair_square(keep.z), pair_square(keep.w));
   }
-  float ss = 0.f;
-#pragma unroll
-  for (int i = 0; i < V; ++i) ss = square_sum8(keep[i], ss);
-  ss = warp_sum(ss);
-  const int warps = blockDim.x >> 5;
-  if (warps > 1) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) red[warp] = ss;
-    __syncthreads();
-    ss = warp_sum(lane < warps ? red[lane] : 0.f);
+  __syncthreads();
+  if (v < 32) {
+    float ss = 0.f;
+#pragma unroll 4
+    for (int i = v; i < nvec; i += 32) {
+      const float4 q = squares[i];
+      ss = (((ss + q.x) + q.y) + q.z) + q.w;
+    }
+    ss = warp_sum(ss);
+    if (v == 0) rstd_s = rsqrtf(ss / (float)d + eps);
   }
-  const float rstd = rsqrtf(ss / (float)d + eps);
-#pragma unroll
-  for (int i = 0; i < V; ++i) {
-    const int v = threadIdx.x + i * blockDim.x;
-    if (v < nvec) *reinterpret_cast<uint4*>(yr + v * 8) = rms_scaled(keep[i], ww[i], rstd);
-  }
+  __syncthreads();
+  if (v < nvec) *reinterpret_cast<uint4*>(y + blockIdx.x * ldy + v * 8) = rms_scaled(keep, ww, rstd_s);
 }
 
-// Rows of any length, one warp each, read twice.
-__global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+// A warp a row, V vectors of 8 a lane in registers, rows past 2048 (V = 0) read twice. What bounds it is bytes: 8192 rows of 896 6.8 us with eight
+// vectors for every row, now 5.1. Longer rows are not better off in registers (8192 x 4096 29.4 us, with 16 vectors a lane 39.8, with the kernel
+// above 34.7).
+template <int V>
+__global__ void __launch_bounds__(256) rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                __nv_bfloat16* __restrict__ y, long long rows, int d, long long ldx,
                                long long ldy, float eps) {
   pdl_launch_dependents();
@@ -85,11 +80,24 @@ __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
   const __nv_bfloat16* xr = x + row * ldx;
   __nv_bfloat16* yr = y + row * ldy;
   const int nvec = d >> 3;
+  uint4 keep[V > 0 ? V : 1];
   float ss = 0.f;
-  for (int v = lane; v < nvec; v += 32) ss = square_sum8(*reinterpret_cast<const uint4*>(xr + v * 8), ss);
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int v = lane + 32 * i;
+    keep[i] = v < nvec ? *reinterpret_cast<const uint4*>(xr + v * 8) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int i = 0; i < V; ++i) ss = square_sum8(keep[i], ss);
+  for (int v = lane + 32 * V; v < nvec; v += 32) ss = square_sum8(*reinterpret_cast<const uint4*>(xr + v * 8), ss);
   ss = warp_sum(ss);
   const float rstd = rsqrtf(ss / (float)d + eps);
-  for (int v = lane; v < nvec; v += 32)
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int v = lane + 32 * i;
+    if (v < nvec) *reinterpret_cast<uint4*>(yr + v * 8) = rms_scaled(keep[i], *reinterpret_cast<const uint4*>(w + v * 8), rstd);
+  }
+  for (int v = lane + 32 * V; v < nvec; v += 32)
     *reinterpret_cast<uint4*>(yr + v * 8) =
         rms_scaled(*reinterpret_cast<const uint4*>(xr + v * 8), *reinterpret_cast<const uint4*>(w + v * 8), rstd);
 }
@@ -282,6 +290,9 @@ __global__ void rope_kv_append_kernel(const __nv_bfloat16* __restrict__ qkv, __n
 // ------------------------------------------------------------------------------------------
 // `rows_dev` (optional) bounds the row count from device memory: the expert-parallel MoE layer only knows on the
 // device how many routed rows it received.
+// What bounds both directions is bytes, once the index is a 32-bit one (SMALL: fewer than 2^31 vectors) and the quotient has no branch: a 64-bit
+// division a vector and an IEEE division an element took 8192 x 4864 52.9 us, now 39.1; backward 63.2 and 62.0. The values are the same.
+template <bool SMALL>
 __global__ void swiglu_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                               long long T, int F, const int* __restrict__ rows_dev) {
   pdl_launch_dependents();
@@ -290,12 +301,11 @@ __global__ void swiglu_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat1
     const long long r = *rows_dev;
     T = r < T ? (r < 0 ? 0 : r) : T;
   }
-  const long long nvec = T * (F >> 3);
-  const int fv = F >> 3;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
-       i += (long long)gridDim.x * blockDim.x) {
+  using I = std::conditional_t<SMALL, unsigned, long long>;
+  const I nvec = (I)(T * (F >> 3)), fv = F >> 3;
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (I)gridDim.x * blockDim.x) {
     const long long t = i / fv;
-    const int c = (int)(i % fv) * 8;
+    const int c = (int)(i - (I)t * fv) * 8;
     uint4 g = *reinterpret_cast<const uint4*>(gu + t * 2 * F + c);
     uint4 u = *reinterpret_cast<const uint4*>(gu + t * 2 * F + F + c);
     uint32_t gi[4] = {g.x, g.y, g.z, g.w}, ui[4] = {u.x, u.y, u.z, u.w}, oi[4];
@@ -303,8 +313,8 @@ __global__ void swiglu_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat1
     for (int j = 0; j < 4; ++j) {
       float2 a = unpack_bf16x2(gi[j]);
       float2 b = unpack_bf16x2(ui[j]);
-      float s0 = __bfloat162float(__float2bfloat16_rn(a.x / (1.f + __expf(-a.x))));
-      float s1 = __bfloat162float(__float2bfloat16_rn(a.y / (1.f + __expf(-a.y))));
+      float s0 = __bfloat162float(__float2bfloat16_rn(quotient_epi(a.x, a.x * -1.44269504f)));
+      float s1 = __bfloat162float(__float2bfloat16_rn(quotient_epi(a.y, a.y * -1.44269504f)));
       oi[j] = pack_bf16x2(s0 * b.x, s1 * b.y);
     }
     *reinterpret_cast<uint4*>(out + t * F + c) = make_uint4(oi[0], oi[1], oi[2], oi[3]);
@@ -312,15 +322,15 @@ __global__ void swiglu_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat1
 }
 
 // SwiGLU backward: given gate|up [T,2F] and dout [T,F] writes dgate|dup [T,2F].
+template <bool SMALL>
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dout,
                                   __nv_bfloat16* __restrict__ dgu, long long T, int F) {
   // 8 columns (16 bytes) per thread and step; F % 8 == 0 is checked by the launcher
-  const int fv = F >> 3;
-  const long long nvec = T * fv;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
-       i += (long long)gridDim.x * blockDim.x) {
+  using I = std::conditional_t<SMALL, unsigned, long long>;
+  const I fv = F >> 3, nvec = (I)(T * (F >> 3));
+  for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (I)gridDim.x * blockDim.x) {
     const long long t = i / fv;
-    const int c = (int)(i % fv) * 8;
+    const int c = (int)(i - (I)t * fv) * 8;
     const uint4 g4 = *reinterpret_cast<const uint4*>(gu + t * 2 * F + c);
     const uint4 u4 = *reinterpret_cast<const uint4*>(gu + t * 2 * F + F + c);
     const uint4 d4 = *reinterpret_cast<const uint4*>(dout + t * F + c);
@@ -329,7 +339,7 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float2 g = unpack_bf16x2(gi[j]), u = unpack_bf16x2(ui[j]), dy = unpack_bf16x2(di[j]);
-      const float s0 = 1.f / (1.f + __expf(-g.x)), s1 = 1.f / (1.f + __expf(-g.y));
+      const float s0 = quotient_epi(1.f, g.x * -1.44269504f), s1 = quotient_epi(1.f, g.y * -1.44269504f);
       const float l0 = g.x * s0, l1 = g.y * s1;
       og[j] = pack_bf16x2(dy.x * u.x * (s0 + l0 * (1.f - s0)), dy.y * u.y * (s1 + l1 * (1.f - s1)));
       ou[j] = pack_bf16x2(dy.x * l0, dy.y * l1);
@@ -1055,21 +1065,17 @@ extern "C" int rb_rmsnorm(const void* x, const void* w, void* y, long long rows,
                           long long ldy, float eps, cudaStream_t stream) {
   if (d % 8 != 0 || rows <= 0) return -1;
   const int nvec = d >> 3;
-  // few rows: one vector a thread; many: about four, which leaves enough CTAs an SM to hide the reduction
-  const int v = rows <= 148 && nvec <= 1024 ? 1 : 4;
-  if (nvec <= (v == 4 ? 2048 : 1024) && rows <= 0x7fffffffll) {
-    const unsigned a_row = (unsigned)(((nvec + v - 1) / v + 31) / 32 * 32);
-    const dim3 threads(a_row, a_row == 32 && v > 1 ? 8 : 1);
-#define RB_RMSNORM(VV) launch_kernel(rmsnorm_row_kernel<VV>, dim3((unsigned)((rows + threads.y - 1) / threads.y)), threads, 0, stream, (const __nv_bfloat16*)x, \
-                                     (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rows, d, ldx, ldy, eps)
-    const cudaError_t e = v == 1 ? RB_RMSNORM(1) : RB_RMSNORM(4);
-#undef RB_RMSNORM
-    return e == cudaSuccess ? 0 : -11;
+  if (nvec <= 1024 && rows <= 148) {
+    return launch_kernel(rmsnorm_few_kernel, dim3((unsigned)rows), dim3((nvec + 31) / 32 * 32), (size_t)nvec * 16, stream, (const __nv_bfloat16*)x,
+                         (const __nv_bfloat16*)w, (__nv_bfloat16*)y, d, ldx, ldy, eps) == cudaSuccess ? 0 : -11;
   }
-  const int warps = 8;
+  const int warps = rows >= 148 * 8 * 4 ? 8 : 2;   // few rows: spread them over more SMs
   const long long grid = (rows + warps - 1) / warps;
-  return launch_kernel(rmsnorm_kernel, dim3((unsigned)grid), dim3(warps * 32), 0, stream, (const __nv_bfloat16*)x,
-                       (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rows, d, ldx, ldy, eps) == cudaSuccess ? 0 : -11;
+#define RB_RMSNORM(VV) launch_kernel(rmsnorm_kernel<VV>, dim3((unsigned)grid), dim3(warps * 32), 0, stream, (const __nv_bfloat16*)x, \
+                                     (const __nv_bfloat16*)w, (__nv_bfloat16*)y, rows, d, ldx, ldy, eps)
+  const cudaError_t e = nvec <= 128 ? RB_RMSNORM(4) : nvec <= 256 ? RB_RMSNORM(8) : RB_RMSNORM(0);
+#undef RB_RMSNORM
+  return e == cudaSuccess ? 0 : -11;
 }
 
 extern "C" int rb_row_squares(const void* x, float* out, int rows, int d, long long ldx, cudaStream_t stream) {
@@ -1113,7 +1119,7 @@ static int swiglu_launch(const void* gu, void* out, long long T, int F, const in
   const long long nvec = T * (F / 8);
   long long grid = (nvec + 255) / 256;
   if (grid > 148 * 16) grid = 148 * 16;
-  return launch_kernel(swiglu_kernel, dim3((unsigned)grid), dim3(256), 0, stream, (const __nv_bfloat16*)gu,
+  return launch_kernel(nvec < 0x7fffffffll ? swiglu_kernel<true> : swiglu_kernel<false>, dim3((unsigned)grid), dim3(256), 0, stream, (const __nv_bfloat16*)gu,
                        (__nv_bfloat16*)out, T, F, rows_dev) == cudaSuccess ? 0 : -11;
 }
 extern "C" int rb_swiglu(const void* gu, void* out, long long T, int F, cudaStream_t stream) {
@@ -1130,7 +1136,7 @@ extern "C" int rb_swiglu_bwd(const void* gu, const void* dout, void* dgu, long l
   const long long n = T * (F / 8);
   long long grid = (n + 255) / 256;
   if (grid > 148 * 32) grid = 148 * 32;
-  swiglu_bwd_kernel<<<(unsigned)grid, 256, 0, stream>>>((const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout,
+  (n < 0x7fffffffll ? swiglu_bwd_kernel<true> : swiglu_bwd_kernel<false>)<<<(unsigned)grid, 256, 0, stream>>>((const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout,
                                                        (__nv_bfloat16*)dgu, T, F);
   return RB_CHECK_LAUNCH();
 }
