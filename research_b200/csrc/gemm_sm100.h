@@ -144,6 +144,7 @@ typedef struct RbGemmArgs {
   int tail_col;
   float* tail;
   long long tail_ld;
+  int b_static;            // nothing still running on the stream writes B (K-major): its first loads overlap the launch before this one
 } RbGemmArgs;
 
 // Token and log-probability from the per-tile records written by the sampling epilogue.

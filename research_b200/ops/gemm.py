@@ -100,6 +100,7 @@ class RbGemmArgs(ctypes.Structure):
         ("tail_col", ctypes.c_int),
         ("tail", ctypes.c_void_p),
         ("tail_ld", ctypes.c_longlong),
+        ("b_static", ctypes.c_int),
     ]
 
 
@@ -542,6 +543,7 @@ def gemm(
         args.tail, args.tail_col, args.tail_ld = tail.data_ptr(), N - tail.shape[1], tail.stride(0)
     if norm_eps is not None:
         args.norm_fold, args.norm_eps = 1, float(norm_eps)
+    args.b_static = int(constant_b and gather is None)
     if gather is not None:
         assert not swiglu and norm_eps is None and alpha == 1.0 and beta == 1.0 and split_k in (0, 1), "gather launches are plain GEMMs"
         split_k = 1
