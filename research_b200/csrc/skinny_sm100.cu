@@ -167,9 +167,11 @@ __global__ void __launch_bounds__(SK_THREADS, 2) skinny_kernel(const __grid_cons
     }
   };
   pdl_launch_dependents();
-  if (p.b_static) load_w(w[0], s_begin);
-  pdl_wait();
-  if (!p.b_static) load_w(w[0], s_begin);
+  // both batches: a slice of up to four steps then waits for nothing but its activations
+  if (!p.b_static) pdl_wait();
+  load_w(w[0], s_begin);
+  load_w(w[1], s_begin + SK_UNROLL);
+  if (p.b_static) pdl_wait();
 
   float acc[NT][4], sq[NT];
   const __nv_bfloat16* arow[NT];
@@ -204,10 +206,10 @@ __global__ void __launch_bounds__(SK_THREADS, 2) skinny_kernel(const __grid_cons
     }
   };
   for (int s = s_begin; s < s_end; s += 2 * SK_UNROLL) {
-    load_w(w[1], s + SK_UNROLL);
     multiply(w[0], s);
     if (s + 2 * SK_UNROLL < s_end) load_w(w[0], s + 2 * SK_UNROLL);
     if (s + SK_UNROLL < s_end) multiply(w[1], s + SK_UNROLL);
+    if (s + 3 * SK_UNROLL < s_end) load_w(w[1], s + 3 * SK_UNROLL);
   }
 
   float* mine = red + ks * T * LD + rt * 16;
