@@ -1461,7 +1461,7 @@ __device__ __forceinline__ uint32_t outside_mask(int first, int lo, int hi) {
 __device__ __forceinline__ uint32_t packed_column(int k) { return (k >> 1) * 32 + (k & 1) * 8; }
 
 template <int D>
-__global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dkdv_kernel(const __grid_constant__ FlashBwdParams p) {
+__device__ __forceinline__ void flash_bwd_dkdv(const FlashBwdParams& p, const dim3& block, const dim3& grid) {
   using Cfg = FlashBwdCfg<D>;
   constexpr int DCH = D / 64;
   constexpr int ST = Cfg::kQdoStages;
@@ -1476,13 +1476,13 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dkdv_kernel(const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Under a causal mask the first key tiles have the longest loops: hand them out first, across all heads (blocks
   // are scheduled in the order of their linear index)
-  const int lin = blockIdx.x + gridDim.x * blockIdx.y;
-  const int b = blockIdx.z, hy = lin % gridDim.y;
+  const int lin = block.x + grid.x * block.y;
+  const int b = block.z, hy = lin % grid.y;
   const int G = p.Hq / p.Hkv;
   const bool head_split = p.dkv_part != nullptr;
   const int kvh = head_split ? hy / G : hy, g_base = head_split ? hy % G : 0;
   const int k_begin = p.cu_k[b], kv_len = p.cu_k[b + 1] - k_begin;
-  const int k0 = (lin / gridDim.y) * 128;
+  const int k0 = (lin / grid.y) * 128;
   if (k0 >= kv_len) return;
   const int q_begin = p.cu_q[b], q_len = p.cu_q[b + 1] - q_begin;
   const int off = kv_len - q_len;
@@ -1699,7 +1699,7 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dkdv_kernel(const
 }
 
 template <int D>
-__global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dq_kernel(const __grid_constant__ FlashBwdParams p) {
+__device__ __forceinline__ void flash_bwd_dq(const FlashBwdParams& p, const dim3& block, const dim3& grid) {
   using Cfg = FlashBwdCfg<D>;
   constexpr int DCH = D / 64;
   constexpr int ST = Cfg::kKvStages;
@@ -1712,8 +1712,8 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dq_kernel(const _
   __shared__ int abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.z, h = blockIdx.y;
-  const int q_tile = gridDim.x - 1 - blockIdx.x;
+  const int b = block.z, h = block.y;
+  const int q_tile = grid.x - 1 - block.x;
   const int q_begin = p.cu_q[b], q_len = p.cu_q[b + 1] - q_begin;
   const int q0 = q_tile * 128;
   if (q0 >= q_len) return;
@@ -1931,6 +1931,20 @@ __global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_dq_kernel(const _
   }
 }
 
+// Both passes in one launch: the CTAs of dK and dV, whose loops run over all queries of a group's heads, start first, and those of dQ fill the SMs that
+// the last of them leave idle. In launches of their own 24 sequences of up to 640 tokens (14 / 2 heads, D 64) took 73 + 65 us, now 106; 5 of
+// up to 6000 (32 / 8, D 128), which have no such tail, 1526 + 1334, now 2882.
+template <int D>
+__global__ void __launch_bounds__(FA_BWD_THREADS, 1) flash_bwd_kernel(const __grid_constant__ FlashBwdParams p, const dim3 grid_kv, const dim3 grid_q) {
+  const unsigned n_kv = grid_kv.x * grid_kv.y * grid_kv.z;
+  const bool kv = blockIdx.x < n_kv;
+  const dim3 grid = kv ? grid_kv : grid_q;
+  const unsigned lin = kv ? blockIdx.x : blockIdx.x - n_kv, yz = lin / grid.x;
+  const dim3 block(lin - yz * grid.x, yz % grid.y, yz / grid.y);
+  if (kv) flash_bwd_dkdv<D>(p, block, grid);
+  else flash_bwd_dq<D>(p, block, grid);
+}
+
 // dv / dk = sum over the G query heads of a group of their fp32 partials (fixed order), rounded to bf16.
 __global__ void flash_bwd_reduce_kernel(const float* __restrict__ part, int G, long long n, __nv_bfloat16* __restrict__ dv,
                                         __nv_bfloat16* __restrict__ dk) {
@@ -1952,22 +1966,18 @@ __global__ void flash_bwd_reduce_kernel(const float* __restrict__ part, int G, l
 
 template <int D>
 static int launch_flash_bwd(const FlashBwdParams& p, dim3 grid_kv, dim3 grid_q, cudaStream_t stream) {
-  using Cfg = FlashBwdCfg<D>;
+  constexpr int smem = FlashBwdCfg<D>::kSmemDkdv > FlashBwdCfg<D>::kSmemDq ? FlashBwdCfg<D>::kSmemDkdv : FlashBwdCfg<D>::kSmemDq;
   static bool attr_dev[64] = {};       // the shared-memory opt-in is a per-device function attribute
   int dev_i = 0;
   if (cudaGetDevice(&dev_i) != cudaSuccess || dev_i < 0 || dev_i >= 64) return -10;
   bool& attr = attr_dev[dev_i];
   if (!attr) {
-    if (cudaFuncSetAttribute(flash_bwd_dkdv_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemDkdv) !=
-        cudaSuccess)
-      return -10;
-    if (cudaFuncSetAttribute(flash_bwd_dq_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemDq) !=
-        cudaSuccess)
-      return -10;
+    if (cudaFuncSetAttribute(flash_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -10;
     attr = true;
   }
-  if (launch_kernel(flash_bwd_dkdv_kernel<D>, grid_kv, dim3(FA_BWD_THREADS), Cfg::kSmemDkdv, stream, p) != cudaSuccess) return -11;
-  if (launch_kernel(flash_bwd_dq_kernel<D>, grid_q, dim3(FA_BWD_THREADS), Cfg::kSmemDq, stream, p) != cudaSuccess) return -11;
+  const unsigned long long n_kv = (unsigned long long)grid_kv.x * grid_kv.y * grid_kv.z, n_q = (unsigned long long)grid_q.x * grid_q.y * grid_q.z;
+  if (n_kv == 0 || n_q == 0 || n_kv + n_q > 0x7fffffffull) return -11;
+  if (launch_kernel(flash_bwd_kernel<D>, dim3((unsigned)(n_kv + n_q)), dim3(FA_BWD_THREADS), smem, stream, p, grid_kv, grid_q) != cudaSuccess) return -11;
   if (p.dkv_part != nullptr) {
     const long long n = (long long)p.Tk * p.Hkv * D;
     long long blocks = (2 * (n >> 2) + 255) / 256;
