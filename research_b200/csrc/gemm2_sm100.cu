@@ -63,6 +63,11 @@ struct G2Params {
   // group_offsets[g] .. group_offsets[g + 1] (multiples of 64, at least 64 rows each)
   const int* group_offsets;
   int groups;
+  // G2_TOKENS: a tile is {first row of B, rows of it (64, 128, 192 or 256), group, tile of A's 256 rows}; A holds group_a_rows rows (K-major) or
+  // K rows (MN-major) per group
+  const int4* tile_table;
+  const int* num_tiles_ptr;
+  int group_a_rows;
   int silu_cols, tail_col;            // as in RbGemmArgs
   float* tail;
   long long tail_ld;
@@ -94,6 +99,7 @@ struct G2Params {
   long long gather_chunk_bytes;
 };
 constexpr int G2_STORE = 0, G2_DLOGITS = 1, G2_GLU = 2, G2_GROUPS = 3;      // epilogues; the last: plain, of a product per group
+constexpr int G2_TOKENS = 4;          // rows of groups: the groups' weights are the 256-row side, the output is stored transposed (rb_gemm2_tokens)
 constexpr int G2_GATHER_WARPS = 4;      // measured with 2: the copy (159 GB/s over NVLink) set the launch's time
 constexpr int G2_THREADS_GATHER = G2_THREADS + 32 * G2_GATHER_WARPS;
 
@@ -143,7 +149,7 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int m_tiles = (p.M + 255) / 256, n_tiles = (p.N + BN - 1) / BN;
-  const int num_tiles = m_tiles * n_tiles * (EPI == G2_GROUPS ? p.groups : 1);
+  const int num_tiles = EPI == G2_TOKENS ? *p.num_tiles_ptr : m_tiles * n_tiles * (EPI == G2_GROUPS ? p.groups : 1);
   // tile t -> (row tile, column tile); a launch that consumes its own gather starts at the local part's columns
   const int nt_rot = (GATHER && p.consume) ? p.rank * p.n_tiles_per_part : 0;
   auto tile_mn = [&](int t, int& mt, int& nt) {
@@ -197,8 +203,16 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
         int mt, nt, k_first, num_kb;
         tile_mn(t, mt, nt);
         tile_k(t, k_first, num_kb);
-        const int m0 = mt * 256 + (int)cta * G2_BM;        // this CTA's rows of A
-        const int n0 = nt * BN + (int)cta * HALF_N;        // this CTA's rows of B
+        int m0 = mt * 256 + (int)cta * G2_BM;              // this CTA's rows of A
+        int n0 = nt * BN + (int)cta * HALF_N;              // this CTA's rows of B
+        int half = HALF_N, a_k0 = k_first;
+        if constexpr (EPI == G2_TOKENS) {
+          const int4 e = p.tile_table[t];
+          half = e.y >> 1;
+          n0 = e.x + (int)cta * half;
+          m0 = e.w * 256 + (int)cta * G2_BM + (A_MN ? 0 : e.z * p.group_a_rows);
+          a_k0 = A_MN ? e.z * p.K : 0;
+        }
         if (GATHER && p.consume) {
           const int part = nt / p.n_tiles_per_part;
           const int idx = part * p.gather_chunks + (nt - part * p.n_tiles_per_part) / p.gather_chunk_tiles;
@@ -214,15 +228,17 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
           ok = mbar_wait_bounded_cluster(smem_u32(&empty_bar[s]), ph ^ 1u, abortp, p.status, ST_TIMEOUT_SMEM_EMPTY);
           if (!ok) break;
           const uint32_t fb = mapa_cluster(smem_u32(&full_bar[s]), 0);       // the leader's barrier of this stage
-          if (leader) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * Cfg::kStageBytes);
+          if (leader) mbar_expect_tx(smem_u32(&full_bar[s]), EPI == G2_TOKENS ? 2 * (Cfg::kABytes + half * 128) : 2 * Cfg::kStageBytes);
           const uint32_t sa = smem_base + s * Cfg::kStageBytes, sb = sa + Cfg::kABytes;
           if (!A_MN) {
             tma_load_2d_pair(sa, &p.a_map, fb, kb * G2_BK, m0);
           } else {
 #pragma unroll
-            for (int c = 0; c < G2_BM / 64; ++c) tma_load_2d_pair(sa + c * (G2_BK * 128), &p.a_map, fb, m0 + c * 64, k_first + kb * G2_BK);
+            for (int c = 0; c < G2_BM / 64; ++c) tma_load_2d_pair(sa + c * (G2_BK * 128), &p.a_map, fb, m0 + c * 64, a_k0 + kb * G2_BK);
           }
-          if (!B_MN) {
+          if (EPI == G2_TOKENS) {
+            for (int c = 0; c < half; c += 32) tma_load_2d_pair(sb + c * 128, &p.b_map, fb, kb * G2_BK, n0 + c);
+          } else if (!B_MN) {
             tma_load_2d_pair(sb, &p.b_map, fb, kb * G2_BK, n0);
           } else {
 #pragma unroll
@@ -256,6 +272,7 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
         const uint32_t tmem_d = tmem_base + acc * BN;
         int k_first, num_kb;
         tile_k(t, k_first, num_kb);
+        const uint32_t tile_idesc = EPI == G2_TOKENS ? make_idesc_bf16(256, p.tile_table[t].y, A_MN ? 1 : 0, 0) : idesc;
         for (int kb = 0; kb < num_kb; ++kb) {
           ok = mbar_wait_bounded_cluster(smem_u32(&full_bar[s]), ph, abortp, p.status, ST_TIMEOUT_SMEM_FULL);
           if (!ok) break;
@@ -267,7 +284,7 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
                                         : make_smem_desc_sw128(sa + k * 32, 16, 1024);
             const uint64_t bdesc = B_MN ? make_smem_desc_sw128(sb + k * 2048, G2_BK * 128, 1024)
                                         : make_smem_desc_sw128(sb + k * 32, 16, 1024);
-            umma2_bf16(tmem_d, adesc, bdesc, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma2_bf16(tmem_d, adesc, bdesc, tile_idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
           // the stage is free in BOTH CTAs once these MMAs retire
           umma2_commit(mapa_cluster(smem_u32(&empty_bar[s]), 0));
@@ -352,6 +369,37 @@ __global__ void __launch_bounds__(GATHER ? G2_THREADS_GATHER : G2_THREADS, 1) ge
       ok = mbar_wait_bounded_cluster(smem_u32(&tmem_full_bar[acc]), acc_ph, abortp, p.status, ST_TIMEOUT_TMEM_FULL);
       if (!ok) break;
       tc_fence_after();
+      if constexpr (EPI == G2_TOKENS) {
+        // A lane has a row of A, a column of the output: 32 x 32 of the accumulator become rows of 64 bytes in shared memory (a warp's stores of one
+        // token are 64 bytes in a row) and leave as one box.
+        const int4 e = p.tile_table[t];
+        const int col0 = e.w * 256 + (int)cta * G2_BM + q * 32;
+        if (col0 < p.N) {
+#pragma unroll 1
+          for (int c0 = 0; c0 < e.y; c0 += 32) {
+            uint32_t r[32];
+            tmem_ld_32x32(tmem_base + acc * BN + c0 + ((uint32_t)(q * 32) << 16), r);
+            tmem_ld_wait();
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            __syncwarp();
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(out_ptr + out_buf * 4096) + lane;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) dst[j * 32] = __float2bfloat16_rn(__uint_as_float(r[j]));
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(&p.c_map)),
+                           "r"(out_s + out_buf * 4096), "r"(col0), "r"(e.x + c0) : "memory");
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+            out_buf ^= 1;
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(acc == 0 ? leader_empty0 : leader_empty1);
+        continue;
+      }
       const int group_row = EPI == G2_GROUPS ? t / (m_tiles * n_tiles) * p.M : 0;
       const long long row = (long long)group_row + row0 + lane;
       const int n_base = nt * BN;
@@ -704,4 +752,29 @@ extern "C" int rb_gemm2_groups(const void* A, const void* B, void* C, const void
   if (rc != 0) return -40 + rc;
   if (N <= 128) return g2_launch<128, true, true, false, G2_GROUPS>(p, groups * ((M + 255) / 256), stream);
   return g2_launch<256, true, true, false, G2_GROUPS>(p, groups * ((M + 255) / 256) * ((N + 255) / 256), stream);
+}
+
+// C[rows of g, N] = B[rows of g, K] A_g^T for every group g: the products of all experts with their weights. The weights are the 256-row side of the
+// pair's tile and a group's rows, padded to 64, its columns in tiles of 64 to 256: what a 128-row tile spends on rows that a group of some
+// hundred does not have goes away, and a tile's weights are read once for up to 256 rows. A: the groups' [N, K] stacked (K-major), or their
+// [K, N] stacked (a_mn_major, K a multiple of 64). table: {first row, rows (a multiple of 64, at most 256), group, tile of 256 columns of N};
+// num_tiles on the device. 128 experts, 37000 rows, 1536 x 2048 / 2048 x 768: one-CTA kernel 238 / 138 us,
+// here 207 / 119, of which the bytes (every weight once) take 163 / 93.
+extern "C" int rb_gemm2_tokens(const void* A, const void* B, void* C, int groups, int N, int K, int rows, int a_mn_major, long long lda, long long ldb,
+                               long long ldc, const void* table, const int* num_tiles, int max_tiles, int* status, cudaStream_t stream) {
+  if (groups <= 0 || N <= 0 || K <= 0 || rows <= 0 || max_tiles <= 0 || N % 8 != 0 || K % 8 != 0 || table == nullptr || num_tiles == nullptr) return -1;
+  if ((a_mn_major && K % G2_BK != 0) || (reinterpret_cast<uintptr_t>(table) & 15) != 0 || (long long)groups * (N > K ? N : K) > 0x7fffffff) return -1;
+  G2Params p;
+  memset(&p, 0, sizeof(p));
+  p.M = N; p.N = N; p.K = K;
+  p.tile_table = reinterpret_cast<const int4*>(table); p.num_tiles_ptr = num_tiles; p.group_a_rows = N;
+  p.status = status;
+  int rc = a_mn_major ? tma_map_2d_bf16(&p.a_map, A, (unsigned long long)groups * K, N, lda, G2_BK)
+                      : tma_map_2d_bf16(&p.a_map, A, (unsigned long long)groups * N, K, lda, G2_BM);
+  if (rc != 0) return -20 + rc;
+  rc = tma_map_2d_bf16(&p.b_map, B, rows, K, ldb, 32);
+  if (rc != 0) return -30 + rc;
+  rc = tma_map_2d_plain(&p.c_map, C, rows, N, ldc, 32, 32);
+  if (rc != 0) return -40 + rc;
+  return a_mn_major ? g2_launch<256, true, false, false, G2_TOKENS>(p, max_tiles, stream) : g2_launch<256, false, false, false, G2_TOKENS>(p, max_tiles, stream);
 }

@@ -394,7 +394,7 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const fl
 
 struct TrainTableDesc {
   int mode;        // 0 forward {a_row0, valid_rows, e * b_stride + n0, n0}; 1 data gradient {a_row0, valid_rows, e * b_stride, n0};
-                   // 2 weight gradient {row0, rows, e, (m tile << 16) | n tile}
+                   // 2 weight gradient {row0, rows, e, (m tile << 16) | n tile}; 3 rows against 256 columns a tile {row0, rows, e, column tile}
   int n_total;     // output columns per expert
   int bn;          // tile width
   int b_stride;    // rows of the stacked B matrix per expert (modes 0, 1); output rows per expert M (mode 2)
@@ -425,7 +425,7 @@ __global__ void moe_train_plan_kernel(const int* __restrict__ counts, int E, int
     for (int e = 0; e < E; ++e) {
       const int rows = off_s[e + 1];
       base_s[e] = b;
-      b += (d.mode == 2 ? (d.b_stride + 127) / 128 : (rows + 127) / 128) * nt;
+      b += (d.mode == 2 ? (d.b_stride + 127) / 128 : d.mode == 3 ? (rows + 255) / 256 : (rows + 127) / 128) * nt;
       o += rows;
       off_s[e + 1] = o;
     }
@@ -448,6 +448,11 @@ __global__ void moe_train_plan_kernel(const int* __restrict__ counts, int E, int
     }
     const int e = lo, j = t - base_s[e];
     const int rows = off_s[e + 1] - off_s[e];
+    if (d.mode == 3) {      // {first row, rows, group, column tile}: the rows in even shares of whole 64s, tiles of the same weights next to each other
+      const int q = (rows + 255) / 256, i = j % q, blocks = rows / 64, first = blocks * i / q;
+      d.tiles[t] = make_int4(off_s[e] + first * 64, (blocks * (i + 1) / q - first) * 64, e, j / q);
+      continue;
+    }
     const int mt = d.mode == 2 ? (d.b_stride + 127) / 128 : (rows + 127) / 128;
     // consecutive tiles share the B tile (modes 0, 1) or the A tile's k range (mode 2)
     const int in = j / mt, im = j % mt;
@@ -743,7 +748,7 @@ extern "C" int rb_moe_train_plan(const int* counts, int E, int* offsets, const i
   for (int i = 0; i < n_tables; ++i) {
     tabs.t[i].mode = desc[4 * i]; tabs.t[i].n_total = desc[4 * i + 1]; tabs.t[i].bn = desc[4 * i + 2]; tabs.t[i].b_stride = desc[4 * i + 3];
     tabs.t[i].tiles = reinterpret_cast<int4*>(tiles[i]); tabs.t[i].ntiles = ntiles[i];
-    if (tabs.t[i].mode < 0 || tabs.t[i].mode > 2 || tabs.t[i].bn <= 0 || tabs.t[i].n_total <= 0 || tabs.t[i].tiles == nullptr ||
+    if (tabs.t[i].mode < 0 || tabs.t[i].mode > 3 || tabs.t[i].bn <= 0 || tabs.t[i].n_total <= 0 || tabs.t[i].tiles == nullptr ||
         tabs.t[i].ntiles == nullptr)
       return -1;
     if (tabs.t[i].mode == 2 && ((tabs.t[i].b_stride + 127) / 128 > 0xffff || (tabs.t[i].n_total + tabs.t[i].bn - 1) / tabs.t[i].bn > 0xffff)) return -1;

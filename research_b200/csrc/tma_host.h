@@ -28,10 +28,11 @@ inline EncodeTiledFnT tma_encode_fn() {
 // The encoder needs the device's context to be current in the calling thread, which a thread that has made no runtime call of its own
 // yet does not have (autograd's, whose allocations may all come from the cache): selecting the thread's device makes it so.
 inline CUresult tma_encode_2d(EncodeTiledFnT fn, CUtensorMap* out, CUtensorMapDataType type, void* base, const cuuint64_t* dims,
-                              const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapL2promotion promotion) {
+                              const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapL2promotion promotion,
+                              CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   const cuuint32_t estr[2] = {1, 1};
   for (int attempt = 0;; ++attempt) {
-    const CUresult r = fn(out, type, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, promotion,
+    const CUresult r = fn(out, type, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     int device = 0;
     if (r == CUDA_SUCCESS || attempt > 0 || cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return r;
@@ -49,6 +50,20 @@ inline int tma_map_2d_bf16(CUtensorMap* out, const void* base, unsigned long lon
   cuuint32_t box[2] = {64, box_rows};
   const CUresult r = tma_encode_2d(fn, out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, const_cast<void*>(base), dims, strides, box,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+  return r == CUDA_SUCCESS ? 0 : -3;
+}
+
+// bf16 output matrix, boxes of box_rows x box_cols, rows of a box back to back in shared memory.
+inline int tma_map_2d_plain(CUtensorMap* out, void* base, unsigned long long rows, unsigned long long cols, unsigned long long ld, unsigned box_rows,
+                            unsigned box_cols) {
+  EncodeTiledFnT fn = tma_encode_fn();
+  if (fn == nullptr) return -1;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (ld * 2) % 16 != 0) return -2;
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {ld * 2};
+  cuuint32_t box[2] = {box_cols, box_rows};
+  const CUresult r = tma_encode_2d(fn, out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                                   CU_TENSOR_MAP_SWIZZLE_NONE);
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 

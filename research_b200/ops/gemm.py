@@ -127,7 +127,8 @@ def _lib2() -> ctypes.CDLL:
         lib.rb_gemm2_bf16_gather.restype = i
         lib.rb_gemm2_dlogits.argtypes = [vp] * 2 + [i] * 3 + [ll] * 2 + [vp] * 6 + [ll, vp, vp]
         lib.rb_gemm2_groups.argtypes = [vp] * 4 + [i] * 4 + [ll] * 4 + [vp] * 3
-        lib.rb_gemm2_dlogits.restype = lib.rb_gemm2_groups.restype = i
+        lib.rb_gemm2_tokens.argtypes = [vp] * 3 + [i] * 5 + [ll] * 3 + [vp, vp, i, vp, vp]
+        lib.rb_gemm2_dlogits.restype = lib.rb_gemm2_groups.restype = lib.rb_gemm2_tokens.restype = i
         lib._rb_typed = True
     return lib
 

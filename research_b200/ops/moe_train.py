@@ -67,6 +67,15 @@ def _pair_wgrad_pays(E: int, m: int, n: int, accumulate: bool) -> bool:
     return pair <= 1.25 * up(m, 128) * up(n, _tile_width(n)) and (accumulate or n != 128)
 
 
+def _pair_tokens_pays(n: int, k: int, mn_major: bool) -> bool:
+    """Products of the experts' rows with ``[n, k]`` weights on the two-CTA kernel, weights as its 256-row side, or on the one-CTA kernel's 128-row tiles.
+    Microseconds (gate|up forward, down forward, their data gradients), one-CTA / two-CTA: 4096 tokens of 8 of 128 experts, 2048 x 768 238 / 207, 138 / 119,
+    134 / 123, 240 / 203; 16 tokens 160 / 154, 88 / 86, 90 / 92, 146 / 145; 4096 of 2 of 8, 4096 x 3584 386 / 326, 210 / 169, 209 / 169, 406 / 331; 100 tokens
+    108 / 111, 62 / 60, 60 / 61, 95 / 95; 64 of 2 of 8, 1024 x 1408, where the last tile of 1408 columns is half empty, 30 / 26, 28 / 19, 24 / 17, 38 / 28.
+    Widths that would leave more of their tiles empty stay with the narrower ones."""
+    return -(-n // 256) * 256 <= 1.15 * n and (k % 64 == 0 or not mn_major)
+
+
 class GroupedPlan:
     """Row layout and tile tables of one MoE layer call, all on the device.
 
@@ -93,11 +102,15 @@ class GroupedPlan:
                      (1, F, _tile_width(F), d), (1, d, _tile_width(d), 2 * F),
                      (2, F, _tile_width(F), d), (2, d, _tile_width(d), 2 * F)]
         m_tiles = self.cap // 128 + E
+        self.on_pair = {w for w in range(WGRAD_DN) if _pair_tokens_pays(self.desc[w][1], (d, F, d, 2 * F)[w], w >= DGRAD_DN)}
+        for w in self.on_pair:
+            self.desc[w] = (3, self.desc[w][1], 256, self.desc[w][3])
         # tables are written for the launches that read one
         used = [w for w in range(6) if w < WGRAD_DN or not _pair_wgrad_pays(E, self.desc[w][3], self.desc[w][1], False)]
         self.table_of = {which: table for table, which in enumerate(used)}
         written = [self.desc[which] for which in self.table_of]
-        self.max_tiles = max((E * -(-bs // 128) if mode == 2 else m_tiles) * -(-n_total // bn) for mode, n_total, bn, bs in written)
+        self.max_tiles = max((E * -(-bs // 128) if mode == 2 else self.cap // 256 + E if mode == 3 else m_tiles) * -(-n_total // bn)
+                             for mode, n_total, bn, bs in written)
         tables = len(written)
         self.tiles = torch.empty(tables, self.max_tiles, 4, dtype=torch.int32, device=dev)
         self.ntiles = torch.zeros(tables, dtype=torch.int32, device=dev)
@@ -167,10 +180,21 @@ class GroupedPlan:
             args.residual, args.ldr = residual.data_ptr(), residual.stride(0)
         check_rc(_gemm_lib().rb_gemm_bf16_ex(ctypes.byref(args), stream_handle(self.device)), "rb_gemm_bf16_ex(grouped training)")
 
+    def _launch_pair(self, which: int, x, w, out, K: int, mn_major: bool) -> None:
+        table = self.table_of[which]
+        assert x.stride(1) == w.stride(1) == out.stride(1) == 1
+        rc = _gemm2_lib().rb_gemm2_tokens(w.data_ptr(), x.data_ptr(), out.data_ptr(), self.E, out.shape[1], K, self.cap, int(mn_major), w.stride(0), x.stride(0),
+                                          out.stride(0), self.tiles[table].data_ptr(), self.ntiles.data_ptr() + 4 * table, self.max_tiles,
+                                          status_tensor(self.device).data_ptr(), stream_handle(self.device))
+        check_rc(rc, "rb_gemm2_tokens")
+
     def forward(self, which: int, x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
         """``out[rows of e] = x[rows of e] @ w_e^T`` with ``w`` the experts' ``[n, K]`` matrices stacked along the rows."""
         n = self.desc[which][1]
         out = torch.empty(self.cap, n, dtype=torch.bfloat16, device=self.device)
+        if which in self.on_pair:
+            self._launch_pair(which, x, w, out, x.shape[1], False)
+            return out
         self._launch(which, x, w, out, M=self.cap, N=w.shape[0], K=x.shape[1], group_n=n, a_mn=False, b_mn=False, group_mode=0)
         return out
 
@@ -180,6 +204,9 @@ class GroupedPlan:
         kd = self.desc[which][3]
         assert dy.shape[1] == kd and w.shape == (self.E * kd, n)
         out = torch.empty(self.cap, n, dtype=torch.bfloat16, device=self.device)
+        if which in self.on_pair:
+            self._launch_pair(which, dy, w, out, kd, True)
+            return out
         self._launch(which, dy, w, out, M=self.cap, N=n, K=kd, group_n=n, a_mn=False, b_mn=True, group_mode=1, group_b_rows=self.E * kd)
         return out
 
