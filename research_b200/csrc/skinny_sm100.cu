@@ -351,27 +351,29 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
         row = j * 2 * p.glu_half + (col - j * p.glu_half);
         up = row + p.glu_half;
       }
-      auto load_w = [&](int i) {
-        const int s = i % sp.stages, k = (kb0 + i) * 64;
+      auto load_w = [&](int i, int s) {
+        const int k = (kb0 + i) * 64;
         const uint32_t fb = smem_u32(&full[s]), dst = smem_base + s * stage_bytes;
         mbar_expect_tx(fb, stage_bytes);
         tma_load_2d(dst, &sp.w_map, fb, k, row);
         if (p.glu_half > 0) tma_load_2d(dst + 64 * 128, &sp.w_map, fb, k, up);
       };
-      auto load_x = [&](int i) {
-        const int s = i % sp.stages;
+      auto load_x = [&](int i, int s) {
         tma_load_2d(smem_base + s * stage_bytes + ST_ROWS * 128, &sp.x_map, smem_u32(&full[s]), (kb0 + i) * 64, 0);
       };
       const int first = min(sp.stages, n_kb);
       if (!p.b_static) pdl_wait();
-      for (int i = 0; i < first; ++i) load_w(i);
+      for (int i = 0; i < first; ++i) load_w(i, i);
       if (p.b_static) pdl_wait();
-      for (int i = 0; i < first; ++i) load_x(i);
-      int i = first;
+      for (int i = 0; i < first; ++i) load_x(i, i);
+      // (slot and phase go along: a division by the depth a stage stood in the way of one thread's loads)
+      int i = first, s = 0;
+      uint32_t ph = 0;
       for (; i < n_kb; ++i) {
-        if (!mbar_wait_bounded(smem_u32(&empty[i % sp.stages]), ((i / sp.stages) & 1u) ^ 1u, abortp, status, ST_TIMEOUT_SMEM_EMPTY)) break;
-        load_w(i);
-        load_x(i);
+        if (!mbar_wait_bounded(smem_u32(&empty[s]), ph, abortp, status, ST_TIMEOUT_SMEM_EMPTY)) break;
+        load_w(i, s);
+        load_x(i, s);
+        if (++s == sp.stages) { s = 0; ph ^= 1u; }
       }
       issued = i;
     }
@@ -380,9 +382,10 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
       const uint32_t idesc = make_idesc_bf16(ST_ROWS, T, 0, 0);
       bool ok = true;
       pdl_wait();      // no stage is full before: the budget of the first wait is not spent on the kernel before this one
+      int s = 0;
+      uint32_t ph = 0;
       for (int i = 0; i < n_kb; ++i) {
-        const int s = i % sp.stages;
-        ok = mbar_wait_bounded(smem_u32(&full[s]), (i / sp.stages) & 1u, abortp, status, ST_TIMEOUT_SMEM_FULL);
+        ok = mbar_wait_bounded(smem_u32(&full[s]), ph, abortp, status, ST_TIMEOUT_SMEM_FULL);
         if (!ok) break;
         tc_fence_after();
         const uint32_t w_s = smem_base + s * stage_bytes, x_s = w_s + ST_ROWS * 128;
@@ -390,6 +393,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
         for (int k = 0; k < 4; ++k)
           umma_bf16(tmem_base, make_smem_desc_sw128(w_s + k * 32, 16, 1024), make_smem_desc_sw128(x_s + k * 32, 16, 1024), idesc, (i > 0 || k > 0) ? 1u : 0u);
         umma_commit(smem_u32(&empty[s]));
+        if (++s == sp.stages) { s = 0; ph ^= 1u; }
       }
       __threadfence_block();
       umma_commit(smem_u32(&acc_full));      // a wait that ran out has set the flag before
@@ -399,9 +403,10 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
     pdl_wait();
     float sum = 0.f;
     if (p.norm_fold) {
+      int s = 0;
+      uint32_t ph = 0;
       for (int i = 0; i < n_kb; ++i) {
-        const int s = i % sp.stages;
-        const bool ok = mbar_wait_bounded(smem_u32(&full[s]), (i / sp.stages) & 1u, abortp, status, ST_TIMEOUT_SMEM_FULL);
+        const bool ok = mbar_wait_bounded(smem_u32(&full[s]), ph, abortp, status, ST_TIMEOUT_SMEM_FULL);
         if (!__all_sync(0xffffffffu, ok)) break;
         if (tid < T) {
           const uint8_t* x = smem_al + s * stage_bytes + ST_ROWS * 128 + tid * 128;
@@ -419,6 +424,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&empty[s]));
+        if (++s == sp.stages) { s = 0; ph ^= 1u; }
       }
       if (tid < T) ssq[tid] = sum;
     }
