@@ -192,6 +192,21 @@ def _stream_most_rows(N: int, K: int, swiglu: bool, norm: bool) -> int:
     return 56 if tiles > 16 and blocks < 32 else 64
 
 
+def _stream_first(M: int, N: int, K: int, swiglu: bool) -> bool:
+    """``rb_stream`` before the two rules above, for K from 896: at any number of rows (up to 32 past two tiles of 128 columns an SM, 48 below, 64 for gated units)
+    if the output has more than a tile an SM, from 9 rows to 16 if it has more than 1024 columns. Microseconds of a chain of captured launches, best of the
+    others / rb_stream: 1 row 151936 x 896 51.8 / 43.2, 128256 x 4096 174 / 154, 28672 x 4096 gated 43.0 / 38.5, 32000 x 2048 23.0 / 21.1, but 6144 x 4096 11.4 /
+    12.1, 4096 x 4096 7.1 / 9.3, 16384 x 2048 gated 12.6 / 12.9; 16 rows 128256 x 4096 174 / 160, 4096 x 14336 25.0 / 22.4, 6144 x 4096 13.5 / 12.8, 9728 x 896
+    gated 7.4 / 6.5, 2048 x 2048 5.3 / 5.0, but 896 x 4864 6.0 / 6.1, 896 x 896 3.7 / 4.2; 32 rows 151936 x 896 57.9 / 55.1, 128256 x 4096 176 / 168; 48 rows 151936 x
+    896 52.7 / 63.3, 128256 x 4096 179 / 181, 32000 x 2048 27.6 / 27.4."""
+    tiles = -(-N // 128)
+    if K < 896:
+        return False
+    if tiles > 148:
+        return M <= (64 if swiglu else 48 if tiles <= 296 else 32)
+    return 9 <= M <= 16 and N > 1024
+
+
 def _skinny_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail,
                   norm: bool = False) -> bool:
     """What it does not take (a layout the vector loads need, what the one-CTA kernel refuses or leaves unsaid) is left to the others."""
@@ -201,7 +216,11 @@ def _skinny_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu:
 
 def _stream_takes(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail,
                   norm: bool = False) -> bool:
-    return (9 <= M <= _stream_most_rows(N, K, swiglu, norm) and K % 8 == 0 and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0
+    return 9 <= M <= _stream_most_rows(N, K, swiglu, norm) and _stream_form(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail)
+
+
+def _stream_form(a, b, bias, residual, M: int, N: int, K: int, bn: int, swiglu: bool, out_f32: bool, softcap: float, silu_cols: int, tail) -> bool:
+    return (K % 8 == 0 and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0
             and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and (not swiglu or bn >= 128)
             and _few_rows_form(a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail))
 
@@ -507,8 +526,9 @@ def gemm(
     if M <= 64 and gather is None and wait_flag is None and not (a_mn_major or b_mn_major) and alpha == 1.0 and beta == 1.0 and max_ctas == 0 \
             and split_k in (0, 1) and not cluster_split:
         form = (a, b, bias, residual, M, N, K, bn, swiglu, out_f32, softcap, silu_cols, tail, norm_eps is not None)
-        skinny, stream = _skinny_takes(*form), _stream_takes(*form)
-        if skinny or stream:
+        stream = _stream_first(M, N, K, swiglu) and _stream_form(*form[:-1])
+        skinny = not stream and _skinny_takes(*form)
+        if skinny or stream or _stream_takes(*form):
             call = (a.data_ptr(), b.data_ptr(), out.data_ptr(), ptr(bias), ptr(residual), M, N, K, a.stride(0), b.stride(0), out.stride(0),
                     residual.stride(0) if residual is not None else 0, int(out_f32), bn // 2 if swiglu else 0, int(glu_limit is not None),
                     glu_limit or 0.0, int(norm_eps is not None), norm_eps or 0.0, softcap, silu_cols, ptr(tail),

@@ -72,3 +72,23 @@ def test_weights_ahead_of_the_launch_before():
         body()
         assert all(torch.equal(a, b) for a, b in zip(got, (*bufs, act)))
     ops.check_status(torch.device("cuda"))
+
+
+@pytest.mark.parametrize("M", [1, 5, 8, 9, 16, 17, 31, 32, 33])
+@pytest.mark.parametrize("N,K,form", [(19072, 896, {}), (20008, 904, dict(out_f32=True)), (38400, 896, dict(out_f32=True, softcap=30.0)),
+                                      (19200, 1024, dict(bn=256, swiglu=True, norm_eps=1e-6)), (2048, 2048, {})])
+def test_wide_outputs_of_few_rows(M, N, K, form):
+    """Outputs of more than a tile an SM take rb_stream from one row on, others from nine. Against 64 bits, and no less exact than the one-CTA kernel."""
+    x, w = _bf16(M, K, seed=M), _bf16(N, K, seed=N, scale=K ** -0.5)
+    assert ops.gemm_mod._stream_first(M, N, K, bool(form.get("swiglu"))) == (M <= (64 if "swiglu" in form else 48 if N <= 37888 else 32) if N > 148 * 128 else 9 <= M <= 16)
+    got, old = (ops.gemm(x, w, max_ctas=m, **form).double() for m in (0, 148))
+    xd = x.double()
+    if "norm_eps" in form:
+        xd = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6)
+    want = xd @ w.double().t()
+    if "softcap" in form:
+        want = 30.0 * torch.tanh(want / 30.0)
+    if "swiglu" in form:
+        want = ops.gemm_mod.swiglu_interleaved_reference(want, 256, None)
+    assert (got - want).norm() <= 1.05 * (old - want).norm()
+    ops.check_status(torch.device("cuda"))
