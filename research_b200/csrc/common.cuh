@@ -207,6 +207,17 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same with descriptors in halves: the upper one (stride of 8-row groups 1024 bytes, version, 128-byte swizzle) is the same for all of a kernel's
+// tiles, and the lower one moves by additions from one step of K to the next.
+constexpr uint32_t SMEM_DESC_HI = 64u | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t saddr, uint32_t lbo_bytes) { return ((saddr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16); }
+__device__ __forceinline__ void umma_bf16_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(SMEM_DESC_HI)
+      : "memory");
+}
 // Same for 8-bit floating point operands (e4m3 / e5m2, chosen in the instruction descriptor); one
 // instruction consumes K = 32 elements = 32 bytes, the same shared-memory footprint as 16 bf16.
 __device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,

@@ -58,7 +58,6 @@ constexpr int GEMM_THREADS_GATHER = GEMM_THREADS + GATHER_WARPS * 32;
 // groups of 8 K-rows are 1024 bytes apart (stride offset).
 #ifndef RB_MN_LBO
 #define RB_MN_LBO (BK * 128)
-#define RB_MN_SBO 1024
 #endif
 
 template <int BN>
@@ -466,6 +465,7 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
     // ------------------------------ MMA issuer --------------------------------------------
     if (elect_one_sync()) {
       constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      const bool fp8 = p.fp8 != 0;
       const uint32_t idesc8 = make_idesc_f8(BM, BN, (p.fp8 >> 1) & 1, (p.fp8 >> 2) & 1);
       uint32_t it = 0;
       int ring_s = 0;
@@ -498,14 +498,15 @@ gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
           tc_fence_after();
           const uint32_t sa = smem_base + s * Cfg::kStageBytes;
           const uint32_t sb = sa + Cfg::kABytes;
+          if (!A_MN && !B_MN && fp8) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t adesc = A_MN ? make_smem_desc_sw128(sa + k * 2048, RB_MN_LBO, RB_MN_SBO)
-                                        : make_smem_desc_sw128(sa + k * 32, 16, 1024);
-            const uint64_t bdesc = B_MN ? make_smem_desc_sw128(sb + k * 2048, RB_MN_LBO, RB_MN_SBO)
-                                        : make_smem_desc_sw128(sb + k * 32, 16, 1024);
-            if (p.fp8) umma_f8(tmem_d, adesc, bdesc, idesc8, (kb > kb0 || k > 0) ? 1u : 0u);
-            else umma_bf16(tmem_d, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / 16; ++k)
+              umma_f8(tmem_d, make_smem_desc_sw128(sa + k * 32, 16, 1024), make_smem_desc_sw128(sb + k * 32, 16, 1024), idesc8, (kb > kb0 || k > 0) ? 1u : 0u);
+          } else {
+            const uint32_t a_lo = smem_desc_lo(sa, A_MN ? RB_MN_LBO : 16), b_lo = smem_desc_lo(sb, B_MN ? RB_MN_LBO : 16);
+#pragma unroll
+            for (int k = 0; k < BK / 16; ++k)       // 16 of K: 32 bytes of a K-major row, 16 rows of 128 bytes otherwise
+              umma_bf16_lo(tmem_d, a_lo + k * (A_MN ? 128 : 2), b_lo + k * (B_MN ? 128 : 2), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           }
           umma_commit(smem_u32(&empty_bar[s]));  // frees the stage when these MMAs retire
         }

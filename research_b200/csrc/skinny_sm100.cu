@@ -390,8 +390,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) stream_kernel(const __grid_cons
         tc_fence_after();
         const uint32_t w_s = smem_base + s * stage_bytes, x_s = w_s + ST_ROWS * 128;
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma_bf16(tmem_base, make_smem_desc_sw128(w_s + k * 32, 16, 1024), make_smem_desc_sw128(x_s + k * 32, 16, 1024), idesc, (i > 0 || k > 0) ? 1u : 0u);
+        for (int k = 0; k < 4; ++k) umma_bf16_lo(tmem_base, smem_desc_lo(w_s, 16) + 2 * k, smem_desc_lo(x_s, 16) + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
         umma_commit(smem_u32(&empty[s]));
         if (++s == sp.stages) { s = 0; ph ^= 1u; }
       }
