@@ -253,12 +253,17 @@ class _FusedLogprob(torch.autograd.Function):
 
     @staticmethod
     def keeps(h: torch.Tensor, vocabulary: int) -> bool:
-        """Whether the logits of ``h`` may stay until backward: they take at most a quarter of the memory that is free."""
+        """Whether the logits of ``h`` may stay until backward, where they are read first of all: while they live, only the gradient of one chunk joins
+        them. They may where the allocator's pool holds both already, as it does from the second step on, or where they take at most a quarter of the
+        free memory. The driver is asked only in the second case: its answer takes 70 us, but up to 72 ms on a busy host."""
         if not h.is_cuda or not torch.is_grad_enabled() or not h.requires_grad:
             return False
         stats = torch.cuda.memory.memory_stats_as_nested_dict(h.device)
         pooled = stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
-        return 16 * h.shape[0] * vocabulary <= torch.cuda.mem_get_info(h.device)[0] + pooled
+        rows = h.shape[0]
+        if (4 * rows + 2 * min(rows, _FusedLogprob.CHUNK)) * vocabulary + 2 * h.nbytes <= pooled:
+            return True
+        return 16 * rows * vocabulary <= torch.cuda.mem_get_info(h.device)[0] + pooled
 
     @staticmethod
     def forward(ctx, h, w, gw, targets, need_entropy, sink, keep=False):
@@ -266,7 +271,12 @@ class _FusedLogprob(torch.autograd.Function):
         lp = torch.empty(N, dtype=torch.float32, device=h.device)
         lse = torch.empty_like(lp)
         ent = torch.empty_like(lp) if need_entropy else None
-        kept = torch.empty(N, w.shape[0], dtype=torch.float32, device=h.device) if keep else None
+        kept = None
+        if keep:
+            try:
+                kept = torch.empty(N, w.shape[0], dtype=torch.float32, device=h.device)
+            except torch.OutOfMemoryError:      # a pool in pieces on a full device
+                keep = False
         for s in range(0, N, _FusedLogprob.CHUNK):
             e = min(N, s + _FusedLogprob.CHUNK)
             logits = ops.gemm(h[s:e], w, out=kept[s:e] if keep else None, out_f32=True)
