@@ -458,6 +458,10 @@ __global__ void __launch_bounds__(FA_THREADS, 1) flash_fwd_kernel(const __grid_c
 //  * Three warpgroups of 168 registers a thread, redistributed to 88 / 208 / 208: the softmax threads keep their 128 scores
 //    in registers without spills.
 //  * Pairs of fp32 values per instruction (fma / add .f32x2), three-way maxima.
+//  * D = 64: both tiles' scores are there at the same time, so both warpgroups would read, search for maxima and exponentiate together, with the
+//    special-function unit idle in between. Tile b starts a part of a tile later, and they stay so: 1 x 16384 tokens, 14 / 2 heads 691 -> 633 us,
+//    1 x 4096 93 -> 84; 300, 600, 1000, 1500 and 2200 cycles 690, 670, 634, 633, 636. 32 x 300 (three key tiles at most) 51 -> 53, so
+//    it takes four. D = 128 issues the scores of the two tiles apart and measures the same with and without.
 //  * A CTA stays and takes the next query tile from the launch's own queue (cluster launch control: it cancels a CTA that
 //    has not started and does its work), so set-up, the first loads and the epilogue overlap; longest tiles first.
 // Measured rates stand beside the dispatch in launch_flash_fwd.
@@ -469,6 +473,8 @@ struct Flash2Cfg {
   static constexpr int kSmemBytes = 1024 + 2 * kTileBytes + kSlots * kTileBytes;
 };
 constexpr int FA2_THREADS = 384;
+constexpr int FA2_STAGGER_TILES = 4;
+constexpr uint32_t FA2_STAGGER_CYCLES = 1000;
 constexpr int FA2_REGS_LAUNCH = 168, FA2_REGS_OTHER = 88, FA2_REGS_SOFTMAX = 208;     // 88 + 2 x 208 = 3 x 168
 
 struct FlashItem {       // one query tile pair
@@ -834,6 +840,12 @@ __global__ void __launch_bounds__(FA2_THREADS, 1) flash_fwd2_kernel(const __grid
           const int k0 = (t.t_begin + j) * FA_BN;
           ok = wait(&s_full[x], count & 1u);
           if (!ok) break;
+          if (EARLY && x == 1 && j == 0 && n_mine >= FA2_STAGGER_TILES && t.n_a > 0) {
+            const uint32_t begun = (uint32_t)clock();
+            while ((uint32_t)clock() - begun < FA2_STAGGER_CYCLES) {
+            }
+            __syncwarp();
+          }
           tc_fence_after();
           const bool need_mask = (k0 + FA_BN > t.kv_len) || (p.causal && k0 + FA_BN - 1 > t.off + q0x) || k0 < last_first;
           uint32_t v[FA_BN];

@@ -224,6 +224,28 @@ def test_flash_forward_tile_edges_many_items_a_block(D, H, Hkv, window, paged):
     ops.check_status(torch.device("cuda"))
 
 
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("keys", [256, 384, 385, 512, 513, 640, 1411])
+def test_flash_forward_second_tile_apart(keys, causal):
+    """Query rows 128 to 255 are tile b, which starts late from four key tiles on. Alone they are tile a: the same key tiles in the same order, so the
+    same bytes. Both against 64 bits: probabilities and the result in bf16, 2^-8 relative each, and the denominator is theirs in fp32."""
+    D, H, Hkv, B = 64, 4, 2, 40
+    q = _rand((B * 256, H, D), "cuda", seed=keys)
+    k, v = (_rand((B * keys, Hkv, D), "cuda", seed=keys + i) for i in (1, 2))
+    cu_q, cu_k, half = _cu([256] * B, "cuda"), _cu([keys] * B, "cuda"), _cu([128] * B, "cuda")
+    both = flash.flash_attn_varlen(q, k, v, cu_q, cu_k, 256, causal=causal).view(B, 256, H, D)
+    late = q.view(B, 256, H, D)[:, 128:].reshape(B * 128, H, D)
+    assert torch.equal(both[:, 128:], flash.flash_attn_varlen(late, k, v, half, cu_k, 256, causal=causal).view(B, 128, H, D))
+    kd, vd = (t.double().view(B, keys, Hkv, D).repeat_interleave(H // Hkv, 2) for t in (k, v))
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double().view(B, 256, H, D), kd) / math.sqrt(D)
+    if causal:
+        s = s.masked_fill(torch.arange(keys, device="cuda") > torch.arange(keys - 256, keys, device="cuda")[:, None], -math.inf)
+    p = s.softmax(-1)
+    want, terms = torch.einsum("bhqk,bkhd->bqhd", p, vd), torch.einsum("bhqk,bkhd->bqhd", p, vd.abs())
+    assert ((both.double() - want).abs() <= 2.0 ** -8 * (want.abs() + terms) + 1e-4 * terms).all()
+    ops.check_status(torch.device("cuda"))
+
+
 @pytest.mark.parametrize("causal,window", [(True, 0), (True, 100), (True, 129), (False, 0)])
 @pytest.mark.parametrize("D,H,Hkv", [(64, 4, 2), (128, 2, 2)])
 def test_flash_backward_tile_edges(D, H, Hkv, causal, window):
