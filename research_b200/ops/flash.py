@@ -153,18 +153,17 @@ _HEAD_SPLIT = os.environ.get("RB_FLASH_BWD_HEAD_SPLIT", "auto")     # auto | 0 |
 def head_split_pays(B: int, max_seqlen_q: int, max_seqlen_k: int, Hq: int, Hkv: int) -> bool:
     """dK/dV as one CTA per (key tile, QUERY head) + a reduction over each group, instead of one CTA per (key tile,
     key/value head) looping over its G query heads and 128-query tiles. The split costs 2 * G * Tk * Hkv * D floats of
-    workspace and one pass over them; it pays where the longest of the whole loops is well above the average per SM, as dQ's blocks fill the SMs
-    that the others leave.
-    Counted in 128 x 128 tiles: the longest whole loop has ``T G`` (``T`` query tiles), a causal pass over all heads with dQ's tiles beside it
-    ``1.75 B Hq T (T + 1) / 2`` over 148 SMs, the workspace of a (key tile, query head) costs 0.06 tiles of time, the pass over it 3.5.
-    Backward in microseconds, whole / split. Taken: 1 x 256 tokens, 14 / 2 heads, D 64 40 / 30; 1 x 512 60 / 32; 1 x 4096 347 / 200; 1 x 8192 673 / 599;
-    2 x 3072 271 / 228; 4 x 512 60 / 50; 4 x 1024 106 / 97; 1 x 1536, 8 / 4 56 / 46; 2 x 3072, 24 / 2, D 128 553 / 519. Refused: 2 x 4096, 14 / 2, D 64 351 / 357;
-    4 x 2048 189 / 230; 16 x 512 91 / 134; 1 x 1024, 32 / 8, D 128 83 / 87; 1 x 2048 155 / 200; 1 x 4096 464 / 556; 2 x 1024 106 / 148;
-    4 x 1536, 24 / 2 308 / 376. Not sharp: 4 x 1024, 24 / 2, taken, loses (210 / 220)."""
-    G, tiles = Hq // Hkv, -(-max_seqlen_q // 128)
+    workspace and one pass over them; it pays where the longest of the whole loops is well above the average per SM.
+    The rule asks for fewer CTAs than the GPU has SMs and a longest loop of at least 32 iterations (counted as 64
+    half tiles). Backward in microseconds, whole / split. Taken: 1 x 4096 tokens, 14 / 2 heads, D 64 414 / 189; 1 x 2048, 32 / 8, D 128
+    200 / 194; 1 x 8192, 16 / 2 1284 / 901. Refused: 1 x 4096, 32 / 8 (256 CTAs, the longest 128 iterations against 114 per SM) 469 / 546;
+    16 x 512, 14 / 2 104 / 131. The line is not sharp: below it 1 x 512, 14 / 2 would gain (60 / 30), above it several
+    sequences lose where their average comes near the longest loop (2 x 1024, 32 / 8 121 / 141; 16 x 512, 16 / 2 174 / 254)."""
+    G = Hq // Hkv
     if _HEAD_SPLIT in ("0", "1"):
         return G > 1 and _HEAD_SPLIT == "1"
-    return G > 1 and tiles * G * (1 - B * Hkv * (1.75 / 296 * (-(-max_seqlen_k // 128) + 1) + 0.06)) > 3.5
+    ctas = -(-max_seqlen_k // 128) * Hkv * B
+    return G > 1 and ctas < 148 and (max_seqlen_q // 64) * G >= 64
 
 
 class FlashAttnVarlen(torch.autograd.Function):
