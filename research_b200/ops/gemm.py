@@ -640,8 +640,7 @@ _STREAM_GBS = {32: 80e3, 64: 85e3, 128: 98e3, 256: 114e3}     # bytes per micros
 def _cluster_split_choice(M: int, N: int, K: int, min_bn: int = 32) -> tuple[int, int]:
     """Cheapest (split, bn) under a model fitted to 100 timed B200 launches (mean error 10 %): per k-block a CTA
     streams ``(128 + bn) * 128`` bytes at the per-SM rate above; a cluster reduction costs 1 + 0.045 bn (2 slices),
-    1.5 + 0.025 bn (4) or 1.5 + 0.03 bn microseconds (8); split launches must fit one wave, of clusters that lie within a group of SMs: 36 clusters of
-    4 or 16 of 8 no longer do (128 x 1152 x 896 in 4 slices 11.2 us, in 2 6.2; 128 x 2048 x 8192 in 8 of 128 columns 24.2, in 4 of 64 14.1)."""
+    1.5 + 0.025 bn (4) or 3 + 0.03 bn microseconds (8); split launches must fit one wave."""
     m_tiles = -(-M // 128)
     num_kb = -(-K // 64)
     best = None
@@ -657,10 +656,10 @@ def _cluster_split_choice(M: int, N: int, K: int, min_bn: int = 32) -> tuple[int
                 continue
             units = m_tiles * n_tiles * s
             grid = min(units, 148 - 148 % s)
-            if s > 1 and units > {2: 148, 4: 132, 8: 112}[s]:
+            if s > 1 and units > grid:
                 continue
             waves = -(-units // grid)
-            red = {1: 0.0, 2: 1 + 0.045 * bn, 4: 1.5 + 0.025 * bn, 8: 1.5 + 0.03 * bn}[s]
+            red = {1: 0.0, 2: 1 + 0.045 * bn, 4: 1.5 + 0.025 * bn, 8: 3 + 0.03 * bn}[s]
             cost = waves * (per * max(stage_us, mma_us) + 1.0 + red)
             if best is None or cost < best[0] - 0.5:
                 best = (cost, s, bn)
