@@ -155,10 +155,11 @@ def head_split_pays(B: int, max_seqlen_q: int, max_seqlen_k: int, Hq: int, Hkv: 
     key/value head) looping over its G query heads and 128-query tiles. The split costs 2 * G * Tk * Hkv * D floats of
     workspace and one pass over them; it pays where the longest of the whole loops is well above the average per SM.
     The rule asks for fewer CTAs than the GPU has SMs and a longest loop of at least 32 iterations (counted as 64
-    half tiles). Backward in microseconds, whole / split. Taken: 1 x 4096 tokens, 14 / 2 heads, D 64 414 / 189; 1 x 2048, 32 / 8, D 128
-    200 / 194; 1 x 8192, 16 / 2 1284 / 901. Refused: 1 x 4096, 32 / 8 (256 CTAs, the longest 128 iterations against 114 per SM) 469 / 546;
-    16 x 512, 14 / 2 104 / 131. The line is not sharp: below it 1 x 512, 14 / 2 would gain (60 / 30), above it several
-    sequences lose where their average comes near the longest loop (2 x 1024, 32 / 8 121 / 141; 16 x 512, 16 / 2 174 / 254)."""
+    half tiles). Backward in microseconds, whole / split. Taken: 1 x 4096 tokens, 14 / 2 heads, D 64 347 / 200; 1 x 8192 673 / 599; 1 x 2048, 24 / 2, D 128
+    349 / 155. Refused: 1 x 4096, 32 / 8 (256 CTAs, the longest 128 iterations against 114 per SM) 464 / 556; 16 x 512, 14 / 2, D 64 91 / 134. The line is
+    not sharp: below it 1 x 512, 14 / 2 would gain (60 / 32), and above it loops near their average lose since dQ's blocks fill the SMs that dK/dV leaves
+    (1 x 2048, 32 / 8 155 / 200; 2 x 1024 106 / 148; 4 x 2048, 14 / 2, D 64 189 / 230). It stays there because the two forms add the heads of a group in
+    another order, and one rounding of dK or dV moves single rows of a deep model's embedding gradient by up to half of the largest value."""
     G = Hq // Hkv
     if _HEAD_SPLIT in ("0", "1"):
         return G > 1 and _HEAD_SPLIT == "1"
